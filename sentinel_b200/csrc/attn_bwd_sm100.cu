@@ -119,7 +119,7 @@ inline int bwd_split_tiles(const AttnShape& s)
 struct BwdBarriers {
     uint64_t kv_full;
     uint64_t q_full[3], q_empty[3], do_full[2], do_empty[2];
-    uint64_t s_ready[2], p_ready, dp_ready, ds_ready, dq_ready, dq_drained, final_bar;
+    uint64_t s_ready[2], p_ready[2], dp_ready, ds_ready, dq_ready, dq_drained, final_bar;
     uint32_t tmem_base;
     uint32_t abort_flag;
 };
@@ -405,8 +405,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             mbar_init(&bars->do_full[i], 1);
             mbar_init(&bars->do_empty[i], 2);
             mbar_init(&bars->s_ready[i], 1);
+            mbar_init(&bars->p_ready[i], 256);
         }
-        mbar_init(&bars->p_ready, 256);
         mbar_init(&bars->dp_ready, 1);
         mbar_init(&bars->ds_ready, 256);
         mbar_init(&bars->dq_ready, 1);
@@ -530,7 +530,9 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             for (int i = 0; ok && i < n_iter; ++i) {
                 const int sq = i % kQStages, sd = i % kDoStages, sb = i % kSBufs;
                 const uint32_t tm_Si = tm_S + (uint32_t)sb * kSBufStride;
-                if (!(ok = wait(&bars->p_ready, (uint32_t)(i & 1), kSiteP))) break;
+                // one barrier per S^T buffer: with two buffers the threads of one warpgroup can be through step i + 1 while a
+                // warp of the other has not stored its P^T_i yet, and a single barrier would count their second arrival for it
+                if (!(ok = wait(&bars->p_ready[sb], (uint32_t)((i / kSBufs) & 1), kSiteP))) break;
                 if (!(ok = wait(&bars->do_full[sd], (uint32_t)((i / kDoStages) & 1), kSiteDoFull))) break;
                 SNTL_TRACE_EV(tl, 0, tn, 1);
                 tc_fence_after();
@@ -763,7 +765,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             tmem_st32(tm_Si + lane_off + col0, pk);
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(&bars->p_ready);
+            mbar_arrive(&bars->p_ready[i % kSBufs]);
             SNTL_TRACE_EV(tw, 1 + wg, tn, 4);
             // ---- dS^T ----
             ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_ready, ph, abort_flag, kSiteDP));

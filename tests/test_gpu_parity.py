@@ -338,6 +338,20 @@ def test_backward_head_dim_64_buffers_and_cut_tiles_vs_oracle(sb, oracle):
     _check_bf16(_np(dv), wdv, "dv (one tile)")
 
 
+def test_backward_head_dim_64_warpgroups_drift_apart(sb):
+    """Many equal CTAs starting at the same moment make the two compute warpgroups of the head_dim-64 backward drift apart by
+    more than a step (each has S^T of the next step ready): dK and dV have one owner per element and must not vary."""
+    w = sb.WORKLOADS["gpt2_small"]
+    q, k, v, do = (t.cuda() for t in _bf16_case(w, batch=8, q_heads=48, kv_heads=48, seq=512))
+    o, lse = sb.attention_forward(q, k, v)
+    _, dk, dv = sb.attention_backward(q, k, v, o, lse, do)
+    assert bool(torch.isfinite(dk).all()) and bool(torch.isfinite(dv).all())
+    for _ in range(30):
+        _, dk2, dv2 = sb.attention_backward(q, k, v, o, lse, do)
+        assert torch.equal(dk, dk2) and torch.equal(dv, dv2)
+    assert sb.poll_device_status() == 0
+
+
 @pytest.mark.parametrize("wname,kw", [
     ("llama1b_gqa", dict(batch=2, q_heads=8, kv_heads=2, seq=768)),      # head_dim 64
     ("gqa7b_d128", dict(batch=1, q_heads=6, kv_heads=2, seq=512)),       # head_dim 128

@@ -3,6 +3,7 @@ compute entry point fails loudly, and the library itself refuses to run on anyth
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -34,11 +35,33 @@ class Desc(C.Structure):
                 ("column_start", C.c_int32), ("flags", C.c_int32), ("window_size", C.c_int32), ("global_tokens", C.c_int32)]
 
 
+HOST_MODULE_PATH = os.path.join(HERE, "lib", "_sntl_host.so")   # csrc/torch_host.cpp
+
+
 class LibraryMissing(RuntimeError):
     pass
 
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native module behind the Python entry points (csrc/torch_host.cpp), bound to the library load() returns."""
+    global _host
+    if _host is None:
+        lib = load()
+        if not os.path.exists(HOST_MODULE_PATH):
+            raise LibraryMissing(f"{HOST_MODULE_PATH} is missing: run `python -m sentinel_b200.build`.")
+        spec = importlib.util.spec_from_file_location("_sntl_host", HOST_MODULE_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(*(C.cast(getattr(lib, n), C.c_void_p).value for n in
+                      ("sntl_attn_fwd", "sntl_attn_bwd", "sntl_attn_cached_fwd", "sntl_attn_fwd_workspace_bytes",
+                       "sntl_attn_bwd_workspace_bytes", "sntl_attn_cached_fwd_workspace_bytes", "sntl_attn_pack_heads",
+                       "sntl_attn_unpack_heads")))
+        _host = module
+    return _host
 
 
 def load():

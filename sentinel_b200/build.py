@@ -2,6 +2,7 @@
 
 nvcc is invoked directly (one object per ``.cu`` file, then a shared link against the static CUDA
 runtime), so the result has no Python or torch dependency and can be bound from C, C++ or ctypes.
+Beside it ``sentinel_b200/lib/_sntl_host.so``, the CPython module that puts torch tensors into that ABI (host code only).
 """
 from __future__ import annotations
 
@@ -9,6 +10,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -16,6 +18,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libsntl_attn.so")
+HOST_MODULE = os.path.join(LIB_DIR, "_sntl_host.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = ["attn_api.cu", "attn_simt.cu", "layout_convert.cu", "attn_fwd_sm100.cu", "attn_bwd_sm100.cu",
@@ -38,6 +41,26 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_host_module(force: bool = False) -> str:
+    """The CPython module of csrc/torch_host.cpp, against the headers and libraries of the torch that is installed."""
+    src = os.path.join(CSRC, "torch_host.cpp")
+    if not force and not _stale(HOST_MODULE, [src, os.path.join(ROOT, "include", "sntl_attn.h")]):
+        return HOST_MODULE
+    import torch
+    from torch.utils import cpp_extension
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc()))), "include")
+    includes = cpp_extension.include_paths() + [sysconfig.get_path("include"), cuda, os.path.join(ROOT, "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           src, "-o", HOST_MODULE] + [x for d in includes for x in ("-isystem", d)]
+    cmd += ["-L" + libs, "-Wl,-rpath," + libs, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on torch_host.cpp")
+    return HOST_MODULE
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIB_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -56,8 +79,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 raise RuntimeError(f"nvcc failed on {src}")
         return obj
 
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
+        host = ex.submit(build_host_module, force)
         objs = list(ex.map(compile_one, srcs))
+        host.result()
     if force or _stale(LIB, objs):
         cmd = [nvcc(), "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static", "-ldl"]
         r = subprocess.run(cmd, capture_output=True, text=True)

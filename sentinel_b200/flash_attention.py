@@ -10,6 +10,10 @@ Two levels:
 
 Nothing here computes attention: every result comes from ``lib/libsntl_attn.so``.  torch supplies memory and
 the current stream.
+
+The calls below hand their arguments to the native module first (``csrc/torch_host.cpp``: checks, allocation and the C ABI
+call in native code, about 20 us less per call).  It declines with ``None`` when anything is not as it expects; the Python
+code that follows then names the error, or makes the call for arguments it alone accepts.
 """
 from __future__ import annotations
 
@@ -18,9 +22,6 @@ import ctypes as C
 import torch
 
 from . import _lib
-
-_ws_cache: dict = {}
-
 
 def _stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
@@ -31,12 +32,8 @@ def _workspace(nbytes: int, device) -> torch.Tensor | None:
     Calls on different streams may overlap on the GPU, so each stream gets scratch of its own."""
     if nbytes == 0:
         return None
-    key = (device.type, device.index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _ws_cache.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _ws_cache[key] = buf
-    return buf
+    with torch.cuda.device(device):
+        return _lib.host().workspace(nbytes)
 
 
 def _dtype_code(t: torch.Tensor) -> int:
@@ -88,6 +85,9 @@ def attention_forward(q, k, v, *, causal=True, scale=None, flags=0, out=None, ls
     ``window`` / ``global_tokens``: the reference layer's sliding window and always-visible first keys
     (CausalSelfAttention.cpp:95-100); key j is visible to query i iff j <= i and (j < global_tokens or window <= 0 or
     j >= i - window + 1)."""
+    r = _lib.host().forward(q, k, v, causal, scale, flags, out, lse, window, global_tokens)
+    if r is not None:
+        return r if r.__class__ is tuple else _lib.check(r, "sntl_attn_fwd")
     lib = _lib.load()
     for t, n in ((q, "q"), (k, "k"), (v, "v")):
         _require(t, n)
@@ -113,6 +113,9 @@ def attention_cached_forward(q, k_cache, v_cache, cache_length, *, scale=None, f
     q: [B,Hq,T,D], the T newest tokens; k_cache, v_cache: [B,Hkv,capacity,D] with the first ``cache_length`` rows in use,
     the new tokens' keys already appended at the end.  Query i sits at position cache_length - T + i.  Returns
     (O [B,Hq,T,D], LSE [B,Hq,T])."""
+    r = _lib.host().cached_forward(q, k_cache, v_cache, cache_length, scale, flags, out, lse, window, global_tokens)
+    if r is not None:
+        return r if r.__class__ is tuple else _lib.check(r, "sntl_attn_cached_fwd")
     lib = _lib.load()
     for t, n in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache")):
         _require(t, n)
@@ -157,6 +160,9 @@ def pack_heads(matrix, batch, heads, seq, head_dim, *, column_start=0, cos_table
     """fp32 feature-major ``(heads*head_dim) x stride`` matrix -> bf16 ``[batch, heads, seq, head_dim]``, rotated by the
     angle tables on the way (``None``: no rotation).  One kernel in place of the reference's rotaryRotateInPlace
     (CudaOps.cu:362-381) plus a relayout and a cast."""
+    r = _lib.host().pack_heads(matrix, batch, heads, seq, head_dim, column_start, cos_table, sin_table, position_offset, out)
+    if r is not None:
+        return r if r.__class__ is not int else _lib.check(r, "sntl_attn_pack_heads")
     lib = _lib.load()
     _require(matrix, "matrix")
     if matrix.dtype != torch.float32 or matrix.dim() != 2 or matrix.shape[0] != heads * head_dim:
@@ -173,6 +179,9 @@ def pack_heads(matrix, batch, heads, seq, head_dim, *, column_start=0, cos_table
 def unpack_heads(tensor, matrix, *, column_start=0, cos_table=None, sin_table=None, position_offset=0, inverse=False):
     """bf16 ``[batch, heads, seq, head_dim]`` -> columns of an fp32 feature-major matrix (written in place), with the
     forward or (``inverse=True``, for dQ and dK) inverse rotation on the way."""
+    r = _lib.host().unpack_heads(tensor, matrix, column_start, cos_table, sin_table, position_offset, inverse)
+    if r is not None:
+        return r if r.__class__ is not int else _lib.check(r, "sntl_attn_unpack_heads")
     lib = _lib.load()
     _require(tensor, "tensor")
     _require(matrix, "matrix")
@@ -191,6 +200,9 @@ def unpack_heads(tensor, matrix, *, column_start=0, cos_table=None, sin_table=No
 def attention_backward(q, k, v, o, lse, dout, *, causal=True, scale=None, flags=0, dq=None, dk=None, dv=None, window=0,
                        global_tokens=0):
     """dQ, dK, dV from dO (P recomputed from LSE).  Shapes as in attention_forward."""
+    r = _lib.host().backward(q, k, v, o, lse, dout, causal, scale, flags, dq, dk, dv, window, global_tokens)
+    if r is not None:
+        return r if r.__class__ is tuple else _lib.check(r, "sntl_attn_bwd")
     lib = _lib.load()
     for t, n in ((q, "q"), (k, "k"), (v, "v"), (o, "o"), (lse, "lse"), (dout, "dout")):
         _require(t, n)
@@ -386,6 +398,11 @@ class CudaFlashAttention:
     @staticmethod
     def forwardMultiHead(query, key, value, out, logSumExp, headCount, headDimension, scale, causal=True, columnStart=0,
                          columnCount=0, packCount=1, windowSize=0, globalTokenCount=0):
+        r = _lib.host().matrix_forward(query, key, value, out, logSumExp, headCount, headDimension, scale, causal, columnStart, columnCount,
+                                       packCount, windowSize, globalTokenCount,
+                                       _lib.FLAG_ALLOW_BF16_COMPUTE if CudaFlashAttention.allow_reduced_precision else 0)
+        if r is not None:
+            return r if r.__class__ is tuple else _lib.check(r, "CudaFlashAttention::forwardMultiHead")
         lib = _lib.load()
         if key.shape != value.shape:
             raise ValueError("CudaFlashAttention key/value rows mismatch")
@@ -416,6 +433,11 @@ class CudaFlashAttention:
     def backwardMultiHead(query, key, value, out, logSumExp, outGradient, queryGradient, keyGradient, valueGradient,
                           deltaWorkspace, headCount, headDimension, scale, causal=True, columnStart=0, columnCount=0,
                           packCount=1, windowSize=0, globalTokenCount=0):
+        r = _lib.host().matrix_backward(query, key, value, out, logSumExp, outGradient, queryGradient, keyGradient, valueGradient,
+                                        headCount, headDimension, scale, causal, columnStart, columnCount, packCount, windowSize,
+                                        globalTokenCount, _lib.FLAG_ALLOW_BF16_COMPUTE if CudaFlashAttention.allow_reduced_precision else 0)
+        if r is not None:
+            return r if r.__class__ is tuple else _lib.check(r, "CudaFlashAttention::backwardMultiHead")
         lib = _lib.load()
         d = CudaFlashAttention._desc(query, key, headCount, headDimension, scale, causal, columnStart, columnCount, packCount,
                                      windowSize, globalTokenCount)

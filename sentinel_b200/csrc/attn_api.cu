@@ -6,6 +6,7 @@
 #include "common.cuh"
 
 #include <atomic>
+#include <initializer_list>
 #include <string.h>
 
 namespace sntl {
@@ -74,6 +75,20 @@ void views(const sntl_attn_desc* d, View4& vq, View4& vkv, View3& vlse)
         vkv = View4{(long long)d->seq_kv, D * C, 1, C};
         vlse = View3{(long long)d->seq_q, C, 1};
     }
+}
+
+// Whether rows of D elements can be accessed four at a time in every one of these tensors (null: not used by the call).
+bool rows_of_four(const View4& v, int D, bool is_bf16, std::initializer_list<const void*> tensors)
+{
+    const uintptr_t bytes = is_bf16 ? 8 : 16;
+    bool ok = v.sd == 1 && D % 4 == 0;   // sb, sh, ss are multiples of D then
+    for (const void* t : tensors) ok = ok && (uintptr_t)t % bytes == 0;
+    return ok;
+}
+void set_vector_access(SimtArgs& a)
+{
+    a.vec_q = rows_of_four(a.vq, a.s.D, a.is_bf16, {a.q, a.o, a.dout, a.o_out, a.dq});
+    a.vec_kv = rows_of_four(a.vkv, a.s.D, a.is_bf16, {a.k, a.v, a.dk, a.dv});
 }
 
 struct Carve {
@@ -188,6 +203,7 @@ int sntl_attn_fwd(const sntl_attn_desc* d, const void* q, const void* k, const v
         a.q = (const char*)q + off; a.k = (const char*)k + off; a.v = (const char*)v + off;
         a.o_out = (char*)o + off; a.lse_out = (float*)((char*)lse + off);
         views(d, a.vq, a.vkv, a.vlse);
+        set_vector_access(a);
         g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
         return cuda_status(simt_forward(a, st));
     }
@@ -294,6 +310,7 @@ int sntl_attn_cached_fwd(const sntl_attn_desc* d, const void* q, const void* k_c
     views(d, a.vq, a.vkv, a.vlse);
     const long long D = d->head_dim, C = cache_capacity;
     a.vkv = d->layout == SNTL_LAYOUT_BHSD ? View4{(long long)d->kv_heads * C * D, C * D, D, 1} : View4{0, D * C, 1, C};
+    set_vector_access(a);
     g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
     return cuda_status(simt_forward(a, st));
 }
@@ -320,10 +337,8 @@ int sntl_attn_bwd(const sntl_attn_desc* d, const void* q, const void* k, const v
         a.q = (const char*)q + off; a.k = (const char*)k + off; a.v = (const char*)v + off;
         a.o = (const char*)o + off; a.dout = (const char*)dout + off; a.lse = (const float*)((const char*)lse + off);
         a.dq = (char*)dq + off; a.dk = (char*)dk + off; a.dv = (char*)dv + off;
-        a.delta = (float*)c.take(4 * nlse(d));
-        if (!c.ok) return SNTL_ERR_WORKSPACE;
         views(d, a.vq, a.vkv, a.vlse);
-        a.vdelta = View3{(long long)d->q_heads * d->seq_q, (long long)d->seq_q, 1};
+        set_vector_access(a);
         g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
         return cuda_status(simt_backward(a, st));
     }

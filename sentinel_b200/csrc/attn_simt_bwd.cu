@@ -1,0 +1,208 @@
+// Exact-fp32 backward: one launch whose CTAs have one of two roles.
+//   dK/dV   8*TM key rows of one (batch, KV head); visits the query tiles that see them, for every query head of the group:
+//           S^T, dP^T, then dV += P^T dO and dK += dS^T Q.  One owner per element: deterministic, no atomics.
+//   dQ      8*TM query rows of one (batch, head); visits the key tiles they see: S, dP, then dQ += dS K.
+// (sentinel/NeuralNet/Layers/CausalSelfAttention.cpp:333-352.)  Both recompute P from the saved log-sum-exp and take
+// delta = rowsum(dO o O) from the O rows that are read along with dO: 1/64 of a tile's FMAs instead of a launch of its own.
+// Seven products where a backward with dQ reductions needs five, but dQ stays reproducible without scratch.
+//
+// Bound by the fp32 FMA pipes.  The dK/dV CTAs come first: they are the longer ones (four products per pair against three,
+// times the heads of the group).
+#include "attn_simt.cuh"
+
+namespace sntl {
+using namespace simt;
+namespace {
+
+template <int TM, int TN, int DP> struct BwdSmem {
+    static constexpr int kRows = 8 * TM, kLoop = 16 * TN, P = DP + 4;
+    // own rows (K, V or Q, dO), loop rows (Q, dO or K, V), P and dS weights, partial sums of delta, per-row terms
+    static constexpr int own0 = 0, own1 = own0 + kRows * P, in0 = own1 + kRows * P, in1 = in0 + kLoop * P;
+    static constexpr int w0 = in1 + kLoop * P, w1 = w0 + kLoop * (kRows + 4);
+    static constexpr int kDeltaRows = kRows > kLoop ? kRows : kLoop;
+    static constexpr int part = w1 + kLoop * (kRows + 4), lse = part + kDeltaRows * (DP / 4 + 1), delta = lse + kDeltaRows;
+    static constexpr size_t bytes = (delta + kDeltaRows) * sizeof(float);
+};
+
+template <typename T, int TM, int TN, int DP>
+__device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* smem)
+{
+    using L = BwdSmem<TM, TN, DP>;
+    using M = OutMap<DP>;
+    const AttnShape& s = a.s;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, group = s.Hq / s.Hkv;
+    const int slabs = s.B * s.Hkv, slab = tile % slabs, b = slab / s.Hkv, hk = slab - b * s.Hkv;
+    const int key0 = (tile / slabs) * L::kRows;               // causal: the first key tiles are seen by the most queries
+    const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
+    const long long kvoff = b * a.vkv.sb + hk * a.vkv.sh;
+    stage<T, DP, L::kRows>(smem + L::own0, (const T*)a.k + kvoff, mk, key0);
+    stage<T, DP, L::kRows>(smem + L::own1, (const T*)a.v + kvoff, mk, key0);
+    float dk[TM][M::N], dv[TM][M::N];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int n = 0; n < M::N; ++n) dk[i][n] = dv[i][n] = 0.f;
+
+    const int shift = s.Skv - s.Sq;                           // first query that sees key j: j - shift
+    const int q_first = s.causal ? max(0, key0 - shift) / L::kLoop * L::kLoop : 0;
+    for (int g = 0; g < group; ++g) {
+        const int h = hk * group + g;
+        const long long qoff = b * a.vq.sb + h * a.vq.sh;
+        for (int q0 = q_first; q0 < s.Sq; q0 += L::kLoop) {
+            // past the window of the last key (and no key is global): no later query sees these keys
+            if (s.window > 0 && key0 >= s.global_tokens && q0 + shift > key0 + L::kRows - 1 + s.window - 1) break;
+            __syncthreads();
+            stage<T, DP, L::kLoop>(smem + L::in0, (const T*)a.q + qoff, mq, q0);
+            stage_with_delta<T, DP, L::kLoop>(smem + L::in1, smem + L::part, (const T*)a.dout + qoff, (const T*)a.o + qoff, mq, q0);
+            if (threadIdx.x < L::kLoop) {
+                const int r = q0 + threadIdx.x;
+                smem[L::lse + threadIdx.x] = r < s.Sq ? a.lse[b * a.vlse.sb + h * a.vlse.sh + (long long)r * a.vlse.ss] : -INFINITY;
+            }
+            __syncthreads();
+            if (threadIdx.x < L::kLoop) smem[L::delta + threadIdx.x] = delta_of<DP>(smem + L::part, threadIdx.x);
+            float p[TM][TN], ds[TM][TN];
+            scores<TM, TN, DP>(p, smem + L::own0, smem + L::in0);
+            scores<TM, TN, DP>(ds, smem + L::own1, smem + L::in1);
+            __syncthreads();
+            // every (query, key) pair of the tile is visible: no masks
+            const bool cut = (s.causal && q0 + shift < key0 + L::kRows - 1) || s.window > 0 || key0 + L::kRows > s.Skv;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int q = q0 + tx + 16 * j;
+                const float lse = smem[L::lse + tx + 16 * j], delta = smem[L::delta + tx + 16 * j];
+                float wp[TM], ws[TM];
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const int key = key0 + ty + 8 * i;
+                    const bool vis = lse > -INFINITY && (!cut || ((!s.causal || key <= q + shift) && window_allows(s, q + shift, key)));
+                    wp[i] = vis ? expf(fmaf(p[i][j], s.scale, -lse)) : 0.f;
+                    ws[i] = wp[i] * (ds[i][j] - delta) * s.scale;
+                }
+                put_weights<TM>(smem + L::w0, tx + 16 * j, wp);
+                put_weights<TM>(smem + L::w1, tx + 16 * j, ws);
+            }
+            __syncwarp();
+            outputs<TM, DP, L::kLoop>(dv, smem + L::w0, smem + L::in1);
+            outputs<TM, DP, L::kLoop>(dk, smem + L::w1, smem + L::in0);
+        }
+    }
+    __syncthreads();
+    store_rows<T, TM, DP>((T*)a.dk + kvoff, mk, key0, dk, smem + L::own0);
+    store_rows<T, TM, DP>((T*)a.dv + kvoff, mk, key0, dv, smem + L::own1);
+}
+
+template <typename T, int TM, int TN, int DP>
+__device__ __forceinline__ void dq_role(const SimtArgs& a, int tile, int n_qt, float* smem)
+{
+    using L = BwdSmem<TM, TN, DP>;
+    using M = OutMap<DP>;
+    const AttnShape& s = a.s;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int slabs = s.B * s.Hq, bh = tile % slabs, b = bh / s.Hq, h = bh - b * s.Hq, hk = h / (s.Hq / s.Hkv);
+    const int row0 = (n_qt - 1 - tile / slabs) * L::kRows;    // longest query tiles first
+    const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
+    const long long qoff = b * a.vq.sb + h * a.vq.sh;
+    const T* kb = (const T*)a.k + b * a.vkv.sb + hk * a.vkv.sh;
+    const T* vb = (const T*)a.v + b * a.vkv.sb + hk * a.vkv.sh;
+    stage<T, DP, L::kRows>(smem + L::own0, (const T*)a.q + qoff, mq, row0);
+    stage_with_delta<T, DP, L::kRows>(smem + L::own1, smem + L::part, (const T*)a.dout + qoff, (const T*)a.o + qoff, mq, row0);
+    __syncthreads();
+    float lse[TM], delta[TM], dq[TM][M::N];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int row = row0 + ty + 8 * i;
+        lse[i] = row < s.Sq ? a.lse[b * a.vlse.sb + h * a.vlse.sh + (long long)row * a.vlse.ss] : -INFINITY;
+        delta[i] = delta_of<DP>(smem + L::part, ty + 8 * i);
+#pragma unroll
+        for (int n = 0; n < M::N; ++n) dq[i][n] = 0.f;
+    }
+    const int shift = s.causal ? s.Skv - s.Sq : 0;
+    const int n_keys = visible_keys(s, min(row0 + L::kRows, s.Sq) - 1);
+    for (int k0 = 0; k0 < n_keys; k0 += L::kLoop) {
+        // tiles between the global tokens and the window of the first row are visible to no row
+        if (s.window > 0 && k0 >= s.global_tokens && k0 + L::kLoop - 1 < row0 + shift - s.window + 1) continue;
+        __syncthreads();
+        stage<T, DP, L::kLoop>(smem + L::in0, kb, mk, k0);
+        stage<T, DP, L::kLoop>(smem + L::in1, vb, mk, k0);
+        __syncthreads();
+        float p[TM][TN], ds[TM][TN];
+        scores<TM, TN, DP>(p, smem + L::own0, smem + L::in0);
+        scores<TM, TN, DP>(ds, smem + L::own1, smem + L::in1);
+        const bool cut = k0 + L::kLoop > visible_keys(s, row0) || s.window > 0;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int key = k0 + tx + 16 * j;
+            float w[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const int row = row0 + ty + 8 * i;
+                const bool vis = lse[i] > -INFINITY && (!cut || (key < visible_keys(s, row) && window_allows(s, row + shift, key)));
+                const float x = vis ? expf(fmaf(p[i][j], s.scale, -lse[i])) : 0.f;
+                w[i] = x * (ds[i][j] - delta[i]) * s.scale;
+            }
+            put_weights<TM>(smem + L::w0, tx + 16 * j, w);
+        }
+        __syncwarp();
+        outputs<TM, DP, L::kLoop>(dq, smem + L::w0, smem + L::in0);
+    }
+    __syncthreads();
+    store_rows<T, TM, DP>((T*)a.dq + qoff, mq, row0, dq, smem + L::own0);
+}
+
+template <typename T, int TM, int TN, int DP>
+__global__ void __launch_bounds__(kThreads) simt_bwd_kernel(const SimtArgs a, int n_dkv, int n_qt)
+{
+    extern __shared__ __align__(16) float smem[];
+    if ((int)blockIdx.x < n_dkv) dkv_role<T, TM, TN, DP>(a, blockIdx.x, smem);
+    else dq_role<T, TM, TN, DP>(a, blockIdx.x - n_dkv, n_qt, smem);
+}
+
+template <typename T, int TM, int TN, int DP>
+cudaError_t launch(const SimtArgs& a, cudaStream_t st)
+{
+    using L = BwdSmem<TM, TN, DP>;
+    auto kernel = simt_bwd_kernel<T, TM, TN, DP>;
+    static std::atomic<unsigned long long> configured{0};
+    cudaError_t e = ensure_dynamic_smem(kernel, L::bytes, configured);
+    if (e != cudaSuccess) return e;
+    const int n_qt = (a.s.Sq + L::kRows - 1) / L::kRows, n_kt = (a.s.Skv + L::kRows - 1) / L::kRows;
+    const long long n_dkv = (long long)n_kt * a.s.B * a.s.Hkv, n_dq = (long long)n_qt * a.s.B * a.s.Hq;
+    if (n_dkv + n_dq > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    kernel<<<(unsigned)(n_dkv + n_dq), kThreads, L::bytes, st>>>(a, (int)n_dkv, n_qt);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// Tile height as in the forward: the largest whose grid still gives every SM its two resident CTAs.
+template <typename T, int DP>
+cudaError_t dispatch(const SimtArgs& a, cudaStream_t st)
+{
+    constexpr int TN = DP <= 64 ? 4 : 2, kTop = DP <= 64 ? 8 : 4;
+    auto ctas = [&](int rows) {
+        return ((a.s.Sq + rows - 1) / rows * (long long)a.s.Hq + (a.s.Skv + rows - 1) / rows * (long long)a.s.Hkv) * a.s.B;
+    };
+    const int sms = sm_count();
+    if (kTop == 8 && ctas(64) >= 4 * sms) return launch<T, kTop, TN, DP>(a, st);
+    if (ctas(32) >= 4 * sms) return launch<T, 4, TN, DP>(a, st);
+    return launch<T, 2, TN, DP>(a, st);
+}
+
+template <typename T>
+cudaError_t dispatch_dim(const SimtArgs& a, cudaStream_t st)
+{
+    if (a.s.D <= 16) return dispatch<T, 16>(a, st);
+    if (a.s.D <= 32) return dispatch<T, 32>(a, st);
+    if (a.s.D <= 64) return dispatch<T, 64>(a, st);
+    if (a.s.D <= 96) return dispatch<T, 96>(a, st);
+    if (a.s.D <= 128) return dispatch<T, 128>(a, st);
+    return dispatch<T, 256>(a, st);
+}
+
+}  // namespace
+
+cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st)
+{
+    return a.is_bf16 ? dispatch_dim<__nv_bfloat16>(a, st) : dispatch_dim<float>(a, st);
+}
+
+}  // namespace sntl

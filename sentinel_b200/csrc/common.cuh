@@ -53,19 +53,34 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, size_t bytes, std::atomic<
     return cudaSuccess;
 }
 
-// Exact-fp32 SIMT kernels (attn_simt.cu).  T = float or __nv_bfloat16 element type.
+// SMs of the current device (148 on a B200), read once per device ordinal
+inline int sm_count()
+{
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = cached[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        cached[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// Exact-fp32 SIMT kernels (attn_simt_fwd.cu, attn_simt_bwd.cu).  T = float or __nv_bfloat16 element type.
 struct SimtArgs {
     AttnShape s;
     int is_bf16;
     const void *q, *k, *v, *o, *dout;
     void *o_out, *dq, *dk, *dv;
-    float *lse_out, *delta;
+    float* lse_out;
     const float* lse;
     View4 vq, vkv;     // q-like tensors (Q, O, dO, dQ) and kv-like tensors (K, V, dK, dV)
-    View3 vlse, vdelta;
+    View3 vlse;
+    bool vec_q, vec_kv;   // every row of all q-like / kv-like tensors can be accessed four elements at a time
 };
 cudaError_t simt_forward(const SimtArgs& a, cudaStream_t st);
-cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st);  // delta pass + dQ kernel + dK/dV kernel
+cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st);  // one launch
 
 // Tensor-core kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu): bf16, BHSD contiguous, D in {64,128}.
 struct TcArgs {

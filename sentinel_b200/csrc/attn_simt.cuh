@@ -136,16 +136,30 @@ __device__ __forceinline__ float delta_of(const float* part, int r)
     return s;
 }
 
+// Two fp32 FMAs in one instruction, each rounded as the scalar one.  The products below use nothing else: three-operand
+// scalar FMAs stall in dispatch on their register reads (forward B8 H12 S512 D64: 129 us with them, the FMA pipes 45 % busy).
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+          "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
+}
+
+// (the two halves of an accumulator take the even and the odd features)
 template <int TM, int TN, int DP>
-__device__ __forceinline__ void scores(float (&acc)[TM][TN], const float* A, const float* B)
+__device__ __forceinline__ void scores(float (&out)[TM][TN], const float* A, const float* B)
 {
     constexpr int P = DP + 4;
     const float* a0 = A + (threadIdx.x >> 4) * P;
     const float* b0 = B + (threadIdx.x & 15) * P;
+    float2 acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 4
     for (int d = 0; d < DP; d += 4) {
         float4 b[TN];
@@ -155,14 +169,15 @@ __device__ __forceinline__ void scores(float (&acc)[TM][TN], const float* A, con
         for (int i = 0; i < TM; ++i) {
             const float4 a = *reinterpret_cast<const float4*>(a0 + i * 8 * P + d);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                acc[i][j] = fmaf(a.x, b[j].x, acc[i][j]);
-                acc[i][j] = fmaf(a.y, b[j].y, acc[i][j]);
-                acc[i][j] = fmaf(a.z, b[j].z, acc[i][j]);
-                acc[i][j] = fmaf(a.w, b[j].w, acc[i][j]);
-            }
+            for (int j = 0; j < TN; ++j) acc[i][j] = ffma2(make_float2(a.x, a.y), make_float2(b[j].x, b[j].y), acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = ffma2(make_float2(a.z, a.w), make_float2(b[j].z, b[j].w), acc[i][j]);
         }
     }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) out[i][j] = acc[i][j].x + acc[i][j].y;
 }
 
 // columns of the outputs a thread owns: NV vectors of VW, starting at tx*VW + 16*VW*c
@@ -189,24 +204,31 @@ template <int V> __device__ __forceinline__ void load_vec(float* x, const float*
     }
 }
 
-// W: [K][8*TM + 4], B: [K][DP + 4]
+// W: [K][8*TM + 4], B: [K][DP + 4].  acc[i] holds rows 2i and 2i + 1 of the thread: their weights are neighbours in W.
 template <int TM, int DP, int K>
-__device__ __forceinline__ void outputs(float (&acc)[TM][OutMap<DP>::N], const float* W, const float* B)
+__device__ __forceinline__ void outputs(float2 (&acc)[TM / 2][OutMap<DP>::N], const float* W, const float* B)
 {
     using M = OutMap<DP>;
     const float* w0 = W + (threadIdx.x >> 4) * TM;
     const float* b0 = B + (threadIdx.x & 15) * M::VW;
-#pragma unroll 8
+#pragma unroll 4
     for (int k = 0; k < K; ++k) {
         float w[TM], b[M::N];
         load_vec<TM>(w, w0 + k * (8 * TM + 4));
 #pragma unroll
         for (int c = 0; c < M::NV; ++c) load_vec<M::VW>(b + c * M::VW, b0 + k * (DP + 4) + c * 16 * M::VW);
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+        for (int n = 0; n < M::N; ++n)
 #pragma unroll
-            for (int n = 0; n < M::N; ++n) acc[i][n] = fmaf(w[i], b[n], acc[i][n]);
+            for (int i = 0; i < TM / 2; ++i) acc[i][n] = ffma2(make_float2(w[2 * i], w[2 * i + 1]), make_float2(b[n], b[n]), acc[i][n]);
     }
+}
+template <int TM, int N> __device__ __forceinline__ void clear(float2 (&acc)[TM][N])
+{
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[i][n] = make_float2(0.f, 0.f);
 }
 template <int TM> __device__ __forceinline__ void put_weights(float* W, int k, const float (&w)[TM])
 {
@@ -222,14 +244,14 @@ template <int TM> __device__ __forceinline__ void put_weights(float* W, int k, c
 
 // The CTA's 8*TM rows of outputs, through `buf` ([8*TM][DP + 4], free of readers) so that stores coalesce in either layout.
 template <typename T, int TM, int DP>
-__device__ __forceinline__ void store_rows(T* base, const Slab& m, int row0, const float (&acc)[TM][OutMap<DP>::N], float* buf)
+__device__ __forceinline__ void store_rows(T* base, const Slab& m, int row0, const float2 (&acc)[TM / 2][OutMap<DP>::N], float* buf)
 {
     using M = OutMap<DP>;
     const int ty = threadIdx.x >> 4;
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int n = 0; n < M::N; ++n) buf[(ty + 8 * i) * (DP + 4) + M::col(n)] = acc[i][n];
+        for (int n = 0; n < M::N; ++n) buf[(ty + 8 * i) * (DP + 4) + M::col(n)] = i & 1 ? acc[i / 2][n].y : acc[i / 2][n].x;
     __syncthreads();
     constexpr int kUnits = 8 * TM * DP / 4;
     for (int u = threadIdx.x; u < kUnits; u += kThreads) {

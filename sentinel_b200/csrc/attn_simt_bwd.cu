@@ -6,7 +6,9 @@
 // delta = rowsum(dO o O) from the O rows that are read along with dO: 1/64 of a tile's FMAs instead of a launch of its own.
 // Seven products where a backward with dQ reductions needs five, but dQ stays reproducible without scratch.
 //
-// Bound by the fp32 FMA pipes.  The dK/dV CTAs come first: they are the longer ones (four products per pair against three,
+// Bound by the fp32 FMA pipes (B8 H12 S512 D64: 424 us against 195 us of packed FMAs at the 112 lanes per clock that they
+// reach in isolation; staging and exponentials are 10 % each, the rest is shared-memory latency at eight warps per SM; 2740 us
+// with one warp per row).  Twice the warps with half the rows each take as long: they load twice as much per FMA.  The dK/dV CTAs come first: they are the longer ones (four products per pair against three,
 // times the heads of the group).
 #include "attn_simt.cuh"
 
@@ -37,11 +39,9 @@ __device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* sme
     const long long kvoff = b * a.vkv.sb + hk * a.vkv.sh;
     stage<T, DP, L::kRows>(smem + L::own0, (const T*)a.k + kvoff, mk, key0);
     stage<T, DP, L::kRows>(smem + L::own1, (const T*)a.v + kvoff, mk, key0);
-    float dk[TM][M::N], dv[TM][M::N];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int n = 0; n < M::N; ++n) dk[i][n] = dv[i][n] = 0.f;
+    float2 dk[TM / 2][M::N], dv[TM / 2][M::N];
+    clear(dk);
+    clear(dv);
 
     const int shift = s.Skv - s.Sq;                           // first query that sees key j: j - shift
     const int q_first = s.causal ? max(0, key0 - shift) / L::kLoop * L::kLoop : 0;
@@ -107,14 +107,14 @@ __device__ __forceinline__ void dq_role(const SimtArgs& a, int tile, int n_qt, f
     stage<T, DP, L::kRows>(smem + L::own0, (const T*)a.q + qoff, mq, row0);
     stage_with_delta<T, DP, L::kRows>(smem + L::own1, smem + L::part, (const T*)a.dout + qoff, (const T*)a.o + qoff, mq, row0);
     __syncthreads();
-    float lse[TM], delta[TM], dq[TM][M::N];
+    float lse[TM], delta[TM];
+    float2 dq[TM / 2][M::N];
+    clear(dq);
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int row = row0 + ty + 8 * i;
         lse[i] = row < s.Sq ? a.lse[b * a.vlse.sb + h * a.vlse.sh + (long long)row * a.vlse.ss] : -INFINITY;
         delta[i] = delta_of<DP>(smem + L::part, ty + 8 * i);
-#pragma unroll
-        for (int n = 0; n < M::N; ++n) dq[i][n] = 0.f;
     }
     const int shift = s.causal ? s.Skv - s.Sq : 0;
     const int n_keys = visible_keys(s, min(row0 + L::kRows, s.Sq) - 1);

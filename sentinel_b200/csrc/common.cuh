@@ -80,6 +80,9 @@ struct SimtArgs {
     bool vec_q, vec_kv;   // every row of all q-like / kv-like tensors can be accessed four elements at a time
 };
 cudaError_t simt_forward(const SimtArgs& a, cudaStream_t st);
+// few query rows per KV head (decode): simt_forward takes this path by itself where it applies
+bool simt_decode_supported(const SimtArgs& a);
+cudaError_t simt_decode(const SimtArgs& a, cudaStream_t st);
 cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st);  // one launch
 
 // Tensor-core kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu): bf16, BHSD contiguous, D in {64,128}.

@@ -57,6 +57,26 @@ def test_exact_cached_forward_matches_reference_rows(sb, name, T):
     assert max_abs(_np(lse), g["lse"][:, :, L - T:L]) <= F32_TOL
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,T,L,D,window", [
+    (1, 12, 12, 1, 777, 64, 0),      # a cluster of eight, the last piece shorter
+    (3, 2, 2, 1, 128, 32, 0),        # exactly one pass of keys
+    (1, 6, 2, 2, 129, 128, 0),       # six of eight rows in use, one key past a pass
+    (2, 8, 1, 1, 2100, 64, 300),     # most pieces hidden by the window
+    (1, 9, 1, 1, 500, 64, 0),        # too many rows: the tiles of the general kernel, keys split over a cluster
+])
+def test_exact_decode_vs_oracle(sb, oracle, B, Hq, Hkv, T, L, D, window):
+    rng = np.random.default_rng(L + D)
+    q = rng.standard_normal((B, Hq, T, D), dtype=np.float32)
+    k, v = (rng.standard_normal((B, Hkv, L, D), dtype=np.float32) for _ in range(2))
+    full = np.zeros((B, Hq, L, D), dtype=np.float32)      # the new tokens are the last T rows of full causal attention
+    full[:, :, L - T:] = q
+    wo, wl = oracle.attn_fwd(full, k, v, window=window, global_tokens=0)
+    o, lse = sb.attention_cached_forward(torch.from_numpy(q).cuda(), _cache(k, L + 7, torch.float32), _cache(v, L + 7, torch.float32), L,
+                                         window=window)
+    assert sb.last_path() == "simt_f32"
+    assert max_abs(_np(o), wo[:, :, L - T:]) <= F32_TOL and max_abs(_np(lse), wl[:, :, L - T:]) <= F32_TOL
+
+
 def test_exact_cached_forward_reference_matrix_layout(sb):
     """The reference's own shapes: query (Hq*D) x 1, caches (Hkv*D) x maximumPositionCount feature-major (CudaKvCache)."""
     lib = sb._lib.load()

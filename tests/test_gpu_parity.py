@@ -72,6 +72,30 @@ def test_f32_exact_path_edge_shapes_vs_oracle(sb, oracle, shape):
         assert max_abs(_np(got), want) <= F32_TOL, (key, max_abs(_np(got), want))
 
 
+@pytest.mark.parametrize("shape", [
+    (8, 12, 12, 200, 64),     # 64-row tiles, ragged
+    (4, 12, 4, 129, 32),      # 32-row tiles, one row past a tile; grouped-query heads
+    (2, 4, 4, 64, 16),        # 16-row tiles, no remainder
+    (1, 2, 1, 513, 64),       # 16-row tiles with the keys of the forward split over a cluster
+    (2, 3, 3, 70, 80),        # head_dim between two compiled sizes
+    (4, 10, 5, 97, 128),
+])
+@pytest.mark.parametrize("window,globals_", [(0, 0), (33, 5)])
+def test_f32_tile_heights_vs_oracle(sb, oracle, shape, window, globals_):
+    """Every tile height of the exact kernels at its edges.  fp32 sums of at most a few hundred terms of order one: 1e-4
+    absolute is far above their rounding (about 1e-6) and far below any misplaced element."""
+    B, Hq, Hkv, S, D = shape
+    rng = np.random.default_rng(S + D)
+    q, k, v, do = (rng.standard_normal((B, H, S, D), dtype=np.float32) for H in (Hq, Hkv, Hkv, Hq))
+    kw = dict(window=window, global_tokens=globals_)
+    o, lse = sb.attention_forward(_dev(q), _dev(k), _dev(v), **kw)
+    dq, dk, dv = sb.attention_backward(_dev(q), _dev(k), _dev(v), o, lse, _dev(do), **kw)
+    wo, wl = oracle.attn_fwd(q, k, v, **kw)
+    wdq, wdk, wdv, _ = oracle.attn_bwd(q, k, v, do, **kw)
+    for got, want, key in ((o, wo, "o"), (lse, wl, "lse"), (dq, wdq, "dq"), (dk, wdk, "dk"), (dv, wdv, "dv")):
+        assert max_abs(_np(got), want) <= F32_TOL, (key, max_abs(_np(got), want))
+
+
 def test_f32_noncausal_rectangular_and_merge(sb, oracle):
     """Ring building blocks: non-causal attention with Sq != Skv, and the LSE merge of two key halves."""
     rng = np.random.default_rng(21)

@@ -120,18 +120,14 @@ bool device_ok()
     return major == 10;
 }
 
-// Stage one tensor of `heads` heads into bf16 BHSD.
-cudaError_t stage_in(const sntl_attn_desc* d, const void* src, __nv_bfloat16* dst, int heads, int S, cudaStream_t st)
+// the three conversions every feature-major call starts with
+void stage_qkv(const sntl_attn_desc* d, MatrixStage& m, const void* q, __nv_bfloat16* qb, const void* k, __nv_bfloat16* kb, const void* v,
+               __nv_bfloat16* vb)
 {
-    if (d->layout == SNTL_LAYOUT_SENTINEL)
-        return sentinel_to_bhsd_bf16((const float*)src, dst, d->batch, heads, S, d->head_dim, d->stride_columns, d->column_start, st);
-    return f32_to_bf16((const float*)src, dst, (size_t)d->batch * heads * S * d->head_dim, st);
-}
-cudaError_t stage_out(const sntl_attn_desc* d, const __nv_bfloat16* src, void* dst, int heads, int S, cudaStream_t st)
-{
-    if (d->layout == SNTL_LAYOUT_SENTINEL)
-        return bhsd_bf16_to_sentinel(src, (float*)dst, d->batch, heads, S, d->head_dim, d->stride_columns, d->column_start, st);
-    return bf16_to_f32(src, (float*)dst, (size_t)d->batch * heads * S * d->head_dim, st);
+    m.n = 3;
+    m.src[0] = (const float*)q; m.dst[0] = qb; m.heads[0] = d->q_heads;
+    m.src[1] = (const float*)k; m.dst[1] = kb; m.heads[1] = d->kv_heads;
+    m.src[2] = (const float*)v; m.dst[2] = vb; m.heads[2] = d->kv_heads;
 }
 
 }  // namespace
@@ -167,8 +163,8 @@ size_t sntl_attn_fwd_workspace_bytes(const sntl_attn_desc* d)
 {
     if (validate(d) != SNTL_OK) return 0;
     if (!wants_tc(d, false) || !needs_staging(d)) return 0;
-    // bf16 copies of Q, K, V, O and a [B][Hq][S] LSE when the caller's LSE is feature-major
-    return align_up(2 * nq_elems(d)) * 2 + align_up(2 * nkv_elems(d)) * 2 + align_up(4 * nlse(d));
+    // bf16 copies of Q, K, V; of O too unless it leaves the kernel as a matrix
+    return align_up(2 * nq_elems(d)) * (d->layout == SNTL_LAYOUT_SENTINEL ? 1 : 2) + align_up(2 * nkv_elems(d)) * 2;
 }
 
 size_t sntl_attn_bwd_workspace_bytes(const sntl_attn_desc* d)
@@ -177,8 +173,10 @@ size_t sntl_attn_bwd_workspace_bytes(const sntl_attn_desc* d)
     size_t bytes = align_up(4 * nlse(d));  // delta (exact path) -- the tensor-core path sizes its own below
     if (!wants_tc(d, true)) return bytes;
     bytes = align_up(tc_backward_workspace_bytes(shape_of(d)));
-    if (needs_staging(d))  // bf16 Q,O,dO,dQ + K,V,dK,dV + LSE
-        bytes += align_up(2 * nq_elems(d)) * 4 + align_up(2 * nkv_elems(d)) * 4 + align_up(4 * nlse(d));
+    if (d->layout == SNTL_LAYOUT_SENTINEL)   // bf16 Q, dO, K, V
+        bytes += align_up(2 * nq_elems(d)) * 2 + align_up(2 * nkv_elems(d)) * 2;
+    else if (needs_staging(d))               // bf16 Q, O, dO, dQ, K, V, dK, dV
+        bytes += align_up(2 * nq_elems(d)) * 4 + align_up(2 * nkv_elems(d)) * 4;
     return bytes;
 }
 
@@ -219,23 +217,28 @@ int sntl_attn_fwd(const sntl_attn_desc* d, const void* q, const void* k, const v
     g_last_path = "tcgen05_staged";
     Carve c{(char*)workspace, workspace_bytes};
     auto* qb = (__nv_bfloat16*)c.take(2 * nq_elems(d));
-    auto* ob = (__nv_bfloat16*)c.take(2 * nq_elems(d));
     auto* kb = (__nv_bfloat16*)c.take(2 * nkv_elems(d));
     auto* vb = (__nv_bfloat16*)c.take(2 * nkv_elems(d));
-    auto* lb = (float*)c.take(4 * nlse(d));
+    t.q = qb; t.k = kb; t.v = vb;
+    if (d->layout == SNTL_LAYOUT_SENTINEL) {
+        if (!c.ok) return SNTL_ERR_WORKSPACE;
+        MatrixStage m{};
+        stage_qkv(d, m, q, qb, k, kb, v, vb);
+        if (stage_matrices(m, d->batch, d->q_heads, d->seq_q, d->head_dim, d->stride_columns, d->column_start, d->scale, st) != cudaSuccess)
+            return SNTL_ERR_CUDA;
+        t.mat.o = (float*)o + d->column_start;
+        t.mat.lse = lse + d->column_start;
+        t.mat.stride = d->stride_columns;
+        return cuda_status(tc_forward(t, st));
+    }
+    auto* ob = (__nv_bfloat16*)c.take(2 * nq_elems(d));
     if (!c.ok) return SNTL_ERR_WORKSPACE;
-    cudaError_t e;
-    if ((e = stage_in(d, q, qb, d->q_heads, d->seq_q, st)) != cudaSuccess) return SNTL_ERR_CUDA;
-    if ((e = stage_in(d, k, kb, d->kv_heads, d->seq_kv, st)) != cudaSuccess) return SNTL_ERR_CUDA;
-    if ((e = stage_in(d, v, vb, d->kv_heads, d->seq_kv, st)) != cudaSuccess) return SNTL_ERR_CUDA;
-    t.q = qb; t.k = kb; t.v = vb; t.o_out = ob;
-    t.lse_out = d->layout == SNTL_LAYOUT_SENTINEL ? lb : lse;
-    if ((e = tc_forward(t, st)) != cudaSuccess) return SNTL_ERR_CUDA;
-    if ((e = stage_out(d, ob, o, d->q_heads, d->seq_q, st)) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (d->layout == SNTL_LAYOUT_SENTINEL &&
-        (e = lse_bhs_to_sentinel(lb, lse, d->batch, d->q_heads, d->seq_q, d->stride_columns, d->column_start, st)) != cudaSuccess)
-        return SNTL_ERR_CUDA;
-    return SNTL_OK;
+    t.o_out = ob; t.lse_out = lse;
+    if (f32_to_bf16((const float*)q, qb, nq_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (f32_to_bf16((const float*)k, kb, nkv_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (f32_to_bf16((const float*)v, vb, nkv_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (tc_forward(t, st) != cudaSuccess) return SNTL_ERR_CUDA;
+    return cuda_status(bf16_to_f32(ob, (float*)o, nq_elems(d), st));
 }
 
 namespace sntl {
@@ -359,32 +362,44 @@ int sntl_attn_bwd(const sntl_attn_desc* d, const void* q, const void* k, const v
     }
     g_last_path = "tcgen05_staged";
     auto* qb = (__nv_bfloat16*)c.take(2 * nq_elems(d));
-    auto* ob = (__nv_bfloat16*)c.take(2 * nq_elems(d));
     auto* gb = (__nv_bfloat16*)c.take(2 * nq_elems(d));
-    auto* dqb = (__nv_bfloat16*)c.take(2 * nq_elems(d));
     auto* kb = (__nv_bfloat16*)c.take(2 * nkv_elems(d));
     auto* vb = (__nv_bfloat16*)c.take(2 * nkv_elems(d));
+    t.q = qb; t.k = kb; t.v = vb; t.dout = gb; t.lse = lse;
+    if (d->layout == SNTL_LAYOUT_SENTINEL) {
+        if (!c.ok) return SNTL_ERR_WORKSPACE;
+        MatrixStage m{};
+        stage_qkv(d, m, q, qb, k, kb, v, vb);
+        m.n = 4;
+        m.src[3] = (const float*)dout; m.dst[3] = gb; m.heads[3] = d->q_heads;
+        m.o_mat = (const float*)o; m.do_mat = (const float*)dout; m.lse_mat = lse;
+        m.row_terms = t.delta;
+        m.dq_accum = t.dq_accum;
+        m.accum_bytes = (t.s.deterministic ? 8 : 4) * (size_t)d->batch * d->q_heads * sq_pad * d->head_dim;
+        if (stage_matrices(m, d->batch, d->q_heads, d->seq_q, d->head_dim, d->stride_columns, d->column_start, d->scale, st) != cudaSuccess)
+            return SNTL_ERR_CUDA;
+        t.mat.dq = (float*)dq + d->column_start;
+        t.mat.dk = (float*)dk + d->column_start;
+        t.mat.dv = (float*)dv + d->column_start;
+        t.mat.stride = d->stride_columns;
+        t.phases = kBwdMain | kBwdPost;
+        return cuda_status(tc_backward(t, st));
+    }
+    auto* ob = (__nv_bfloat16*)c.take(2 * nq_elems(d));
+    auto* dqb = (__nv_bfloat16*)c.take(2 * nq_elems(d));
     auto* dkb = (__nv_bfloat16*)c.take(2 * nkv_elems(d));
     auto* dvb = (__nv_bfloat16*)c.take(2 * nkv_elems(d));
-    auto* lb = (float*)c.take(4 * nlse(d));
     if (!c.ok) return SNTL_ERR_WORKSPACE;
-    if (stage_in(d, q, qb, d->q_heads, d->seq_q, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_in(d, o, ob, d->q_heads, d->seq_q, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_in(d, dout, gb, d->q_heads, d->seq_q, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_in(d, k, kb, d->kv_heads, d->seq_kv, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_in(d, v, vb, d->kv_heads, d->seq_kv, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    t.lse = lse;
-    if (d->layout == SNTL_LAYOUT_SENTINEL) {
-        if (lse_sentinel_to_bhs(lse, lb, d->batch, d->q_heads, d->seq_q, d->stride_columns, d->column_start, st) != cudaSuccess)
-            return SNTL_ERR_CUDA;
-        t.lse = lb;
-    }
-    t.q = qb; t.k = kb; t.v = vb; t.o = ob; t.dout = gb; t.dq = dqb; t.dk = dkb; t.dv = dvb;
+    t.o = ob; t.dq = dqb; t.dk = dkb; t.dv = dvb;
+    if (f32_to_bf16((const float*)q, qb, nq_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (f32_to_bf16((const float*)o, ob, nq_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (f32_to_bf16((const float*)dout, gb, nq_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (f32_to_bf16((const float*)k, kb, nkv_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (f32_to_bf16((const float*)v, vb, nkv_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
     if (tc_backward(t, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_out(d, dqb, dq, d->q_heads, d->seq_q, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_out(d, dkb, dk, d->kv_heads, d->seq_kv, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    if (stage_out(d, dvb, dv, d->kv_heads, d->seq_kv, st) != cudaSuccess) return SNTL_ERR_CUDA;
-    return SNTL_OK;
+    if (bf16_to_f32(dqb, (float*)dq, nq_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    if (bf16_to_f32(dkb, (float*)dk, nkv_elems(d), st) != cudaSuccess) return SNTL_ERR_CUDA;
+    return cuda_status(bf16_to_f32(dvb, (float*)dv, nkv_elems(d), st));
 }
 
 // ---- backward in pieces ----

@@ -42,6 +42,7 @@
 // TMEM map (512 columns): S^T/P^T [0,128)  dP^T/dQ [128,256)  then dV [256,384) dK [384,512) at head_dim 128, and
 // dV [256,320) dK [320,384) plus a second S^T/P^T buffer [384,512) at head_dim 64.
 #include "common.cuh"
+#include "row_terms.cuh"
 #include "sm100_ptx.cuh"
 
 namespace sntl {
@@ -75,6 +76,9 @@ struct BwdParams {
     int split_tiles;       // the first split_tiles key tiles are cut into one CTA per query head of the group
     float* dkv_part;       // [split tile][slab][head of group][dV, dK][128][D] fp32
     float *dk_acc, *dv_acc;   // non-null: dK*scale / dV are ADDED into these fp32 [B*Hkv][Skv][D] tensors (no bf16 store)
+    // non-null: dK / dV leave as fp32 feature-major matrices (see MatrixOut)
+    float *dk_mat, *dv_mat;
+    long long mat_stride;
     float scale, scale_log2;
 };
 
@@ -109,12 +113,6 @@ struct BwdBarriers {
     uint32_t tmem_base;
     uint32_t abort_flag;
 };
-
-// Whether the per-query terms (LSE, delta) are folded into the S^T and dP^T products as one extra contraction step (see
-// kAugBytes in the kernel).  That trades shared-memory loads and arithmetic in the compute warps for 2 x 65 tensor-pipe
-// cycles per step on the two chains of products: a clear gain at head_dim 64, where the compute warps set the pace
-// (-11 % kernel time), a loss at 128, where the chains do (+3 %).
-__host__ __device__ constexpr bool bwd_folds_row_terms(int D) { return D == 64; }
 
 // Shared-memory descriptor of an unswizzled K-major operand of ONE contraction step (16 bf16 = two 8-element column
 // blocks): a column block is rows of 16 bytes, eight rows forming one 128-byte core matrix (SBO = 128 to the next eight
@@ -189,7 +187,7 @@ __device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile
 // Epilogue of a compute warpgroup: its accumulator (dV for warpgroup 0, dK for warpgroup 1; `src` = TMEM address of this
 // thread's row) leaves as an fp32 partial (cut tiles), is added into the caller's fp32 accumulators, or is stored as bf16
 // through `stage_base` (a shared-memory tile no product reads any more).
-template <int D>
+template <int D, bool kMat>
 __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool split, int n_iter, int wg, int warp, int lane, int row,
                                           uint32_t src, int kt, int slab, int slabs, int group, int g0, int k0, uint8_t* stage_base)
 {
@@ -211,7 +209,7 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
             for (int v = 0; v < 8; ++v)
                 *reinterpret_cast<uint4*>(dst + c * 32 + v * 4) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
         }
-    } else if (ok && p.dk_acc != nullptr) {
+    } else if (!kMat && ok && p.dk_acc != nullptr) {
         // accumulate form: this CTA is the only writer of its 128 key rows in this launch
         tc_fence_after();
         const int key = k0 + row;
@@ -233,6 +231,23 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
                     a.w = fmaf(__uint_as_float(r[4 * v + 3]), mul, a.w);
                     *reinterpret_cast<float4*>(dst + c * 32 + v * 4) = a;
                 }
+            }
+        }
+    } else if (kMat && ok) {
+        // feature-major matrices: the 32 keys of a warp are 128 contiguous bytes of every feature's row
+        tc_fence_after();
+        const int key = k0 + row;
+        const float mul = wg == 0 ? 1.0f : p.scale;
+        const int b = slab / p.Hkv, hk = slab - b * p.Hkv;
+        float* dst = (wg == 0 ? p.dv_mat : p.dk_mat) + (long long)hk * D * p.mat_stride + (long long)b * p.Skv + key;
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld32(src + (uint32_t)(c * 32), r);
+            tmem_ld_wait();
+            if (key < p.Skv) {
+#pragma unroll
+                for (int v = 0; v < 32; ++v) dst[(c * 32 + v) * p.mat_stride] = __uint_as_float(r[v]) * mul;
             }
         }
     } else if (ok) {
@@ -278,7 +293,11 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
     } else if (n_iter == 0 && p.dk_acc == nullptr) {
         // a key tile no query can see (cannot happen for causal with Sq == Skv; kept for safety): zero grads
         const int key = k0 + row;
-        if (key < p.Skv) {
+        if (key < p.Skv && kMat) {
+            const int b = slab / p.Hkv, hk = slab - b * p.Hkv;
+            float* dst = (wg == 0 ? p.dv_mat : p.dk_mat) + (long long)hk * D * p.mat_stride + (long long)b * p.Skv + key;
+            for (int d = 0; d < D; ++d) dst[d * p.mat_stride] = 0.0f;
+        } else if (key < p.Skv) {
             __nv_bfloat16* dst = (wg == 0 ? p.dv : p.dk) + ((size_t)slab * p.Skv + key) * D;
             for (int d = 0; d < D; d += 8) *reinterpret_cast<uint4*>(dst + d) = make_uint4(0, 0, 0, 0);
         }
@@ -288,7 +307,9 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
 // kSplit: the grid may hold key tiles cut by query head (a separate instantiation, so that the plain kernel carries none
 // of that bookkeeping)
 // kDet: dQ contributions leave as 64-bit fixed point (see the drain warpgroup)
-template <int D, bool kWin, bool kSplit, bool kDet>
+// kMat: dK and dV leave as feature-major fp32 matrices (an instantiation of its own: with that store in the common kernel it is
+// 3 % slower at head_dim 128; the accumulate form, in contrast, is better left in: without it the kernel is 3 % slower too)
+template <int D, bool kWin, bool kSplit, bool kDet, bool kMat>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do, const BwdParams p)
@@ -347,6 +368,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if ((smem_u32(smem_raw) & 1023u) != 0u) {      // uniform over the CTA: nothing has been set up yet
         if (threadIdx.x == 0) atomicCAS(&g_device_status, 0u, (0x3fu << 24) | (blockIdx.x & 0xffffffu));
+        wait_for_stream();
         return;
     }
 
@@ -414,6 +436,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
+    wait_for_stream();      // nothing before this reads or writes global memory
     // S^T / P^T [0,128)   dP^T / dQ [128,256)   head_dim 128: dV [256,384) dK [384,512)   64: dV [256,320) dK [320,384) 2nd S^T [384,512)
     const uint32_t tm_S = tmem, tm_dP = tmem + 128u, tm_dV = tmem + 256u, tm_dK = tmem + (D == 128 ? 384u : 320u);
     constexpr uint32_t kSBufStride = 384u;         // columns from the first S^T buffer to the second
@@ -796,7 +819,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         // ---- epilogue: dV (warpgroup 0) and dK (warpgroup 1) ----
         ok = __all_sync(0xffffffffu, ok && n_iter > 0 && mbar_wait(&bars->final_bar, 0, abort_flag, kSiteFinal));
-        write_dkv<D>(p, ok, split, n_iter, wg, warp, lane, row, (wg == 0 ? tm_dV : tm_dK) + lane_off, kt, slab, slabs, group, g0, k0,
+        write_dkv<D, kMat>(p, ok, split, n_iter, wg, warp, lane, row, (wg == 0 ? tm_dV : tm_dK) + lane_off, kt, slab, slabs, group, g0, k0,
                      wg == 0 ? sV : sK);
     }
 
@@ -812,104 +835,83 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
 }
 
-// Per padded query row: the two 16-byte records the main kernel feeds to its extra contraction step -- bf16 (hi, mid, lo, 0 x 5)
-// with hi + mid + lo = -rowsum(dO o O) (delta) and = -LSE / scale (a large negative number for padded rows and for rows without
-// visible keys, so that they produce P = 0) -- and the dQ accumulator zeroed.  D/4 lanes per (b, h, padded row), 8 bytes of O
-// and of dO per lane: a warp covers one row at head_dim 128 and two at 64, every lane busy either way.
+template <int D> constexpr int kPreRows = D == 64 ? 128 : 64;   // query rows per block of bwd_pre_kernel
+
+// Per padded query row: the terms the main kernel wants (store_row_terms) from delta = rowsum(dO o O) and LSE, and the dQ
+// accumulator zeroed.  Bound by HBM: D/8 lanes per row with 16 bytes of O and of dO each and four rows per lane group in flight,
+// 8 warps x 8 (16 at head_dim 64) rows per block, whose part of the accumulator is contiguous.
 template <int D>
-__global__ void bwd_pre_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                               const float* __restrict__ lse, void* __restrict__ lse_out, void* __restrict__ delta_out,
-                               float* __restrict__ dq_accum, int Sq, int Sq_pad, long long rows_padded, int acc_words_per_row,
-                               float inv_scale)
+__global__ void __launch_bounds__(256) bwd_pre_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
+                                                      const float* __restrict__ lse, const RowTerms terms, float* __restrict__ dq_accum, int Sq,
+                                                      int Sq_pad, int acc_words_per_row)
 {
-    constexpr int kLanesPerRow = D / 4, kRowsPerWarp = 32 / kLanesPerRow;
-    const int lane = threadIdx.x & 31, sub = lane / kLanesPerRow, l = lane % kLanesPerRow;
-    const long long r = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * kRowsPerWarp + sub;
-    const bool live = r < rows_padded;
-    const long long bh = live ? r / Sq_pad : 0;
-    const int s = live ? (int)(r - bh * Sq_pad) : 0;
-    if (live) {
-        // the accumulator is tile-permuted but covers exactly acc_words_per_row 32-bit words per padded row (D, or 2*D
-        // when it is 64-bit fixed point): zero it linearly
-        float4* z = reinterpret_cast<float4*>(dq_accum + r * acc_words_per_row);
-        for (int i = l; i < acc_words_per_row / 4; i += kLanesPerRow) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    float acc = 0.0f;
-    if (live && s < Sq) {
-        const size_t off = ((size_t)bh * Sq + s) * D + l * 4;
-        const uint2 a = __ldg(reinterpret_cast<const uint2*>(o + off));
-        const uint2 g = __ldg(reinterpret_cast<const uint2*>(dout + off));
-        acc = fmaf(__uint_as_float(a.x << 16), __uint_as_float(g.x << 16), acc);
-        acc = fmaf(__uint_as_float(a.x & 0xffff0000u), __uint_as_float(g.x & 0xffff0000u), acc);
-        acc = fmaf(__uint_as_float(a.y << 16), __uint_as_float(g.y << 16), acc);
-        acc = fmaf(__uint_as_float(a.y & 0xffff0000u), __uint_as_float(g.y & 0xffff0000u), acc);
-    }
+    wait_for_stream();
+    constexpr int kLanes = D / 8, kGroups = 32 / kLanes, kPer = 4, kRows = 8 * kGroups * kPer;   // rows per block
+    static_assert(kRows == kPreRows<D>, "grid");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % kLanes;
+    const long long r0 = (long long)blockIdx.x * kRows;
+    uint4 x[kPer], y[kPer];
+    int s[kPer];
+    long long bh[kPer];
 #pragma unroll
-    for (int m = kLanesPerRow / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    if (live && l == 0) {
-        if constexpr (bwd_folds_row_terms(D)) {
-            uint4* qaug = static_cast<uint4*>(lse_out);
-            uint4* doaug = static_cast<uint4*>(delta_out);
-            // value -> three bf16 (hi, mid, lo) whose sum is the fp32 value exactly (3 x 8 significant bits), as the first
-            // three slots of a record
-            auto split = [](float x) {
-                const __nv_bfloat16 hi = __float2bfloat16_rn(x);
-                const float r1 = x - __bfloat162float(hi);
-                const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
-                const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-                return make_uint4((uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(mid) << 16),
-                                  (uint32_t)__bfloat16_as_ushort(lo), 0u, 0u);
-            };
-            constexpr float kMasked = -1.0e30f;   // times scale*log2(e) still far below the exponent range: P = 0, and finite
-            if (s >= Sq) { qaug[r] = split(kMasked); doaug[r] = make_uint4(0u, 0u, 0u, 0u); }
-            else {
-                const float lv = lse[(size_t)bh * Sq + s];
-                qaug[r] = split((lv == -INFINITY) ? kMasked : -lv * inv_scale);
-                doaug[r] = split(-acc);
-            }
-        } else {
-            float* lse2 = static_cast<float*>(lse_out);
-            float* delta = static_cast<float*>(delta_out);
-            if (s >= Sq) { lse2[r] = -INFINITY; delta[r] = 0.0f; }
-            else {
-                const float lv = lse[(size_t)bh * Sq + s];
-                lse2[r] = (lv == -INFINITY) ? -INFINITY : -lv * 1.4426950408889634f;
-                delta[r] = -acc;
-            }
+    for (int i = 0; i < kPer; ++i) {
+        const long long r = r0 + (i * 8 + warp) * kGroups + lane / kLanes;
+        bh[i] = r / Sq_pad;
+        s[i] = (int)(r - bh[i] * Sq_pad);
+        const bool live = s[i] < Sq;
+        const size_t off = ((size_t)bh[i] * Sq + s[i]) * D + l * 8;
+        x[i] = live ? __ldg(reinterpret_cast<const uint4*>(o + off)) : make_uint4(0, 0, 0, 0);
+        y[i] = live ? __ldg(reinterpret_cast<const uint4*>(dout + off)) : make_uint4(0, 0, 0, 0);
+    }
+    const int words = kRows * acc_words_per_row;       // (rows_padded is a multiple of 128: every block has all its rows)
+    float4* z = reinterpret_cast<float4*>(dq_accum + r0 * acc_words_per_row);
+    for (int i = threadIdx.x; i < words / 4; i += 256) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const uint32_t xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+        float acc = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            acc = fmaf(__uint_as_float(xs[k] << 16), __uint_as_float(ys[k] << 16), acc);
+            acc = fmaf(__uint_as_float(xs[k] & 0xffff0000u), __uint_as_float(ys[k] & 0xffff0000u), acc);
         }
+#pragma unroll
+        for (int m = kLanes / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+        const long long r = r0 + (i * 8 + warp) * kGroups + lane / kLanes;
+        if (l == 0) store_row_terms<D>(terms, r, s[i] < Sq, s[i] < Sq ? lse[(size_t)bh[i] * Sq + s[i]] : 0.0f, acc);
     }
 }
 
-// dQ (bf16, [B][Hq][Sq][D]) = scale * accumulator, undoing the per-tile [d/4][row][4] order.
-// One CTA per (tile, 32-row group): for a fixed d/4 chunk its 32 rows are 512 contiguous bytes of the accumulator.
+// dQ (bf16, [B][Hq][Sq][D]) = scale * accumulator, undoing the per-tile [d/4][row][4] order; one block per tile.  A thread
+// takes 16 features of a row at a time: four loads that are contiguous over the rows of a warp, one whole 32-byte sector out,
+// and all its loads (16 at head_dim 128) in flight before the first store.
 template <int D>
-__global__ void __launch_bounds__(256) bwd_post_kernel(const float* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq, int Sq,
+__global__ void __launch_bounds__(256, 2) bwd_post_kernel(const float* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq, int Sq,
                                                        int n_qt, float scale)
 {
-    constexpr int kRows = 32;
-    __shared__ float tile[kRows][D + 4];
-    const size_t t = blockIdx.x >> 2;
-    const int r0 = (int)(blockIdx.x & 3) * kRows;
-    const size_t bh = t / n_qt;
-    const int qt = (int)(t - bh * n_qt);
-    const float4* src = reinterpret_cast<const float4*>(dq_accum + t * (size_t)(kT * D));
-    for (int e = threadIdx.x; e < kRows * D / 4; e += blockDim.x) {
-        const int chunk = e / kRows, row = e - chunk * kRows;   // consecutive threads -> consecutive 16-byte units
-        const float4 v = src[(size_t)chunk * kT + r0 + row];
-        *reinterpret_cast<float4*>(&tile[row][chunk * 4]) = v;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < kRows * D / 8; e += blockDim.x) {
-        const int row = e / (D / 8), d8 = (e - row * (D / 8)) * 8;
-        const int s = qt * kT + r0 + row;
-        if (s >= Sq) continue;
-        const float* x = &tile[row][d8];
-        uint4 w;
-        w.x = pack_bf16(x[0] * scale, x[1] * scale);
-        w.y = pack_bf16(x[2] * scale, x[3] * scale);
-        w.z = pack_bf16(x[4] * scale, x[5] * scale);
-        w.w = pack_bf16(x[6] * scale, x[7] * scale);
-        *reinterpret_cast<uint4*>(dq + (bh * Sq + s) * D + d8) = w;
+    wait_for_stream();
+    const size_t t = blockIdx.x, bh = t / n_qt;
+    const int qt = (int)(t - bh * n_qt), row = threadIdx.x & 127, half = threadIdx.x >> 7, s = qt * kT + row;
+    if (s >= Sq) return;
+    const float4* src = reinterpret_cast<const float4*>(dq_accum + t * (size_t)(kT * D)) + row;
+    constexpr int kPer = D / 32;
+    float4 x[kPer][4];
+#pragma unroll
+    for (int g = 0; g < kPer; ++g)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[g][i] = src[(size_t)((2 * g + half) * 4 + i) * kT];
+    __nv_bfloat16* dst = dq + (bh * Sq + s) * D;
+#pragma unroll
+    for (int g = 0; g < kPer; ++g) {
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[2 * i] = pack_bf16(x[g][i].x * scale, x[g][i].y * scale);
+            w[2 * i + 1] = pack_bf16(x[g][i].z * scale, x[g][i].w * scale);
+        }
+        uint4* out = reinterpret_cast<uint4*>(dst + (2 * g + half) * 16);
+        out[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        out[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
 
@@ -919,31 +921,24 @@ template <int D>
 __global__ void __launch_bounds__(256) bwd_post_det_kernel(const unsigned long long* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq,
                                                            int Sq, int n_qt, float scale)
 {
-    constexpr int kRows = 32;
-    __shared__ float tile[kRows][D + 4];
-    const size_t t = blockIdx.x >> 2;
-    const int r0 = (int)(blockIdx.x & 3) * kRows;
-    const size_t bh = t / n_qt;
-    const int qt = (int)(t - bh * n_qt);
-    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(dq_accum + t * (size_t)(kT * D));
-    for (int e = threadIdx.x; e < kRows * D / 2; e += blockDim.x) {
-        const int chunk = e / kRows, row = e - chunk * kRows;   // consecutive threads -> consecutive 16-byte units
-        const ulonglong2 v = src[(size_t)chunk * kT + r0 + row];
-        tile[row][chunk * 2] = (float)((double)(long long)v.x * (1.0 / 4294967296.0));
-        tile[row][chunk * 2 + 1] = (float)((double)(long long)v.y * (1.0 / 4294967296.0));
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < kRows * D / 8; e += blockDim.x) {
-        const int row = e / (D / 8), d8 = (e - row * (D / 8)) * 8;
-        const int s = qt * kT + r0 + row;
-        if (s >= Sq) continue;
-        const float* x = &tile[row][d8];
-        uint4 w;
-        w.x = pack_bf16(x[0] * scale, x[1] * scale);
-        w.y = pack_bf16(x[2] * scale, x[3] * scale);
-        w.z = pack_bf16(x[4] * scale, x[5] * scale);
-        w.w = pack_bf16(x[6] * scale, x[7] * scale);
-        *reinterpret_cast<uint4*>(dq + (bh * Sq + s) * D + d8) = w;
+    wait_for_stream();
+    const size_t t = blockIdx.x, bh = t / n_qt;
+    const int qt = (int)(t - bh * n_qt), row = threadIdx.x & 127, half = threadIdx.x >> 7, s = qt * kT + row;
+    if (s >= Sq) return;
+    const longlong2* src = reinterpret_cast<const longlong2*>(dq_accum + t * (size_t)(kT * D)) + row;
+    __nv_bfloat16* dst = dq + (bh * Sq + s) * D;
+#pragma unroll 2
+    for (int g = half; g < D / 16; g += 2) {
+        longlong2 x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = src[(size_t)(g * 8 + i) * kT];
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            w[i] = pack_bf16((float)((double)x[i].x * (1.0 / 4294967296.0)) * scale, (float)((double)x[i].y * (1.0 / 4294967296.0)) * scale);
+        uint4* out = reinterpret_cast<uint4*>(dst + g * 16);
+        out[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        out[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
 
@@ -956,6 +951,7 @@ __global__ void __launch_bounds__(256) bwd_dkv_reduce_kernel(const float* __rest
                                                              __nv_bfloat16* __restrict__ dv, int slabs, int group, int Skv,
                                                              float scale, long long n_units)
 {
+    wait_for_stream();
     const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= n_units) return;
     constexpr int kPerRow = D / 8;
@@ -984,7 +980,70 @@ __global__ void __launch_bounds__(256) bwd_dkv_reduce_kernel(const float* __rest
     *reinterpret_cast<uint4*>((which ? dk : dv) + ((size_t)slab * Skv + key) * D + d8) = w;
 }
 
-template <int D, bool kWin, bool kSplit, bool kDet>
+// The same sums into fp32 feature-major matrices: consecutive threads take consecutive keys.
+template <int D>
+__global__ void __launch_bounds__(256) bwd_dkv_reduce_matrix_kernel(const float* __restrict__ part, float* __restrict__ dk, float* __restrict__ dv,
+                                                                    long long stride, int Hkv, int slabs, int group, int Skv, float scale,
+                                                                    long long n_units)
+{
+    wait_for_stream();
+    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= n_units) return;
+    constexpr int kPerRow = D / 8;
+    const int row = (int)(u % kT);
+    long long r = u / kT;
+    const int d8 = (int)(r % kPerRow) * 8; r /= kPerRow;
+    const int which = (int)(r & 1); r >>= 1;              // 0: dV, 1: dK
+    const int slab = (int)(r % slabs), kt = (int)(r / slabs), key = kt * kT + row;
+    if (key >= Skv) return;
+    const float* src = part + (((size_t)kt * slabs + slab) * group * 2 + which) * (size_t)(kT * D) + (size_t)row * D + d8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int g = 0; g < group; ++g)
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(src + (size_t)g * 2 * kT * D + i);
+            acc[i] += x.x; acc[i + 1] += x.y; acc[i + 2] += x.z; acc[i + 3] += x.w;
+        }
+    const int b = slab / Hkv, hk = slab - b * Hkv;
+    float* dst = (which ? dk : dv) + (long long)(hk * D + d8) * stride + (long long)b * Skv + key;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dst[i * stride] = acc[i] * (which ? scale : 1.0f);
+}
+
+// dQ as an fp32 feature-major matrix = scale * accumulator: four features of one query per thread, consecutive threads on
+// consecutive queries, in either form of the accumulator (fp32 [d/4][row][4] or 2^-32 fixed point [d/2][row][2]).
+template <int D, bool kDet>
+__global__ void __launch_bounds__(256) bwd_post_matrix_kernel(const float* __restrict__ dq_accum, float* __restrict__ dq, long long stride, int Hq,
+                                                              int Sq, int n_qt, float scale)
+{
+    wait_for_stream();
+    const size_t t = blockIdx.x;                          // tile: (b, h, query tile)
+    const int bh = (int)(t / n_qt), qt = (int)(t - (size_t)bh * n_qt), b = bh / Hq, h = bh - b * Hq;
+    const int row = threadIdx.x & 127, s = qt * kT + row;
+    if (s >= Sq) return;
+    const float* src = dq_accum + t * (size_t)(kT * D) * (kDet ? 2 : 1);
+    float* dst = dq + (long long)h * D * stride + (long long)b * Sq + s;
+#pragma unroll 4
+    for (int c = threadIdx.x >> 7; c < D / 4; c += 2) {
+        float x[4];
+        if constexpr (!kDet) {
+            const float4 v = *reinterpret_cast<const float4*>(src + ((size_t)c * kT + row) * 4);
+            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+        } else {
+            const longlong2* w = reinterpret_cast<const longlong2*>(src);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const longlong2 v = w[(size_t)(2 * c + i) * kT + row];
+                x[2 * i] = (float)((double)v.x * (1.0 / 4294967296.0));
+                x[2 * i + 1] = (float)((double)v.y * (1.0 / 4294967296.0));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[(4 * c + i) * stride] = x[i] * scale;
+    }
+}
+
+template <int D, bool kWin, bool kSplit, bool kDet, bool kMat>
 cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
 {
     const AttnShape& s = a.s;
@@ -993,20 +1052,15 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     const long long rows_padded = (long long)s.B * s.Hq * Sq_pad;
     // workspace: [delta records | LSE records] then the accumulator (see tc_backward_workspace_bytes)
     constexpr bool kAug = bwd_folds_row_terms(D);
-    uint4* doaug = reinterpret_cast<uint4*>(a.delta);
-    uint4* qaug = doaug + rows_padded;
-    float* lse2 = a.delta + rows_padded;           // the plain-column form takes the head of the same region
+    const RowTerms terms = row_terms_of(a.delta, rows_padded, D, s.scale);
     cudaError_t e;
     const int phases = a.phases ? a.phases : (kBwdPre | kBwdMain | kBwdPost);
     if (phases & kBwdPre) {
-        const int warps = 8;
-        const long long rows_per_block = (long long)warps * (32 / (D / 4));
-        const long long blocks = (rows_padded + rows_per_block - 1) / rows_per_block;
-        bwd_pre_kernel<D><<<(unsigned)blocks, warps * 32, 0, st>>>(a.o, a.dout, a.lse, kAug ? (void*)qaug : (void*)lse2,
-                                                                    kAug ? (void*)doaug : (void*)a.delta, a.dq_accum, s.Sq, Sq_pad,
-                                                                    rows_padded, kDet ? 2 * D : D, 1.0f / s.scale);
-        count_launch();
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const long long blocks = rows_padded / kPreRows<D>;
+        if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+        if ((e = launch_kernel(bwd_pre_kernel<D>, (unsigned)blocks, 256, 0, st, 1, a.o, a.dout, a.lse, terms, a.dq_accum, s.Sq, Sq_pad,
+                               kDet ? 2 * D : D)) != cudaSuccess)
+            return e;
     }
     if (phases & kBwdMain) {
     CUtensorMap tq, tk, tv, tdo;
@@ -1016,7 +1070,8 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     if ((e = encode_tmap_bf16_3d(&tv, a.v, D, s.Skv, s.B * s.Hkv, 128)) != cudaSuccess) return e;
     BwdParams p{};
     p.dk = a.dk; p.dv = a.dv;
-    p.qaug = qaug; p.doaug = doaug; p.lse2 = lse2; p.delta = a.delta; p.dq_accum = a.dq_accum;
+    p.qaug = (const uint4*)terms.lse; p.doaug = (const uint4*)terms.delta; p.lse2 = (const float*)terms.lse;
+    p.delta = (const float*)terms.delta; p.dq_accum = a.dq_accum;
     p.B = s.B; p.Hq = s.Hq; p.Hkv = s.Hkv; p.Sq = s.Sq; p.Skv = s.Skv; p.Sq_pad = Sq_pad;
     p.causal = s.causal;
     p.window = s.causal ? s.window : 0;
@@ -1025,6 +1080,7 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     p.split_tiles = kSplit ? bwd_split_tiles(s) : 0;
     p.dkv_part = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dq_accum) + align256((kDet ? 8 : 4) * (size_t)rows_padded * D));
     p.dk_acc = a.dk_acc; p.dv_acc = a.dv_acc;
+    p.dk_mat = a.mat.dk; p.dv_mat = a.mat.dv; p.mat_stride = a.mat.stride;
     p.scale = s.scale;
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const int group = s.Hq / s.Hkv, slabs = s.B * s.Hkv;
@@ -1037,27 +1093,31 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
         constexpr int kQStages = (D == 128) ? 2 : 3;
         const size_t smem = (size_t)(128 * D * 2) * (2 + kQStages + kDoStages) + (D == 128 ? 1 : 2) * 128 * 128 * 2 + 32 * 1024 +
                             (kAug ? (size_t)(2 + kQStages + kDoStages) * 128 * 16 : (size_t)2 * kQStages * 128 * 4) + sizeof(BwdBarriers);
-        if ((e = ensure_dynamic_smem(attn_bwd_tc_kernel<D, kWin, kSplit, kDet>, smem, configured)) != cudaSuccess) return e;
-        attn_bwd_tc_kernel<D, kWin, kSplit, kDet><<<(unsigned)ctas, kBwdThreads, smem, st>>>(tq, tk, tv, tdo, p);
+        if ((e = ensure_dynamic_smem(attn_bwd_tc_kernel<D, kWin, kSplit, kDet, kMat>, smem, configured)) != cudaSuccess) return e;
+        if ((e = launch_kernel(attn_bwd_tc_kernel<D, kWin, kSplit, kDet, kMat>, (unsigned)ctas, kBwdThreads, smem, st, 1, tq, tk, tv, tdo, p)) !=
+            cudaSuccess)
+            return e;
     }
-    count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (p.split_tiles > 0) {
         const long long n_units = (long long)p.split_tiles * slabs * 2 * kT * (D / 8);
-        bwd_dkv_reduce_kernel<D><<<(unsigned)((n_units + 255) / 256), 256, 0, st>>>(p.dkv_part, a.dk, a.dv, slabs, group, s.Skv,
-                                                                                   s.scale, n_units);
-        count_launch();
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const unsigned blocks = (unsigned)((n_units + 255) / 256);
+        if constexpr (kMat)
+            e = launch_kernel(bwd_dkv_reduce_matrix_kernel<D>, blocks, 256, 0, st, 1, p.dkv_part, a.mat.dk, a.mat.dv, a.mat.stride, s.Hkv, slabs,
+                              group, s.Skv, s.scale, n_units);
+        else
+            e = launch_kernel(bwd_dkv_reduce_kernel<D>, blocks, 256, 0, st, 1, p.dkv_part, a.dk, a.dv, slabs, group, s.Skv, s.scale, n_units);
+        if (e != cudaSuccess) return e;
     }
     }   // kBwdMain
     if (!(phases & kBwdPost)) return cudaSuccess;
-    if (kDet)
-        bwd_post_det_kernel<D><<<(unsigned)((long long)s.B * s.Hq * n_qt * 4), 256, 0, st>>>(
-            reinterpret_cast<const unsigned long long*>(a.dq_accum), a.dq, s.Sq, n_qt, s.scale);
+    const unsigned tiles = (unsigned)((long long)s.B * s.Hq * n_qt);
+    if constexpr (kMat)
+        return launch_kernel(bwd_post_matrix_kernel<D, kDet>, tiles, 256, 0, st, 1, a.dq_accum, a.mat.dq, a.mat.stride, s.Hq, s.Sq, n_qt, s.scale);
+    else if constexpr (kDet)
+        return launch_kernel(bwd_post_det_kernel<D>, tiles, 256, 0, st, 1, reinterpret_cast<const unsigned long long*>(a.dq_accum), a.dq, s.Sq,
+                             n_qt, s.scale);
     else
-        bwd_post_kernel<D><<<(unsigned)((long long)s.B * s.Hq * n_qt * 4), 256, 0, st>>>(a.dq_accum, a.dq, s.Sq, n_qt, s.scale);
-    count_launch();
-    return cudaGetLastError();
+        return launch_kernel(bwd_post_kernel<D>, tiles, 256, 0, st, 1, a.dq_accum, a.dq, s.Sq, n_qt, s.scale);
 }
 
 }  // namespace
@@ -1077,20 +1137,30 @@ size_t tc_backward_workspace_bytes(const AttnShape& s)
     return align256(kBwdRowAuxBytes * rows) + align256((s.deterministic ? 8 : 4) * rows * (size_t)s.D) + align256(part);
 }
 
-cudaError_t tc_backward(const TcArgs& a, cudaStream_t st)
+namespace {
+template <int D, bool kMat>
+cudaError_t dispatch_bwd(const TcArgs& a, cudaStream_t st)
 {
     const bool win = a.s.causal && a.s.window > 0;
-    if (a.s.deterministic) {   // (bwd_split_tiles is 0 for this form)
-        if (a.s.D == 64) return win ? launch_bwd<64, true, false, true>(a, st) : launch_bwd<64, false, false, true>(a, st);
-        return win ? launch_bwd<128, true, false, true>(a, st) : launch_bwd<128, false, false, true>(a, st);
-    }
-    // the accumulate form has no cut key tiles: their fp32 partials would need a second adding pass
-    if (a.dk_acc == nullptr && bwd_split_tiles(a.s) > 0) {
-        if (a.s.D == 64) return win ? launch_bwd<64, true, true, false>(a, st) : launch_bwd<64, false, true, false>(a, st);
-        return win ? launch_bwd<128, true, true, false>(a, st) : launch_bwd<128, false, true, false>(a, st);
-    }
-    if (a.s.D == 64) return win ? launch_bwd<64, true, false, false>(a, st) : launch_bwd<64, false, false, false>(a, st);
-    return win ? launch_bwd<128, true, false, false>(a, st) : launch_bwd<128, false, false, false>(a, st);
+    if (a.s.deterministic)   // (bwd_split_tiles is 0 for this form)
+        return win ? launch_bwd<D, true, false, true, kMat>(a, st) : launch_bwd<D, false, false, true, kMat>(a, st);
+    if (bwd_split_tiles(a.s) > 0)
+        return win ? launch_bwd<D, true, true, false, kMat>(a, st) : launch_bwd<D, false, true, false, kMat>(a, st);
+    return win ? launch_bwd<D, true, false, false, kMat>(a, st) : launch_bwd<D, false, false, false, kMat>(a, st);
+}
+template <int D>
+cudaError_t dispatch_bwd_out(const TcArgs& a, cudaStream_t st)
+{
+    // the accumulate form (backward in pieces) has no window, no fixed-point dQ and no cut key tiles: their fp32 partials
+    // would need a second adding pass
+    if (a.dk_acc) return launch_bwd<D, false, false, false, false>(a, st);
+    return a.mat.dk ? dispatch_bwd<D, true>(a, st) : dispatch_bwd<D, false>(a, st);
+}
+}  // namespace
+
+cudaError_t tc_backward(const TcArgs& a, cudaStream_t st)
+{
+    return a.s.D == 64 ? dispatch_bwd_out<64>(a, st) : dispatch_bwd_out<128>(a, st);
 }
 
 #ifdef SNTL_TRACE

@@ -59,6 +59,9 @@ struct FwdParams {
     int new_tokens, n_splits, tiles_per_split;
     int n_qblk;       // 256-row query blocks per (b, h)
     float scale_log2; // scale * log2(e)
+    // non-null: O and LSE leave as fp32 feature-major matrices (see MatrixOut; not in KV-cache mode)
+    float *o_mat, *lse_mat;
+    long long mat_stride;
 };
 
 struct FwdBarriers {
@@ -77,7 +80,8 @@ struct FwdBarriers {
 // the rows of one tile, keys split over CTAs.
 enum FwdMode : int { kPlain = 0, kWindow = 1, kCache = 2 };
 
-template <int D, int kMode>
+// kMat: O and LSE leave as fp32 feature-major matrices
+template <int D, int kMode, bool kMat>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const FwdParams p)
@@ -174,6 +178,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
+    wait_for_stream();      // nothing before this reads or writes global memory
     // head_dim 64 (plain / window kernels) leaves room for P in columns of its own: S_t [192t, 192t+128), P_t the next 64,
     // O_t [384+64t, +64).  The next S of a tile is then issued as soon as the softmax warps have READ the current one
     // instead of behind the P V product that consumes P, which takes a tile's two products out of the chain between two of
@@ -509,6 +514,23 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             // (Cache mode: the two streams share ONE query tile, which the other stream may still be reading, but each owns
             // K stage t, and that stage gets no further load once the stream's last tile is done.)
             constexpr int kUnits = D / 8;                       // 16-byte units per row
+            if constexpr (kMat) {
+                // feature-major matrices: the 32 rows of a warp are 128 contiguous bytes of every feature's row
+                const int b = bh / p.Hq, h = bh - b * p.Hq;
+                float* dst = p.o_mat + (long long)h * D * p.mat_stride + (long long)b * p.Sq + grow;
+#pragma unroll
+                for (int c = 0; c < D / 32; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(tmem_O(t) + lane_off + (uint32_t)(c * 32), o);
+                    tmem_ld_wait();
+                    if (store) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) dst[(c * 32 + i) * p.mat_stride] = __uint_as_float(o[i]) * inv;
+                    }
+                }
+                if (store)
+                    p.lse_mat[(long long)h * p.mat_stride + (long long)b * p.Sq + grow] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
+            } else {
             uint8_t* stage = (kMode == kCache ? sK : sQ) + t * kTileBytes + (warp & 3) * 32 * (D * 2);
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
@@ -542,6 +564,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             if (store)
                 p.lse[out_row] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
+            }
         } else if (kMode == kCache && ok && n_mine == 0 && grow < p.Sq) {
             // a stream that got no key tile (a piece of one tile): its partial result weighs nothing in the merge
             p.lse[((size_t)(2 * split + t) * bh_count + bh) * p.Sq + grow] = -INFINITY;
@@ -579,7 +602,7 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-template <int D, int kMode>
+template <int D, int kMode, bool kMat>
 cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
 {
     const AttnShape& s = a.s;
@@ -591,6 +614,7 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     FwdParams p{};
     p.o = a.o_out;
     p.lse = a.lse_out;
+    p.o_mat = a.mat.o; p.lse_mat = a.mat.lse; p.mat_stride = a.mat.stride;
     p.B = s.B; p.Hq = s.Hq; p.Hkv = s.Hkv; p.Sq = s.Sq; p.Skv = s.Skv;
     p.causal = s.causal;
     p.window = s.causal ? s.window : 0;
@@ -601,10 +625,8 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const size_t smem = 6 * (size_t)(128 * D * 2) + sizeof(FwdBarriers) + 1024;
     static std::atomic<unsigned long long> configured{0};   // per instantiation, one bit per device
-    if ((e = ensure_dynamic_smem(attn_fwd_tc_kernel<D, kMode>, smem, configured)) != cudaSuccess) return e;
-    attn_fwd_tc_kernel<D, kMode><<<(unsigned)ctas, kFwdThreads, smem, st>>>(tq, tk, tv, p);
-    count_launch();
-    return cudaGetLastError();
+    if ((e = ensure_dynamic_smem(attn_fwd_tc_kernel<D, kMode, kMat>, smem, configured)) != cudaSuccess) return e;
+    return launch_kernel(attn_fwd_tc_kernel<D, kMode, kMat>, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p);
 }
 
 // ---- KV-cache mode ----------------------------------------------------------------------------------------------
@@ -615,6 +637,7 @@ __global__ void __launch_bounds__(256) cache_merge_kernel(const __nv_bfloat16* _
                                                           int n_splits, long long rows, __nv_bfloat16* __restrict__ o,
                                                           float* __restrict__ lse)
 {
+    wait_for_stream();
     const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (r >= rows) return;
@@ -677,15 +700,11 @@ cudaError_t launch_cache(const TcArgs& a, int capacity, void* workspace, cudaStr
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const size_t smem = 6 * (size_t)(128 * D * 2) + sizeof(FwdBarriers) + 1024;
     static std::atomic<unsigned long long> configured{0};   // one bit per device
-    if ((e = ensure_dynamic_smem(attn_fwd_tc_kernel<D, kCache>, smem, configured)) != cudaSuccess) return e;
+    if ((e = ensure_dynamic_smem(attn_fwd_tc_kernel<D, kCache, false>, smem, configured)) != cudaSuccess) return e;
     const long long ctas = (long long)plan.n_splits * p.n_qblk * slabs;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    attn_fwd_tc_kernel<D, kCache><<<(unsigned)ctas, kFwdThreads, smem, st>>>(tq, tk, tv, p);
-    count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    cache_merge_kernel<D><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(o_part, lse_part, n_parts, rows, a.o_out, a.lse_out);
-    count_launch();
-    return cudaGetLastError();
+    if ((e = launch_kernel(attn_fwd_tc_kernel<D, kCache, false>, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p)) != cudaSuccess) return e;
+    return launch_kernel(cache_merge_kernel<D>, (unsigned)((rows + 7) / 8), 256, 0, st, 1, o_part, lse_part, n_parts, rows, a.o_out, a.lse_out);
 }
 
 }  // namespace
@@ -798,11 +817,19 @@ bool tc_fwd_supported(const AttnShape& s)
     return (s.D == 64 || s.D == 128) && (!s.causal || s.Sq == s.Skv);
 }
 
-cudaError_t tc_forward(const TcArgs& a, cudaStream_t st)
+namespace {
+template <int D>
+cudaError_t dispatch_fwd(const TcArgs& a, cudaStream_t st)
 {
     const bool win = a.s.causal && a.s.window > 0;
-    if (a.s.D == 64) return win ? launch_fwd<64, kWindow>(a, st) : launch_fwd<64, kPlain>(a, st);
-    return win ? launch_fwd<128, kWindow>(a, st) : launch_fwd<128, kPlain>(a, st);
+    if (a.mat.o) return win ? launch_fwd<D, kWindow, true>(a, st) : launch_fwd<D, kPlain, true>(a, st);
+    return win ? launch_fwd<D, kWindow, false>(a, st) : launch_fwd<D, kPlain, false>(a, st);
+}
+}  // namespace
+
+cudaError_t tc_forward(const TcArgs& a, cudaStream_t st)
+{
+    return a.s.D == 64 ? dispatch_fwd<64>(a, st) : dispatch_fwd<128>(a, st);
 }
 
 #ifdef SNTL_TRACE

@@ -153,6 +153,7 @@ template <typename T, int TM, int TN, int DP>
 __global__ void __launch_bounds__(kThreads) simt_bwd_kernel(const SimtArgs a, int n_dkv, int n_qt)
 {
     extern __shared__ __align__(16) float smem[];
+    wait_for_stream();
     if ((int)blockIdx.x < n_dkv) dkv_role<T, TM, TN, DP>(a, blockIdx.x, smem);
     else dq_role<T, TM, TN, DP>(a, blockIdx.x - n_dkv, n_qt, smem);
 }
@@ -168,9 +169,7 @@ cudaError_t launch(const SimtArgs& a, cudaStream_t st)
     const int n_qt = (a.s.Sq + L::kRows - 1) / L::kRows, n_kt = (a.s.Skv + L::kRows - 1) / L::kRows;
     const long long n_dkv = (long long)n_kt * a.s.B * a.s.Hkv, n_dq = (long long)n_qt * a.s.B * a.s.Hq;
     if (n_dkv + n_dq > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    kernel<<<(unsigned)(n_dkv + n_dq), kThreads, L::bytes, st>>>(a, (int)n_dkv, n_qt);
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(kernel, (unsigned)(n_dkv + n_dq), kThreads, L::bytes, st, 1, a, (int)n_dkv, n_qt);
 }
 
 // Tile height as in the forward: the largest whose grid still gives every SM its two resident CTAs.

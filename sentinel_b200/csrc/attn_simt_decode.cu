@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
     using L = DecodeSmem<DP, R>;
     constexpr int kCols = DP / 32;                            // features per lane in the P V product
     extern __shared__ __align__(16) float smem[];
+    wait_for_stream();
     const AttnShape& s = a.s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slab = blockIdx.x / n_split, rank = blockIdx.x - slab * n_split;
@@ -211,20 +212,7 @@ cudaError_t launch(const SimtArgs& a, cudaStream_t st)
     const long long slabs = (long long)a.s.B * a.s.Hkv;
     int split = 1;
     while (split < 8 && slabs * split * 2 <= 3 * sm_count() && a.s.Skv >= split * kChunk) split *= 2;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(slabs * split));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = L::bytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)split;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if ((e = cudaLaunchKernelEx(&cfg, kernel, a, split)) != cudaSuccess) return e;
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(kernel, (unsigned)(slabs * split), kThreads, L::bytes, st, split, a, split);
 }
 
 template <int DP>

@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(kThreads, DP <= 64 ? 3 : 2) simt_fwd_kernel(co
     using L = FwdSmem<TM, TN, DP>;
     using M = OutMap<DP>;
     extern __shared__ __align__(16) float smem[];
+    wait_for_stream();
     const AttnShape& s = a.s;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int tile = kSplit ? blockIdx.x / n_split : blockIdx.x, rank = kSplit ? blockIdx.x - tile * n_split : 0;
@@ -161,22 +162,7 @@ cudaError_t launch(const SimtArgs& a, int n_qt, int n_split, cudaStream_t st)
     if (e != cudaSuccess) return e;
     const long long ctas = (long long)n_qt * a.s.B * a.s.Hq * n_split;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    if (kSplit) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)n_split;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    if ((e = cudaLaunchKernelEx(&cfg, kernel, a, n_qt, n_split)) != cudaSuccess) return e;
-    count_launch();
-    return cudaGetLastError();
+    return launch_kernel(kernel, (unsigned)ctas, kThreads, smem, st, kSplit ? n_split : 1, a, n_qt, n_split);
 }
 
 // Tile height: 64 rows keep the FMA pipes busiest, but a grid that does not give every SM a CTA or two loses more than the

@@ -6,10 +6,14 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 
 #include "sntl_attn.h"
 
 namespace sntl {
+
+// Launch accounting (attn_api.cu).
+void count_launch(int n = 1);
 
 // Element strides of a [B][H][S][D]-indexed tensor; covers both layouts of the C ABI.
 struct View4 {
@@ -53,6 +57,38 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, size_t bytes, std::atomic<
     return cudaSuccess;
 }
 
+// Programmatic dependent launch: a kernel's blocks may start as soon as all blocks of the one before it in the stream have
+// exited or are running out, before that one has been flushed, so that launch latency, barrier set-up and tensor-memory
+// allocation overlap its end (1-3 us a launch).  wait_for_stream() comes before the first access to global memory in every
+// block of every kernel launched this way: it returns when all earlier work of the stream has completed and its writes are
+// visible, so ordering is what it would be without.  (Triggering the next launch explicitly at the start of a kernel was slower
+// everywhere: 126 vs 121 us on the B8 H12 S1024 D64 training step, 242 vs 218 on a ragged head_dim-128 one.)
+__device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cluster, A&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cluster > 1) {
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = cluster;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    if (e == cudaSuccess) count_launch();
+    return e;
+}
+
 // SMs of the current device (148 on a B200), read once per device ordinal
 inline int sm_count()
 {
@@ -85,6 +121,13 @@ bool simt_decode_supported(const SimtArgs& a);
 cudaError_t simt_decode(const SimtArgs& a, cudaStream_t st);
 cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st);  // one launch
 
+// Results in the reference's feature-major layout: element (b, h, s, d) at ((h*D + d)*stride + b*S + s), LSE (b, h, s) at
+// (h*stride + b*S + s); the pointers include the first column of the window.
+struct MatrixOut {
+    float *o, *lse, *dq, *dk, *dv;
+    long long stride;
+};
+
 // Tensor-core kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu): bf16, BHSD contiguous, D in {64,128}.
 struct TcArgs {
     AttnShape s;
@@ -103,6 +146,7 @@ struct TcArgs {
     int phases = 0;
     float* dk_acc = nullptr;
     float* dv_acc = nullptr;
+    MatrixOut mat{};   // non-null members: results leave as fp32 feature-major matrices instead of bf16 [B][H][S][D]
 };
 enum : int { kBwdPre = 1, kBwdMain = 2, kBwdPost = 4 };
 bool tc_fwd_supported(const AttnShape& s);
@@ -133,18 +177,24 @@ cudaError_t sentinel_to_bhsd_bf16(const float* src, __nv_bfloat16* dst, int B, i
                                   int column_start, cudaStream_t st);
 cudaError_t bhsd_bf16_to_sentinel(const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
                                   int column_start, cudaStream_t st);
+// Everything a tensor-core call needs from feature-major fp32 matrices, in one launch: up to four of them converted to bf16
+// [B][H][S][D], and for the backward (o_mat non-null) the per-query terms from O, dO and LSE, and the dQ accumulator zeroed.
+struct MatrixStage {
+    const float* src[4];
+    __nv_bfloat16* dst[4];
+    int heads[4];
+    int n;
+    const float *o_mat, *do_mat, *lse_mat;
+    void* row_terms;          // start of the backward workspace
+    float* dq_accum;
+    size_t accum_bytes;
+};
+cudaError_t stage_matrices(const MatrixStage& m, int B, int Hq, int S, int D, int stride_columns, int column_start, float scale, cudaStream_t st);
 cudaError_t f32_to_bf16(const float* src, __nv_bfloat16* dst, size_t n, cudaStream_t st);
 cudaError_t bf16_to_f32(const __nv_bfloat16* src, float* dst, size_t n, cudaStream_t st);
-cudaError_t lse_bhs_to_sentinel(const float* src, float* dst, int B, int H, int S, int stride_columns, int column_start,
-                                cudaStream_t st);
-cudaError_t lse_sentinel_to_bhs(const float* src, float* dst, int B, int H, int S, int stride_columns, int column_start,
-                                cudaStream_t st);
 cudaError_t accumulate_f32(int part_dtype, float* acc, const void* part, size_t n, cudaStream_t st);
 cudaError_t merge_partials(int acc_dtype, int part_dtype, long long rows, int D, void* o_acc, float* lse_acc,
                            const void* o_part, const float* lse_part, cudaStream_t st);
-
-// Launch accounting (attn_api.cu).
-void count_launch(int n = 1);
 
 // A one-warp kernel whose only wait can never complete, limited to limit_ns (attn_fwd_sm100.cu): exercises the
 // give-up path of the bounded waits without hanging or faulting anything.  *gave_up (device memory, optional) <- 1.

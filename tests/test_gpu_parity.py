@@ -240,6 +240,45 @@ def test_bf16_tensor_core_noncausal_rectangular(sb, oracle):
     _check_bf16(_np(dv), wdv, "dv")
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,col0,tail,window", [
+    (1, 2, 2, 1, 64, 0, 0, 0),         # one token
+    (2, 4, 2, 129, 64, 3, 5, 0),       # unaligned window: 4-byte accesses; key tiles cut by query head
+    (3, 6, 1, 384, 128, 32, 0, 0),     # head_dim 128: fp32 row-term columns, two feature tiles per head
+    (5, 3, 3, 300, 64, 0, 4, 70),      # sliding window, 16-byte accesses, ragged tiles
+])
+def test_staged_matrices_vs_exact_kernels(sb, B, Hq, Hkv, S, D, col0, tail, window):
+    """One conversion launch, results stored as matrices by the kernels that compute them: against the exact kernels on the
+    same matrices.  Relative L2 of bf16 operands and bf16 P / dS (8 significant bits each, errors independent over the sums):
+    at most 3 x 2^-9 = 6e-3; columns outside the window stay as they were."""
+    FA = sb.CudaFlashAttention
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    C_ = col0 + B * S + tail
+    q, k, v, do = (torch.randn(H * D, C_, generator=g, device="cuda") * std for H, std in ((Hq, 0.5), (Hkv, 0.5), (Hkv, 1.0), (Hq, 1e-2)))
+    shape = (Hq, D, D ** -0.5, True, col0, S, B, window)
+    got = {}
+    try:
+        for reduced in (False, True):
+            FA.allow_reduced_precision = reduced
+            o, lse = torch.full_like(q, 9.0), torch.full((Hq, C_), 9.0, device="cuda")
+            grads = torch.full_like(q, 9.0), torch.full_like(k, 9.0), torch.full_like(v, 9.0)
+            FA.forwardMultiHead(q, k, v, o, lse, *shape)
+            assert sb.last_path() == ("tcgen05_staged" if reduced else "simt_f32")
+            FA.backwardMultiHead(q, k, v, o, lse, do, *grads, None, *shape)
+            got[reduced] = (o, lse) + grads
+    finally:
+        FA.allow_reduced_precision = False
+    assert sb.poll_device_status() == 0
+    for name, x, y in zip(("o", "lse", "dq", "dk", "dv"), got[True], got[False]):
+        assert bool((x[:, :col0] == 9).all()) and bool((x[:, col0 + B * S:] == 9).all()), name
+        x, y = x[:, col0:col0 + B * S], y[:, col0:col0 + B * S]
+        if name == "lse":                        # a difference of exponents: |ds| <= scale |q| |k| 2^-8 <= 8 x 2^-8 / 2 here, typically 1e-3
+            assert float((x - y).abs().max()) <= BF16_ABS
+        elif float(y.abs().max()) > 1e-6:
+            assert float((x - y).norm() / y.norm()) <= 6e-3, (name, float((x - y).norm() / y.norm()))
+        else:                                    # one visible key: dQ = dK = 0 up to rounding
+            assert float(x.abs().max()) <= 1e-4, name
+
+
 def test_bf16_golden_inputs_tensor_core_vs_reference_cpu(sb):
     """Golden fixtures whose inputs are bf16-exact: the tensor-core path against the reference CPU outputs."""
     for name in ("gqa_h4_kv1_s200_d64_bf16in", "gqa_h4_kv2_s136_d128_bf16in"):

@@ -629,124 +629,7 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     return launch_kernel(attn_fwd_tc_kernel<D, kMode, kMat>, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p);
 }
 
-// ---- KV-cache mode ----------------------------------------------------------------------------------------------
-// Combines the per-split partial results: LSE = log sum_s exp(lse_s), O = sum_s exp(lse_s - LSE) * O_s.  One warp per
-// row; a split that saw no visible key for the row carries LSE = -inf and weighs nothing.
-template <int D>
-__global__ void __launch_bounds__(256) cache_merge_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __restrict__ lse_part,
-                                                          int n_splits, long long rows, __nv_bfloat16* __restrict__ o,
-                                                          float* __restrict__ lse)
-{
-    wait_for_stream();
-    const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (r >= rows) return;
-    float m = -INFINITY;
-    for (int sp = lane; sp < n_splits; sp += 32) m = fmaxf(m, lse_part[(size_t)sp * rows + r]);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    float sum = 0.0f;
-    if (m > -INFINITY)
-        for (int sp = lane; sp < n_splits; sp += 32) sum += __expf(lse_part[(size_t)sp * rows + r] - m);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    const float total = m > -INFINITY ? m + __logf(sum) : -INFINITY;
-    constexpr int kPer = D / 32;   // consecutive elements per lane
-    float acc[kPer];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) acc[i] = 0.0f;
-    for (int sp = 0; sp < n_splits; ++sp) {
-        const float l = lse_part[(size_t)sp * rows + r];
-        if (!(l > -INFINITY)) continue;
-        const float w = __expf(l - total);
-        const __nv_bfloat16* src = o_part + ((size_t)sp * rows + r) * D + lane * kPer;
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) acc[i] = fmaf(w, __bfloat162float(src[i]), acc[i]);
-    }
-    __nv_bfloat16* dst = o + (size_t)r * D + lane * kPer;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) dst[i] = __float2bfloat16(acc[i]);
-    if (lane == 0) lse[r] = total;
-}
-
-template <int D>
-cudaError_t launch_cache(const TcArgs& a, int capacity, void* workspace, cudaStream_t st)
-{
-    const AttnShape& s = a.s;
-    const CachePlan plan = tc_cache_plan(s);
-    const int group = s.Hq / s.Hkv, rows_per_slab = group * s.Sq, slabs = s.B * s.Hkv;
-    const long long rows = (long long)slabs * rows_per_slab;
-    CUtensorMap tq, tk, tv;
-    cudaError_t e;
-    // Q [B][Hq][new][D] read as [B*Hkv][group*new][D]: the query heads of a group are consecutive heads
-    if ((e = encode_tmap_bf16_3d(&tq, a.q, D, rows_per_slab, slabs, 128)) != cudaSuccess) return e;
-    if ((e = encode_tmap_bf16_3d(&tk, a.k, D, s.Skv, slabs, 128, capacity)) != cudaSuccess) return e;
-    if ((e = encode_tmap_bf16_3d(&tv, a.v, D, s.Skv, slabs, 128, capacity)) != cudaSuccess) return e;
-    const int n_parts = 2 * plan.n_splits;   // two key streams per CTA
-    float* lse_part = reinterpret_cast<float*>(workspace);
-    __nv_bfloat16* o_part = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<uint8_t*>(workspace) +
-                                                             (((size_t)n_parts * rows * sizeof(float) + 255) / 256) * 256);
-    FwdParams p{};
-    p.o = o_part;
-    p.lse = lse_part;
-    p.B = s.B; p.Hq = s.Hq; p.Hkv = s.Hkv; p.Sq = rows_per_slab; p.Skv = s.Skv;
-    p.causal = 1;
-    p.window = s.window;
-    p.global_tokens = s.global_tokens;
-    p.new_tokens = s.Sq;
-    p.n_splits = plan.n_splits;
-    p.tiles_per_split = plan.tiles_per_split;
-    p.n_qblk = (rows_per_slab + kM - 1) / kM;
-    p.scale_log2 = s.scale * 1.4426950408889634f;
-    const size_t smem = 6 * (size_t)(128 * D * 2) + sizeof(FwdBarriers) + 1024;
-    static std::atomic<unsigned long long> configured{0};   // one bit per device
-    if ((e = ensure_dynamic_smem(attn_fwd_tc_kernel<D, kCache, false>, smem, configured)) != cudaSuccess) return e;
-    const long long ctas = (long long)plan.n_splits * p.n_qblk * slabs;
-    if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if ((e = launch_kernel(attn_fwd_tc_kernel<D, kCache, false>, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p)) != cudaSuccess) return e;
-    return launch_kernel(cache_merge_kernel<D>, (unsigned)((rows + 7) / 8), 256, 0, st, 1, o_part, lse_part, n_parts, rows, a.o_out, a.lse_out);
-}
-
 }  // namespace
-
-// Key tiles the cache-mode kernel visits (global-token tiles, then the window of the oldest new token up to the end of
-// the cache) and how they are dealt to CTAs: about one CTA per SM in total.
-CachePlan tc_cache_plan(const AttnShape& s)
-{
-    const int n_tiles = (s.Skv + kN - 1) / kN;
-    int n_list = n_tiles;
-    if (s.window > 0) {
-        const int g_tiles = (s.global_tokens + kN - 1) / kN;
-        const int first_pos = s.Skv - s.Sq;
-        const int w_first = std::max(g_tiles, std::max(0, first_pos - s.window + 1) / kN);
-        n_list = std::min(g_tiles, n_tiles) + std::max(0, n_tiles - w_first);
-    }
-    const int group = s.Hq / s.Hkv;
-    const long long base = (long long)s.B * s.Hkv * ((group * s.Sq + kM - 1) / kM);
-    // pieces of at least two tiles (one per stream of a CTA), about one CTA per SM in total
-    int want = (int)std::max(1LL, std::min<long long>((n_list + 1) / 2, 148 / std::max(1LL, base)));
-    CachePlan plan;
-    plan.tiles_per_split = (n_list + want - 1) / want;
-    plan.n_splits = (n_list + plan.tiles_per_split - 1) / plan.tiles_per_split;
-    return plan;
-}
-
-size_t tc_cache_workspace_bytes(const AttnShape& s)
-{
-    const size_t n_parts = 2 * (size_t)tc_cache_plan(s).n_splits;
-    const size_t rows = (size_t)s.B * s.Hq * s.Sq;
-    return ((n_parts * rows * sizeof(float) + 255) / 256) * 256 + n_parts * rows * s.D * 2;
-}
-
-bool tc_cache_supported(const AttnShape& s)
-{
-    return (s.D == 64 || s.D == 128) && s.causal && s.Sq <= s.Skv;
-}
-
-cudaError_t tc_cache_forward(const TcArgs& a, int capacity, void* workspace, cudaStream_t st)
-{
-    return a.s.D == 64 ? launch_cache<64>(a, capacity, workspace, st) : launch_cache<128>(a, capacity, workspace, st);
-}
 
 // A training loop calls with the same tensors step after step (the reference's trainer even replays a captured graph
 // with identical pointers, CudaLanguageModel.cu:2176-2209), and on small problems the seven driver calls that encode
@@ -876,7 +759,9 @@ cudaError_t read_and_clear_fwd_status(cudaStream_t st, uint32_t* word)
     unsigned int w = 0, zero = 0;
     if ((e = cudaMemcpyFromSymbol(&w, ptx::g_device_status, sizeof(w))) != cudaSuccess) return e;
     if (w != 0 && (e = cudaMemcpyToSymbol(ptx::g_device_status, &zero, sizeof(zero))) != cudaSuccess) return e;
-    *word = w;
+    uint32_t cache = 0;
+    if ((e = read_and_clear_cache_status(&cache)) != cudaSuccess) return e;
+    *word = w ? w : cache;
     return cudaSuccess;
 }
 

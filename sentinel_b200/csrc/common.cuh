@@ -152,11 +152,8 @@ enum : int { kBwdPre = 1, kBwdMain = 2, kBwdPost = 4 };
 bool tc_fwd_supported(const AttnShape& s);
 bool tc_bwd_supported(const AttnShape& s);
 cudaError_t tc_forward(const TcArgs& a, cudaStream_t st);
-// New tokens against a KV cache (forward only): s.Sq new tokens per head at positions Skv-Sq .. Skv-1, K/V slabs
-// `capacity` rows apart.  The keys are dealt to n_splits CTAs per (KV head, 128-row query block), each running two key
-// streams; the 2 * n_splits partial results go through `workspace` (tc_cache_workspace_bytes) and a merge kernel.
-struct CachePlan { int n_splits, tiles_per_split; };
-CachePlan tc_cache_plan(const AttnShape& s);
+// New tokens against a KV cache (attn_cache_sm100.cu, forward only): s.Sq new tokens per head at positions Skv-Sq .. Skv-1, K/V
+// slabs `capacity` rows apart.  Partial results go through `workspace` (tc_cache_workspace_bytes) and a merge kernel.
 size_t tc_cache_workspace_bytes(const AttnShape& s);
 bool tc_cache_supported(const AttnShape& s);
 cudaError_t tc_cache_forward(const TcArgs& a, int capacity, void* workspace, cudaStream_t st);
@@ -200,8 +197,9 @@ cudaError_t merge_partials(int acc_dtype, int part_dtype, long long rows, int D,
 // give-up path of the bounded waits without hanging or faulting anything.  *gave_up (device memory, optional) <- 1.
 cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned int* gave_up, cudaStream_t st);
 
-// Device status words written by bounded waits (one per tensor-core translation unit).
+// Device status words written by bounded waits (one per tensor-core translation unit; the first reports the KV-cache kernel's too).
 cudaError_t read_and_clear_fwd_status(cudaStream_t st, uint32_t* word);
+cudaError_t read_and_clear_cache_status(uint32_t* word);   // after a synchronisation of the stream
 cudaError_t read_and_clear_bwd_status(cudaStream_t st, uint32_t* word);
 
 }  // namespace sntl

@@ -327,7 +327,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // dS_i -> dQ_i -> drain -> dP^T_{i+1} -> dS_{i+1} then no longer carries the issue time of dK_i (with one buffer dK_i must
     // have read the tile before dP^T_{i+1} lets the compute warps overwrite it)
     constexpr int kDsBufs = (D == 128) ? 1 : 2;
-    constexpr bool kElect14 = D == 64;             // issue form of the dS-side warp (see there)
     // columns of a dQ tile per bulk reduction (kStageCols columns x 128 rows fp32 = one piece): 8 KB pieces at head_dim 128,
     // where the tile loads of Q and dO queue behind the reductions on the SM's path to L2 and shorter pieces let them through
     // sooner (-3 % kernel time); 16 KB pieces at head_dim 64 (there the finer split costs 1 %, and 4 KB pieces cost 10-20 %
@@ -365,7 +364,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     BwdBarriers* bars = (BwdBarriers*)(sTail + kTailBytes);
     volatile uint32_t* abort_flag = &bars->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp-uniform for the compiler)
     if ((smem_u32(smem_raw) & 1023u) != 0u) {      // uniform over the CTA: nothing has been set up yet
         if (threadIdx.x == 0) atomicCAS(&g_device_status, 0u, (0x3fu << 24) | (blockIdx.x & 0xffffffu));
         wait_for_stream();
@@ -498,33 +497,24 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         // accumulator, and a third issuing warp for dK measured 7-20 % slower than this split at either head size.)
         if (warp == 12 && n_iter > 0) {
             // P side: all 32 lanes walk the loop (warp-uniform control flow lets descriptors and addresses live in uniform
-            // registers) and one elected lane issues each tcgen05 instruction.  dV_i and S^T_{i+1} head the chain the compute
-            // warps wait on, and this form issues 8 MMAs in ~720 cycles against ~1100 for a single-lane loop.
+            // registers) and one elected lane issues the products four k-steps at a time (mma_ss_4).
             SNTL_TRACE_DECL(tn);
             const bool tl = lane == 0;
             (void)tl;
             constexpr uint32_t idesc_st = make_idesc(kT, kT, false, false);
             constexpr uint32_t idesc_kv = make_idesc(kT, D, false, true);
-            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
-                return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site));
-            };
+            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_warp(bar, parity, abort_flag, site); };
             const uint64_t d_ones = make_sdesc_plain(smem_u32(sOnes), kAugBytes), d_qaug0 = make_sdesc_plain(smem_u32(sQaug), 0);
             // the D/16 steps over the head dimension, then the extra step that subtracts LSE/scale (see kAugBytes)
             auto issue_kmajor = [&](uint32_t d_tmem, uint64_t a, uint64_t b, uint64_t aug) {
-                mma_ss_e<false>(d_tmem, a, b, idesc_st);
 #pragma unroll
-                for (int ks = 1; ks < D / 16; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * kChunkBytes + (ks & 3) * 32);
-                    mma_ss_e<true>(d_tmem, sdesc_advance(a, off), sdesc_advance(b, off), idesc_st);
-                }
-                if constexpr (kAug) mma_ss_e<true>(d_tmem, d_ones, aug, idesc_st);
+                for (int c = 0; c < kChunks; ++c)
+                    mma_ss_4<2, 2>(d_tmem, sdesc_advance(a, (uint32_t)(c * kChunkBytes)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_st, c > 0);
+                if constexpr (kAug) mma_ss_1(d_tmem, d_ones, aug, idesc_st);
             };
             auto issue_from_tmem = [&](uint32_t d_tmem, uint32_t a_tmem, uint64_t b, bool accumulate) {
-                if (accumulate) mma_ts_e<true>(d_tmem, a_tmem, b, idesc_kv);
-                else mma_ts_e<false>(d_tmem, a_tmem, b, idesc_kv);
-#pragma unroll
-                for (int ks = 1; ks < kT / 16; ++ks)
-                    mma_ts_e<true>(d_tmem, a_tmem + (uint32_t)((ks >> 2) * 64 + (ks & 3) * 8), sdesc_advance(b, ks * 2048), idesc_kv);
+                mma_ts_4<8, 128>(d_tmem, a_tmem, b, idesc_kv, accumulate);
+                mma_ts_4<8, 128>(d_tmem, a_tmem + 64u, sdesc_advance(b, 4 * 2048), idesc_kv, 1);
             };
             bool ok = wait(&bars->kv_full, 0, kSiteKV);
             const uint64_t dK_k = make_sdesc(smem_u32(sK), 16, 1024);
@@ -534,7 +524,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if (!(ok = wait(&bars->q_full[j], 0, kSiteQFull))) break;
                 tc_fence_after();
                 issue_kmajor(tm_S + (uint32_t)j * kSBufStride, dK_k, sdesc_advance(dQ_k0, j * kTileBytes), sdesc_advance(d_qaug0, j * kAugBytes));
-                tc_commit_e(&bars->s_ready[j]);
+                tc_commit_p(&bars->s_ready[j]);
             }
             for (int i = 0; ok && i < n_iter; ++i) {
                 const int sq = i % kQStages, sd = i % kDoStages, sb = i % kSBufs;
@@ -546,48 +536,37 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 SNTL_TRACE_EV(tl, 0, tn, 1);
                 tc_fence_after();
                 issue_from_tmem(tm_dV, tm_Si, sdesc_advance(dDo_mn0, sd * kTileBytes), i > 0);
-                tc_commit_e(&bars->do_empty[sd]);
-                tc_commit_e(&bars->q_empty[sq]);
+                tc_commit_p(&bars->do_empty[sd]);
+                tc_commit_p(&bars->q_empty[sq]);
                 SNTL_TRACE_EV(tl, 0, tn, 2);
                 if (i + kSBufs < n_iter) {
                     const int nq = (i + kSBufs) % kQStages;
                     if (!(ok = wait(&bars->q_full[nq], (uint32_t)(((i + kSBufs) / kQStages) & 1), kSiteQFull))) break;
                     tc_fence_after();
                     issue_kmajor(tm_Si, dK_k, sdesc_advance(dQ_k0, nq * kTileBytes), sdesc_advance(d_qaug0, nq * kAugBytes));
-                    tc_commit_e(&bars->s_ready[sb]);
+                    tc_commit_p(&bars->s_ready[sb]);
                     SNTL_TRACE_EV(tl, 0, tn, 9);
                 }
             }
-            tc_commit_e(&bars->final_bar);
+            tc_commit_p(&bars->final_bar);
             wait(&bars->final_bar, 0, kSiteFinal);
-        } else if (warp == 14 && (kElect14 || lane == 0) && n_iter > 0) {
-            // dS side.  At head_dim 64 it takes the same warp-uniform form as the P side (-4 % kernel time); at 128 a single
-            // lane walks the loop: there the faster form costs 8 % (2.81 vs 2.59 ms) -- these products then get into the
-            // tensor pipe ahead of the P side's, whose chain sets the step at that head size.
+        } else if (warp == 14 && n_iter > 0) {
+            // dS side, in the same form
             const bool tl14 = lane == 0;
             (void)tl14;
-            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
-                if constexpr (kElect14) return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site));
-                else return mbar_wait(bar, parity, abort_flag, site);
-            };
+            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_warp(bar, parity, abort_flag, site); };
             SNTL_TRACE_DECL(tn);
             constexpr uint32_t idesc_st = make_idesc(kT, kT, false, false);   // S^T, dP^T
             constexpr uint32_t idesc_kv = make_idesc(kT, D, false, true);     // dV, dK: A in TMEM, B MN-major
             constexpr uint32_t idesc_dq = make_idesc(kT, D, true, true);      // dQ: both operands MN-major
-            // C[128 x 128] = A[128 x D] * B[128 x D]^T, both K-major tiles; one descriptor per tile, advanced per k-step
-            // by a 64-bit add (the empty asm keeps the compiler from hoisting every advanced descriptor out of the main
-            // loop, which would cost this warp more registers than it is allotted)
             const uint64_t d_ones = make_sdesc_plain(smem_u32(sOnes), kAugBytes), d_doaug0 = make_sdesc_plain(smem_u32(sDoaug), 0);
-            // the D/16 steps over the head dimension, then the extra step that subtracts delta (see kAugBytes)
+            // C[128 x 128] = A[128 x D] * B[128 x D]^T, both K-major tiles: the D/16 steps over the head dimension, then the extra
+            // step that subtracts delta (see kAugBytes)
             auto issue_kmajor = [&](uint32_t d_tmem, uint64_t a, uint64_t b, uint64_t aug) {
-                asm volatile("" : "+l"(a), "+l"(b), "+l"(aug));
-                mma_ss_x<kElect14, false>(d_tmem, a, b, idesc_st);
 #pragma unroll
-                for (int ks = 1; ks < D / 16; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * kChunkBytes + (ks & 3) * 32);
-                    mma_ss_x<kElect14, true>(d_tmem, sdesc_advance(a, off), sdesc_advance(b, off), idesc_st);
-                }
-                if constexpr (kAug) mma_ss_x<kElect14, true>(d_tmem, d_ones, aug, idesc_st);
+                for (int c = 0; c < kChunks; ++c)
+                    mma_ss_4<2, 2>(d_tmem, sdesc_advance(a, (uint32_t)(c * kChunkBytes)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_st, c > 0);
+                if constexpr (kAug) mma_ss_1(d_tmem, d_ones, aug, idesc_st);
             };
             bool ok = wait(&bars->kv_full, 0, kSiteKV);
             {
@@ -599,8 +578,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if (ok) {
                     tc_fence_after();
                     issue_kmajor(tm_dP, dV_k, dDo_k0, d_doaug0);
-                    tc_commit_x<kElect14>(&bars->dp_ready);
-                    tc_commit_x<kElect14>(&bars->do_empty[0]);   // this warp's share of releasing dO_0: dP^T_0
+                    tc_commit_p(&bars->dp_ready);
+                    tc_commit_p(&bars->do_empty[0]);   // this warp's share of releasing dO_0: dP^T_0
                 }
                 for (int i = 0; ok && i < n_iter; ++i) {
                     const uint32_t ph = (uint32_t)(i & 1);
@@ -610,15 +589,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     tc_fence_after();
                     // dQ first: it gates the drain and with it the next dP^T
                     const uint32_t ds_off = (uint32_t)((i % kDsBufs) * kDsBytes);
-                    {
-                        uint64_t a = sdesc_advance(dDs_mn, ds_off), bq = dK_mn;
-                        asm volatile("" : "+l"(a), "+l"(bq));
-                        mma_ss_x<kElect14, false>(tm_dP, a, bq, idesc_dq);
-#pragma unroll
-                        for (int ks = 1; ks < kT / 16; ++ks)
-                            mma_ss_x<kElect14, true>(tm_dP, sdesc_advance(a, ks * 2048), sdesc_advance(bq, ks * 2048), idesc_dq);
-                    }
-                    tc_commit_x<kElect14>(&bars->dq_ready);
+                    const uint64_t ds_mn = sdesc_advance(dDs_mn, ds_off);
+                    mma_ss_4<128, 128>(tm_dP, ds_mn, dK_mn, idesc_dq, 0);
+                    mma_ss_4<128, 128>(tm_dP, sdesc_advance(ds_mn, 4 * 2048), sdesc_advance(dK_mn, 4 * 2048), idesc_dq, 1);
+                    tc_commit_p(&bars->dq_ready);
                     SNTL_TRACE_EV(tl14, 4, tn, 4);
                     // dK += dS^T Q with dS^T read from its shared-memory tile as a K-major A operand (rows = keys, the 64
                     // contiguous elements run along the queries).  Q_i is ready: ds_ready implies its load was seen.  With
@@ -626,14 +600,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     // tile, this product has read it (one thread's MMAs run in order).  With two it goes after, and the
                     // buffer it reads is rewritten only behind dP^T_{i+2}, which this thread issues later still.
                     auto issue_dk = [&]() {
-                        uint64_t a = sdesc_advance(dDs_k, ds_off), bq = sdesc_advance(dQ_mn0, sq * kTileBytes);
-                        asm volatile("" : "+l"(a), "+l"(bq));
-                        if (i > 0) mma_ss_x<kElect14, true>(tm_dK, a, bq, idesc_kv);
-                        else mma_ss_x<kElect14, false>(tm_dK, a, bq, idesc_kv);
-#pragma unroll
-                        for (int ks = 1; ks < kT / 16; ++ks)
-                            mma_ss_x<kElect14, true>(tm_dK, sdesc_advance(a, (ks >> 2) * kChunkBytes + (ks & 3) * 32), sdesc_advance(bq, ks * 2048), idesc_kv);
-                        tc_commit_x<kElect14>(&bars->q_empty[sq]);    // this warp's share: dK_i
+                        const uint64_t a = sdesc_advance(dDs_k, ds_off), bq = sdesc_advance(dQ_mn0, sq * kTileBytes);
+                        mma_ss_4<2, 128>(tm_dK, a, bq, idesc_kv, i > 0);
+                        mma_ss_4<2, 128>(tm_dK, sdesc_advance(a, kChunkBytes), sdesc_advance(bq, 4 * 2048), idesc_kv, 1);
+                        tc_commit_p(&bars->q_empty[sq]);    // this warp's share: dK_i
                     };
                     if constexpr (kDsBufs == 1) issue_dk();
                     if (i + 1 < n_iter) {
@@ -643,17 +613,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                         if (!(ok = wait(&bars->do_full[nd], (uint32_t)(((i + 1) / kDoStages) & 1), kSiteDoFull))) break;
                         tc_fence_after();
                         issue_kmajor(tm_dP, dV_k, sdesc_advance(dDo_k0, nd * kTileBytes), sdesc_advance(d_doaug0, nd * kAugBytes));
-                        tc_commit_x<kElect14>(&bars->dp_ready);
+                        tc_commit_p(&bars->dp_ready);
                         // this warp's share of releasing dO_{i+1}, committed at once: with a single dO stage the load of the
                         // next tile starts as soon as this product and dV_{i+1} have read the stage
-                        tc_commit_x<kElect14>(&bars->do_empty[nd]);
+                        tc_commit_p(&bars->do_empty[nd]);
                         SNTL_TRACE_EV(tl14, 4, tn, 6);
                     }
                     if constexpr (kDsBufs == 2) issue_dk();
                 }
             }
             // every MMA of this thread has retired once its commit lands; the epilogue waits for both issuers
-            tc_commit_x<kElect14>(&bars->final_bar);
+            tc_commit_p(&bars->final_bar);
             wait(&bars->final_bar, 0, kSiteFinal);
         }
     } else if (warp >= 8) {

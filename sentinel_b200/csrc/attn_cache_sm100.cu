@@ -25,6 +25,7 @@
 // written over S.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
+#include "softmax_tile.cuh"
 
 #include <algorithm>
 
@@ -124,7 +125,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint8_t *sK = smem + L::k, *sV = smem + L::v, *sQ = smem + L::q;
     CacheBarriers* bars = (CacheBarriers*)(smem + L::bars);
     volatile uint32_t* abort_flag = &bars->abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp-uniform for the compiler)
 
     // Key tiles a unit visits, in ascending order: those holding global tokens, then from the window of the oldest new token
     // to the end of the cache.
@@ -201,45 +202,35 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     } else if (warp == 8) {
         setmaxnreg_dec<72>();
         // =========================== MMA issuer ===========================
-        // All 32 lanes walk the loops, one elected lane issues each tcgen05 instruction: descriptors then live in uniform
-        // registers.  With a single-lane loop 16 products took 2200 cycles to issue, and a tile of a 512-token continuation 5600.
+        // All 32 lanes walk the loops, one elected lane issues the products four k-steps at a time: descriptors then live in
+        // uniform registers.  With a single-lane loop 16 products took 2200 cycles to issue, and a tile of a 512-token continuation 5600.
         {
             constexpr uint32_t idesc_s = make_idesc(kM, kN, false, false);
             constexpr uint32_t idesc_pv = make_idesc(kM, D, false, true);
             const uint64_t dq0 = make_sdesc(smem_u32(sQ), 16, 1024), dk0 = make_sdesc(smem_u32(sK), 16, 1024);
             const uint64_t dv0 = make_sdesc(smem_u32(sV), kChunkBytes, 1024);
             auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
-                return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site));
+                return mbar_wait_warp(bar, parity, abort_flag, site);
             };
             auto issue_s = [&](int t, int st, int slot) {
-                uint64_t a = dq0 + (uint64_t)((slot * L::kQBytes - (kMode == kSmall ? (t + 1) * kSmallRows * 128 : 0)) >> 4);
-                uint64_t b = sdesc_advance(dk0, (uint32_t)(st * L::kTileBytes));
-                asm volatile("" : "+l"(a), "+l"(b));
-                mma_ss_e<false>(tmem_S(t), a, b, idesc_s);
+                const uint64_t a = dq0 + (uint64_t)((slot * L::kQBytes - (kMode == kSmall ? (t + 1) * kSmallRows * 128 : 0)) >> 4);
+                const uint64_t b = sdesc_advance(dk0, (uint32_t)(st * L::kTileBytes));
 #pragma unroll
-                for (int ks = 1; ks < D / 16; ++ks)
-                    mma_ss_e<true>(tmem_S(t), sdesc_advance(a, (uint32_t)((ks >> 2) * L::kQChunk + (ks & 3) * 32)),
-                                   sdesc_advance(b, (uint32_t)((ks >> 2) * kChunkBytes + (ks & 3) * 32)), idesc_s);
-                tc_commit_e(&bars->s_ready[t]);
+                for (int c = 0; c < kChunks; ++c)
+                    mma_ss_4<2, 2>(tmem_S(t), sdesc_advance(a, (uint32_t)(c * L::kQChunk)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_s, c > 0);
+                tc_commit_p(&bars->s_ready[t]);
             };
             // kPair: the first half of the contraction goes out as soon as the first 64 columns of P are there (the caller has
             // waited for them), the rest behind p_ready.  Returns false when a wait gave up.
             auto issue_pv = [&](int t, int st, bool accumulate, uint32_t parity) {
-                uint64_t b = sdesc_advance(dv0, (uint32_t)(st * L::kTileBytes));
-                asm volatile("" : "+l"(b));
-                if (accumulate) mma_ts_e<true>(tmem_O(t), tmem_S(t), b, idesc_pv);
-                else mma_ts_e<false>(tmem_O(t), tmem_S(t), b, idesc_pv);
-#pragma unroll
-                for (int ks = 1; ks < kN / 32; ++ks)
-                    mma_ts_e<true>(tmem_O(t), tmem_S(t) + (uint32_t)(ks * 8), sdesc_advance(b, (uint32_t)(ks * 2048)), idesc_pv);
+                const uint64_t b = sdesc_advance(dv0, (uint32_t)(st * L::kTileBytes));
+                mma_ts_4<8, 128>(tmem_O(t), tmem_S(t), b, idesc_pv, accumulate);
                 if (kMode == kPair) {
                     if (!wait(&bars->p_ready[t], parity, kSitePReady)) return false;
                     tc_fence_after();
                 }
-#pragma unroll
-                for (int ks = kN / 32; ks < kN / 16; ++ks)
-                    mma_ts_e<true>(tmem_O(t), tmem_S(t) + (uint32_t)(ks * 8), sdesc_advance(b, (uint32_t)(ks * 2048)), idesc_pv);
-                tc_commit_e(&bars->o_ready[t]);
+                mma_ts_4<8, 128>(tmem_O(t), tmem_S(t) + 32u, sdesc_advance(b, 4 * 2048), idesc_pv, 1);
+                tc_commit_p(&bars->o_ready[t]);
                 return true;
             };
             // S runs ahead of P V: one load, or two when the streams take turns.  Each side walks the piece by itself.
@@ -269,8 +260,8 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 return true;
             };
             auto s_done = [&]() {         // S products are issued in load order: behind the unit's last one its Q is free
-                tc_commit_e(&bars->k_empty[s.st]);
-                if (s.last()) tc_commit_e(&bars->q_empty[kMode == kPair ? 0 : s.seg & 1]);
+                tc_commit_p(&bars->k_empty[s.st]);
+                if (s.last()) tc_commit_p(&bars->q_empty[kMode == kPair ? 0 : s.seg & 1]);
                 s.advance();
             };
             if constexpr (kMode == kPair) {
@@ -297,7 +288,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                         }
                     }
                     if (!ok) break;
-                    tc_commit_e(&bars->v_empty[v.st]);
+                    tc_commit_p(&bars->v_empty[v.st]);
                     v.advance();
                     if (s.more) s_done();
                 }
@@ -314,7 +305,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     tc_fence_after();
                     // a stream's first tile of a unit overwrites its O: the unit's loads are dealt to the streams in turn
                     issue_pv(t, v.st, v.j >= 2, 0);
-                    tc_commit_e(&bars->v_empty[v.st]);
+                    tc_commit_p(&bars->v_empty[v.st]);
                     v.advance();
                     // into the S columns this product has just read P from: one thread's products run in order
                     if (s.more && (ok = s_operands())) {
@@ -323,7 +314,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     }
                 }
             }
-            tc_commit_e(&bars->final_bar);
+            tc_commit_p(&bars->final_bar);
             wait(&bars->final_bar, 0, kSiteFinal);
         }
     } else {
@@ -365,17 +356,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                                 if (c < lo && c >= glim) s[c] = 0xff800000u;
                         }
                     }
-                    float mx8[8];
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) mx8[c] = __uint_as_float(s[c]);
-#pragma unroll
-                    for (int c = 8; c + 16 <= kN; c += 16)
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) mx8[i] = fmax3(mx8[i], __uint_as_float(s[c + i]), __uint_as_float(s[c + 8 + i]));
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(mx8[i], __uint_as_float(s[kN - 8 + i]));
-                    const float mx = fmax3(fmax3(mx8[0], mx8[1], mx8[2]), fmax3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]));
-                    const float m_new = fmaxf(m_ref, mx * p.scale_log2);
+                    const float m_new = fmaxf(m_ref, row_max(s) * p.scale_log2);
                     const bool need = (m_new - m_ref) > kRescaleThreshold && live;   // false when both are -inf (NaN compare)
                     if (count == 0) {
                         m_ref = m_new;
@@ -397,26 +378,19 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                         tmem_st_wait();
                     }
                     const float neg_m = (m_ref == -INFINITY) ? 0.0f : -m_ref;
-                    float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(neg_m, neg_m);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        uint32_t pk[32];
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) {
-                            const float2 x = ffma2(make_float2(__uint_as_float(s[h * 64 + 2 * c]), __uint_as_float(s[h * 64 + 2 * c + 1])), sc2, nm2);
-                            const float p0 = ex2(x.x), p1 = ex2(x.y);
-                            l4[c & 3] += p0 + p1;
-                            pk[c] = pack_bf16(p0, p1);
-                        }
-                        tmem_st32(tmem_S(t) + lane_off + (uint32_t)(h * 32), pk);
-                        if (kMode == kPair && h == 0) {
-                            tmem_st_wait();
-                            tc_fence_before();
-                            mbar_arrive(&bars->p_half[t]);
-                        }
+                    uint32_t pk[32];
+                    float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                    RowMax unused;
+                    exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, unused);
+                    tmem_st32(tmem_S(t) + lane_off, pk);
+                    if (kMode == kPair) {
+                        tmem_st_wait();
+                        tc_fence_before();
+                        mbar_arrive(&bars->p_half[t]);
                     }
-                    l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+                    exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, unused);
+                    tmem_st32(tmem_S(t) + lane_off + 32u, pk);
+                    l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
                     tmem_st_wait();
                     tc_fence_before();
                     mbar_arrive(&bars->p_ready[t]);

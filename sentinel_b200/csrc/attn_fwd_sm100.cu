@@ -23,10 +23,11 @@
 //     heads of one group are adjacent in launch order so they share K/V tiles in L2.
 //
 // Layout: bf16 token-major [B][H][S][D], D in {64,128}; LSE [B][Hq][Sq] fp32 (natural log).
-// TMEM map (512 columns): head_dim 128 and KV-cache mode S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D);
+// TMEM map (512 columns): head_dim 128 S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D);
 // head_dim 64 S0 [0,128) P0 [128,192) S1 [192,320) P1 [320,384) O0 [384,448) O1 [448,512).
 #include "common.cuh"
 #include "sm100_ptx.cuh"
+#include "softmax_tile.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -44,7 +45,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 enum WaitSite : uint32_t {
-    kSiteQ = 1, kSiteKFull, kSiteVFull, kSiteKEmpty, kSiteVEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue
+    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue
 };
 
 struct FwdParams {
@@ -53,32 +54,30 @@ struct FwdParams {
     int B, Hq, Hkv, Sq, Skv;
     int causal;
     int window, global_tokens;   // sliding window and always-visible first keys (0, 0: plain causal)
-    // KV-cache mode: the rows of one slab are the (query head of the group, new token) pairs of one KV head, row r
-    // sits at position Skv - new_tokens + r % new_tokens, and the key tiles are dealt to n_splits CTAs whose partial
-    // (O, LSE) land in o / lse as [split][slab][row]
-    int new_tokens, n_splits, tiles_per_split;
     int n_qblk;       // 256-row query blocks per (b, h)
     float scale_log2; // scale * log2(e)
-    // non-null: O and LSE leave as fp32 feature-major matrices (see MatrixOut; not in KV-cache mode)
+    // non-null: O and LSE leave as fp32 feature-major matrices (see MatrixOut)
     float *o_mat, *lse_mat;
     long long mat_stride;
 };
 
 struct FwdBarriers {
-    uint64_t q_full;
-    uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
-    uint64_t s_ready[2], p_ready[2], o_ready[2];
+    uint64_t q_full, k0_full;
+    // Loads come in pairs {K_{j+1}, V_j} (K_0 alone first) and are released in the same pairs, {K_0} counting as pair -1: one
+    // wait and one commit per key tile for the issuing warp instead of two each.  Barrier j & 1.
+    uint64_t pair_full[2], pair_empty[2];
+    uint64_t s_ready[2], p_ready[2];
+    uint64_t o_ready[2];     // head_dim 64: after every P V product; 128: after the tile's last one (s_ready covers the others)
     uint64_t p_half[2];      // the first 64 columns of P_t are written
     uint64_t final_bar;
     uint32_t tmem_base;
     uint32_t abort_flag;
-    uint64_t s_free[2];      // head_dim 64 (plain / window): the softmax warps have read S_j of tile t
+    uint64_t s_free[2];      // head_dim 64: the softmax warps have read S_j of tile t
 };
 
 // kMode: kPlain = causal / full attention of a whole sequence; kWindow adds the sliding window (separate so that the
-// plain kernel carries none of its bookkeeping); kCache = new tokens against a KV cache, grouped-query heads packed into
-// the rows of one tile, keys split over CTAs.
-enum FwdMode : int { kPlain = 0, kWindow = 1, kCache = 2 };
+// plain kernel carries none of its bookkeeping).
+enum FwdMode : int { kPlain = 0, kWindow = 1 };
 
 // kMat: O and LSE leave as fp32 feature-major matrices
 template <int D, int kMode, bool kMat>
@@ -97,57 +96,35 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     FwdBarriers* bars = (FwdBarriers*)(sV + 2 * kTileBytes);
     volatile uint32_t* abort_flag = &bars->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp-uniform for the compiler)
 
     // ---- work decode: heaviest query blocks first; the heads of one KV group are adjacent ----
     constexpr bool kWin = kMode != kPlain;
-    const int bh_count = kMode == kCache ? p.B * p.Hkv : p.B * p.Hq;
-    int qblk_rank = blockIdx.x / bh_count;
+    const int bh_count = p.B * p.Hq;
+    const int qblk_rank = blockIdx.x / bh_count;
     const int bh = blockIdx.x - qblk_rank * bh_count;
-    int split = 0;
-    if (kMode == kCache) {
-        split = qblk_rank / p.n_qblk;
-        qblk_rank -= split * p.n_qblk;
-    }
-    const int qblk = (p.causal && kMode != kCache) ? (p.n_qblk - 1 - qblk_rank) : qblk_rank;
-    int bh_kv = bh;
-    if (kMode != kCache) {
-        const int b = bh / p.Hq, h = bh - b * p.Hq;
-        bh_kv = b * p.Hkv + h / (p.Hq / p.Hkv);
-    }
-    // plain / window: the CTA owns two consecutive 128-row tiles.  Cache mode: it owns ONE 128-row tile and its two
-    // softmax warpgroups take alternate key tiles of the CTA's piece (two independent streams, each with its own K/V
-    // stage, S and O columns and running max / sum), so one stream's softmax overlaps the other's MMAs.
-    const int q0 = kMode == kCache ? qblk * kM : qblk * 2 * kM;
+    const int qblk = p.causal ? (p.n_qblk - 1 - qblk_rank) : qblk_rank;
+    const int b = bh / p.Hq, h = bh - b * p.Hq;
+    const int bh_kv = b * p.Hkv + h / (p.Hq / p.Hkv);
+    const int q0 = qblk * 2 * kM;                    // the CTA owns two consecutive 128-row tiles
     const int n_ktiles_all = (p.Skv + kN - 1) / kN;
-    // position of a row in its sequence (what the causal and window masks compare keys with)
-    auto row_pos = [&](int r) { return kMode == kCache ? p.Skv - p.new_tokens + r % p.new_tokens : r; };
     // Key tiles this CTA visits, in ascending order: the tiles holding global tokens, then the tiles from the window
     // of the block's first query row up to the diagonal.  Without a window that is simply 0 .. diagonal.
-    // In cache mode every row of the slab sees keys up to (almost) the end of the cache; the list is cut into
-    // tiles_per_split pieces and this CTA takes piece `split`.
-    const int first_pos = kMode == kCache ? p.Skv - p.new_tokens : q0;   // lowest position among the CTA's rows
     const bool windowed = kWin && p.window > 0;
     const int g_tiles = windowed ? (p.global_tokens + kN - 1) / kN : 0;
-    const int w_first = windowed ? max(g_tiles, max(0, first_pos - p.window + 1) / kN) : 0;
-    const int list0 = kMode == kCache ? split * p.tiles_per_split : 0;
-    auto key_tile = [&](int j) { j += list0; return j < g_tiles ? j : w_first + (j - g_tiles); };   // j-th load of the CTA
+    const int w_first = windowed ? max(g_tiles, max(0, q0 - p.window + 1) / kN) : 0;
+    auto key_tile = [&](int j) { return j < g_tiles ? j : w_first + (j - g_tiles); };   // j-th load of the CTA
     int n_t[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        const int row0 = kMode == kCache ? q0 : q0 + t * kM;
+        const int row0 = q0 + t * kM;
         if (row0 >= p.Sq) n_t[t] = 0;
-        else if (kMode == kCache) {
-            const int n_list = min(g_tiles, n_ktiles_all) + max(0, n_ktiles_all - w_first);
-            const int mine = max(0, min(p.tiles_per_split, n_list - list0));
-            n_t[t] = (mine + 1 - t) / 2;       // stream t takes loads t, t + 2, ...
-        } else if (p.causal) {
+        else if (p.causal) {
             const int diag = min(n_ktiles_all - 1, row0 / kN);
             n_t[t] = min(g_tiles, diag + 1) + max(0, diag - w_first + 1);
         } else n_t[t] = n_ktiles_all;
     }
-    const int n_max = max(n_t[0], n_t[1]);
-    const int n_loads = kMode == kCache ? n_t[0] + n_t[1] : n_max;   // K/V tiles the producer brings in
+    const int n_max = max(n_t[0], n_t[1]);           // K/V tiles the producer brings in
 
     // ---- setup ----
     if (warp == 9 && lane == 0) {
@@ -155,13 +132,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         prefetch_tensormap(&tmap_k);
         prefetch_tensormap(&tmap_v);
         mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->k0_full, 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&bars->k_full[i], 1);
-            mbar_init(&bars->k_empty[i], 1);
-            mbar_init(&bars->v_full[i], 1);
-            mbar_init(&bars->v_empty[i], 1);
+            mbar_init(&bars->pair_full[i], 1);
+            mbar_init(&bars->pair_empty[i], 1);
             mbar_init(&bars->s_ready[i], 1);
-            if (D == 64 && kMode != kCache) mbar_init(&bars->s_free[i], 128);
+            if (D == 64) mbar_init(&bars->s_free[i], 128);
             mbar_init(&bars->p_ready[i], 128);
             mbar_init(&bars->p_half[i], 128);
             mbar_init(&bars->o_ready[i], 1);
@@ -184,13 +160,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // instead of behind the P V product that consumes P, which takes a tile's two products out of the chain between two of
     // its softmax passes.  Otherwise (512 columns full at head_dim 128): S_t [128t, +128) with P written over it,
     // O_t [256+128t, +128).
-    constexpr bool kOwnP = D == 64 && kMode != kCache;
+    constexpr bool kOwnP = D == 64;
     // (computed, not looked up: a two-element array indexed by the warp's tile would live in local memory)
     auto tmem_S = [&](int t) { return tmem + (uint32_t)t * (kOwnP ? 192u : 128u); };
     constexpr uint32_t kPOff = kOwnP ? 128u : 0u;   // P relative to the S of its tile
     // head_dim 128 (plain / window): P is written over S, so a tile's P V product and next S stay in the chain between two of
     // its softmax passes; there the first half of P V is issued as soon as the first 64 columns of P are written (-6 %)
-    constexpr bool kHalfP = !kOwnP && kMode != kCache;
+    constexpr bool kHalfP = !kOwnP;
     auto tmem_O = [&](int t) { return tmem + (kOwnP ? 384u : 256u) + (uint32_t)t * (kOwnP ? 64u : 128u); };
 
     // 384 threads start with 168 registers each; each role re-allocates inside its own branch
@@ -200,27 +176,30 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         setmaxnreg_dec<72>();
         // =========================== TMA producer ===========================
         if (lane == 0) {
-            if (kMode == kCache) {      // one query tile, shared by both streams
-                if (n_loads > 0) mbar_arrive_expect_tx(&bars->q_full, (uint32_t)kTileBytes);
-                for (int c = 0; c < kChunks && n_loads > 0; ++c) tma_load_3d(sQ + c * kChunkBytes, &tmap_q, &bars->q_full, c * 64, q0, bh);
-            } else {
+            {
                 int n_valid = (n_t[0] > 0) + (n_t[1] > 0);
                 mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(n_valid * kTileBytes));
+#pragma unroll
                 for (int t = 0; t < 2; ++t)
                     if (n_t[t] > 0)
                         for (int c = 0; c < kChunks; ++c)
                             tma_load_3d(sQ + t * kTileBytes + c * kChunkBytes, &tmap_q, &bars->q_full, c * 64, q0 + t * kM, bh);
             }
-            for (int j = 0; j < n_loads; ++j) {
-                const int st = j & 1;
-                if (j >= 2 && !mbar_wait(&bars->k_empty[st], ((j >> 1) - 1) & 1, abort_flag, kSiteKEmpty)) break;
-                mbar_arrive_expect_tx(&bars->k_full[st], (uint32_t)kTileBytes);
-                for (int c = 0; c < kChunks; ++c)
-                    tma_load_3d(sK + st * kTileBytes + c * kChunkBytes, &tmap_k, &bars->k_full[st], c * 64, key_tile(j) * kN, bh_kv);
-                if (j >= 2 && !mbar_wait(&bars->v_empty[st], ((j >> 1) - 1) & 1, abort_flag, kSiteVEmpty)) break;
-                mbar_arrive_expect_tx(&bars->v_full[st], (uint32_t)kTileBytes);
-                for (int c = 0; c < kChunks; ++c)
-                    tma_load_3d(sV + st * kTileBytes + c * kChunkBytes, &tmap_v, &bars->v_full[st], c * 64, key_tile(j) * kN, bh_kv);
+            auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int j) {
+                for (int c = 0; c < kChunks; ++c) tma_load_3d(dst + (j & 1) * kTileBytes + c * kChunkBytes, map, bar, c * 64, key_tile(j) * kN, bh_kv);
+            };
+            if (n_max > 0) {
+                mbar_arrive_expect_tx(&bars->k0_full, (uint32_t)kTileBytes);
+                load(sK, &tmap_k, &bars->k0_full, 0);
+            }
+            for (int j = 0; j < n_max; ++j) {
+                // K_{j+1} and V_j go where K_{j-1} and V_{j-2} were: pair j - 2, the (j >> 1)-th release of this barrier for odd j
+                // (pair -1 was the first), the one before for even j
+                if (j >= 1 && !mbar_wait(&bars->pair_empty[j & 1], (uint32_t)((j >> 1) - (j & 1 ? 0 : 1)) & 1u, abort_flag, kSitePairEmpty)) break;
+                const bool k_too = j + 1 < n_max;
+                mbar_arrive_expect_tx(&bars->pair_full[j & 1], (uint32_t)(k_too ? 2 * kTileBytes : kTileBytes));
+                if (k_too) load(sK, &tmap_k, &bars->pair_full[j & 1], j + 1);
+                load(sV, &tmap_v, &bars->pair_full[j & 1], j);
             }
         }
     } else if (warp == 8) {
@@ -229,13 +208,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         // All 32 lanes walk the loops (warp-uniform control flow keeps descriptors and addresses in uniform registers) and
         // one elected lane issues each tcgen05 instruction: the warp shares its scheduler with two softmax warps and this
         // form needs fewer of the issue slots it is given per MMA than a single-lane loop (-3.7 % at head_dim 64, where
-        // the issue order below makes this warp's pace count; no change at 128).  The KV-cache kernel, which is bound by
-        // HBM, keeps a single lane.
-        constexpr bool kElectF = kMode != kCache;
-        if (kElectF || lane == 0) {
+        // the issue order below makes this warp's pace count; no change at 128).
+        {
             auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
-                if constexpr (kElectF) return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site));
-                else return mbar_wait(bar, parity, abort_flag, site);
+                return mbar_wait_warp(bar, parity, abort_flag, site);
             };
             const bool tl8 = lane == 0;
             (void)tl8;
@@ -247,140 +223,99 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             const uint64_t dk0 = make_sdesc(smem_u32(sK), 16, 1024), dk1 = sdesc_advance(dk0, kTileBytes);
             const uint64_t dv0 = make_sdesc(smem_u32(sV), kChunkBytes, 1024), dv1 = sdesc_advance(dv0, kTileBytes);
             auto issue_s = [&](int t, int st) {
-                uint64_t a = (t && kMode != kCache) ? dq1 : dq0, b = st ? dk1 : dk0;
-                asm volatile("" : "+l"(a), "+l"(b));   // keeps the advanced descriptors from being hoisted into registers
-                const uint32_t d = tmem_S(t);
-                mma_ss_x<kElectF, false>(d, a, b, idesc_s);
+                const uint64_t a = t ? dq1 : dq0, b = st ? dk1 : dk0;
 #pragma unroll
-                for (int ks = 1; ks < D / 16; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * kChunkBytes + (ks & 3) * 32);
-                    mma_ss_x<kElectF, true>(d, sdesc_advance(a, off), sdesc_advance(b, off), idesc_s);
-                }
-                tc_commit_x<kElectF>(&bars->s_ready[t]);
+                for (int c = 0; c < kChunks; ++c)
+                    mma_ss_4<2, 2>(tmem_S(t), sdesc_advance(a, (uint32_t)(c * kChunkBytes)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_s, c > 0);
+                tc_commit_p(&bars->s_ready[t]);
             };
             // With kHalfP, P V in two halves of the contraction: the first four k-steps need only the first 64 columns of P
             // (p_half, which the caller has waited for), the rest the whole of it (p_ready) -- so half the product is issued
             // while the softmax warps still compute the second half of their exponentials.  Otherwise the caller has waited
             // for the whole of P.  Returns false when a wait gave up.
             auto issue_pv = [&](int t, int st, bool accumulate, uint32_t parity) {
-                uint64_t b = st ? dv1 : dv0;
-                asm volatile("" : "+l"(b));
+                const uint64_t b = st ? dv1 : dv0;
                 const uint32_t d = tmem_O(t), a = tmem_S(t) + kPOff;
-                if (accumulate) mma_ts_x<kElectF, true>(d, a, b, idesc_pv);
-                else mma_ts_x<kElectF, false>(d, a, b, idesc_pv);
-#pragma unroll
-                for (int ks = 1; ks < kN / 32; ++ks) mma_ts_x<kElectF, true>(d, a + (uint32_t)(ks * 8), sdesc_advance(b, ks * 2048), idesc_pv);
+                mma_ts_4<8, 128>(d, a, b, idesc_pv, accumulate);
                 if constexpr (kHalfP) {
                     if (!wait(&bars->p_ready[t], parity, kSitePReady)) return false;
                     tc_fence_after();
                 }
-#pragma unroll
-                for (int ks = kN / 32; ks < kN / 16; ++ks) mma_ts_x<kElectF, true>(d, a + (uint32_t)(ks * 8), sdesc_advance(b, ks * 2048), idesc_pv);
-                tc_commit_x<kElectF>(&bars->o_ready[t]);
+                mma_ts_4<8, 128>(d, a + 32u, sdesc_advance(b, 4 * 2048), idesc_pv, 1);
                 return true;
             };
-            if constexpr (kMode == kCache) {
-                // two independent streams: stream t owns K/V stage t, S_t and O_t; its jj-th key tile is load 2*jj + t
-                bool ok = n_max > 0 && wait(&bars->q_full, 0, kSiteQ);
-                for (int t = 0; t < 2 && ok; ++t) {
-                    if (n_t[t] == 0) continue;
-                    if (!(ok = wait(&bars->k_full[t], 0, kSiteKFull))) break;
-                    tc_fence_after();
-                    issue_s(t, t);
-                    tc_commit_x<kElectF>(&bars->k_empty[t]);
-                }
-                for (int jj = 0; ok && jj < n_max; ++jj) {
-                    const uint32_t ph = (uint32_t)(jj & 1), nph = ph ^ 1u;
-                    for (int t = 0; t < 2 && ok; ++t) {
-                        if (jj >= n_t[t]) continue;
-                        if (!(ok = wait(&bars->v_full[t], ph, kSiteVFull))) break;
-                        if (!(ok = wait(kHalfP ? &bars->p_half[t] : &bars->p_ready[t], ph, kSitePReady))) break;
-                        tc_fence_after();
-                        if (!(ok = issue_pv(t, t, jj > 0, ph))) break;
-                        tc_commit_x<kElectF>(&bars->v_empty[t]);
-                        if (jj + 1 < n_t[t]) {
-                            if (!(ok = wait(&bars->k_full[t], nph, kSiteKFull))) break;
-                            tc_fence_after();
-                            issue_s(t, t);
-                            tc_commit_x<kElectF>(&bars->k_empty[t]);
-                        }
-                    }
-                }
-            } else if constexpr (kOwnP) {
-                // With P in columns of its own the next S of a tile no longer waits for the P V product that consumes P:
-                // per key tile j the thread first issues S_{j+1} of both query tiles, each as soon as its softmax warps have
-                // READ S_j (s_free, early in their pass), then the two P V products of step j as their P arrive.
-                bool ok = n_max > 0 && wait(&bars->q_full, 0, kSiteQ) &&
-                          wait(&bars->k_full[0], 0, kSiteKFull);
-                if (ok) {
-                    tc_fence_after();
-                    if (n_t[0] > 0) issue_s(0, 0);
-                    if (n_t[1] > 0) issue_s(1, 0);
-                    tc_commit_x<kElectF>(&bars->k_empty[0]);
-                }
-                for (int j = 0; ok && j < n_max; ++j) {
-                    const int st = j & 1, nst = st ^ 1;
-                    if (j + 1 < n_max) {
-                        if (!(ok = wait(&bars->k_full[nst], (uint32_t)(((j + 1) >> 1) & 1), kSiteKFull))) break;
-                        for (int t = 0; t < 2 && ok; ++t) {
-                            if (j + 1 >= n_t[t]) continue;
-                            if (!(ok = wait(&bars->s_free[t], (uint32_t)(j & 1), kSiteIssue))) break;
-                            tc_fence_after();
-                            issue_s(t, nst);
-                        }
-                        if (!ok) break;
-                        tc_commit_x<kElectF>(&bars->k_empty[nst]);
-                    }
-                    if (!(ok = wait(&bars->v_full[st], (uint32_t)((j >> 1) & 1), kSiteVFull))) break;
-                    for (int t = 0; t < 2 && ok; ++t) {
-                        if (j >= n_t[t]) continue;
-                        if (!(ok = wait(kHalfP ? &bars->p_half[t] : &bars->p_ready[t], (uint32_t)(j & 1), kSitePReady))) break;
-                        tc_fence_after();
-                        if (!(ok = issue_pv(t, st, j > 0, (uint32_t)(j & 1)))) break;
-                    }
-                    if (!ok) break;
-                    tc_commit_x<kElectF>(&bars->v_empty[st]);
-                }
-            } else {
-            bool ok = n_max > 0 && wait(&bars->q_full, 0, kSiteQ) &&
-                      wait(&bars->k_full[0], 0, kSiteKFull);
+            const int n0 = n_t[0], n1 = n_t[1];
+            bool ok = n_max > 0 && wait(&bars->q_full, 0, kSiteQ) && wait(&bars->k0_full, 0, kSiteK0);
             if (ok) {
                 tc_fence_after();
-                if (n_t[0] > 0) issue_s(0, 0);
-                if (n_t[1] > 0) issue_s(1, 0);
-                tc_commit_x<kElectF>(&bars->k_empty[0]);
+                issue_s(0, 0);          // (a block has rows in its first tile)
             }
-            for (int j = 0; ok && j < n_max; ++j) {
-                const int st = j & 1, nst = st ^ 1;
-                const uint32_t ph = (uint32_t)((j >> 1) & 1), nph = (uint32_t)(((j + 1) >> 1) & 1);
-                if (!(ok = wait(&bars->v_full[st], ph, kSiteVFull))) break;
-                bool next_k_ready = false;
-                for (int t = 0; t < 2 && ok; ++t) {
-                    if (j >= n_t[t]) continue;
-                    if (!(ok = wait(kHalfP ? &bars->p_half[t] : &bars->p_ready[t], (uint32_t)(j & 1), kSitePReady))) break;
-                    SNTL_TRACE_EV(tl8, 0, tn, 10 + t);
-                    tc_fence_after();
-                    if (!(ok = issue_pv(t, st, j > 0, (uint32_t)(j & 1)))) break;
-                    SNTL_TRACE_EV(tl8, 0, tn, 20 + t);
-                    if (j + 1 < n_t[t]) {
-                        if (!next_k_ready) {
-                            SNTL_TRACE_EV(tl8, 0, tn, 40);
-                            if (!(ok = wait(&bars->k_full[nst], nph, kSiteKFull))) break;
+            if constexpr (kOwnP) {
+                // With P in columns of its own the next S of a tile does not wait for the P V product that consumes P, and the two
+                // tiles are kept half a pass apart: S of tile 1 starts behind the first half of tile 0's first pass, and per key tile
+                // the order is S0_{j+1}, P1_{j-1} V, P0_j V, S1_{j+1}, which is the order in which their operands are ready then.
+                // One tile's loads, stores and hand-offs so fall into the other's exponentials.
+                const bool apart = n_max >= 4;   // short rows would pay more for the late start than they gain
+                if (ok && !apart && n1 > 0) issue_s(1, 0);
+                for (int j = 0; ok && j <= n_max; ++j) {
+                    if (j < n_max) {
+                        if (!(ok = wait(&bars->pair_full[j & 1], (uint32_t)((j >> 1) & 1), kSitePairFull))) break;
+                    }
+                    const bool late = j == 0 && apart && n1 > 0;
+                    if (j + 1 < n0 || late) {
+                        if (!(ok = wait(&bars->s_free[0], (uint32_t)(j & 1), kSiteIssue))) break;
+                        tc_fence_after();
+                        if (j + 1 < n0) issue_s(0, (j + 1) & 1);
+                        if (late) issue_s(1, 0);
+                    }
+                    if (j == 0) {
+                        tc_commit_p(&bars->pair_empty[1]);        // K_0
+                    } else {
+                        if (j - 1 < n1) {
+                            if (!(ok = wait(&bars->p_ready[1], (uint32_t)((j - 1) & 1), kSitePReady))) break;
                             tc_fence_after();
-                            SNTL_TRACE_EV(tl8, 0, tn, 41);
-                            next_k_ready = true;
+                            issue_pv(1, (j - 1) & 1, j > 1, 0);
+                            tc_commit_p(&bars->o_ready[1]);
                         }
-                        issue_s(t, nst);
-                        SNTL_TRACE_EV(tl8, 0, tn, 30 + t);
+                        tc_commit_p(&bars->pair_empty[(j - 1) & 1]);
+                    }
+                    if (j < n0) {
+                        if (!(ok = wait(&bars->p_ready[0], (uint32_t)(j & 1), kSitePReady))) break;
+                        tc_fence_after();
+                        issue_pv(0, j & 1, j > 0, 0);
+                        tc_commit_p(&bars->o_ready[0]);
+                    }
+                    if (j + 1 < n1) {
+                        if (!(ok = wait(&bars->s_free[1], (uint32_t)(j & 1), kSiteIssue))) break;
+                        tc_fence_after();
+                        issue_s(1, (j + 1) & 1);
                     }
                 }
-                if (!ok) break;
-                if (j + 1 < n_max) tc_commit_x<kElectF>(&bars->k_empty[nst]);
-                tc_commit_x<kElectF>(&bars->v_empty[st]);
-            }
+            } else {
+                // P is written over S: a tile's P V product, then its next S, as its P arrives
+                if (ok && n1 > 0) issue_s(1, 0);
+                if (ok) tc_commit_p(&bars->pair_empty[1]);        // K_0
+                for (int j = 0; ok && j < n_max; ++j) {
+                    if (!(ok = wait(&bars->pair_full[j & 1], (uint32_t)((j >> 1) & 1), kSitePairFull))) break;
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const int n = t ? n1 : n0;
+                        if (!ok || j >= n) continue;
+                        if (!(ok = wait(&bars->p_half[t], (uint32_t)(j & 1), kSitePReady))) continue;
+                        SNTL_TRACE_EV(tl8, 0, tn, 10 + t);
+                        tc_fence_after();
+                        if (!(ok = issue_pv(t, j & 1, j > 0, (uint32_t)(j & 1)))) continue;
+                        SNTL_TRACE_EV(tl8, 0, tn, 20 + t);
+                        if (j + 1 < n) issue_s(t, (j + 1) & 1);
+                        else tc_commit_p(&bars->o_ready[t]);
+                        SNTL_TRACE_EV(tl8, 0, tn, 30 + t);
+                    }
+                    if (!ok) break;
+                    tc_commit_p(&bars->pair_empty[j & 1]);
+                }
             }
             // every MMA issued above must have retired before shared memory / TMEM are given up
-            tc_commit_x<kElectF>(&bars->final_bar);
+            tc_commit_p(&bars->final_bar);
             wait(&bars->final_bar, 0, kSiteFinal);
         }
     } else {
@@ -389,70 +324,58 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const int t = warp >> 2;                       // tile 0 or 1
         const int row = (warp & 3) * 32 + lane;        // row inside the tile == TMEM lane
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-        const int grow = kMode == kCache ? q0 + row : q0 + t * kM + row;   // query row inside the (batch, head) slab
-        const int n_mine = n_t[t];
+        const int grow = q0 + t * kM + row;   // query row inside the (batch, head) slab
+        const int n_mine = t ? n_t[1] : n_t[0];        // (an index would put the array in local memory)
         SNTL_TRACE_DECL(tn);
         const bool tw = (warp & 3) == 0 && lane == 0;
         (void)tw;
         float m_ref = -INFINITY, l = 0.0f;
         bool ok = true;
+        // Barrier tests queue behind the exponentials in the same unit and take 200-400 cycles here; where a result is likely to be
+        // there already it is asked for ahead of its use, with other work in between.
+        bool s_seen = false;
+        const int row_lo = q0 + t * kM + (warp & 3) * 32;      // first row of the warp
         for (int j = 0; j < n_mine; ++j) {
-            if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_ready[t], (uint32_t)(j & 1), abort_flag, kSiteSReady)))) break;
+            if (!(ok = __all_sync(0xffffffffu, s_seen || mbar_wait(&bars->s_ready[t], (uint32_t)(j & 1), abort_flag, kSiteSReady)))) break;
             SNTL_TRACE_EV(tw, 1 + t, tn, 1);
             tc_fence_after();
             uint32_t s[128];
 #pragma unroll
             for (int c = 0; c < 4; ++c) tmem_ld32(tmem_S(t) + lane_off + (uint32_t)(c * 32), s + c * 32);
             tmem_ld_wait();
-            if constexpr (kOwnP) {      // S_j is in registers: the next S of this tile may overwrite it
-                tc_fence_before();
-                mbar_arrive(&bars->s_free[t]);
-            }
             SNTL_TRACE_EV(tw, 1 + t, tn, 2);
             // number of visible keys of this row inside this tile
-            const int key0 = key_tile(kMode == kCache ? 2 * j + t : j) * kN;
-            const int qpos = row_pos(grow);
-            int limit = (p.causal ? min(p.Skv, qpos + 1) : p.Skv) - key0;
-            if (limit < kN) {
-#pragma unroll
-                for (int c = 0; c < kN; ++c)
-                    if (c >= limit) s[c] = 0xff800000u;  // -inf
-            }
-            if (kWin && (kMode != kCache || p.window > 0)) {
-                // keys below the row's window are hidden unless they are global tokens
-                const int lo = qpos - p.window + 1 - key0, glim = p.global_tokens - key0;
-                if (lo > 0 && glim < min(lo, kN)) {
-#pragma unroll
-                    for (int c = 0; c < kN; ++c)
-                        if (c < lo && c >= glim) s[c] = 0xff800000u;
+            const int key0 = key_tile(j) * kN;
+            int limit = (p.causal ? min(p.Skv, grow + 1) : p.Skv) - key0;
+            const int lo = kWin ? grow - p.window + 1 - key0 : 0, glim = kWin ? p.global_tokens - key0 : 0;
+            const bool below = kWin && lo > 0 && glim < min(lo, kN);   // keys below the window that are no global tokens
+            // Once a row has a reference maximum, a tile that the mask does not cut is exponentiated against it at once, with the
+            // tile's own maximum taken on the way: only if some row of the warp then needs a rescale (its maximum grew by more
+            // than 2^8, which the lazy rule below leaves rare) is the first half done again.  The maximum and the decision were
+            // a quarter of a tile's time in front of the exponentials.
+            const int limit_lo = (p.causal ? min(p.Skv, row_lo + 1) : p.Skv) - key0, lo_hi = row_lo + 31 - p.window + 1 - key0;
+            const bool ahead = (kOwnP || kMode == kPlain) && j > 0 && limit_lo >= kN && !(kWin && lo_hi > 0 && glim < min(lo_hi, kN));   // (no row of the warp is cut)
+            uint32_t pk[32];
+            float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+            RowMax mx;
+            float neg_m = -m_ref;
+            // whether some row of the warp has outgrown its reference (false when both are -inf: NaN compare)
+            auto outgrown = [&](float m_new) { return j > 0 && __any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold); };
+            auto s_read = [&]() {       // nothing reads S_j any more: the next S of this tile may overwrite it
+                if constexpr (kOwnP) {
+                    tc_fence_before();
+                    mbar_arrive(&bars->s_free[t]);
                 }
-            }
-            // row max with eight independent chains (a single 128-long dependent chain costs ~600 cycles) of
-            // three-input maxima: half the instructions of a two-input reduction
-            float mx8[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) mx8[c] = __uint_as_float(s[c]);
-#pragma unroll
-            for (int c = 8; c + 16 <= kN; c += 16)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) mx8[i] = fmax3(mx8[i], __uint_as_float(s[c + i]), __uint_as_float(s[c + 8 + i]));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(mx8[i], __uint_as_float(s[kN - 8 + i]));
-            const float mx = fmax3(fmax3(mx8[0], mx8[1], mx8[2]), fmax3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]));
-            const float m_new = fmaxf(m_ref, mx * p.scale_log2);
-            SNTL_TRACE_EV(tw, 1 + t, tn, 3);
-            const bool need = (m_new - m_ref) > kRescaleThreshold;   // false when both are -inf (NaN compare)
-            if constexpr (kOwnP) {      // P_{j-1} has been consumed (and O holds its product): P_j may be written
-                if (j > 0) {
-                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_ready[t], (uint32_t)((j - 1) & 1), abort_flag, kSiteOReady)))) break;
+            };
+            bool o_seen = false;
+            auto o_done = [&]() {       // P_{j-1} has been consumed and O holds its product (head_dim 128: S_j was issued behind it)
+                if constexpr (kOwnP) {
+                    ok = __all_sync(0xffffffffu, o_seen || mbar_wait(&bars->o_ready[t], (uint32_t)((j - 1) & 1), abort_flag, kSiteOReady));
                     tc_fence_after();
                 }
-            }
-            if (j == 0) {
-                m_ref = m_new;
-            } else if (__any_sync(0xffffffffu, need)) {
-                if (!kOwnP && !(ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_ready[t], (uint32_t)((j - 1) & 1), abort_flag, kSiteOReady)))) break;
-                tc_fence_after();
+            };
+            auto rescale = [&](float m_new) {
+                const bool need = (m_new - m_ref) > kRescaleThreshold;
                 const float factor = need ? ex2(m_ref - m_new) : 1.0f;
                 if (need) m_ref = m_new;
                 l *= factor;
@@ -466,44 +389,68 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     tmem_st32(tmem_O(t) + lane_off + (uint32_t)(c * 32), o);
                 }
                 tmem_st_wait();
-            }
-            SNTL_TRACE_EV(tw, 1 + t, tn, 4);
-            const float neg_m = (m_ref == -INFINITY) ? 0.0f : -m_ref;
-            // exp2, row sum (four independent partial sums) and bf16 packing, 64 columns at a time so the packed half
-            // can be stored while the other half is computed
-            float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(neg_m, neg_m);
+                neg_m = -m_ref;
+            };
+            if (ahead) {
+                exp_half<0, true>(s, p.scale_log2, neg_m, pk, sum, mx);
+                SNTL_TRACE_EV(tw, 1 + t, tn, 3);
+                if (kOwnP) o_seen = mbar_try_wait(&bars->o_ready[t], (uint32_t)((j - 1) & 1));
+                const float m_new = fmaxf(m_ref, mx.value() * p.scale_log2);
+                const bool again = outgrown(m_new);
+                if (!again) s_read();
+                o_done();
+                if (!ok) break;
+                if (again) {            // (S is read again: kept, it would take 64 registers more than there are)
+                    rescale(m_new);
+                    sum[0] = sum[1] = make_float2(0.0f, 0.0f);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t pk[32];
+                    for (int c = 0; c < 2; ++c) tmem_ld32(tmem_S(t) + lane_off + (uint32_t)(c * 32), s + c * 32);
+                    tmem_ld_wait();
+                    s_read();
+                    exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
+                }
+            } else {
+                s_read();
+                if (limit < kN) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const float2 x = ffma2(make_float2(__uint_as_float(s[h * 64 + 2 * c]), __uint_as_float(s[h * 64 + 2 * c + 1])), sc2, nm2);
-                    const float p0 = ex2(x.x), p1 = ex2(x.y);
-                    l4[c & 3] += p0 + p1;
-                    pk[c] = pack_bf16(p0, p1);
+                    for (int c = 0; c < kN; ++c)
+                        if (c >= limit) s[c] = 0xff800000u;  // -inf
                 }
-                tmem_st32(tmem_S(t) + kPOff + lane_off + (uint32_t)(h * 32), pk);
-                if (kHalfP && h == 0) {   // the P V product may start on the first 64 keys while the rest is computed
-                    tmem_st_wait();
-                    tc_fence_before();
-                    mbar_arrive(&bars->p_half[t]);
+                if (below) {
+#pragma unroll
+                    for (int c = 0; c < kN; ++c)
+                        if (c < lo && c >= glim) s[c] = 0xff800000u;
                 }
+                const float m_new = fmaxf(m_ref, row_max(s) * p.scale_log2);
+                const bool again = outgrown(m_new);
+                if (j > 0) o_done();
+                if (!ok) break;
+                if (j == 0) m_ref = m_new;
+                else if (again) rescale(m_new);
+                neg_m = (m_ref == -INFINITY) ? 0.0f : -m_ref;
+                SNTL_TRACE_EV(tw, 1 + t, tn, 4);
+                exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
             }
-            l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+            tmem_st32(tmem_S(t) + kPOff + lane_off, pk);
+            if (kHalfP) {   // the P V product may start on the first 64 keys while the rest is computed
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(&bars->p_half[t]);
+            }
+            exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, mx);
+            if (kOwnP) s_seen = j + 1 < n_mine && mbar_try_wait(&bars->s_ready[t], (uint32_t)((j + 1) & 1));
+            tmem_st32(tmem_S(t) + kPOff + lane_off + 32u, pk);
+            l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             SNTL_TRACE_EV(tw, 1 + t, tn, 5);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&bars->p_ready[t]);
             SNTL_TRACE_EV(tw, 1 + t, tn, 6);
         }
-        if (__all_sync(0xffffffffu, ok && n_mine > 0 && mbar_wait(&bars->o_ready[t], (uint32_t)((n_mine - 1) & 1), abort_flag, kSiteOReady))) {
+        if (__all_sync(0xffffffffu, ok && n_mine > 0 && mbar_wait(&bars->o_ready[t], (uint32_t)(kOwnP ? (n_mine - 1) & 1 : 0), abort_flag, kSiteOReady))) {
             tc_fence_after();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             const bool store = grow < p.Sq;
-            // cache mode: each stream of each split writes its own partial result, [2 * split + t][slab][row]
-            const size_t part = kMode == kCache ? (size_t)(2 * split + t) : 0;
-            const size_t out_row = (part * bh_count + bh) * p.Sq + (size_t)(store ? grow : 0);
             // Coalesced store of O.  A thread holds one whole row (2*D bytes); written straight from there a warp's store
             // instruction would touch 32 rows, 16 bytes each.  So the warp's 32 rows go through shared memory -- this tile's
             // Q buffer, free since the last S product of this tile retired (o_ready of the last step implies it) -- and
@@ -511,12 +458,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             // rows: 16 lanes x 16 bytes = one 256-byte row at head_dim 128, 8 lanes per 128-byte row at 64.  Only the rows of
             // this warp are exchanged, so a warp-level sync is all it takes; 16-byte units are XOR-swizzled by the row so
             // that both the row-wise writes and the row-wise reads spread over the banks.
-            // (Cache mode: the two streams share ONE query tile, which the other stream may still be reading, but each owns
-            // K stage t, and that stage gets no further load once the stream's last tile is done.)
             constexpr int kUnits = D / 8;                       // 16-byte units per row
             if constexpr (kMat) {
                 // feature-major matrices: the 32 rows of a warp are 128 contiguous bytes of every feature's row
-                const int b = bh / p.Hq, h = bh - b * p.Hq;
                 float* dst = p.o_mat + (long long)h * D * p.mat_stride + (long long)b * p.Sq + grow;
 #pragma unroll
                 for (int c = 0; c < D / 32; ++c) {
@@ -531,7 +475,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if (store)
                     p.lse_mat[(long long)h * p.mat_stride + (long long)b * p.Sq + grow] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
             } else {
-            uint8_t* stage = (kMode == kCache ? sK : sQ) + t * kTileBytes + (warp & 3) * 32 * (D * 2);
+            uint8_t* stage = sQ + t * kTileBytes + (warp & 3) * 32 * (D * 2);
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
                 uint32_t o[32];
@@ -553,7 +497,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 constexpr int kRowsPerStore = 32 / kUnits;       // rows one store instruction of the warp covers
                 const int sub = lane / kUnits, unit = lane % kUnits;
                 const int warp_row0 = grow - lane;                // first row of this warp inside the slab
-                const size_t part_base = (part * bh_count + bh) * (size_t)p.Sq;
+                const size_t part_base = (size_t)bh * p.Sq;
 #pragma unroll
                 for (int i = 0; i < 32 / kRowsPerStore; ++i) {
                     const int r = i * kRowsPerStore + sub;        // row inside the warp's 32
@@ -563,11 +507,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 }
             }
             if (store)
-                p.lse[out_row] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
+                p.lse[(size_t)bh * p.Sq + grow] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
             }
-        } else if (kMode == kCache && ok && n_mine == 0 && grow < p.Sq) {
-            // a stream that got no key tile (a piece of one tile): its partial result weighs nothing in the merge
-            p.lse[((size_t)(2 * split + t) * bh_count + bh) * p.Sq + grow] = -INFINITY;
         }
     }
 

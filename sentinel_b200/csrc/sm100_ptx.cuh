@@ -134,12 +134,6 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem_sr
                  "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-// fire-and-forget fp32 vector reduction into global memory (16-byte aligned)
-__device__ __forceinline__ void red_add_v4(float* gptr, float a, float b, float c, float d)
-{
-    asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(gptr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // asynchronous fp32 add-reduction of a contiguous shared-memory block into global memory (both 16-byte aligned,
 // bytes a multiple of 16); tracked by bulk groups
 __device__ __forceinline__ void bulk_reduce_add_f32(float* gmem_dst, const void* smem_src, uint32_t bytes)
@@ -215,12 +209,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)  //
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// mbarrier arrives once every MMA issued so far by this thread has completed
-__device__ __forceinline__ void tc_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // ---------------------------------------------------------------------------------------------------
 // UMMA descriptors (bf16 operands, fp32 accumulate)
 // ---------------------------------------------------------------------------------------------------
@@ -251,100 +239,72 @@ __device__ __forceinline__ uint64_t make_sdesc(uint32_t smem_addr, uint32_t lbo_
     return d;
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]; A holds bf16 pairs packed in 32-bit TMEM columns (K/2 columns per row)
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// Lean issue forms.  The single issuing thread shares its scheduler with busy softmax warps, so every instruction
-// it spends per MMA shows up as tensor-pipe idle time: descriptors are built once per tile and advanced with one
-// 64-bit add (the start-address field is in 16-byte units and never carries out of its 14 bits for addresses below
-// 256 KB), and the accumulate flag is a compile-time constant wherever the k-step is known.
+// Descriptors are built once per tile and advanced with one 64-bit add (the start-address field is in 16-byte units and never
+// carries out of its 14 bits for addresses below 256 KB).
 __device__ __forceinline__ uint64_t sdesc_advance(uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); }
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ss_c(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
-{
-    if (kAccumulate)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                     "l"(a_desc), "l"(b_desc), "r"(idesc)
-                     : "memory");
-    else
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                     "l"(a_desc), "l"(b_desc), "r"(idesc)
-                     : "memory");
-}
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
-{
-    if (kAccumulate)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-                     "r"(a_tmem), "l"(b_desc), "r"(idesc)
-                     : "memory");
-    else
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-                     "r"(a_tmem), "l"(b_desc), "r"(idesc)
-                     : "memory");
-}
 
-// One lane of a fully active warp (always the same one): lets an MMA-issuing warp run its loop with all 32 lanes --
-// warp-uniform control flow, so descriptors and addresses can live in uniform registers -- with only the tcgen05
-// instruction itself behind the election.
-__device__ __forceinline__ bool elect_one()
+// D[tmem] (+)= A * B with A and B in shared memory (ss), or with A as bf16 pairs packed in 32-bit TMEM columns (ts).
+// Four k-steps of a product, issued by the elected lane of a fully active warp: one election for all of them and nothing but
+// predicated instructions in between.  Step i reads A at +i * kA and B at +i * kB (descriptor units of 16 bytes; for the form
+// with A in TMEM, kA counts columns); `first` = whether step 0 accumulates.  The issuing warp shares its scheduler with
+// ALU-dense warps, so its instruction count is tensor-pipe idle time: with an election and a branch around every single MMA it
+// needed 90 cycles for each, and the forward ran at the pace of this one warp at both head sizes.
+template <int kA, int kB>
+__device__ __forceinline__ void mma_ss_4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t first)
 {
-    uint32_t pred = 0;
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred != 0;
+        "{\n\t.reg .pred e, f, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.u32 f, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+        "add.u64 a1, %1, %5;\n\tadd.u64 b1, %2, %8;\n\t"
+        "add.u64 a2, %1, %6;\n\tadd.u64 b2, %2, %9;\n\t"
+        "add.u64 a3, %1, %7;\n\tadd.u64 b3, %2, %10;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, f;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(first), "n"(kA), "n"(2 * kA), "n"(3 * kA), "n"(kB), "n"(2 * kB), "n"(3 * kB)
+        : "memory");
 }
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ss_e(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+template <int kA, int kB>
+__device__ __forceinline__ void mma_ts_4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t first)
 {
-    if (elect_one()) mma_ss_c<kAccumulate>(d_tmem, a_desc, b_desc, idesc);
+    asm volatile(
+        "{\n\t.reg .pred e, f, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.u32 f, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+        "add.u32 a1, %1, %5;\n\tadd.u64 b1, %2, %8;\n\t"
+        "add.u32 a2, %1, %6;\n\tadd.u64 b2, %2, %9;\n\t"
+        "add.u32 a3, %1, %7;\n\tadd.u64 b3, %2, %10;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, f;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(first), "n"(kA), "n"(2 * kA), "n"(3 * kA), "n"(kB), "n"(2 * kB), "n"(3 * kB)
+        : "memory");
 }
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ts_e(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
+// one accumulating step, likewise
+__device__ __forceinline__ void mma_ss_1(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
 {
-    if (elect_one()) mma_ts_c<kAccumulate>(d_tmem, a_tmem, b_desc, idesc);
+    asm volatile(
+        "{\n\t.reg .pred e, t;\n\telect.sync _|e, 0xffffffff;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, t;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc)
+        : "memory");
 }
-__device__ __forceinline__ void tc_commit_e(uint64_t* bar)
+// mbarrier arrives once every MMA issued so far by this warp's elected lane (always the same one) has completed
+__device__ __forceinline__ void tc_commit_p(uint64_t* bar)
 {
-    if (elect_one()) tc_commit(bar);
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
 }
-// either form, chosen at compile time: kElect = a fully active warp with an elected lane, else the calling thread itself
-template <bool kElect, bool kAccumulate>
-__device__ __forceinline__ void mma_ss_x(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+// mbar_wait for a fully active warp: the usual case is one instruction and a vote, with warp-uniform control flow
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t site)
 {
-    if constexpr (kElect) mma_ss_e<kAccumulate>(d_tmem, a_desc, b_desc, idesc);
-    else mma_ss_c<kAccumulate>(d_tmem, a_desc, b_desc, idesc);
-}
-template <bool kElect, bool kAccumulate>
-__device__ __forceinline__ void mma_ts_x(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
-{
-    if constexpr (kElect) mma_ts_e<kAccumulate>(d_tmem, a_tmem, b_desc, idesc);
-    else mma_ts_c<kAccumulate>(d_tmem, a_tmem, b_desc, idesc);
-}
-template <bool kElect>
-__device__ __forceinline__ void tc_commit_x(uint64_t* bar)
-{
-    if constexpr (kElect) tc_commit_e(bar);
-    else tc_commit(bar);
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site));
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -34,16 +34,17 @@
 // huge LSE so they produce P = 0) and zeroes the dQ accumulator; a post-pass converts the accumulator to bf16 dQ (times
 // scale).
 //
-// Long key tiles.  The CTA of key tile 0 visits every query tile of every head of its group; when the grid is small
-// (few batch elements x KV heads, as in the chunks of the host-buffer pipeline) or a sliding window leaves only the
-// global-token tiles long, that one CTA outlasts the average SM's whole load and bounds the kernel.  Such tiles are
-// cut by query head: one CTA per (key tile, KV head, query head of the group), each leaving its dK/dV as an fp32
-// partial in scratch, and a small kernel adds the partials in head order (deterministic) and writes bf16.
+// Long key tiles are cut into pieces (BwdCut): one CTA per (key tile, KV head, piece), each leaving its dK/dV as an fp32
+// partial in scratch, and a small kernel adds the partials in piece order (deterministic) and writes the result.
 // TMEM map (512 columns): S^T/P^T [0,128)  dP^T/dQ [128,256)  then dV [256,384) dK [384,512) at head_dim 128, and
 // dV [256,320) dK [320,384) plus a second S^T/P^T buffer [384,512) at head_dim 64.
 #include "common.cuh"
 #include "row_terms.cuh"
 #include "sm100_ptx.cuh"
+
+#include <string.h>
+
+#include <algorithm>
 
 namespace sntl {
 
@@ -73,8 +74,9 @@ struct BwdParams {
     int causal;
     int window, global_tokens;   // sliding window and always-visible first keys (0, 0: plain causal)
     int n_qt, n_kt;
-    int split_tiles;       // the first split_tiles key tiles are cut into one CTA per query head of the group
-    float* dkv_part;       // [split tile][slab][head of group][dV, dK][128][D] fp32
+    int split_tiles;       // the first split_tiles key tiles are cut into pieces (see BwdCut) of about split_steps steps,
+    int split_steps, split_pieces, whole_first;   // at most split_pieces of a tile
+    float* dkv_part;       // [split tile][slab][piece][dV, dK][128][D] fp32
     float *dk_acc, *dv_acc;   // non-null: dK*scale / dV are ADDED into these fp32 [B*Hkv][Skv][D] tensors (no bf16 store)
     // non-null: dK / dV leave as fp32 feature-major matrices (see MatrixOut)
     float *dk_mat, *dv_mat;
@@ -91,19 +93,109 @@ __host__ __device__ inline int bwd_tiles_per_head(int kt, int n_qt, int causal, 
     return max(0, qt_last - qt_first + 1);
 }
 
-// How many leading key tiles to cut by query head: those whose CTA would run longer than the average load of an SM.
-inline int bwd_split_tiles(const AttnShape& s)
+// A key tile's CTA visits `steps` (head of the group, query tile) pairs in order; a cut tile deals them to pieces of equal
+// length, one CTA each.
+__host__ __device__ inline int bwd_piece_count(int steps, int split_steps) { return (steps + split_steps - 1) / split_steps; }
+
+// Which key tiles to cut, and how fine.  The CTA of key tile 0 visits every query tile of every head of its group; on a small
+// grid (few sequences x KV heads, one layer's strong-scaling share, short batches) or where a window leaves only the tiles with
+// global tokens long, that one CTA outlasts the average SM's whole load.  Cutting balances the grid and costs each piece its
+// set-up and an fp32 partial of dK and dV: about two steps for a CTA, one more for a piece.  The estimate below weighs the
+// two for a few piece lengths.  B3 Hq16 Hkv4 S1237 D128 with reproducible dQ: 120 CTAs of up to 40 steps on 148 SMs took
+// 158 us, 108 us cut.
+struct BwdCut {
+    int tiles = 0, steps = 1, pieces = 0;
+    bool whole_first = false;      // some whole tile is longer than the pieces
+};
+inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+size_t bwd_base_bytes(const AttnShape& s)      // without the partials
 {
-    const int group = s.Hq / s.Hkv;
-    if (group <= 1 || s.deterministic) return 0;   // (the order-independent dQ form is not instantiated with cut tiles)
+    const size_t sq_pad = ((size_t)s.Sq + kT - 1) / kT * kT, rows = (size_t)s.B * s.Hq * sq_pad;
+    return align256(kBwdRowAuxBytes * rows) + align256((s.deterministic ? 8 : 4) * rows * (size_t)s.D);
+}
+size_t bwd_part_bytes(const AttnShape& s, const BwdCut& c) { return (size_t)c.tiles * c.pieces * s.B * s.Hkv * 2 * kT * (size_t)s.D * 4; }
+
+BwdCut bwd_cut_uncached(const AttnShape& s)
+{
+    const int group = s.Hq / s.Hkv, slabs = s.B * s.Hkv, sms = sm_count(), window = s.causal ? s.window : 0;
     const int n_qt = (s.Sq + kT - 1) / kT, n_kt = (s.Skv + kT - 1) / kT;
-    const int window = s.causal ? s.window : 0;
+    auto steps = [&](int kt) { return bwd_tiles_per_head(kt, n_qt, s.causal, window, s.global_tokens) * group; };
+    constexpr double kCta = 2.0, kPiece = 5.0;       // overhead in steps
+    const int longest = steps(0);
     double total = 0.0;
-    for (int kt = 0; kt < n_kt; ++kt) total += bwd_tiles_per_head(kt, n_qt, s.causal, window, s.global_tokens);
-    const double avg = total * group * s.B * s.Hkv / sm_count();
+    for (int kt = 0; kt < n_kt; ++kt) total += steps(kt);
+    BwdCut cut;
+    if (s.whole_tiles) return cut;
+    if (s.deterministic) {
+        // dK and dV must not depend on how a caller cuts the batch (their partials are summed in another order than whole tiles):
+        // the rule looks at the tile alone.  At most four pieces of 24 steps or so cost a large grid little.
+        if (longest < 24) return cut;
+        cut.steps = (longest + 1) / std::max(2, std::min(4, longest / 32));
+        cut.pieces = bwd_piece_count(longest, cut.steps);
+        while (cut.tiles < n_kt && steps(cut.tiles) * 4 > cut.steps * 5) ++cut.tiles;
+        cut.whole_first = cut.tiles < n_kt && steps(cut.tiles) > cut.steps;
+        return cut;
+    }
+    if (total * slabs / sms > 3.0 * longest) return cut;       // balanced by its many CTAs
+    // Time of a cut in steps: the longest CTA, or the SMs' average load and a tail (short: the longest CTAs go first), or the
+    // whole waves that the CTAs of about the longest kind need.
+    auto estimate = [&](BwdCut& c) {
+        double work = 0.0, last = 0.0, long_sum = 0.0, long_n = 0.0;
+        c.tiles = 0;
+        auto visit = [&](auto&& f) {
+            bool cutting = c.steps > 0;
+            for (int kt = 0; kt < n_kt; ++kt) {
+                const int n = steps(kt);
+                cutting = cutting && n * 4 > c.steps * 5;
+                const int pieces = cutting ? bwd_piece_count(n, c.steps) : 1;
+                f(cutting, (n + pieces - 1) / pieces + (cutting ? kPiece : kCta), pieces);
+            }
+        };
+        double piece_longest = 0.0;
+        visit([&](bool cutting, double len, int pieces) {
+            work += len * pieces;
+            last = std::max(last, len);
+            c.tiles += cutting;
+            if (cutting) piece_longest = std::max(piece_longest, len);
+        });
+        visit([&](bool, double len, int pieces) {
+            if (len >= 0.75 * last) { long_sum += len * pieces; long_n += pieces; }
+        });
+        c.whole_first = c.tiles < n_kt && steps(c.tiles) + kCta > piece_longest;
+        const double waves = (double)(((long long)long_n * slabs + sms - 1) / sms);
+        return std::max({last, work * slabs / sms + 0.25 * last, waves * long_sum / long_n});
+    };
+    BwdCut none;
+    none.steps = 0;
+    BwdCut tried[17];
+    double time[17], best = 0.9 * estimate(none);              // cut for a clear gain only
     int n = 0;
-    while (n < n_kt && (double)bwd_tiles_per_head(n, n_qt, s.causal, window, s.global_tokens) * group > avg) ++n;
-    return n;
+    for (int k = 2; k <= 16; ++k) {
+        BwdCut c;
+        c.steps = (longest + k - 1) / k;
+        if (c.steps < 3) break;
+        c.pieces = bwd_piece_count(longest, c.steps);
+        time[n] = estimate(c);
+        best = std::min(best, time[n]);
+        tried[n++] = c;
+    }
+    for (int i = 0; i < n; ++i)                                // the coarsest of those that are about as good
+        if (time[i] <= 1.03 * best) return tried[i];
+    return cut;
+}
+
+// (asked for several times per call)
+BwdCut bwd_cut(const AttnShape& s)
+{
+    struct Key { int B, Hq, Hkv, Sq, Skv, D, causal, window, global_tokens, deterministic, whole_tiles, sms; };
+    static thread_local Key last{};
+    static thread_local BwdCut cut;
+    const Key key{s.B, s.Hq, s.Hkv, s.Sq, s.Skv, s.D, s.causal, s.window, s.global_tokens, s.deterministic, s.whole_tiles, sm_count()};
+    if (memcmp(&key, &last, sizeof key) != 0) {
+        cut = bwd_cut_uncached(s);
+        last = key;
+    }
+    return cut;
 }
 
 struct BwdBarriers {
@@ -189,11 +281,11 @@ __device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile
 // through `stage_base` (a shared-memory tile no product reads any more).
 template <int D, bool kMat>
 __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool split, int n_iter, int wg, int warp, int lane, int row,
-                                          uint32_t src, int kt, int slab, int slabs, int group, int g0, int k0, uint8_t* stage_base)
+                                          uint32_t src, int kt, int slab, int slabs, int piece, int k0, uint8_t* stage_base)
 {
     if (split) {
         // this CTA's share of dV (warpgroup 0) / dK (warpgroup 1) as an fp32 partial; zeros if it saw no query
-        float* dst = p.dkv_part + ((((size_t)kt * slabs + slab) * group + g0) * 2 + wg) * (size_t)(kT * D) + (size_t)row * D;
+        float* dst = p.dkv_part + ((((size_t)kt * slabs + slab) * p.split_pieces + piece) * 2 + wg) * (size_t)(kT * D) + (size_t)row * D;
         if (ok) tc_fence_after();
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -374,21 +466,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // ---- work decode: key tile 0 sees every query tile, so low key tiles go first ----
     const int slabs = p.B * p.Hkv;
     const int group = p.Hq / p.Hkv;
-    // the first split_tiles key tiles come as one CTA per (tile, head of the group, slab), the rest as one per (tile, slab)
-    const int n_split_ctas = kSplit ? p.split_tiles * group * slabs : 0;
-    int kt, slab, g0 = 0, n_heads = group;
-    const bool split = kSplit && (int)blockIdx.x < n_split_ctas;
-    if (split) {
-        kt = blockIdx.x / (group * slabs);
-        const int rem = blockIdx.x - kt * group * slabs;
-        g0 = rem / slabs;
-        slab = rem - g0 * slabs;
-        n_heads = 1;
-    } else {
-        const int idx = blockIdx.x - n_split_ctas;
-        kt = p.split_tiles + idx / slabs;
-        slab = idx - (idx / slabs) * slabs;             // b * Hkv + hk
-    }
+    // whole tiles as one CTA per (tile, slab), cut ones as one per (tile, piece, slab); the kind with the longest CTAs first
+    const int n_whole = (p.n_kt - p.split_tiles) * slabs, n_pieces = kSplit ? p.split_tiles * p.split_pieces * slabs : 0;
+    const bool split = kSplit && (p.whole_first ? (int)blockIdx.x >= n_whole : (int)blockIdx.x < n_pieces);
+    const int idx = (int)blockIdx.x - (!kSplit ? 0 : p.whole_first ? (split ? n_whole : 0) : (split ? 0 : n_pieces)), rest = idx / slabs;
+    const int slab = idx - rest * slabs;                // b * Hkv + hk
+    const int kt = split ? rest / p.split_pieces : p.split_tiles + rest, piece = split ? rest - kt * p.split_pieces : 0;
     const int b = slab / p.Hkv, hk = slab - b * p.Hkv;
     const int k0 = kt * kT;
     const int qt_first = p.causal ? kt : 0;
@@ -396,7 +479,15 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // global tokens, which every later query sees
     const int qt_last = (kWin && k0 >= p.global_tokens) ? min(p.n_qt - 1, (k0 + kT - 1 + p.window - 1) / kT) : p.n_qt - 1;
     const int per_head = qt_last - qt_first + 1;        // query tiles per head this CTA visits
-    const int n_iter = per_head > 0 ? per_head * n_heads : 0;
+    int n_iter = per_head > 0 ? per_head * group : 0;   // steps of this CTA: all of the tile's, or its piece of them from step i0 on
+    int i0 = 0;
+    if (split) {
+        const int pieces = bwd_piece_count(n_iter, p.split_steps), len = (n_iter + pieces - 1) / pieces;
+        i0 = piece * len;
+        n_iter = min(len, n_iter - i0);
+        if (piece >= pieces || n_iter <= 0) return;     // (uniform over the CTA, before anything is set up)
+    }
+    const int g_first = per_head > 0 ? i0 / per_head : 0, r_first = i0 - g_first * per_head;   // head and query tile of the first step
 
     if (warp == 13 && lane == 0) {
         prefetch_tensormap(&tmap_q);
@@ -456,9 +547,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 tma_load_3d(sK + c * kChunkBytes, &tmap_k, &bars->kv_full, c * 64, k0, slab);
                 tma_load_3d(sV + c * kChunkBytes, &tmap_v, &bars->kv_full, c * 64, k0, slab);
             }
+            int g = g_first, r = r_first;
             for (int i = 0; i < n_iter; ++i) {
-                const int g = i / per_head, qt = qt_first + (i - g * per_head);
-                const int bh = b * p.Hq + hk * group + g0 + g;
+                const int qt = qt_first + r, bh = b * p.Hq + hk * group + g;
+                if (++r == per_head) { r = 0; ++g; }
                 const int sq = i % kQStages;
                 if (i >= kQStages && !mbar_wait(&bars->q_empty[sq], (uint32_t)(((i / kQStages) - 1) & 1), abort_flag, kSiteQEmpty)) break;
                 mbar_arrive_expect_tx(&bars->q_full[sq], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 2 * kT * 4)));
@@ -637,9 +729,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const bool elected = warp == 8 && lane == 0;
         bool ok = true;
         uint32_t piece = 0;
+        int g = g_first, tile_r = r_first;
         for (int i = 0; i < n_iter; ++i) {
-            const int g = i / per_head, qt = qt_first + (i - g * per_head);
-            const int bh = b * p.Hq + hk * group + g0 + g;
+            const int qt = qt_first + tile_r, bh = b * p.Hq + hk * group + g;
+            if (++tile_r == per_head) { tile_r = 0; ++g; }
             // fp32 accumulator: kT*D words per tile; fixed-point accumulator: kT*D 64-bit words per tile
             float* tile = p.dq_accum + ((size_t)bh * p.n_qt + qt) * (size_t)(kT * D) * (kDet ? 2 : 1);
             ok = __all_sync(0xffffffffu, mbar_wait(&bars->dq_ready, (uint32_t)(i & 1), abort_flag, kSiteDQ));
@@ -677,8 +770,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const uint32_t col0 = (uint32_t)(wg * 64);
         uint8_t* ds_row0 = sDs + wg * kChunkBytes + row * 128;   // this thread's 128-byte row of its 64-query chunk
         bool ok = true;
+        int tile_r = r_first;
         for (int i = 0; i < n_iter; ++i) {
-            const int qt = qt_first + (i % per_head);
+            const int qt = qt_first + tile_r;
+            if (++tile_r == per_head) tile_r = 0;
             const uint32_t ph = (uint32_t)(i & 1);
             // ---- P^T ----
             const uint32_t tm_Si = tm_S + (uint32_t)(i % kSBufs) * kSBufStride;
@@ -789,7 +884,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         // ---- epilogue: dV (warpgroup 0) and dK (warpgroup 1) ----
         ok = __all_sync(0xffffffffu, ok && n_iter > 0 && mbar_wait(&bars->final_bar, 0, abort_flag, kSiteFinal));
-        write_dkv<D, kMat>(p, ok, split, n_iter, wg, warp, lane, row, (wg == 0 ? tm_dV : tm_dK) + lane_off, kt, slab, slabs, group, g0, k0,
+        write_dkv<D, kMat>(p, ok, split, n_iter, wg, warp, lane, row, (wg == 0 ? tm_dV : tm_dK) + lane_off, kt, slab, slabs, piece, k0,
                      wg == 0 ? sV : sK);
     }
 
@@ -912,13 +1007,18 @@ __global__ void __launch_bounds__(256) bwd_post_det_kernel(const unsigned long l
     }
 }
 
-inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// dV / dK of the key tiles that were cut by query head: the partials of a tile are added in head order and written as
+// How many partials each cut key tile has.
+struct BwdPieces {
+    int n_qt, causal, window, global_tokens, group, steps, stride;
+    __device__ int of(int kt) const { return bwd_piece_count(bwd_tiles_per_head(kt, n_qt, causal, window, global_tokens) * group, steps); }
+};
+
+// dV / dK of the key tiles that were cut: the partials of a tile are added in piece order and written as
 // bf16 (dK times the softmax scale).  One thread per 8 consecutive features of one key row.
 template <int D>
 __global__ void __launch_bounds__(256) bwd_dkv_reduce_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ dk,
-                                                             __nv_bfloat16* __restrict__ dv, int slabs, int group, int Skv,
+                                                             __nv_bfloat16* __restrict__ dv, const BwdPieces pieces, int slabs, int Skv,
                                                              float scale, long long n_units)
 {
     wait_for_stream();
@@ -933,9 +1033,11 @@ __global__ void __launch_bounds__(256) bwd_dkv_reduce_kernel(const float* __rest
     const int kt = (int)(r / slabs);
     const int key = kt * kT + row;
     if (key >= Skv) return;
-    const float* src = part + (((size_t)kt * slabs + slab) * group * 2 + which) * (size_t)(kT * D) + (size_t)row * D + d8;
+    const float* src = part + (((size_t)kt * slabs + slab) * pieces.stride * 2 + which) * (size_t)(kT * D) + (size_t)row * D + d8;
+    const int n = pieces.of(kt);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int g = 0; g < group; ++g) {
+#pragma unroll 4
+    for (int g = 0; g < n; ++g) {
         const float4 a = *reinterpret_cast<const float4*>(src + (size_t)g * 2 * kT * D);
         const float4 c = *reinterpret_cast<const float4*>(src + (size_t)g * 2 * kT * D + 4);
         acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
@@ -953,7 +1055,7 @@ __global__ void __launch_bounds__(256) bwd_dkv_reduce_kernel(const float* __rest
 // The same sums into fp32 feature-major matrices: consecutive threads take consecutive keys.
 template <int D>
 __global__ void __launch_bounds__(256) bwd_dkv_reduce_matrix_kernel(const float* __restrict__ part, float* __restrict__ dk, float* __restrict__ dv,
-                                                                    long long stride, int Hkv, int slabs, int group, int Skv, float scale,
+                                                                    long long stride, const BwdPieces pieces, int Hkv, int slabs, int Skv, float scale,
                                                                     long long n_units)
 {
     wait_for_stream();
@@ -966,9 +1068,11 @@ __global__ void __launch_bounds__(256) bwd_dkv_reduce_matrix_kernel(const float*
     const int which = (int)(r & 1); r >>= 1;              // 0: dV, 1: dK
     const int slab = (int)(r % slabs), kt = (int)(r / slabs), key = kt * kT + row;
     if (key >= Skv) return;
-    const float* src = part + (((size_t)kt * slabs + slab) * group * 2 + which) * (size_t)(kT * D) + (size_t)row * D + d8;
+    const float* src = part + (((size_t)kt * slabs + slab) * pieces.stride * 2 + which) * (size_t)(kT * D) + (size_t)row * D + d8;
+    const int n = pieces.of(kt);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int g = 0; g < group; ++g)
+#pragma unroll 4
+    for (int g = 0; g < n; ++g)
 #pragma unroll
         for (int i = 0; i < 8; i += 4) {
             const float4 x = *reinterpret_cast<const float4*>(src + (size_t)g * 2 * kT * D + i);
@@ -1047,14 +1151,15 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     p.window = s.causal ? s.window : 0;
     p.global_tokens = s.global_tokens;
     p.n_qt = n_qt; p.n_kt = n_kt;
-    p.split_tiles = kSplit ? bwd_split_tiles(s) : 0;
+    const BwdCut cut = kSplit ? bwd_cut(s) : BwdCut{};
+    p.split_tiles = cut.tiles; p.split_steps = cut.steps; p.split_pieces = cut.pieces; p.whole_first = cut.whole_first;
     p.dkv_part = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dq_accum) + align256((kDet ? 8 : 4) * (size_t)rows_padded * D));
     p.dk_acc = a.dk_acc; p.dv_acc = a.dv_acc;
     p.dk_mat = a.mat.dk; p.dv_mat = a.mat.dv; p.mat_stride = a.mat.stride;
     p.scale = s.scale;
     p.scale_log2 = s.scale * 1.4426950408889634f;
-    const int group = s.Hq / s.Hkv, slabs = s.B * s.Hkv;
-    const long long ctas = (long long)p.split_tiles * group * slabs + (long long)(n_kt - p.split_tiles) * slabs;
+    const int slabs = s.B * s.Hkv;
+    const long long ctas = (long long)p.split_tiles * cut.pieces * slabs + (long long)(n_kt - p.split_tiles) * slabs;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     static std::atomic<unsigned long long> configured{0};   // per instantiation, one bit per device
     {
@@ -1071,11 +1176,12 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     if (p.split_tiles > 0) {
         const long long n_units = (long long)p.split_tiles * slabs * 2 * kT * (D / 8);
         const unsigned blocks = (unsigned)((n_units + 255) / 256);
+        const BwdPieces pieces{n_qt, p.causal, p.window, p.global_tokens, s.Hq / s.Hkv, cut.steps, cut.pieces};
         if constexpr (kMat)
-            e = launch_kernel(bwd_dkv_reduce_matrix_kernel<D>, blocks, 256, 0, st, 1, p.dkv_part, a.mat.dk, a.mat.dv, a.mat.stride, s.Hkv, slabs,
-                              group, s.Skv, s.scale, n_units);
+            e = launch_kernel(bwd_dkv_reduce_matrix_kernel<D>, blocks, 256, 0, st, 1, p.dkv_part, a.mat.dk, a.mat.dv, a.mat.stride, pieces,
+                              s.Hkv, slabs, s.Skv, s.scale, n_units);
         else
-            e = launch_kernel(bwd_dkv_reduce_kernel<D>, blocks, 256, 0, st, 1, p.dkv_part, a.dk, a.dv, slabs, group, s.Skv, s.scale, n_units);
+            e = launch_kernel(bwd_dkv_reduce_kernel<D>, blocks, 256, 0, st, 1, p.dkv_part, a.dk, a.dv, pieces, slabs, s.Skv, s.scale, n_units);
         if (e != cudaSuccess) return e;
     }
     }   // kBwdMain
@@ -1098,24 +1204,20 @@ bool tc_bwd_supported(const AttnShape& s)
 }
 
 // [delta records: B*Hq*Sq_pad x 16 bytes][LSE records: same], 256-byte aligned, then the fp32 dQ accumulator B*Hq*Sq_pad*D, then the fp32
-// dK/dV partials of the key tiles that are cut by query head (none for most shapes)
-size_t tc_backward_workspace_bytes(const AttnShape& s)
-{
-    const size_t sq_pad = ((size_t)s.Sq + kT - 1) / kT * kT;
-    const size_t rows = (size_t)s.B * s.Hq * sq_pad;
-    const size_t part = (size_t)bwd_split_tiles(s) * s.B * s.Hq * 2 * kT * (size_t)s.D * 4;   // slabs * group = B * Hq
-    return align256(kBwdRowAuxBytes * rows) + align256((s.deterministic ? 8 : 4) * rows * (size_t)s.D) + align256(part);
-}
+// dK/dV partials of the key tiles that are cut into pieces (none for most shapes)
+size_t tc_backward_workspace_bytes(const AttnShape& s) { return bwd_base_bytes(s) + align256(bwd_part_bytes(s, bwd_cut(s))); }
 
 namespace {
 template <int D, bool kMat>
 cudaError_t dispatch_bwd(const TcArgs& a, cudaStream_t st)
 {
     const bool win = a.s.causal && a.s.window > 0;
-    if (a.s.deterministic)   // (bwd_split_tiles is 0 for this form)
+    const bool cut = bwd_cut(a.s).tiles > 0;
+    if (a.s.deterministic) {
+        if (cut) return win ? launch_bwd<D, true, true, true, kMat>(a, st) : launch_bwd<D, false, true, true, kMat>(a, st);
         return win ? launch_bwd<D, true, false, true, kMat>(a, st) : launch_bwd<D, false, false, true, kMat>(a, st);
-    if (bwd_split_tiles(a.s) > 0)
-        return win ? launch_bwd<D, true, true, false, kMat>(a, st) : launch_bwd<D, false, true, false, kMat>(a, st);
+    }
+    if (cut) return win ? launch_bwd<D, true, true, false, kMat>(a, st) : launch_bwd<D, false, true, false, kMat>(a, st);
     return win ? launch_bwd<D, true, false, false, kMat>(a, st) : launch_bwd<D, false, false, false, kMat>(a, st);
 }
 template <int D>

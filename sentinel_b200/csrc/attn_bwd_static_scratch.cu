@@ -25,7 +25,7 @@
 
 #include <cuda_runtime.h>
 
-#include "sntl_attn.h"
+#include "common.cuh"
 
 namespace {
 
@@ -64,14 +64,20 @@ int sntl_attn_bwd_static_scratch(const sntl_attn_desc* desc, const void* q, cons
                                  const float* lse, const void* dout, void* dq, void* dk, void* dv, void* stream)
 {
     if (!desc) return SNTL_ERR_BAD_ARGUMENT;
-    const size_t need = sntl_attn_bwd_workspace_bytes(desc);
+    // key tiles stay whole where the partials of cut ones would not fit
+    bool whole = false;
+    size_t need = sntl_attn_bwd_workspace_bytes(desc);
+    if (need > kStaticScratchBytes) {
+        whole = true;
+        need = sntl::bwd_workspace_bytes(desc, true);
+    }
     if (need == 0)  // the descriptor does not validate: let the normal entry point name the reason (it launches nothing)
         return sntl_attn_bwd(desc, q, k, v, o, lse, dout, dq, dk, dv, nullptr, 0, stream);
     if (need > kStaticScratchBytes) return SNTL_ERR_SCRATCH_LIMIT;
     void* scratch = nullptr;
     const int rc = static_scratch_pointer(&scratch);
     if (rc != SNTL_OK) return rc;
-    return sntl_attn_bwd(desc, q, k, v, o, lse, dout, dq, dk, dv, scratch, kStaticScratchBytes, stream);
+    return sntl::bwd_run(desc, q, k, v, o, lse, dout, dq, dk, dv, scratch, kStaticScratchBytes, stream, whole);
 }
 
 }  // extern "C"

@@ -372,6 +372,31 @@ def test_backward_long_key_tiles_cut_by_query_head(sb, oracle):
         _check_bf16(_np(got), _np(want), what + " slice vs exact kernels")
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,kw", [
+    (1, 2, 2, 1100, 128, {}),                                    # one head per group: tiles cut along the queries, ragged
+    (1, 6, 2, 700, 64, dict(window=200, global_tokens=5)),       # pieces that end inside a head's query range
+    (1, 4, 1, 900, 128, dict(flags=4)),                          # cut tiles with reproducible dQ
+    (2, 3, 1, 1024, 64, dict(flags=4)),                          # a step count that is no multiple of the pieces
+])
+def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
+    """Key tiles cut into pieces against the exact kernels on the same bf16 values.  P, dS and the operands are bf16 (2^-9 each,
+    independent): dQ, dK within 8e-3 relative L2, dV within 4e-3; dK, dV bit-identical from run to run."""
+    w = sb.WORKLOADS["gqa7b_d128"]
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v, do = ((torch.randn(B, H, S, D, generator=g, device="cuda") * std).to(torch.bfloat16)
+                   for H, std in ((Hq, 0.5), (Hkv, 0.5), (Hkv, 1.0), (Hq, w.do_std)))
+    mask = {n: x for n, x in kw.items() if n != "flags"}
+    o, lse = sb.attention_forward(q, k, v, **mask)
+    dq, dk, dv = sb.attention_backward(q, k, v, o, lse, do, **kw)
+    again = sb.attention_backward(q, k, v, o, lse, do, **kw)
+    assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+    assert torch.equal(dk, again[1]) and torch.equal(dv, again[2]) and (torch.equal(dq, again[0]) or "flags" not in kw)
+    qf, kf, vf, dof = (t.float() for t in (q, k, v, do))
+    of, lf = sb.attention_forward(qf, kf, vf, **mask)
+    for got, want, tol in zip((dq, dk, dv), sb.attention_backward(qf, kf, vf, of, lf, dof, **mask), (8e-3, 8e-3, 4e-3)):
+        assert float((got.float() - want).norm() / want.norm()) <= tol
+
+
 def test_backward_head_dim_64_buffers_and_cut_tiles_vs_oracle(sb, oracle):
     """head_dim 64 takes a path of its own inside the backward kernel (LSE and delta folded into the S^T / dP^T products,
     two S^T buffers, three Q stages, two dS tiles).  B1 / Hq8 / Hkv2 / S1400 is a grid small enough that every key tile is

@@ -112,9 +112,7 @@ __global__ void rope_unpack_kernel(const __nv_bfloat16* __restrict__ src, float*
     }
 }
 
-// Head sizes that are multiples of 64 (the tensor-core kernels' sizes) take 64-token x 64-feature tiles: every global
-// access is a full 128-byte line per warp (32 tokens of one feature on the fp32 side, the 64 features of one token as
-// bf16 pairs on the other), each thread keeps 16 loads in flight, and a rotation pair lives in one thread.
+// Head sizes that are multiples of 64 (the tensor-core kernels' sizes) take the kernels below: a rotation pair lives in one thread.
 // kRot: 0 no rotation, 1 forward, 2 inverse.
 template <int kRot>
 __device__ __forceinline__ void rotate_pair(float& even, float& odd, float c, float sn)
@@ -130,16 +128,11 @@ __device__ __forceinline__ void rotate_pair(float& even, float& odd, float c, fl
     }
 }
 
-// Tiles of kTok tokens x DT = 64 features, every global access 16 bytes wide: on the bf16 side a thread moves eight
-// consecutive features of one token, on the fp32 side four consecutive tokens of one feature (runs of kTok * 4 = 512
-// contiguous bytes per feature).  (A tile covering a whole 128-feature head makes the bf16 side one contiguous block,
-// but its 66 KB of shared memory leave three CTAs per SM and it measured 35 % slower.)  The angle tables come as float4 (four
-// pairs).  Lane maps are chosen so that, with the tile's odd row pitch, the 32 lanes of a warp hit 32 different banks in
-// both transposing directions: 8 token quads x 4 features on the fp32 side, 8 tokens x 4 eight-feature units on the
-// bf16 side.  kVec = false is the same kernel with 4-byte accesses on the fp32 side, for windows whose first column,
-// length or row pitch is not a multiple of four elements.
+// Tiles of kTok tokens x DT = 64 features: on the bf16 side a thread moves eight consecutive features of one token, on the fp32
+// side runs of kTok tokens of one feature.  (A tile covering a whole 128-feature head makes the bf16 side one contiguous block,
+// but its shared memory leaves too few CTAs per SM: 35 % slower.)  The angle tables come as float4 (four pairs).
 constexpr int kTok = 128;
-constexpr int kHeadsPerCta = 4;   // heads one CTA converts in turn: the angle tables then cost a quarter of the L2 traffic
+constexpr int kHeadsPerCta = 8;   // heads one CTA converts in turn, at most
 
 // lane maps (see above): fp32 side -> (first of four tokens, feature); bf16 side -> (token, 8-feature unit)
 template <int DT> struct PackMap {
@@ -178,45 +171,47 @@ __device__ __forceinline__ void load_angles(float4* cs, float4* sn, const float*
     }
 }
 
-template <int kRot, bool kVec, int DT>
+// eight features of one token, rotated and stored as bf16
+template <int kRot>
+__device__ __forceinline__ void store_unit(__nv_bfloat16* dst, float (&x)[8], const float4& cs, const float4& sn)
+{
+    if (kRot != 0) {
+        rotate_pair<kRot>(x[0], x[1], cs.x, sn.x);
+        rotate_pair<kRot>(x[2], x[3], cs.y, sn.y);
+        rotate_pair<kRot>(x[4], x[5], cs.z, sn.z);
+        rotate_pair<kRot>(x[6], x[7], cs.w, sn.w);
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 y = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&y);
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Scalar form, for windows whose first column, length or row pitch is not a multiple of four elements: 4-byte accesses on the
+// fp32 side, one tile at a time.
+template <int kRot, int DT>
 __global__ void __launch_bounds__(256, 4) pack64_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int H, int S, int D,
                                                      int stride_columns, int column_start, const float* __restrict__ cos_t,
-                                                     const float* __restrict__ sin_t, int position_offset)
+                                                     const float* __restrict__ sin_t, int position_offset, int heads_per_cta)
 {
     using M = PackMap<DT>;
     extern __shared__ float tile_raw[];
     wait_for_stream();
     float (*tile)[DT + 1] = reinterpret_cast<float (*)[DT + 1]>(tile_raw);   // [token][feature]
-    const int groups = (H + kHeadsPerCta - 1) / kHeadsPerCta;
-    const int b = blockIdx.z / groups, h_first = (blockIdx.z % groups) * kHeadsPerCta;
+    const int groups = (H + heads_per_cta - 1) / heads_per_cta;
+    const int b = blockIdx.z / groups, h_first = (blockIdx.z % groups) * heads_per_cta;
     const int s0 = blockIdx.x * kTok, d0 = blockIdx.y * DT;
     float4 cs[M::kUnits], sn[M::kUnits];
     load_angles<kRot, DT>(cs, sn, cos_t, sin_t, s0, d0, S, D >> 1, position_offset);
-    for (int h = h_first; h < min(H, h_first + kHeadsPerCta); ++h) {
+    for (int h = h_first; h < min(H, h_first + heads_per_cta); ++h) {
         const float* base = src + (long long)(h * D + d0) * stride_columns + column_start + (long long)b * S + s0;
-        if (kVec) {
-            // all of a thread's loads are issued before the first one is used (S is a multiple of four here, so a quad
-            // of tokens is inside the sequence or outside it as a whole)
-            float4 x[M::kQuads];
-#pragma unroll
-            for (int r = 0; r < M::kQuads; ++r) {
-                int s4, d;
-                M::quad(r, s4, d);
-                x[r] = (s0 + s4 < S) ? __ldg(reinterpret_cast<const float4*>(base + (long long)d * stride_columns + s4))
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int r = 0; r < M::kQuads; ++r) {
-                int s4, d;
-                M::quad(r, s4, d);
-                tile[s4][d] = x[r].x; tile[s4 + 1][d] = x[r].y; tile[s4 + 2][d] = x[r].z; tile[s4 + 3][d] = x[r].w;
-            }
-        } else {
 #pragma unroll 4
-            for (int r = 0; r < kTok * DT / 256; ++r) {
-                const int idx = r * 256 + threadIdx.x, d = idx / kTok, sl = idx % kTok;
-                tile[sl][d] = (s0 + sl < S) ? base[(long long)d * stride_columns + sl] : 0.0f;
-            }
+        for (int r = 0; r < kTok * DT / 256; ++r) {
+            const int idx = r * 256 + threadIdx.x, d = idx / kTok, sl = idx % kTok;
+            tile[sl][d] = (s0 + sl < S) ? base[(long long)d * stride_columns + sl] : 0.0f;
         }
         __syncthreads();
         __nv_bfloat16* out = dst + ((long long)(b * H + h) * S + s0) * D + d0;
@@ -228,38 +223,27 @@ __global__ void __launch_bounds__(256, 4) pack64_kernel(const float* __restrict_
             float x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = tile[sl][8 * u + i];
-            if (kRot != 0) {
-                rotate_pair<kRot>(x[0], x[1], cs[r].x, sn[r].x);
-                rotate_pair<kRot>(x[2], x[3], cs[r].y, sn[r].y);
-                rotate_pair<kRot>(x[4], x[5], cs[r].z, sn[r].z);
-                rotate_pair<kRot>(x[6], x[7], cs[r].w, sn[r].w);
-            }
-            __nv_bfloat162 o0 = __floats2bfloat162_rn(x[0], x[1]), o1 = __floats2bfloat162_rn(x[2], x[3]);
-            __nv_bfloat162 o2 = __floats2bfloat162_rn(x[4], x[5]), o3 = __floats2bfloat162_rn(x[6], x[7]);
-            uint4 w;
-            w.x = *reinterpret_cast<uint32_t*>(&o0); w.y = *reinterpret_cast<uint32_t*>(&o1);
-            w.z = *reinterpret_cast<uint32_t*>(&o2); w.w = *reinterpret_cast<uint32_t*>(&o3);
-            *reinterpret_cast<uint4*>(out + (long long)sl * D + 8 * u) = w;
+            store_unit<kRot>(out + (long long)sl * D + 8 * u, x, cs[r], sn[r]);
         }
         __syncthreads();      // the tile is refilled for the next head
     }
 }
 
-template <int kRot, bool kVec, int DT>
+template <int kRot, int DT>
 __global__ void __launch_bounds__(256, 4) unpack64_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst, int H, int S, int D,
                                                        int stride_columns, int column_start, const float* __restrict__ cos_t,
-                                                       const float* __restrict__ sin_t, int position_offset)
+                                                       const float* __restrict__ sin_t, int position_offset, int heads_per_cta)
 {
     using M = PackMap<DT>;
     extern __shared__ float tile_raw[];
     wait_for_stream();
     float (*tile)[DT + 1] = reinterpret_cast<float (*)[DT + 1]>(tile_raw);
-    const int groups = (H + kHeadsPerCta - 1) / kHeadsPerCta;
-    const int b = blockIdx.z / groups, h_first = (blockIdx.z % groups) * kHeadsPerCta;
+    const int groups = (H + heads_per_cta - 1) / heads_per_cta;
+    const int b = blockIdx.z / groups, h_first = (blockIdx.z % groups) * heads_per_cta;
     const int s0 = blockIdx.x * kTok, d0 = blockIdx.y * DT;
     float4 cs[M::kUnits], sn[M::kUnits];
     load_angles<kRot, DT>(cs, sn, cos_t, sin_t, s0, d0, S, D >> 1, position_offset);
-    for (int h = h_first; h < min(H, h_first + kHeadsPerCta); ++h) {
+    for (int h = h_first; h < min(H, h_first + heads_per_cta); ++h) {
         const __nv_bfloat16* in = src + ((long long)(b * H + h) * S + s0) * D + d0;
         uint4 win[M::kUnits];
 #pragma unroll
@@ -290,63 +274,189 @@ __global__ void __launch_bounds__(256, 4) unpack64_kernel(const __nv_bfloat16* _
         }
         __syncthreads();
         float* base = dst + (long long)(h * D + d0) * stride_columns + column_start + (long long)b * S + s0;
-        if (kVec) {
-#pragma unroll
-            for (int r = 0; r < M::kQuads; ++r) {
-                int s4, d;
-                M::quad(r, s4, d);
-                if (s0 + s4 < S)
-                    *reinterpret_cast<float4*>(base + (long long)d * stride_columns + s4) =
-                        make_float4(tile[s4][d], tile[s4 + 1][d], tile[s4 + 2][d], tile[s4 + 3][d]);
-            }
-        } else {
 #pragma unroll 4
-            for (int r = 0; r < kTok * DT / 256; ++r) {
-                const int idx = r * 256 + threadIdx.x, d = idx / kTok, sl = idx % kTok;
-                if (s0 + sl < S) base[(long long)d * stride_columns + sl] = tile[sl][d];
-            }
+        for (int r = 0; r < kTok * DT / 256; ++r) {
+            const int idx = r * 256 + threadIdx.x, d = idx / kTok, sl = idx % kTok;
+            if (s0 + sl < S) base[(long long)d * stride_columns + sl] = tile[sl][d];
         }
         __syncthreads();      // the tile is refilled for the next head
     }
 }
 
-// launches pack64_kernel / unpack64_kernel (one tile column of 64 features per blockIdx.y)
-#define SNTL_PACK_CASE(KERNEL, ROT, VEC, DTV)                                                                                      \
-    do {                                                                                                                           \
-        constexpr size_t smem = (size_t)kTok * (DTV + 1) * sizeof(float);                                                          \
-        static std::atomic<unsigned long long> configured{0};                                                                      \
-        if ((e = ensure_dynamic_smem(KERNEL<ROT, VEC, DTV>, smem, configured)) != cudaSuccess) return e;                           \
-        dim3 grid((S + kTok - 1) / kTok, D / DTV, B * ((H + kHeadsPerCta - 1) / kHeadsPerCta));                                    \
-        return launch_kernel(KERNEL<ROT, VEC, DTV>, grid, 256, smem, st, 1, src, dst, H, S, D, stride_columns, column_start, cos_t, sin_t, position_offset); \
+// The usual form: every global access 16 bytes, and the next head's tile on its way into shared memory (asynchronous copies, two
+// buffers) while this one is converted.  Bound by HBM: 6 bytes per element; B2 H28 S8192 D128 (352 MB): rotated 95 us with the
+// tile loaded, converted and stored in turn, 62 us here (0.87 of the copy rate), plain 63 and 60.  The tile lies in shared memory as it came; its 16-byte units are XOR-permuted
+// by row so that the reads across the grain (eight tokens x four units, or eight quads of tokens x four pairs) hit all banks.
+__device__ __forceinline__ void copy16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_left() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <int kRot, int DT>
+__global__ void __launch_bounds__(256, 3) pack64_pipe_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int H, int S, int D,
+                                                          int stride_columns, int column_start, const float* __restrict__ cos_t,
+                                                          const float* __restrict__ sin_t, int position_offset, int heads_per_cta)
+{
+    using M = PackMap<DT>;
+    extern __shared__ float tile_raw[];            // [2][feature][128 tokens], token quad q of feature d at quad q ^ (d >> 3) * 2
+    wait_for_stream();
+    const int groups = (H + heads_per_cta - 1) / heads_per_cta;
+    const int b = blockIdx.z / groups, h_first = (blockIdx.z % groups) * heads_per_cta, h_end = min(H, h_first + heads_per_cta);
+    const int s0 = blockIdx.x * kTok, d0 = blockIdx.y * DT;
+    auto fetch = [&](int h, float* tile) {
+        const float* base = src + (long long)(h * D + d0) * stride_columns + column_start + (long long)b * S + s0;
+#pragma unroll
+        for (int r = 0; r < M::kQuads; ++r) {
+            const int d = r * 8 + (threadIdx.x >> 5), q = threadIdx.x & 31;      // a warp: the 512 bytes of one feature
+            if (s0 + 4 * q < S) copy16(tile + d * kTok + ((q ^ ((d >> 3) << 1)) << 2), base + (long long)d * stride_columns + 4 * q);
+        }
+        copies_commit();
+    };
+    fetch(h_first, tile_raw);
+    float4 cs[M::kUnits], sn[M::kUnits];
+    load_angles<kRot, DT>(cs, sn, cos_t, sin_t, s0, d0, S, D >> 1, position_offset);
+    for (int h = h_first; h < h_end; ++h) {
+        const float* tile = tile_raw + ((h - h_first) & 1) * (DT * kTok);
+        if (h + 1 < h_end) {
+            fetch(h + 1, tile_raw + ((h + 1 - h_first) & 1) * (DT * kTok));
+            copies_left<1>();
+        } else copies_left<0>();
+        __syncthreads();
+        __nv_bfloat16* out = dst + ((long long)(b * H + h) * S + s0) * D + d0;
+#pragma unroll
+        for (int r = 0; r < M::kUnits; ++r) {
+            int sl, u;
+            M::unit(r, sl, u);
+            if (s0 + sl >= S) continue;
+            const float* p = tile + 8 * u * kTok + (((sl >> 2) ^ (u << 1)) << 2) + (sl & 3);
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = p[i * kTok];
+            store_unit<kRot>(out + (long long)sl * D + 8 * u, x, cs[r], sn[r]);
+        }
+        __syncthreads();
+    }
+}
+
+template <int kRot, int DT>
+__global__ void __launch_bounds__(256, 4) unpack64_pipe_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst, int H, int S, int D,
+                                                            int stride_columns, int column_start, const float* __restrict__ cos_t,
+                                                            const float* __restrict__ sin_t, int position_offset, int heads_per_cta)
+{
+    static_assert(DT == 64, "eight 16-byte units per token");
+    constexpr int kWords = DT / 2, kItems = kTok / 4 * kWords / 256;   // an item: four tokens of one feature pair
+    extern __shared__ float tile_raw[];
+    uint32_t* tiles = reinterpret_cast<uint32_t*>(tile_raw);           // [2][token][32 pairs], unit c of token t at c ^ (t >> 2 & 7)
+    wait_for_stream();
+    const int groups = (H + heads_per_cta - 1) / heads_per_cta;
+    const int b = blockIdx.z / groups, h_first = (blockIdx.z % groups) * heads_per_cta, h_end = min(H, h_first + heads_per_cta);
+    const int s0 = blockIdx.x * kTok, d0 = blockIdx.y * DT;
+    auto fetch = [&](int h, uint32_t* tile) {
+        const __nv_bfloat16* in = src + ((long long)(b * H + h) * S + s0) * D + d0;
+#pragma unroll
+        for (int r = 0; r < kTok * 8 / 256; ++r) {
+            const int t = r * 32 + (threadIdx.x >> 3), c = threadIdx.x & 7;
+            if (s0 + t < S) copy16(tile + t * kWords + ((c ^ ((t >> 2) & 7)) << 2), in + (long long)t * D + 8 * c);
+        }
+        copies_commit();
+    };
+    fetch(h_first, tiles);
+    const int q8 = threadIdx.x & 7, p4 = (threadIdx.x >> 3) & 3, warp = threadIdx.x >> 5;
+    auto item = [&](int r, int& quad, int& pair) {
+        const int rest = r * 8 + warp;
+        quad = (rest & 3) * 8 + q8;
+        pair = (rest >> 2) * 4 + p4;
+    };
+    float cs[kItems][4], sn[kItems][4];
+    if (kRot != 0) {
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+            int quad, pair;
+            item(r, quad, pair);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const long long ti = (long long)(position_offset + min(s0 + 4 * quad + k, S - 1)) * (D >> 1) + (d0 >> 1) + pair;
+                cs[r][k] = __ldg(cos_t + ti);
+                sn[r][k] = __ldg(sin_t + ti);
+            }
+        }
+    }
+    for (int h = h_first; h < h_end; ++h) {
+        const uint32_t* tile = tiles + ((h - h_first) & 1) * (kTok * kWords);
+        if (h + 1 < h_end) {
+            fetch(h + 1, tiles + ((h + 1 - h_first) & 1) * (kTok * kWords));
+            copies_left<1>();
+        } else copies_left<0>();
+        __syncthreads();
+        float* base = dst + (long long)(h * D + d0) * stride_columns + column_start + (long long)b * S + s0;
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+            int quad, pair;
+            item(r, quad, pair);
+            if (s0 + 4 * quad >= S) continue;
+            const uint32_t* p = tile + 4 * quad * kWords + (((pair >> 2) ^ q8) << 2) + p4;
+            float e[4], o[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t w = p[k * kWords];
+                e[k] = __uint_as_float(w << 16);
+                o[k] = __uint_as_float(w & 0xffff0000u);
+                if (kRot != 0) rotate_pair<kRot>(e[k], o[k], cs[r][k], sn[r][k]);
+            }
+            float* out = base + (long long)(2 * pair) * stride_columns + 4 * quad;
+            *reinterpret_cast<float4*>(out) = make_float4(e[0], e[1], e[2], e[3]);
+            *reinterpret_cast<float4*>(out + stride_columns) = make_float4(o[0], o[1], o[2], o[3]);
+        }
+        __syncthreads();
+    }
+}
+
+// One tile column of 64 features per blockIdx.y.  A CTA converts several heads in turn: the angles cost it one fetch and the
+// pipeline runs; fewer heads where the grid would leave SMs without CTAs.
+template <typename Kernel, typename Src, typename Dst>
+cudaError_t launch_convert64(Kernel kernel, size_t smem, std::atomic<unsigned long long>& configured, const Src* src, Dst* dst, int B, int H, int S,
+                             int D, int stride_columns, int column_start, const float* cos_t, const float* sin_t, int position_offset, cudaStream_t st)
+{
+    const cudaError_t e = ensure_dynamic_smem(kernel, smem, configured);
+    if (e != cudaSuccess) return e;
+    const long long tiles = (long long)((S + kTok - 1) / kTok) * (D / 64) * B, want = (4LL * sm_count() + tiles - 1) / tiles;
+    int groups = (int)(want < H ? want : H);
+    if (groups * kHeadsPerCta < H) groups = (H + kHeadsPerCta - 1) / kHeadsPerCta;
+    const int per = (H + groups - 1) / groups;
+    const dim3 grid((S + kTok - 1) / kTok, D / 64, B * ((H + per - 1) / per));
+    return launch_kernel(kernel, grid, 256, smem, st, 1, src, dst, H, S, D, stride_columns, column_start, cos_t, sin_t, position_offset, per);
+}
+#define SNTL_CONVERT(KERNEL, ROT, SMEM)                                                                                                   \
+    do {                                                                                                                                  \
+        static std::atomic<unsigned long long> configured{0};                                                                             \
+        return launch_convert64(KERNEL<ROT, 64>, SMEM, configured, src, dst, B, H, S, D, stride_columns, column_start, cos_t, sin_t,      \
+                                position_offset, st);                                                                                     \
     } while (0)
-#define SNTL_PACK_ROT(KERNEL, VEC, DTV)                                 \
-    do {                                                                \
-        if (rot == 0) SNTL_PACK_CASE(KERNEL, 0, VEC, DTV);              \
-        else if (rot == 1) SNTL_PACK_CASE(KERNEL, 1, VEC, DTV);         \
-        else SNTL_PACK_CASE(KERNEL, 2, VEC, DTV);                       \
+#define SNTL_CONVERT_ROT(KERNEL, SMEM)                          \
+    do {                                                        \
+        if (rot == 0) SNTL_CONVERT(KERNEL, 0, SMEM);            \
+        else if (rot == 1) SNTL_CONVERT(KERNEL, 1, SMEM);       \
+        else SNTL_CONVERT(KERNEL, 2, SMEM);                     \
     } while (0)
-#define SNTL_PACK_ALL(KERNEL)                                                            \
-    do {                                                                                 \
-        if (vec) SNTL_PACK_ROT(KERNEL, true, 64); else SNTL_PACK_ROT(KERNEL, false, 64);                         \
-    } while (0)
+
+constexpr size_t kTileBytes = (size_t)kTok * 65 * sizeof(float);
 
 cudaError_t launch_pack64(int rot, bool vec, const float* src, __nv_bfloat16* dst, int B, int H, int S, int D, int stride_columns,
                           int column_start, const float* cos_t, const float* sin_t, int position_offset, cudaStream_t st)
 {
-    cudaError_t e;
-    SNTL_PACK_ALL(pack64_kernel);
-    return cudaErrorInvalidValue;
+    if (vec) SNTL_CONVERT_ROT(pack64_pipe_kernel, 2 * kTok * 64 * sizeof(float));
+    SNTL_CONVERT_ROT(pack64_kernel, kTileBytes);
 }
 cudaError_t launch_unpack64(int rot, bool vec, const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
                             int column_start, const float* cos_t, const float* sin_t, int position_offset, cudaStream_t st)
 {
-    cudaError_t e;
-    SNTL_PACK_ALL(unpack64_kernel);
-    return cudaErrorInvalidValue;
+    if (vec) SNTL_CONVERT_ROT(unpack64_pipe_kernel, 2 * kTok * 64 * sizeof(__nv_bfloat16));
+    SNTL_CONVERT_ROT(unpack64_kernel, kTileBytes);
 }
-#undef SNTL_PACK_ALL
-#undef SNTL_PACK_ROT
-#undef SNTL_PACK_CASE
+#undef SNTL_CONVERT_ROT
+#undef SNTL_CONVERT
 
 // ---- everything a tensor-core call needs from feature-major matrices (see MatrixStage) ----
 // One launch instead of one per tensor: on the sizes of a training microstep (16 MB a matrix) a conversion takes as long as the

@@ -84,6 +84,14 @@ def test_pack_windows_offsets_and_ragged_shapes_vs_oracle(sb, oracle, B, H, S, D
     assert max_abs(o[:, col0:col0 + B * S], window) <= 2.0 ** -7 * float(np.abs(window).max())
 
 
+@pytest.mark.parametrize("B,H,S,D,col0,extra,offset", [(1, 1, 4, 64, 0, 0, 0), (2, 19, 132, 64, 4, 4, 3), (1, 200, 128, 64, 0, 0, 0),
+                                                       (2, 9, 260, 128, 8, 0, 0)])
+def test_pack_pipelined_tiles_vs_oracle(sb, oracle, B, H, S, D, col0, extra, offset):
+    """Windows whose rows are 16-byte aligned take the pipelined kernels: one quad of tokens, a tile and a quad, several heads per
+    CTA (200 heads: the pipeline's buffers go round), two feature tiles per head."""
+    test_pack_windows_offsets_and_ragged_shapes_vs_oracle(sb, oracle, B, H, S, D, col0, extra, offset)
+
+
 def test_rotary_layer_path_matches_reference_layer(sb):
     """The whole neighbourhood of the hot path as the reference layer runs it (CudaCausalSelfAttention.cu:181-253, :392-509):
     un-rotated fp32 feature-major Q/K/V -> rotate + pack -> attention forward/backward on the tensor cores -> unpack with the

@@ -84,7 +84,7 @@ def test_pack_windows_offsets_and_ragged_shapes_vs_oracle(sb, oracle, B, H, S, D
     assert max_abs(o[:, col0:col0 + B * S], window) <= 2.0 ** -7 * float(np.abs(window).max())
 
 
-@pytest.mark.parametrize("B,H,S,D,col0,extra,offset", [(1, 1, 4, 64, 0, 0, 0), (2, 19, 132, 64, 4, 4, 3), (1, 200, 128, 64, 0, 0, 0),
+@pytest.mark.parametrize("B,H,S,D,col0,extra,offset", [(1, 1, 4, 64, 0, 0, 0), (2, 19, 132, 64, 4, 4, 0), (1, 5, 100, 64, 4, 0, 3), (1, 200, 128, 64, 0, 0, 0),
                                                        (2, 9, 260, 128, 8, 0, 0)])
 def test_pack_pipelined_tiles_vs_oracle(sb, oracle, B, H, S, D, col0, extra, offset):
     """Windows whose rows are 16-byte aligned take the pipelined kernels: one quad of tokens, a tile and a quad, several heads per

@@ -5,7 +5,7 @@
 // (sentinel/NeuralNet/Cuda/CudaFlashAttention.cu:1105-1266): same math -- S = scale*Q K^T, causal mask,
 // online softmax, O = P V, LSE = m + ln(l) -- re-designed for Blackwell:
 //
-//   * one CTA owns 256 consecutive query rows of one (batch, head) as two 128-row tiles; each tile has its
+//   * one CTA owns 256 (small grids: 128) consecutive query rows of one (batch, head) as two 128-row tiles; each tile has its
 //     own softmax warpgroup (one thread per query row: tcgen05.ld's 32x32b shape hands thread i row i, so the
 //     row max / row sum need no shuffles) while a single MMA-issuing warp (one elected lane) feeds the tensor core for both,
 //     so one tile's softmax overlaps the other tile's MMAs;
@@ -54,7 +54,7 @@ struct FwdParams {
     int B, Hq, Hkv, Sq, Skv;
     int causal;
     int window, global_tokens;   // sliding window and always-visible first keys (0, 0: plain causal)
-    int n_qblk;       // 256-row query blocks per (b, h)
+    int n_qblk, tiles_per_cta;   // query blocks of that many 128-row tiles per (b, h)
     float scale_log2; // scale * log2(e)
     // non-null: O and LSE leave as fp32 feature-major matrices (see MatrixOut)
     float *o_mat, *lse_mat;
@@ -106,7 +106,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const int qblk = p.causal ? (p.n_qblk - 1 - qblk_rank) : qblk_rank;
     const int b = bh / p.Hq, h = bh - b * p.Hq;
     const int bh_kv = b * p.Hkv + h / (p.Hq / p.Hkv);
-    const int q0 = qblk * 2 * kM;                    // the CTA owns two consecutive 128-row tiles
+    const int q0 = qblk * p.tiles_per_cta * kM;      // the CTA owns two consecutive 128-row tiles, or one (fwd_tiles_per_cta)
     const int n_ktiles_all = (p.Skv + kN - 1) / kN;
     // Key tiles this CTA visits, in ascending order: the tiles holding global tokens, then the tiles from the window
     // of the block's first query row up to the diagonal.  Without a window that is simply 0 .. diagonal.
@@ -118,7 +118,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const int row0 = q0 + t * kM;
-        if (row0 >= p.Sq) n_t[t] = 0;
+        if (row0 >= p.Sq || t >= p.tiles_per_cta) n_t[t] = 0;
         else if (p.causal) {
             const int diag = min(n_ktiles_all - 1, row0 / kN);
             n_t[t] = min(g_tiles, diag + 1) + max(0, diag - w_first + 1);
@@ -543,6 +543,29 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
+// Two query tiles per CTA overlap one tile's softmax with the other's products; on a grid that leaves SMs idle or ends with one
+// long CTA, one tile per CTA finishes sooner: a step of one tile takes 0.7 (head_dim 64) or 0.83 (128) of a step of two.  The
+// estimate counts steps of two tiles: the longest CTA, or the SMs' average load and a short tail, with 1.3 steps per CTA of
+// set-up.  Cold, B1 Hq8 S2048: 33 -> 28 us at head_dim 128, 30 -> 21 at 64; B1 Hq4 S8192 D128 110 -> 92; equal at 128 CTAs of
+// 1024 rows, worse beyond (B8 Hq12 S1024 D64 37 -> 49).
+int fwd_tiles_per_cta(const AttnShape& s)
+{
+    const int n = (s.Sq + kM - 1) / kM, n_keys = (s.Skv + kN - 1) / kN, heads = s.B * s.Hq, sms = sm_count();
+    const long long pairs = (long long)((n + 1) / 2) * heads;
+    if (pairs > 2 * sms) return 2;
+    const int reach = s.causal && s.window > 0 ? (s.window + kN - 1) / kN + 1 + (s.global_tokens + kN - 1) / kN : n_keys;
+    auto steps = [&](int tile) { return std::min(s.causal ? tile + 1 : n_keys, reach); };
+    double two = 0.0, one = 0.0;
+    for (int i = 0; i < n; ++i) {
+        one += steps(i);
+        if (i + 1 == n || (i & 1)) two += steps(i);
+    }
+    const double cost = s.D == 64 ? 0.7 : 0.83, set_up = 1.3, longest = steps(n - 1);
+    const double t2 = std::max(longest + set_up, (two * heads + set_up * pairs) / sms + 0.1 * longest);
+    const double t1 = std::max(cost * longest + set_up, (cost * one + set_up * n) * heads / sms + 0.1 * cost * longest);
+    return t1 < 0.95 * t2 ? 1 : 2;
+}
+
 template <int D, int kMode, bool kMat>
 cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
 {
@@ -560,7 +583,8 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     p.causal = s.causal;
     p.window = s.causal ? s.window : 0;
     p.global_tokens = s.global_tokens;
-    p.n_qblk = (s.Sq + 2 * kM - 1) / (2 * kM);
+    p.tiles_per_cta = fwd_tiles_per_cta(s);
+    p.n_qblk = (s.Sq + p.tiles_per_cta * kM - 1) / (p.tiles_per_cta * kM);
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const long long ctas = (long long)p.n_qblk * s.B * s.Hq;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;

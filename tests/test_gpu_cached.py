@@ -131,6 +131,32 @@ def test_bf16_cached_forward_vs_oracle(sb, oracle, wname, B, Hq, Hkv, L, T, wind
     assert max_abs(_np(o32), wo) <= F32_TOL and max_abs(_np(lse32), wl) <= F32_TOL
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,T,L,D,window,global_tokens", [
+    (2, 8, 2, 8, 300, 128, 0, 0),           # 32 rows per KV head: the last size of the decode layout
+    (1, 6, 2, 11, 11, 64, 0, 0),            # 33 rows, every query in one tile
+    (1, 8, 2, 32, 700, 128, 0, 0),          # 128 rows
+    (1, 6, 2, 43, 900, 64, 0, 0),           # 129 rows: the second stream has one
+    (2, 2, 2, 257, 600, 128, 300, 3),       # the second unit of a KV head has one row
+    (25, 16, 4, 1, 3800, 64, 0, 0),         # pieces that end one unit and begin the next
+    (25, 16, 4, 1, 3800, 128, 1000, 130),
+    (1, 4, 1, 1, 40000, 128, 0, 0),         # one KV head on every SM: more than a hundred partial results per row
+])
+def test_bf16_cached_plan_edges_vs_exact_kernels(sb, B, Hq, Hkv, T, L, D, window, global_tokens):
+    """The row layouts and the two ways the keys are dealt to CTAs, against the exact kernels on the same bf16 values: P, the
+    partial results and O are rounded to bf16 (2^-9 each, independent), so O is within 4e-3 relative L2; the LSE stays fp32."""
+    g = torch.Generator(device="cuda").manual_seed(L + T)
+    q = torch.randn(B, Hq, T, D, generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.full((B, Hkv, L + 9, D), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for c in (kc, vc):
+        c[:, :, :L] = torch.randn(B, Hkv, L, D, generator=g, device="cuda").to(torch.bfloat16)
+    kw = dict(window=window, global_tokens=global_tokens)
+    o, lse = sb.attention_cached_forward(q, kc, vc, L, **kw)
+    assert sb.last_path() == "tcgen05_cache" and sb.poll_device_status() == 0
+    of, lf = sb.attention_cached_forward(q.float(), kc.float(), vc.float(), L, **kw)
+    assert float((o.float() - of).norm() / of.norm()) <= 4e-3
+    assert float((lse - lf).abs().max()) <= 1e-3
+
+
 def test_cached_forward_equals_rows_of_full_attention(sb):
     """Decoding token L-1 from a cache is row L-1 of causal attention over the first L tokens."""
     w = sb.WORKLOADS["gqa7b_d128"]

@@ -372,6 +372,27 @@ def test_backward_long_key_tiles_cut_by_query_head(sb, oracle):
         _check_bf16(_np(got), _np(want), what + " slice vs exact kernels")
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,kw", [
+    (1, 2, 1, 1, 1, 128, {}),
+    (1, 4, 2, 129, 129, 64, {}),                                  # the second block holds one row
+    (1, 2, 2, 1300, 1300, 128, {}),                               # ragged, one 128-row block per CTA
+    (1, 6, 2, 1000, 1000, 64, dict(window=200, global_tokens=5)),
+    (1, 4, 4, 300, 900, 128, dict(causal=False)),
+    (1, 37, 37, 257, 257, 64, {}),                                # the last two sizes lie on either side of the rule:
+    (1, 80, 80, 257, 257, 64, {}),                                # 74 and 160 CTAs of 256 rows
+])
+def test_forward_query_tiles_per_cta_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, kw):
+    """Query blocks of 128 rows (small grids) and of 256 against the exact kernels on the same bf16 values: P and O are rounded to
+    bf16 (2^-9 each, independent), so O is within 4e-3 relative L2; the LSE only sees fp32 sums of exact products."""
+    g = torch.Generator(device="cuda").manual_seed(Sq + Hq)
+    q, k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").to(torch.bfloat16) for H, S in ((Hq, Sq), (Hkv, Sk), (Hkv, Sk)))
+    o, lse = sb.attention_forward(q, k, v, **kw)
+    assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+    of, lf = sb.attention_forward(q.float(), k.float(), v.float(), **kw)
+    assert float((o.float() - of).norm() / of.norm()) <= 4e-3
+    assert float((lse - lf).abs().max()) <= 1e-3
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,S,D,kw", [
     (1, 2, 2, 1100, 128, {}),                                    # one head per group: tiles cut along the queries, ragged
     (1, 6, 2, 700, 64, dict(window=200, global_tokens=5)),       # pieces that end inside a head's query range

@@ -52,13 +52,14 @@ using namespace ptx;
 
 namespace {
 
+constexpr int kMaxPieces = 16;          // of one key tile
 constexpr int kT = 128;                 // tile edge: keys per CTA, queries per step
 constexpr int kBwdThreads = 512;        // 2 compute WGs + drain WG + 1 WG holding the MMA warp and the producer warp
 constexpr uint32_t kTmemCols = 512;
 
 enum BwdSite : uint32_t {
     kSiteKV = 0x21, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty, kSiteS, kSiteP, kSiteDP, kSiteDS, kSiteDQ,
-    kSiteDrained, kSiteFinal
+    kSiteDrained, kSiteFinal, kSiteNext
 };
 
 struct BwdParams {
@@ -76,6 +77,8 @@ struct BwdParams {
     int n_qt, n_kt;
     int split_tiles;       // the first split_tiles key tiles are cut into pieces (see BwdCut) of about split_steps steps,
     int split_steps, split_pieces, whole_first;   // at most split_pieces of a tile
+    int piece_end[kMaxPieces];                    // blocks of all pieces up to this one (piece 0 of every cut tile, then piece 1, ...)
+    int several_waves;     // more blocks than SMs
     float* dkv_part;       // [split tile][slab][piece][dV, dK][128][D] fp32
     float *dk_acc, *dv_acc;   // non-null: dK*scale / dV are ADDED into these fp32 [B*Hkv][Skv][D] tensors (no bf16 store)
     // non-null: dK / dV leave as fp32 feature-major matrices (see MatrixOut)
@@ -100,8 +103,9 @@ __host__ __device__ inline int bwd_piece_count(int steps, int split_steps) { ret
 // Which key tiles to cut, and how fine.  The CTA of key tile 0 visits every query tile of every head of its group; on a small
 // grid (few sequences x KV heads, one layer's strong-scaling share, short batches) or where a window leaves only the tiles with
 // global tokens long, that one CTA outlasts the average SM's whole load.  Cutting balances the grid and costs each piece its
-// set-up and an fp32 partial of dK and dV: about two steps for a CTA, one more for a piece.  The estimate below weighs the
-// two for a few piece lengths.  B3 Hq16 Hkv4 S1237 D128 with reproducible dQ: 120 CTAs of up to 40 steps on 148 SMs took
+// set-up and an fp32 partial of dK and dV: about two steps for a CTA, four for a piece.  The estimate below weighs the
+// two for a few piece lengths (a CTA's cost counts once per block, although blocks that follow one another in a CTA hide part of
+// it).  B3 Hq16 Hkv4 S1237 D128 with reproducible dQ: 120 CTAs of up to 40 steps on 148 SMs took
 // 158 us, 108 us cut.
 struct BwdCut {
     int tiles = 0, steps = 1, pieces = 0;
@@ -120,7 +124,7 @@ BwdCut bwd_cut_uncached(const AttnShape& s)
     const int group = s.Hq / s.Hkv, slabs = s.B * s.Hkv, sms = sm_count(), window = s.causal ? s.window : 0;
     const int n_qt = (s.Sq + kT - 1) / kT, n_kt = (s.Skv + kT - 1) / kT;
     auto steps = [&](int kt) { return bwd_tiles_per_head(kt, n_qt, s.causal, window, s.global_tokens) * group; };
-    constexpr double kCta = 2.0, kPiece = 5.0;       // overhead in steps
+    constexpr double kCta = 1.5, kPiece = 4.0;       // overhead in steps
     const int longest = steps(0);
     double total = 0.0;
     for (int kt = 0; kt < n_kt; ++kt) total += steps(kt);
@@ -198,8 +202,56 @@ BwdCut bwd_cut(const AttnShape& s)
     return cut;
 }
 
+// What one block of the grid computes.  A CTA computes its own block and then takes over blocks that have not started yet, one at
+// a time (clc_try_cancel), so that the loads and first products of one run under the epilogue of the one before, and barriers
+// and TMEM are set up once.  A block's fixed cost of about 2 us was a third of a short one: B8 Hq12 S1024 D64, 768 blocks of 1 to 8
+// steps, took 83 us for the whole backward and takes 73; B2 Hq32 S1024 D64 54 -> 49; a 300-key window over B1 Hq16 Hkv4 S4096
+// D128 159 -> 149.  Grids that fit the SMs at once have nothing to take over and do not ask.
+struct BwdWork {
+    int kt, slab, piece;       // key tile, b * Hkv + hk, piece of a cut tile
+    int n_iter;                // steps
+    int qt_first, per_head;    // query tiles of a head: from qt_first, per_head of them
+    int g_first, r_first;      // head and query tile of the first step
+    int split;
+
+    template <bool kWin, bool kSplit> __device__ __forceinline__ void decode(const BwdParams& p, int block)
+    {
+        // whole tiles as one block per (tile, slab), cut ones as one per (piece, tile, slab); the kind with the longest blocks
+        // first, and key tile 0, which sees every query tile, before the others
+        const int slabs = p.B * p.Hkv, group = p.Hq / p.Hkv;
+        const int n_whole = (p.n_kt - p.split_tiles) * slabs, n_pieces = kSplit ? p.piece_end[p.split_pieces - 1] : 0;
+        split = kSplit && (p.whole_first ? block >= n_whole : block < n_pieces);
+        int idx = block - (!kSplit ? 0 : p.whole_first ? (split ? n_whole : 0) : (split ? 0 : n_pieces));
+        piece = 0;
+        if (split) {
+            while (idx >= p.piece_end[piece]) ++piece;
+            if (piece > 0) idx -= p.piece_end[piece - 1];
+        }
+        kt = idx / slabs;
+        slab = idx - kt * slabs;
+        if (!split) kt += p.split_tiles;
+        qt_first = p.causal ? kt : 0;
+        // with a sliding window the last query that sees this tile is (last key + window - 1), unless the tile holds
+        // global tokens, which every later query sees
+        const int qt_last = (kWin && kt * kT >= p.global_tokens) ? min(p.n_qt - 1, (kt * kT + kT - 1 + p.window - 1) / kT) : p.n_qt - 1;
+        per_head = qt_last - qt_first + 1;
+        n_iter = per_head > 0 ? per_head * group : 0;
+        int i0 = 0;
+        if (split) {
+            const int pieces = bwd_piece_count(n_iter, p.split_steps), len = (n_iter + pieces - 1) / pieces;
+            i0 = piece * len;
+            n_iter = min(len, n_iter - i0);
+        }
+        g_first = per_head > 0 ? i0 / per_head : 0;
+        r_first = i0 - g_first * per_head;
+    }
+};
+
 struct BwdBarriers {
-    uint64_t kv_full;
+    uint4 response;           // of the block scheduler
+    uint64_t response_full, work_full[2], work_empty[2];
+    BwdWork work[2];          // blocks in turn
+    uint64_t k_full, v_full;
     uint64_t q_full[3], q_empty[3], do_full[2], do_empty[2];
     uint64_t s_ready[2], p_ready[2], dp_ready, ds_ready, dq_ready, dq_drained, final_bar;
     uint32_t tmem_base;
@@ -278,10 +330,10 @@ __device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile
 
 // Epilogue of a compute warpgroup: its accumulator (dV for warpgroup 0, dK for warpgroup 1; `src` = TMEM address of this
 // thread's row) leaves as an fp32 partial (cut tiles), is added into the caller's fp32 accumulators, or is stored as bf16
-// through `stage_base` (a shared-memory tile no product reads any more).
+// through `stage` (4 KB of shared memory of this warp's own).
 template <int D, bool kMat>
 __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool split, int n_iter, int wg, int warp, int lane, int row,
-                                          uint32_t src, int kt, int slab, int slabs, int piece, int k0, uint8_t* stage_base)
+                                          uint32_t src, int kt, int slab, int slabs, int piece, int k0, uint8_t* stage)
 {
     if (split) {
         // this CTA's share of dV (warpgroup 0) / dK (warpgroup 1) as an fp32 partial; zeros if it saw no query
@@ -345,42 +397,38 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
     } else if (ok) {
         tc_fence_after();
         const int key = k0 + row;
-        const bool store = key < p.Skv;
         const float mul = wg == 0 ? 1.0f : p.scale;
-        // Coalesced bf16 store: a thread holds one whole key row, so the warp's 32 rows go through shared memory (the V
-        // tile's buffer for dV, the K tile's for dK: every product has retired) and leave with each store instruction
-        // covering whole rows; 16-byte units are XOR-swizzled by the row against bank conflicts.
-        (void)store;
+        // Coalesced bf16 store: a thread holds one whole key row, so the warp's 32 rows go through shared memory, 64 columns at a
+        // time, and leave with each store instruction covering 128 bytes of four rows; 16-byte units are XOR-swizzled by the row
+        // against bank conflicts.  The staging rows are the warp's own rows of the dS tile: every product that read them has
+        // retired, and only this warp writes them again.  (K and V are not: the next block's may be on their way.)
         __nv_bfloat16* out = (wg == 0 ? p.dv : p.dk) + (size_t)slab * p.Skv * D;
-        constexpr int kUnits = D / 8;
-        uint8_t* stage = stage_base + (warp & 3) * 32 * (D * 2);
+        const int sub = lane >> 3, unit0 = lane & 7, key_warp0 = key - lane;
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld32(src + (uint32_t)(c * 32), r);
-            tmem_ld_wait();
+        for (int half = 0; half < D / 64; ++half) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                uint4 w;
-                w.x = pack_bf16(__uint_as_float(r[8 * v + 0]) * mul, __uint_as_float(r[8 * v + 1]) * mul);
-                w.y = pack_bf16(__uint_as_float(r[8 * v + 2]) * mul, __uint_as_float(r[8 * v + 3]) * mul);
-                w.z = pack_bf16(__uint_as_float(r[8 * v + 4]) * mul, __uint_as_float(r[8 * v + 5]) * mul);
-                w.w = pack_bf16(__uint_as_float(r[8 * v + 6]) * mul, __uint_as_float(r[8 * v + 7]) * mul);
-                const int unit = c * 4 + v;
-                *reinterpret_cast<uint4*>(stage + lane * (D * 2) + ((unit ^ (lane & 7)) << 4)) = w;
+            for (int c = 0; c < 2; ++c) {
+                uint32_t r[32];
+                tmem_ld32(src + (uint32_t)(half * 64 + c * 32), r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    uint4 w;
+                    w.x = pack_bf16(__uint_as_float(r[8 * v + 0]) * mul, __uint_as_float(r[8 * v + 1]) * mul);
+                    w.y = pack_bf16(__uint_as_float(r[8 * v + 2]) * mul, __uint_as_float(r[8 * v + 3]) * mul);
+                    w.z = pack_bf16(__uint_as_float(r[8 * v + 4]) * mul, __uint_as_float(r[8 * v + 5]) * mul);
+                    w.w = pack_bf16(__uint_as_float(r[8 * v + 6]) * mul, __uint_as_float(r[8 * v + 7]) * mul);
+                    *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + v) ^ (lane & 7)) << 4)) = w;
+                }
             }
-        }
-        __syncwarp();
-        {
-            constexpr int kRowsPerStore = 32 / kUnits;
-            const int sub = lane / kUnits, unit = lane % kUnits;
-            const int key_warp0 = key - lane;               // first key row of this warp
+            __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 32 / kRowsPerStore; ++i) {
-                const int rr = i * kRowsPerStore + sub;
-                const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * (D * 2) + ((unit ^ (rr & 7)) << 4));
-                if (key_warp0 + rr < p.Skv) *reinterpret_cast<uint4*>(out + (size_t)(key_warp0 + rr) * D + unit * 8) = w;
+            for (int i = 0; i < 8; ++i) {
+                const int rr = i * 4 + sub;
+                const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((unit0 ^ (rr & 7)) << 4));
+                if (key_warp0 + rr < p.Skv) *reinterpret_cast<uint4*>(out + (size_t)(key_warp0 + rr) * D + half * 64 + unit0 * 8) = w;
             }
+            __syncwarp();
         }
     } else if (n_iter == 0 && p.dk_acc == nullptr) {
         // a key tile no query can see (cannot happen for causal with Sq == Skv; kept for safety): zero grads
@@ -463,43 +511,25 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         return;
     }
 
-    // ---- work decode: key tile 0 sees every query tile, so low key tiles go first ----
-    const int slabs = p.B * p.Hkv;
     const int group = p.Hq / p.Hkv;
-    // whole tiles as one CTA per (tile, slab), cut ones as one per (tile, piece, slab); the kind with the longest CTAs first
-    const int n_whole = (p.n_kt - p.split_tiles) * slabs, n_pieces = kSplit ? p.split_tiles * p.split_pieces * slabs : 0;
-    const bool split = kSplit && (p.whole_first ? (int)blockIdx.x >= n_whole : (int)blockIdx.x < n_pieces);
-    const int idx = (int)blockIdx.x - (!kSplit ? 0 : p.whole_first ? (split ? n_whole : 0) : (split ? 0 : n_pieces)), rest = idx / slabs;
-    const int slab = idx - rest * slabs;                // b * Hkv + hk
-    const int kt = split ? rest / p.split_pieces : p.split_tiles + rest, piece = split ? rest - kt * p.split_pieces : 0;
-    const int b = slab / p.Hkv, hk = slab - b * p.Hkv;
-    const int k0 = kt * kT;
-    const int qt_first = p.causal ? kt : 0;
-    // with a sliding window the last query that sees this tile is (last key + window - 1), unless the tile holds
-    // global tokens, which every later query sees
-    const int qt_last = (kWin && k0 >= p.global_tokens) ? min(p.n_qt - 1, (k0 + kT - 1 + p.window - 1) / kT) : p.n_qt - 1;
-    const int per_head = qt_last - qt_first + 1;        // query tiles per head this CTA visits
-    int n_iter = per_head > 0 ? per_head * group : 0;   // steps of this CTA: all of the tile's, or its piece of them from step i0 on
-    int i0 = 0;
-    if (split) {
-        const int pieces = bwd_piece_count(n_iter, p.split_steps), len = (n_iter + pieces - 1) / pieces;
-        i0 = piece * len;
-        n_iter = min(len, n_iter - i0);
-        if (piece >= pieces || n_iter <= 0) return;     // (uniform over the CTA, before anything is set up)
-    }
-    const int g_first = per_head > 0 ? i0 / per_head : 0, r_first = i0 - g_first * per_head;   // head and query tile of the first step
-
+    BwdWork w;          // (the producer's)
     if (warp == 13 && lane == 0) {
+        w.decode<kWin, kSplit>(p, (int)blockIdx.x);
+        bars->work[0] = w;
         prefetch_tensormap(&tmap_q);
         prefetch_tensormap(&tmap_k);
         prefetch_tensormap(&tmap_v);
         prefetch_tensormap(&tmap_do);
-        mbar_init(&bars->kv_full, 1);
+        mbar_init(&bars->response_full, 1);
+        mbar_init(&bars->k_full, 1);
+        mbar_init(&bars->v_full, 1);
         for (int i = 0; i < 3; ++i) {
             mbar_init(&bars->q_full[i], 1);
             mbar_init(&bars->q_empty[i], 2);
         }
         for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->work_full[i], 1);
+            mbar_init(&bars->work_empty[i], 14);    // every warp but the idle one and the producer
             mbar_init(&bars->do_full[i], 1);
             mbar_init(&bars->do_empty[i], 2);
             mbar_init(&bars->s_ready[i], 1);
@@ -534,6 +564,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // 512 threads start with 128 registers each; the issuing/producer warpgroup needs few, the others get the rest
     // (each role re-allocates registers inside its own branch so that the compiler sees which register count applies where)
 
+    // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Step counters run
+    // on over the blocks (n0: steps before this block, blocks: how many before it had steps), so stages and barrier phases continue
+    // where they are.  next(u): done with block u; whether another follows.
+    auto next = [&](int u) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->work_empty[u & 1]);
+        return mbar_wait_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && bars->work[(u + 1) & 1].n_iter >= 0;
+    };
 
     if (warp == 15) {
         setmaxnreg_dec<56>();
@@ -541,36 +579,66 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     } else if (warp == 13) {
         setmaxnreg_dec<56>();
         // =========================== TMA producer ===========================
-        if (lane == 0 && n_iter > 0) {
-            mbar_arrive_expect_tx(&bars->kv_full, (uint32_t)(2 * kTileBytes));
-            for (int c = 0; c < kChunks; ++c) {
-                tma_load_3d(sK + c * kChunkBytes, &tmap_k, &bars->kv_full, c * 64, k0, slab);
-                tma_load_3d(sV + c * kChunkBytes, &tmap_v, &bars->kv_full, c * 64, k0, slab);
-            }
-            int g = g_first, r = r_first;
-            for (int i = 0; i < n_iter; ++i) {
-                const int qt = qt_first + r, bh = b * p.Hq + hk * group + g;
-                if (++r == per_head) { r = 0; ++g; }
-                const int sq = i % kQStages;
-                if (i >= kQStages && !mbar_wait(&bars->q_empty[sq], (uint32_t)(((i / kQStages) - 1) & 1), abort_flag, kSiteQEmpty)) break;
-                mbar_arrive_expect_tx(&bars->q_full[sq], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 2 * kT * 4)));
-                for (int c = 0; c < kChunks; ++c)
-                    tma_load_3d(sQ + sq * kTileBytes + c * kChunkBytes, &tmap_q, &bars->q_full[sq], c * 64, qt * kT, bh);
-                if constexpr (kAug) {
-                    bulk_load_1d(sQaug + sq * kAugBytes, p.qaug + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kAugBytes, &bars->q_full[sq]);
-                } else {
-                    bulk_load_1d(sLse + sq * kT, p.lse2 + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kT * 4, &bars->q_full[sq]);
-                    bulk_load_1d(sDelta + sq * kT, p.delta + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kT * 4, &bars->q_full[sq]);
+        if (lane == 0) {
+            int n0 = 0, blocks = 0;
+            bool ok = true;
+            for (int u = 0, block = 0; block >= 0; ++u) {
+                // K and V: once every product of the block before has read them
+                if (w.n_iter > 0) {
+                    ok = blocks == 0 || mbar_wait(&bars->final_bar, (uint32_t)((blocks - 1) & 1), abort_flag, kSiteFinal);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&bars->k_full, (uint32_t)kTileBytes);
+                    for (int c = 0; c < kChunks; ++c) tma_load_3d(sK + c * kChunkBytes, &tmap_k, &bars->k_full, c * 64, w.kt * kT, w.slab);
+                    ++blocks;
                 }
-                const int sd = i % kDoStages;
-                if (i >= kDoStages &&
-                    !mbar_wait(&bars->do_empty[sd], (uint32_t)(((i / kDoStages) - 1) & 1), abort_flag, kSiteDoEmpty))
-                    break;
-                mbar_arrive_expect_tx(&bars->do_full[sd], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 0)));
-                if constexpr (kAug)
-                    bulk_load_1d(sDoaug + sd * kAugBytes, p.doaug + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kAugBytes, &bars->do_full[sd]);
-                for (int c = 0; c < kChunks; ++c)
-                    tma_load_3d(sDo + sd * kTileBytes + c * kChunkBytes, &tmap_do, &bars->do_full[sd], c * 64, qt * kT, bh);
+                const int bh0 = w.slab * group;      // b * Hq + hk * group
+                int g = w.g_first, r = w.r_first;
+                for (int i = 0; i < w.n_iter; ++i) {
+                    const int qt = w.qt_first + r, bh = bh0 + g, n = n0 + i;
+                    if (++r == w.per_head) { r = 0; ++g; }
+                    const int sq = n % kQStages;
+                    if (n >= kQStages && !(ok = mbar_wait(&bars->q_empty[sq], (uint32_t)(((n / kQStages) - 1) & 1), abort_flag, kSiteQEmpty))) break;
+                    mbar_arrive_expect_tx(&bars->q_full[sq], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 2 * kT * 4)));
+                    for (int c = 0; c < kChunks; ++c)
+                        tma_load_3d(sQ + sq * kTileBytes + c * kChunkBytes, &tmap_q, &bars->q_full[sq], c * 64, qt * kT, bh);
+                    if constexpr (kAug) {
+                        bulk_load_1d(sQaug + sq * kAugBytes, p.qaug + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kAugBytes, &bars->q_full[sq]);
+                    } else {
+                        bulk_load_1d(sLse + sq * kT, p.lse2 + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kT * 4, &bars->q_full[sq]);
+                        bulk_load_1d(sDelta + sq * kT, p.delta + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kT * 4, &bars->q_full[sq]);
+                    }
+                    if (i == 0) {
+                        mbar_arrive_expect_tx(&bars->v_full, (uint32_t)kTileBytes);
+                        for (int c = 0; c < kChunks; ++c) tma_load_3d(sV + c * kChunkBytes, &tmap_v, &bars->v_full, c * 64, w.kt * kT, w.slab);
+                    }
+                    const int sd = n % kDoStages;
+                    if (n >= kDoStages &&
+                        !(ok = mbar_wait(&bars->do_empty[sd], (uint32_t)(((n / kDoStages) - 1) & 1), abort_flag, kSiteDoEmpty)))
+                        break;
+                    mbar_arrive_expect_tx(&bars->do_full[sd], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 0)));
+                    if constexpr (kAug)
+                        bulk_load_1d(sDoaug + sd * kAugBytes, p.doaug + (size_t)bh * p.Sq_pad + (size_t)qt * kT, kAugBytes, &bars->do_full[sd]);
+                    for (int c = 0; c < kChunks; ++c)
+                        tma_load_3d(sDo + sd * kTileBytes + c * kChunkBytes, &tmap_do, &bars->do_full[sd], c * 64, qt * kT, bh);
+                }
+                if (!ok) break;
+                n0 += w.n_iter;
+                // The next block is asked for one or two steps before this one ends, in time to have the answer: asked for at its
+                // start, it would go to this CTA even if others are free sooner (B3 Hq16 Hkv4 S1237 D128, reproducible: 183 us instead of
+                // 134; blocks left to the hardware's own order: 138).
+                block = -1;
+                if (p.several_waves) {
+                    mbar_arrive_expect_tx(&bars->response_full, 16);
+                    clc_try_cancel(&bars->response, &bars->response_full);
+                    if (!mbar_wait(&bars->response_full, (uint32_t)(u & 1), abort_flag, kSiteNext)) break;
+                    block = clc_first_block(&bars->response);
+                    fence_proxy_async_smem();
+                }
+                w.n_iter = -1;
+                if (block >= 0) w.decode<kWin, kSplit>(p, block);
+                if (u >= 1 && !mbar_wait(&bars->work_empty[(u + 1) & 1], (uint32_t)(((u - 1) >> 1) & 1), abort_flag, kSiteNext)) break;
+                bars->work[(u + 1) & 1] = w;
+                mbar_arrive(&bars->work_full[(u + 1) & 1]);
             }
         }
     } else if (warp == 12 || warp == 14) {
@@ -587,7 +655,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         // can only be loaded once both have, and dP^T_{i+1} waits for that load.
         // (Two, not more: MMAs issued by different warps interleave in the tensor pipe k-step by k-step, each on another
         // accumulator, and a third issuing warp for dK measured 7-20 % slower than this split at either head size.)
-        if (warp == 12 && n_iter > 0) {
+        if (warp == 12) {
             // P side: all 32 lanes walk the loop (warp-uniform control flow lets descriptors and addresses live in uniform
             // registers) and one elected lane issues the products four k-steps at a time (mma_ss_4).
             SNTL_TRACE_DECL(tn);
@@ -608,41 +676,54 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 mma_ts_4<8, 128>(d_tmem, a_tmem, b, idesc_kv, accumulate);
                 mma_ts_4<8, 128>(d_tmem, a_tmem + 64u, sdesc_advance(b, 4 * 2048), idesc_kv, 1);
             };
-            bool ok = wait(&bars->kv_full, 0, kSiteKV);
             const uint64_t dK_k = make_sdesc(smem_u32(sK), 16, 1024);
             const uint64_t dQ_k0 = make_sdesc(smem_u32(sQ), 16, 1024), dDo_mn0 = make_sdesc(smem_u32(sDo), kChunkBytes, 1024);
-            // S^T of the first kSBufs steps; after that S^T_{i+kSBufs} follows dV_i into the buffer that P^T_i leaves
-            for (int j = 0; ok && j < kSBufs && j < n_iter; ++j) {
-                if (!(ok = wait(&bars->q_full[j], 0, kSiteQFull))) break;
-                tc_fence_after();
-                issue_kmajor(tm_S + (uint32_t)j * kSBufStride, dK_k, sdesc_advance(dQ_k0, j * kTileBytes), sdesc_advance(d_qaug0, j * kAugBytes));
-                tc_commit_p(&bars->s_ready[j]);
-            }
-            for (int i = 0; ok && i < n_iter; ++i) {
-                const int sq = i % kQStages, sd = i % kDoStages, sb = i % kSBufs;
-                const uint32_t tm_Si = tm_S + (uint32_t)sb * kSBufStride;
-                // one barrier per S^T buffer: with two buffers the threads of one warpgroup can be through step i + 1 while a
-                // warp of the other has not stored its P^T_i yet, and a single barrier would count their second arrival for it
-                if (!(ok = wait(&bars->p_ready[sb], (uint32_t)((i / kSBufs) & 1), kSiteP))) break;
-                if (!(ok = wait(&bars->do_full[sd], (uint32_t)((i / kDoStages) & 1), kSiteDoFull))) break;
-                SNTL_TRACE_EV(tl, 0, tn, 1);
-                tc_fence_after();
-                issue_from_tmem(tm_dV, tm_Si, sdesc_advance(dDo_mn0, sd * kTileBytes), i > 0);
-                tc_commit_p(&bars->do_empty[sd]);
-                tc_commit_p(&bars->q_empty[sq]);
-                SNTL_TRACE_EV(tl, 0, tn, 2);
-                if (i + kSBufs < n_iter) {
-                    const int nq = (i + kSBufs) % kQStages;
-                    if (!(ok = wait(&bars->q_full[nq], (uint32_t)(((i + kSBufs) / kQStages) & 1), kSiteQFull))) break;
+            int n0 = 0, blocks = 0;
+            bool ok = true;
+            bool more = true;
+            for (int u = 0; more; more = next(u++)) {
+                const int end = n0 + bars->work[u & 1].n_iter;
+                if (end == n0) continue;
+                if (!(ok = wait(&bars->k_full, (uint32_t)(blocks & 1), kSiteKV))) break;
+                // S^T of the first kSBufs steps; after that S^T_{n+kSBufs} follows dV_n into the buffer that P^T_n leaves
+                for (int n = n0; n < n0 + kSBufs && n < end; ++n) {
+                    const int sq = n % kQStages, sb = n % kSBufs;
+                    if (!(ok = wait(&bars->q_full[sq], (uint32_t)((n / kQStages) & 1), kSiteQFull))) break;
                     tc_fence_after();
-                    issue_kmajor(tm_Si, dK_k, sdesc_advance(dQ_k0, nq * kTileBytes), sdesc_advance(d_qaug0, nq * kAugBytes));
+                    issue_kmajor(tm_S + (uint32_t)sb * kSBufStride, dK_k, sdesc_advance(dQ_k0, sq * kTileBytes), sdesc_advance(d_qaug0, sq * kAugBytes));
                     tc_commit_p(&bars->s_ready[sb]);
-                    SNTL_TRACE_EV(tl, 0, tn, 9);
                 }
+                for (int n = n0; ok && n < end; ++n) {
+                    const int sq = n % kQStages, sd = n % kDoStages, sb = n % kSBufs;
+                    const uint32_t tm_Si = tm_S + (uint32_t)sb * kSBufStride;
+                    // one barrier per S^T buffer: with two buffers the threads of one warpgroup can be through step n + 1 while a
+                    // warp of the other has not stored its P^T_n yet, and a single barrier would count their second arrival for it
+                    if (!(ok = wait(&bars->p_ready[sb], (uint32_t)((n / kSBufs) & 1), kSiteP))) break;
+                    if (!(ok = wait(&bars->do_full[sd], (uint32_t)((n / kDoStages) & 1), kSiteDoFull))) break;
+                    SNTL_TRACE_EV(tl, 0, tn, 1);
+                    tc_fence_after();
+                    // (the first dV of a block overwrites the accumulator: the compute warps arrive at p_ready behind their epilogue)
+                    issue_from_tmem(tm_dV, tm_Si, sdesc_advance(dDo_mn0, sd * kTileBytes), n > n0);
+                    tc_commit_p(&bars->do_empty[sd]);
+                    tc_commit_p(&bars->q_empty[sq]);
+                    SNTL_TRACE_EV(tl, 0, tn, 2);
+                    if (n + kSBufs < end) {
+                        const int nq = (n + kSBufs) % kQStages;
+                        if (!(ok = wait(&bars->q_full[nq], (uint32_t)(((n + kSBufs) / kQStages) & 1), kSiteQFull))) break;
+                        tc_fence_after();
+                        issue_kmajor(tm_Si, dK_k, sdesc_advance(dQ_k0, nq * kTileBytes), sdesc_advance(d_qaug0, nq * kAugBytes));
+                        tc_commit_p(&bars->s_ready[sb]);
+                        SNTL_TRACE_EV(tl, 0, tn, 9);
+                    }
+                }
+                if (!ok) break;
+                tc_commit_p(&bars->final_bar);
+                n0 = end;
+                ++blocks;
             }
-            tc_commit_p(&bars->final_bar);
-            wait(&bars->final_bar, 0, kSiteFinal);
-        } else if (warp == 14 && n_iter > 0) {
+            if (!ok) tc_commit_p(&bars->final_bar);
+            else if (blocks > 0) wait(&bars->final_bar, (uint32_t)((blocks - 1) & 1), kSiteFinal);
+        } else {
             // dS side, in the same form
             const bool tl14 = lane == 0;
             (void)tl14;
@@ -660,63 +741,67 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     mma_ss_4<2, 2>(d_tmem, sdesc_advance(a, (uint32_t)(c * kChunkBytes)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_st, c > 0);
                 if constexpr (kAug) mma_ss_1(d_tmem, d_ones, aug, idesc_st);
             };
-            bool ok = wait(&bars->kv_full, 0, kSiteKV);
-            {
-                const uint64_t dV_k = make_sdesc(smem_u32(sV), 16, 1024), dDo_k0 = make_sdesc(smem_u32(sDo), 16, 1024);
-                const uint64_t dK_mn = make_sdesc(smem_u32(sK), kChunkBytes, 1024), dDs_mn = make_sdesc(smem_u32(sDs), kChunkBytes, 1024);
-                const uint64_t dDs_k = make_sdesc(smem_u32(sDs), 16, 1024);
-                const uint64_t dQ_mn0 = make_sdesc(smem_u32(sQ), kChunkBytes, 1024);
-                ok = ok && wait(&bars->do_full[0], 0, kSiteDoFull);
-                if (ok) {
+            const uint64_t dV_k = make_sdesc(smem_u32(sV), 16, 1024), dDo_k0 = make_sdesc(smem_u32(sDo), 16, 1024);
+            const uint64_t dK_mn = make_sdesc(smem_u32(sK), kChunkBytes, 1024), dDs_mn = make_sdesc(smem_u32(sDs), kChunkBytes, 1024);
+            const uint64_t dDs_k = make_sdesc(smem_u32(sDs), 16, 1024);
+            const uint64_t dQ_mn0 = make_sdesc(smem_u32(sQ), kChunkBytes, 1024);
+            int n0 = 0, blocks = 0;
+            bool ok = true;
+            bool more = true;
+            for (int u = 0; more; more = next(u++)) {
+                const int end = n0 + bars->work[u & 1].n_iter;
+                if (end == n0) continue;
+                // dP^T of step n, into the columns that dQ of the step before has left
+                auto issue_dp = [&](int n) {
+                    const int nd = n % kDoStages;
+                    if (n > 0 && !wait(&bars->dq_drained, (uint32_t)((n - 1) & 1), kSiteDrained)) return false;
+                    SNTL_TRACE_EV(tl14, 4, tn, 5);
+                    if (!wait(&bars->do_full[nd], (uint32_t)((n / kDoStages) & 1), kSiteDoFull)) return false;
                     tc_fence_after();
-                    issue_kmajor(tm_dP, dV_k, dDo_k0, d_doaug0);
+                    issue_kmajor(tm_dP, dV_k, sdesc_advance(dDo_k0, nd * kTileBytes), sdesc_advance(d_doaug0, nd * kAugBytes));
                     tc_commit_p(&bars->dp_ready);
-                    tc_commit_p(&bars->do_empty[0]);   // this warp's share of releasing dO_0: dP^T_0
-                }
-                for (int i = 0; ok && i < n_iter; ++i) {
-                    const uint32_t ph = (uint32_t)(i & 1);
-                    const int sq = i % kQStages;
-                    if (!(ok = wait(&bars->ds_ready, ph, kSiteDS))) break;
+                    // this warp's share of releasing dO_n, committed at once: with a single dO stage the load of the
+                    // next tile starts as soon as this product and dV_n have read the stage
+                    tc_commit_p(&bars->do_empty[nd]);
+                    SNTL_TRACE_EV(tl14, 4, tn, 6);
+                    return true;
+                };
+                if (!(ok = wait(&bars->k_full, (uint32_t)(blocks & 1), kSiteKV) && wait(&bars->v_full, (uint32_t)(blocks & 1), kSiteKV) && issue_dp(n0))) break;
+                for (int n = n0; n < end; ++n) {
+                    const int sq = n % kQStages;
+                    if (!(ok = wait(&bars->ds_ready, (uint32_t)(n & 1), kSiteDS))) break;
                     SNTL_TRACE_EV(tl14, 4, tn, 3);
                     tc_fence_after();
                     // dQ first: it gates the drain and with it the next dP^T
-                    const uint32_t ds_off = (uint32_t)((i % kDsBufs) * kDsBytes);
+                    const uint32_t ds_off = (uint32_t)((n % kDsBufs) * kDsBytes);
                     const uint64_t ds_mn = sdesc_advance(dDs_mn, ds_off);
                     mma_ss_4<128, 128>(tm_dP, ds_mn, dK_mn, idesc_dq, 0);
                     mma_ss_4<128, 128>(tm_dP, sdesc_advance(ds_mn, 4 * 2048), sdesc_advance(dK_mn, 4 * 2048), idesc_dq, 1);
                     tc_commit_p(&bars->dq_ready);
                     SNTL_TRACE_EV(tl14, 4, tn, 4);
                     // dK += dS^T Q with dS^T read from its shared-memory tile as a K-major A operand (rows = keys, the 64
-                    // contiguous elements run along the queries).  Q_i is ready: ds_ready implies its load was seen.  With
+                    // contiguous elements run along the queries).  Q_n is ready: ds_ready implies its load was seen.  With
                     // one dS buffer it goes before the next dP^T: by the time the compute warps see that dP^T and rewrite the
                     // tile, this product has read it (one thread's MMAs run in order).  With two it goes after, and the
-                    // buffer it reads is rewritten only behind dP^T_{i+2}, which this thread issues later still.
+                    // buffer it reads is rewritten only behind dP^T_{n+2}, which this thread issues later still.
                     auto issue_dk = [&]() {
                         const uint64_t a = sdesc_advance(dDs_k, ds_off), bq = sdesc_advance(dQ_mn0, sq * kTileBytes);
-                        mma_ss_4<2, 128>(tm_dK, a, bq, idesc_kv, i > 0);
+                        mma_ss_4<2, 128>(tm_dK, a, bq, idesc_kv, n > n0);
                         mma_ss_4<2, 128>(tm_dK, sdesc_advance(a, kChunkBytes), sdesc_advance(bq, 4 * 2048), idesc_kv, 1);
-                        tc_commit_p(&bars->q_empty[sq]);    // this warp's share: dK_i
+                        tc_commit_p(&bars->q_empty[sq]);    // this warp's share: dK_n
                     };
                     if constexpr (kDsBufs == 1) issue_dk();
-                    if (i + 1 < n_iter) {
-                        const int nd = (i + 1) % kDoStages;
-                        if (!(ok = wait(&bars->dq_drained, ph, kSiteDrained))) break;
-                        SNTL_TRACE_EV(tl14, 4, tn, 5);
-                        if (!(ok = wait(&bars->do_full[nd], (uint32_t)(((i + 1) / kDoStages) & 1), kSiteDoFull))) break;
-                        tc_fence_after();
-                        issue_kmajor(tm_dP, dV_k, sdesc_advance(dDo_k0, nd * kTileBytes), sdesc_advance(d_doaug0, nd * kAugBytes));
-                        tc_commit_p(&bars->dp_ready);
-                        // this warp's share of releasing dO_{i+1}, committed at once: with a single dO stage the load of the
-                        // next tile starts as soon as this product and dV_{i+1} have read the stage
-                        tc_commit_p(&bars->do_empty[nd]);
-                        SNTL_TRACE_EV(tl14, 4, tn, 6);
-                    }
+                    if (n + 1 < end && !(ok = issue_dp(n + 1))) break;
                     if constexpr (kDsBufs == 2) issue_dk();
                 }
+                if (!ok) break;
+                // every MMA of this thread has retired once its commit lands; the epilogue waits for both issuers
+                tc_commit_p(&bars->final_bar);
+                n0 = end;
+                ++blocks;
             }
-            // every MMA of this thread has retired once its commit lands; the epilogue waits for both issuers
-            tc_commit_p(&bars->final_bar);
-            wait(&bars->final_bar, 0, kSiteFinal);
+            if (!ok) tc_commit_p(&bars->final_bar);
+            else if (blocks > 0) wait(&bars->final_bar, (uint32_t)((blocks - 1) & 1), kSiteFinal);
         }
     } else if (warp >= 8) {
         setmaxnreg_inc<152>();
@@ -729,13 +814,18 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const bool elected = warp == 8 && lane == 0;
         bool ok = true;
         uint32_t piece = 0;
-        int g = g_first, tile_r = r_first;
-        for (int i = 0; i < n_iter; ++i) {
-            const int qt = qt_first + tile_r, bh = b * p.Hq + hk * group + g;
-            if (++tile_r == per_head) { tile_r = 0; ++g; }
+        int n = 0;
+        bool more = true;
+        for (int u = 0; ok && more; more = next(u++)) {
+        const BwdWork w = bars->work[u & 1];
+        const int bh0 = w.slab * group;      // b * Hq + hk * group
+        int g = w.g_first, tile_r = w.r_first;
+        for (const int end = n + w.n_iter; n < end; ++n) {
+            const int qt = w.qt_first + tile_r, bh = bh0 + g;
+            if (++tile_r == w.per_head) { tile_r = 0; ++g; }
             // fp32 accumulator: kT*D words per tile; fixed-point accumulator: kT*D 64-bit words per tile
             float* tile = p.dq_accum + ((size_t)bh * p.n_qt + qt) * (size_t)(kT * D) * (kDet ? 2 : 1);
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->dq_ready, (uint32_t)(i & 1), abort_flag, kSiteDQ));
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->dq_ready, (uint32_t)(n & 1), abort_flag, kSiteDQ));
             SNTL_TRACE_EV(tw, 3, tn, 1);
             if (!ok) break;
             tc_fence_after();
@@ -757,6 +847,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             push_dq_tile<D, kDet, kStageCols, kStagingBytes>(r, tile, sStage, row, elected, piece);
             SNTL_TRACE_EV(tw, 3, tn, 3);
         }
+        }
         if (elected) bulk_wait_all();   // the reductions read shared memory and must land before the CTA retires
     } else {
         setmaxnreg_inc<152>();
@@ -770,16 +861,22 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const uint32_t col0 = (uint32_t)(wg * 64);
         uint8_t* ds_row0 = sDs + wg * kChunkBytes + row * 128;   // this thread's 128-byte row of its 64-query chunk
         bool ok = true;
-        int tile_r = r_first;
-        for (int i = 0; i < n_iter; ++i) {
+        int n = 0, blocks = 0;
+        bool more = true;
+        for (int u = 0; ok && more; more = next(u++)) {
+        const BwdWork& w = bars->work[u & 1];
+        const int qt_first = w.qt_first, per_head = w.per_head, n_iter = w.n_iter;
+        const int kt = w.kt, k0 = kt * kT;
+        int tile_r = w.r_first;
+        for (const int end = n + n_iter; n < end; ++n) {
             const int qt = qt_first + tile_r;
             if (++tile_r == per_head) tile_r = 0;
-            const uint32_t ph = (uint32_t)(i & 1);
+            const uint32_t ph = (uint32_t)(n & 1);
             // ---- P^T ----
-            const uint32_t tm_Si = tm_S + (uint32_t)(i % kSBufs) * kSBufStride;
+            const uint32_t tm_Si = tm_S + (uint32_t)(n % kSBufs) * kSBufStride;
             // (the Q stage's barrier also covers the LSE and delta columns this warp reads when they come as plain columns)
-            ok = __all_sync(0xffffffffu, (kAug || mbar_wait(&bars->q_full[i % kQStages], (uint32_t)((i / kQStages) & 1), abort_flag, kSiteQFull)) &&
-                                             mbar_wait(&bars->s_ready[i % kSBufs], (uint32_t)((i / kSBufs) & 1), abort_flag, kSiteS));
+            ok = __all_sync(0xffffffffu, (kAug || mbar_wait(&bars->q_full[n % kQStages], (uint32_t)((n / kQStages) & 1), abort_flag, kSiteQFull)) &&
+                                             mbar_wait(&bars->s_ready[n % kSBufs], (uint32_t)((n / kSBufs) & 1), abort_flag, kSiteS));
             SNTL_TRACE_EV(tw, 1 + wg, tn, 1);
             if (!ok) break;
             tc_fence_after();
@@ -792,7 +889,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             const bool diag = (p.causal && qt == kt) || (kWin && qt * kT + kT - 1 > k0 + p.window - 1);
             uint32_t pk[32];
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-            const float4* lse4 = reinterpret_cast<const float4*>(sLse + (i % kQStages) * kT + col0);
+            const float4* lse4 = reinterpret_cast<const float4*>(sLse + (n % kQStages) * kT + col0);
             // exponents of four columns: with the extra contraction step the product already holds S^T - LSE/scale and one
             // packed multiply per pair gives them; else x = s*scale*log2(e) - LSE*log2(e) is one packed FMA per pair
             auto exponents = [&](int c, float2& x01, float2& x23) {
@@ -839,7 +936,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             tmem_st32(tm_Si + lane_off + col0, pk);
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(&bars->p_ready[i % kSBufs]);
+            mbar_arrive(&bars->p_ready[n % kSBufs]);
             SNTL_TRACE_EV(tw, 1 + wg, tn, 4);
             // ---- dS^T ----
             ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_ready, ph, abort_flag, kSiteDP));
@@ -850,7 +947,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             tmem_ld32(tm_dP + lane_off + col0 + 32u, s + 32);
             tmem_ld_wait();
             SNTL_TRACE_EV(tw, 1 + wg, tn, 6);
-            const float4* dl4 = reinterpret_cast<const float4*>(sDelta + (i % kQStages) * kT + col0);
+            const float4* dl4 = reinterpret_cast<const float4*>(sDelta + (n % kQStages) * kT + col0);
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
                 if constexpr (kAug) {
@@ -870,7 +967,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             // into shared memory, rows of 128 bytes with the 128-byte swizzle the MMA expects (both the dQ and the dK
             // product read this tile)
-            uint8_t* ds_row = ds_row0 + (i % kDsBufs) * kDsBytes;
+            uint8_t* ds_row = ds_row0 + (n % kDsBufs) * kDsBytes;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 uint4 w = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
@@ -883,9 +980,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             SNTL_TRACE_EV(tw, 1 + wg, tn, 8);
         }
         // ---- epilogue: dV (warpgroup 0) and dK (warpgroup 1) ----
-        ok = __all_sync(0xffffffffu, ok && n_iter > 0 && mbar_wait(&bars->final_bar, 0, abort_flag, kSiteFinal));
-        write_dkv<D, kMat>(p, ok, split, n_iter, wg, warp, lane, row, (wg == 0 ? tm_dV : tm_dK) + lane_off, kt, slab, slabs, piece, k0,
-                     wg == 0 ? sV : sK);
+        const bool done = __all_sync(0xffffffffu, ok && n_iter > 0 && mbar_wait(&bars->final_bar, (uint32_t)(blocks & 1), abort_flag, kSiteFinal));
+        if (n_iter > 0) {
+            ok = done;
+            ++blocks;
+        }
+        write_dkv<D, kMat>(p, done, w.split != 0, n_iter, wg, warp, lane, row, (wg == 0 ? tm_dV : tm_dK) + lane_off, kt, w.slab, p.B * p.Hkv, w.piece, k0,
+                               sDs + warp * 32 * 128);
+        }
     }
 
     // ---- teardown ----
@@ -1159,7 +1261,18 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     p.scale = s.scale;
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const int slabs = s.B * s.Hkv;
-    const long long ctas = (long long)p.split_tiles * cut.pieces * slabs + (long long)(n_kt - p.split_tiles) * slabs;
+    long long ctas = (long long)(n_kt - p.split_tiles) * slabs, n_pieces = 0;
+    if (cut.pieces > kMaxPieces) return cudaErrorInvalidValue;
+    for (int piece = 0; piece < cut.pieces; ++piece) {      // (a later tile has no more steps than an earlier one)
+        for (int kt = 0; kt < cut.tiles; ++kt) {
+            const int steps = bwd_tiles_per_head(kt, n_qt, s.causal, p.window, s.global_tokens) * (s.Hq / s.Hkv);
+            const int pieces = bwd_piece_count(steps, cut.steps), len = (steps + pieces - 1) / pieces;
+            if (piece * len < steps) n_pieces += slabs;
+        }
+        p.piece_end[piece] = (int)n_pieces;
+    }
+    ctas += n_pieces;
+    p.several_waves = ctas > sm_count();
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     static std::atomic<unsigned long long> configured{0};   // per instantiation, one bit per device
     {

@@ -154,6 +154,30 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Cluster launch control: asks the block scheduler to hand a block of this grid that has not started yet to the caller.  The
+// 16-byte response arrives like a copy (expect_tx 16); clc_first_block reads it: the block's index, or -1 if none is left (then
+// the caller asks no more).
+__device__ __forceinline__ void clc_try_cancel(void* response, uint64_t* bar)
+{
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(response)),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ int clc_first_block(const void* response)
+{
+    int block;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+        "ld.shared.b128 r, [%1];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+        "mov.b32 %0, -1;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t}"
+        : "=r"(block)
+        : "r"(smem_u32(response))
+        : "memory");
+    return block;
+}
+
 // barrier among a subset of the CTA's warps (id 1..15; `threads` a multiple of 32)
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads)
 {

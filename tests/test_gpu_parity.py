@@ -418,6 +418,32 @@ def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
         assert float((got.float() - want).norm() / want.norm()) <= tol
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,kw", [
+    (40, 8, 8, 100, 100, 64, {}),                                 # 320 blocks of one step each
+    (30, 6, 6, 129, 129, 128, {}),                                # one- and two-step blocks, the last with one query
+    (9, 12, 6, 700, 700, 64, dict(window=150, global_tokens=3)),
+    (3, 36, 12, 640, 640, 128, dict(flags=4)),                    # cut tiles among whole ones
+    (20, 8, 8, 150, 260, 64, dict(causal=False)),
+])
+def test_backward_blocks_taken_over_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, kw):
+    """More blocks than SMs, so that every CTA computes several in turn, of equal and of different lengths, against the exact
+    kernels on the same bf16 values (bounds as for the cut pieces above); dK, dV do not depend on which CTA took which block."""
+    w = sb.WORKLOADS["gqa7b_d128"]
+    g = torch.Generator(device="cuda").manual_seed(Sq + B)
+    q, k, v, do = ((torch.randn(B, H, S, D, generator=g, device="cuda") * std).to(torch.bfloat16)
+                   for H, S, std in ((Hq, Sq, 0.5), (Hkv, Sk, 0.5), (Hkv, Sk, 1.0), (Hq, Sq, w.do_std)))
+    fwd = {n: x for n, x in kw.items() if n != "flags"}
+    o, lse = sb.attention_forward(q, k, v, **fwd)
+    dq, dk, dv = sb.attention_backward(q, k, v, o, lse, do, **kw)
+    again = sb.attention_backward(q, k, v, o, lse, do, **kw)
+    assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+    assert torch.equal(dk, again[1]) and torch.equal(dv, again[2])
+    qf, kf, vf, dof = (t.float() for t in (q, k, v, do))
+    of, lf = sb.attention_forward(qf, kf, vf, **fwd)
+    for got, want, tol in zip((dq, dk, dv), sb.attention_backward(qf, kf, vf, of, lf, dof, **fwd), (8e-3, 8e-3, 4e-3)):
+        assert float((got.float() - want).norm() / want.norm()) <= tol
+
+
 def test_backward_head_dim_64_buffers_and_cut_tiles_vs_oracle(sb, oracle):
     """head_dim 64 takes a path of its own inside the backward kernel (LSE and delta folded into the S^T / dP^T products,
     two S^T buffers, three Q stages, two dS tiles).  B1 / Hq8 / Hkv2 / S1400 is a grid small enough that every key tile is

@@ -205,7 +205,7 @@ BwdCut bwd_cut(const AttnShape& s)
 // What one block of the grid computes.  A CTA computes its own block and then takes over blocks that have not started yet, one at
 // a time (clc_try_cancel), so that the loads and first products of one run under the epilogue of the one before, and barriers
 // and TMEM are set up once.  A block's fixed cost of about 2 us was a third of a short one: B8 Hq12 S1024 D64, 768 blocks of 1 to 8
-// steps, took 83 us for the whole backward and takes 73; B2 Hq32 S1024 D64 54 -> 49; a 300-key window over B1 Hq16 Hkv4 S4096
+// steps, took 83 us for the whole backward and takes 73; B2 Hq32 S1024 D64 54 -> 49; a 300-key window over B2 Hq16 Hkv4 S4096
 // D128 159 -> 149.  Grids that fit the SMs at once have nothing to take over and do not ask.
 struct BwdWork {
     int kt, slab, piece;       // key tile, b * Hkv + hk, piece of a cut tile

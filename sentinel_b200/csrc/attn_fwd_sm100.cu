@@ -42,10 +42,11 @@ constexpr int kM = 128;          // query rows per tile
 constexpr int kN = 128;          // keys per tile
 constexpr int kFwdThreads = 384; // 2 softmax warpgroups + 1 warpgroup holding the MMA warp and the TMA warp
 constexpr uint32_t kTmemCols = 512;
+constexpr int kOutBytes = 8 * 4096;        // staging of O
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 enum WaitSite : uint32_t {
-    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue
+    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue, kSiteQEmpty, kSiteNext
 };
 
 struct FwdParams {
@@ -61,8 +62,47 @@ struct FwdParams {
     long long mat_stride;
 };
 
+// What one block of the grid computes.  A CTA computes its own block and then takes over blocks that have not started yet (as the
+// backward does): K, Q and the first S of one come in under the last softmax passes and the epilogue of the one before.
+// Cold: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108 us; B8 Hq12 S1024 D64 37.1 -> 35.3; B4 Hq32 Hkv8 S4096 D64 421 ->
+// 407.
+struct FwdWork {
+    int bh, bh_kv, q0;         // q0: first of the one or two 128-row tiles
+    int g_tiles, w_first;      // key tiles in ascending order: the g_tiles tiles holding global tokens, then from w_first up to the
+                               // diagonal (without a window simply 0 .. diagonal)
+    int n0, n1;                // key tiles that tile 0 / tile 1 visits; n0 < 0: no more blocks
+
+    template <bool kWin> __device__ __forceinline__ void decode(const FwdParams& p, int block)
+    {
+        // heaviest query blocks first; the heads of one KV group are adjacent
+        const int bh_count = p.B * p.Hq, rank = block / bh_count;
+        bh = block - rank * bh_count;
+        const int b = bh / p.Hq, h = bh - b * p.Hq;
+        bh_kv = b * p.Hkv + h / (p.Hq / p.Hkv);
+        q0 = (p.causal ? p.n_qblk - 1 - rank : rank) * p.tiles_per_cta * kM;
+        const bool windowed = kWin && p.window > 0;
+        g_tiles = windowed ? (p.global_tokens + kN - 1) / kN : 0;
+        w_first = windowed ? max(g_tiles, max(0, q0 - p.window + 1) / kN) : 0;
+        const int n_all = (p.Skv + kN - 1) / kN;
+        auto visits = [&](int t) {
+            const int row0 = q0 + t * kM;
+            if (row0 >= p.Sq || t >= p.tiles_per_cta) return 0;
+            if (!p.causal) return n_all;
+            const int diag = min(n_all - 1, row0 / kN);
+            return min(g_tiles, diag + 1) + max(0, diag - w_first + 1);
+        };
+        n0 = visits(0);
+        n1 = visits(1);
+    }
+    __device__ __forceinline__ int n_max() const { return max(n0, n1); }      // K/V tiles the producer brings in
+    __device__ __forceinline__ int key_tile(int j) const { return j < g_tiles ? j : w_first + (j - g_tiles); }
+};
+
 struct FwdBarriers {
-    uint64_t q_full, k0_full;
+    uint4 response;            // of the block scheduler
+    uint64_t response_full, work_full[2], work_empty[2];
+    FwdWork work[2];           // blocks in turn
+    uint64_t q_full, q_empty, k0_full;
     // Loads come in pairs {K_{j+1}, V_j} (K_0 alone first) and are released in the same pairs, {K_0} counting as pair -1: one
     // wait and one commit per key tile for the issuing warp instead of two each.  Barrier j & 1.
     uint64_t pair_full[2], pair_empty[2];
@@ -80,7 +120,8 @@ struct FwdBarriers {
 enum FwdMode : int { kPlain = 0, kWindow = 1 };
 
 // kMat: O and LSE leave as fp32 feature-major matrices
-template <int D, int kMode, bool kMat>
+// kMany: CTAs take over blocks (FwdWork); without it each computes its own and the bookkeeping folds away
+template <int D, int kMode, bool kMat, bool kMany>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const FwdParams p)
@@ -93,47 +134,29 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     uint8_t* sQ = smem;                               // [2][kTileBytes]
     uint8_t* sK = sQ + 2 * kTileBytes;                // [2][kTileBytes]
     uint8_t* sV = sK + 2 * kTileBytes;                // [2][kTileBytes]
-    FwdBarriers* bars = (FwdBarriers*)(sV + 2 * kTileBytes);
+    uint8_t* sOut = sV + 2 * kTileBytes;              // 4 KB per softmax warp
+    FwdBarriers* bars = (FwdBarriers*)(sOut + (kMat ? 0 : kOutBytes));
     volatile uint32_t* abort_flag = &bars->abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp-uniform for the compiler)
 
-    // ---- work decode: heaviest query blocks first; the heads of one KV group are adjacent ----
     constexpr bool kWin = kMode != kPlain;
-    const int bh_count = p.B * p.Hq;
-    const int qblk_rank = blockIdx.x / bh_count;
-    const int bh = blockIdx.x - qblk_rank * bh_count;
-    const int qblk = p.causal ? (p.n_qblk - 1 - qblk_rank) : qblk_rank;
-    const int b = bh / p.Hq, h = bh - b * p.Hq;
-    const int bh_kv = b * p.Hkv + h / (p.Hq / p.Hkv);
-    const int q0 = qblk * p.tiles_per_cta * kM;      // the CTA owns two consecutive 128-row tiles, or one (fwd_tiles_per_cta)
-    const int n_ktiles_all = (p.Skv + kN - 1) / kN;
-    // Key tiles this CTA visits, in ascending order: the tiles holding global tokens, then the tiles from the window
-    // of the block's first query row up to the diagonal.  Without a window that is simply 0 .. diagonal.
-    const bool windowed = kWin && p.window > 0;
-    const int g_tiles = windowed ? (p.global_tokens + kN - 1) / kN : 0;
-    const int w_first = windowed ? max(g_tiles, max(0, q0 - p.window + 1) / kN) : 0;
-    auto key_tile = [&](int j) { return j < g_tiles ? j : w_first + (j - g_tiles); };   // j-th load of the CTA
-    int n_t[2];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int row0 = q0 + t * kM;
-        if (row0 >= p.Sq || t >= p.tiles_per_cta) n_t[t] = 0;
-        else if (p.causal) {
-            const int diag = min(n_ktiles_all - 1, row0 / kN);
-            n_t[t] = min(g_tiles, diag + 1) + max(0, diag - w_first + 1);
-        } else n_t[t] = n_ktiles_all;
-    }
-    const int n_max = max(n_t[0], n_t[1]);           // K/V tiles the producer brings in
 
     // ---- setup ----
+    FwdWork own;        // (kMany: the producer's)
+    if (!kMany || (warp == 9 && lane == 0)) own.decode<kWin>(p, (int)blockIdx.x);
     if (warp == 9 && lane == 0) {
+        if (kMany) bars->work[0] = own;
         prefetch_tensormap(&tmap_q);
         prefetch_tensormap(&tmap_k);
         prefetch_tensormap(&tmap_v);
         mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->q_empty, 1);
         mbar_init(&bars->k0_full, 1);
+        mbar_init(&bars->response_full, 1);
         for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->work_full[i], 1);
+            mbar_init(&bars->work_empty[i], 9);    // the issuing warp and the softmax warps
             mbar_init(&bars->pair_full[i], 1);
             mbar_init(&bars->pair_empty[i], 1);
             mbar_init(&bars->s_ready[i], 1);
@@ -169,6 +192,19 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     constexpr bool kHalfP = !kOwnP;
     auto tmem_O = [&](int t) { return tmem + (kOwnP ? 384u : 256u) + (uint32_t)t * (kOwnP ? 64u : 128u); };
 
+    // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Counters of key
+    // tiles run on over the blocks (all of them: c0; those of tile t: its steps), so stages and barrier phases continue where they
+    // are.  next(u): done with block u; whether another follows.
+    auto next = [&](int u) {
+        if (!kMany) return false;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->work_empty[u & 1]);
+        return mbar_wait_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && warp_uniform(bars->work[(u + 1) & 1].n0) >= 0;
+    };
+
+    auto work = [&](int u) -> const FwdWork& { return kMany ? bars->work[u & 1] : own; };
+    auto uniform = [&](int x) { return kMany ? warp_uniform(x) : x; };
+
     // 384 threads start with 168 registers each; each role re-allocates inside its own branch
     if (warp >= 10) {
         setmaxnreg_dec<72>();   // idle warps of the last warpgroup
@@ -176,30 +212,51 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         setmaxnreg_dec<72>();
         // =========================== TMA producer ===========================
         if (lane == 0) {
-            {
-                int n_valid = (n_t[0] > 0) + (n_t[1] > 0);
-                mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(n_valid * kTileBytes));
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-                    if (n_t[t] > 0)
-                        for (int c = 0; c < kChunks; ++c)
-                            tma_load_3d(sQ + t * kTileBytes + c * kChunkBytes, &tmap_q, &bars->q_full, c * 64, q0 + t * kM, bh);
-            }
-            auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int j) {
-                for (int c = 0; c < kChunks; ++c) tma_load_3d(dst + (j & 1) * kTileBytes + c * kChunkBytes, map, bar, c * 64, key_tile(j) * kN, bh_kv);
-            };
-            if (n_max > 0) {
+            int c0 = 0;
+            bool ok = true;
+            FwdWork& w = own;
+            for (int u = 0, block = 0; block >= 0; ++u) {
+                const int n_max = w.n_max();
+                auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int j) {
+                    for (int c = 0; c < kChunks; ++c)
+                        tma_load_3d(dst + ((c0 + j) & 1) * kTileBytes + c * kChunkBytes, map, bar, c * 64, w.key_tile(j) * kN, w.bh_kv);
+                };
+                // K_0 goes where the block before had its last K but one, which is free (its last pair has been loaded); Q once that
+                // block's last S product has read it
                 mbar_arrive_expect_tx(&bars->k0_full, (uint32_t)kTileBytes);
                 load(sK, &tmap_k, &bars->k0_full, 0);
-            }
-            for (int j = 0; j < n_max; ++j) {
-                // K_{j+1} and V_j go where K_{j-1} and V_{j-2} were: pair j - 2, the (j >> 1)-th release of this barrier for odd j
-                // (pair -1 was the first), the one before for even j
-                if (j >= 1 && !mbar_wait(&bars->pair_empty[j & 1], (uint32_t)((j >> 1) - (j & 1 ? 0 : 1)) & 1u, abort_flag, kSitePairEmpty)) break;
-                const bool k_too = j + 1 < n_max;
-                mbar_arrive_expect_tx(&bars->pair_full[j & 1], (uint32_t)(k_too ? 2 * kTileBytes : kTileBytes));
-                if (k_too) load(sK, &tmap_k, &bars->pair_full[j & 1], j + 1);
-                load(sV, &tmap_v, &bars->pair_full[j & 1], j);
+                if (u > 0 && !mbar_wait(&bars->q_empty, (uint32_t)((u - 1) & 1), abort_flag, kSiteQEmpty)) break;
+                mbar_arrive_expect_tx(&bars->q_full, (uint32_t)((w.n1 > 0 ? 2 : 1) * kTileBytes));
+                for (int t = 0; t < (w.n1 > 0 ? 2 : 1); ++t)
+                    for (int c = 0; c < kChunks; ++c)
+                        tma_load_3d(sQ + t * kTileBytes + c * kChunkBytes, &tmap_q, &bars->q_full, c * 64, w.q0 + t * kM, w.bh);
+                for (int j = 0; j < n_max; ++j) {
+                    // K_{c+1} and V_c go where K_{c-1} and V_{c-2} were: pair c - 2, the (c >> 1)-th release of this barrier for odd c
+                    // (pair -1 was the first), the one before for even c
+                    const int c = c0 + j;
+                    if (c >= 1 && !(ok = mbar_wait(&bars->pair_empty[c & 1], (uint32_t)((c >> 1) - (c & 1 ? 0 : 1)) & 1u, abort_flag, kSitePairEmpty))) break;
+                    const bool k_too = j + 1 < n_max;
+                    mbar_arrive_expect_tx(&bars->pair_full[c & 1], (uint32_t)(k_too ? 2 * kTileBytes : kTileBytes));
+                    if (k_too) load(sK, &tmap_k, &bars->pair_full[c & 1], j + 1);
+                    load(sV, &tmap_v, &bars->pair_full[c & 1], j);
+                }
+                if (!ok) break;
+                c0 += n_max;
+                // The next block is asked for about two steps before this one ends: in time, and not so early that it would go to
+                // this CTA although others are free sooner.
+                block = -1;
+                if constexpr (kMany) {
+                    mbar_arrive_expect_tx(&bars->response_full, 16);
+                    clc_try_cancel(&bars->response, &bars->response_full);
+                    if (!mbar_wait(&bars->response_full, (uint32_t)(u & 1), abort_flag, kSiteNext)) break;
+                    block = clc_first_block(&bars->response);
+                    fence_proxy_async_smem();
+                    w.n0 = -1;
+                    if (block >= 0) w.decode<kWin>(p, block);
+                    if (u >= 1 && !mbar_wait(&bars->work_empty[(u + 1) & 1], (uint32_t)(((u - 1) >> 1) & 1), abort_flag, kSiteNext)) break;
+                    bars->work[(u + 1) & 1] = w;
+                    mbar_arrive(&bars->work_full[(u + 1) & 1]);
+                }
             }
         }
     } else if (warp == 8) {
@@ -244,75 +301,87 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 mma_ts_4<8, 128>(d, a + 32u, sdesc_advance(b, 4 * 2048), idesc_pv, 1);
                 return true;
             };
-            const int n0 = n_t[0], n1 = n_t[1];
-            bool ok = n_max > 0 && wait(&bars->q_full, 0, kSiteQ) && wait(&bars->k0_full, 0, kSiteK0);
-            if (ok) {
-                tc_fence_after();
-                issue_s(0, 0);          // (a block has rows in its first tile)
-            }
+            int c0 = 0, s0 = 0, s1 = 0;        // key tiles of the blocks before: all, those of tile 0, of tile 1
+            bool ok = true, more = true;
+            for (int u = 0; more; more = next(u++)) {
+            const int n0 = uniform(work(u).n0), n1 = uniform(work(u).n1), n_max = max(n0, n1);
+            if (!(ok = wait(&bars->k0_full, (uint32_t)(u & 1), kSiteK0) && wait(&bars->q_full, (uint32_t)(u & 1), kSiteQ))) break;
+            tc_fence_after();
+            // (S of the last step of the block before has been read, and P over it consumed: this warp waited for p_ready and issued
+            // the product; O is overwritten behind p_ready of the new block, which its warps give after their epilogue)
+            issue_s(0, c0 & 1);          // (a block has rows in its first tile)
             if constexpr (kOwnP) {
                 // With P in columns of its own the next S of a tile does not wait for the P V product that consumes P, and the two
                 // tiles are kept half a pass apart: S of tile 1 starts behind the first half of tile 0's first pass, and per key tile
                 // the order is S0_{j+1}, P1_{j-1} V, P0_j V, S1_{j+1}, which is the order in which their operands are ready then.
                 // One tile's loads, stores and hand-offs so fall into the other's exponentials.
                 const bool apart = n_max >= 4;   // short rows would pay more for the late start than they gain
-                if (ok && !apart && n1 > 0) issue_s(1, 0);
+                if (!apart && n1 > 0) issue_s(1, c0 & 1);
+                if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
                 for (int j = 0; ok && j <= n_max; ++j) {
+                    const int c = c0 + j;
                     if (j < n_max) {
-                        if (!(ok = wait(&bars->pair_full[j & 1], (uint32_t)((j >> 1) & 1), kSitePairFull))) break;
+                        if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
                     }
                     const bool late = j == 0 && apart && n1 > 0;
                     if (j + 1 < n0 || late) {
-                        if (!(ok = wait(&bars->s_free[0], (uint32_t)(j & 1), kSiteIssue))) break;
+                        if (!(ok = wait(&bars->s_free[0], (uint32_t)((s0 + j) & 1), kSiteIssue))) break;
                         tc_fence_after();
-                        if (j + 1 < n0) issue_s(0, (j + 1) & 1);
-                        if (late) issue_s(1, 0);
+                        if (j + 1 < n0) issue_s(0, (c + 1) & 1);
+                        if (late) issue_s(1, c & 1);
                     }
-                    if (j == 0) {
-                        tc_commit_p(&bars->pair_empty[1]);        // K_0
-                    } else {
-                        if (j - 1 < n1) {
-                            if (!(ok = wait(&bars->p_ready[1], (uint32_t)((j - 1) & 1), kSitePReady))) break;
-                            tc_fence_after();
-                            issue_pv(1, (j - 1) & 1, j > 1, 0);
-                            tc_commit_p(&bars->o_ready[1]);
-                        }
-                        tc_commit_p(&bars->pair_empty[(j - 1) & 1]);
+                    if (j > 0 && j - 1 < n1) {
+                        if (!(ok = wait(&bars->p_ready[1], (uint32_t)((s1 + j - 1) & 1), kSitePReady))) break;
+                        tc_fence_after();
+                        issue_pv(1, (c - 1) & 1, j > 1, 0);
+                        tc_commit_p(&bars->o_ready[1]);
                     }
+                    // pair c - 1; K_0 counts into the last pair of the block before, and this block's last into the next block's first
+                    if (j < n_max) tc_commit_p(&bars->pair_empty[(c - 1) & 1]);
                     if (j < n0) {
-                        if (!(ok = wait(&bars->p_ready[0], (uint32_t)(j & 1), kSitePReady))) break;
+                        if (!(ok = wait(&bars->p_ready[0], (uint32_t)((s0 + j) & 1), kSitePReady))) break;
                         tc_fence_after();
-                        issue_pv(0, j & 1, j > 0, 0);
+                        issue_pv(0, c & 1, j > 0, 0);
                         tc_commit_p(&bars->o_ready[0]);
                     }
                     if (j + 1 < n1) {
-                        if (!(ok = wait(&bars->s_free[1], (uint32_t)(j & 1), kSiteIssue))) break;
+                        if (!(ok = wait(&bars->s_free[1], (uint32_t)((s1 + j) & 1), kSiteIssue))) break;
                         tc_fence_after();
-                        issue_s(1, (j + 1) & 1);
+                        issue_s(1, (c + 1) & 1);
                     }
+                    if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
                 }
             } else {
                 // P is written over S: a tile's P V product, then its next S, as its P arrives
-                if (ok && n1 > 0) issue_s(1, 0);
-                if (ok) tc_commit_p(&bars->pair_empty[1]);        // K_0
+                if (n1 > 0) issue_s(1, c0 & 1);
+                tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
+                if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
                 for (int j = 0; ok && j < n_max; ++j) {
-                    if (!(ok = wait(&bars->pair_full[j & 1], (uint32_t)((j >> 1) & 1), kSitePairFull))) break;
+                    const int c = c0 + j;
+                    if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
                         const int n = t ? n1 : n0;
+                        const uint32_t parity = (uint32_t)(((t ? s1 : s0) + j) & 1);
                         if (!ok || j >= n) continue;
-                        if (!(ok = wait(&bars->p_half[t], (uint32_t)(j & 1), kSitePReady))) continue;
+                        if (!(ok = wait(&bars->p_half[t], parity, kSitePReady))) continue;
                         SNTL_TRACE_EV(tl8, 0, tn, 10 + t);
                         tc_fence_after();
-                        if (!(ok = issue_pv(t, j & 1, j > 0, (uint32_t)(j & 1)))) continue;
+                        if (!(ok = issue_pv(t, c & 1, j > 0, parity))) continue;
                         SNTL_TRACE_EV(tl8, 0, tn, 20 + t);
-                        if (j + 1 < n) issue_s(t, (j + 1) & 1);
+                        if (j + 1 < n) issue_s(t, (c + 1) & 1);
                         else tc_commit_p(&bars->o_ready[t]);
                         SNTL_TRACE_EV(tl8, 0, tn, 30 + t);
                     }
                     if (!ok) break;
-                    tc_commit_p(&bars->pair_empty[j & 1]);
+                    if (j + 1 < n_max) tc_commit_p(&bars->pair_empty[c & 1]);
+                    if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
                 }
+            }
+            if (!ok) break;
+            c0 += n_max;
+            s0 += n0;
+            s1 += n1;
             }
             // every MMA issued above must have retired before shared memory / TMEM are given up
             tc_commit_p(&bars->final_bar);
@@ -324,19 +393,24 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const int t = warp >> 2;                       // tile 0 or 1
         const int row = (warp & 3) * 32 + lane;        // row inside the tile == TMEM lane
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-        const int grow = q0 + t * kM + row;   // query row inside the (batch, head) slab
-        const int n_mine = t ? n_t[1] : n_t[0];        // (an index would put the array in local memory)
         SNTL_TRACE_DECL(tn);
         const bool tw = (warp & 3) == 0 && lane == 0;
         (void)tw;
+        bool ok = true, more = true;
+        uint32_t phase = 0, blocks = 0;                // of this tile so far: parity of its key tiles, blocks with rows
+        for (int u = 0; ok && more; more = next(u++)) {
+        const FwdWork& w = work(u);
+        const int n_mine = uniform(t ? w.n1 : w.n0), q0 = uniform(w.q0);
+        const int g_tiles = kWin ? uniform(w.g_tiles) : 0, w_first = kWin ? uniform(w.w_first) : 0;
+        const int grow = q0 + t * kM + row;            // query row inside the (batch, head) slab
+        auto key_tile = [&](int j) { return j < g_tiles ? j : w_first + (j - g_tiles); };
         float m_ref = -INFINITY, l = 0.0f;
-        bool ok = true;
         // Barrier tests queue behind the exponentials in the same unit and take 200-400 cycles here; where a result is likely to be
         // there already it is asked for ahead of its use, with other work in between.
         bool s_seen = false;
         const int row_lo = q0 + t * kM + (warp & 3) * 32;      // first row of the warp
-        for (int j = 0; j < n_mine; ++j) {
-            if (!(ok = __all_sync(0xffffffffu, s_seen || mbar_wait(&bars->s_ready[t], (uint32_t)(j & 1), abort_flag, kSiteSReady)))) break;
+        for (int j = 0; j < n_mine; ++j, phase = kMany ? phase ^ 1u : (uint32_t)(j & 1)) {
+            if (!(ok = __all_sync(0xffffffffu, s_seen || mbar_wait(&bars->s_ready[t], phase, abort_flag, kSiteSReady)))) break;
             SNTL_TRACE_EV(tw, 1 + t, tn, 1);
             tc_fence_after();
             uint32_t s[128];
@@ -370,7 +444,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             bool o_seen = false;
             auto o_done = [&]() {       // P_{j-1} has been consumed and O holds its product (head_dim 128: S_j was issued behind it)
                 if constexpr (kOwnP) {
-                    ok = __all_sync(0xffffffffu, o_seen || mbar_wait(&bars->o_ready[t], (uint32_t)((j - 1) & 1), abort_flag, kSiteOReady));
+                    ok = __all_sync(0xffffffffu, o_seen || mbar_wait(&bars->o_ready[t], phase ^ 1u, abort_flag, kSiteOReady));
                     tc_fence_after();
                 }
             };
@@ -394,7 +468,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             if (ahead) {
                 exp_half<0, true>(s, p.scale_log2, neg_m, pk, sum, mx);
                 SNTL_TRACE_EV(tw, 1 + t, tn, 3);
-                if (kOwnP) o_seen = mbar_try_wait(&bars->o_ready[t], (uint32_t)((j - 1) & 1));
+                if (kOwnP) o_seen = mbar_try_wait(&bars->o_ready[t], phase ^ 1u);
                 const float m_new = fmaxf(m_ref, mx.value() * p.scale_log2);
                 const bool again = outgrown(m_new);
                 if (!again) s_read();
@@ -438,7 +512,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 mbar_arrive(&bars->p_half[t]);
             }
             exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, mx);
-            if (kOwnP) s_seen = j + 1 < n_mine && mbar_try_wait(&bars->s_ready[t], (uint32_t)((j + 1) & 1));
+            if (kOwnP) s_seen = j + 1 < n_mine && mbar_try_wait(&bars->s_ready[t], phase ^ 1u);
             tmem_st32(tmem_S(t) + kPOff + lane_off + 32u, pk);
             l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             SNTL_TRACE_EV(tw, 1 + t, tn, 5);
@@ -447,20 +521,22 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             mbar_arrive(&bars->p_ready[t]);
             SNTL_TRACE_EV(tw, 1 + t, tn, 6);
         }
-        if (__all_sync(0xffffffffu, ok && n_mine > 0 && mbar_wait(&bars->o_ready[t], (uint32_t)(kOwnP ? (n_mine - 1) & 1 : 0), abort_flag, kSiteOReady))) {
+        if (ok && n_mine > 0)
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_ready[t], kOwnP ? phase ^ 1u : blocks & 1u, abort_flag, kSiteOReady));
+        if (ok && n_mine > 0) {
+            ++blocks;
             tc_fence_after();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             const bool store = grow < p.Sq;
             // Coalesced store of O.  A thread holds one whole row (2*D bytes); written straight from there a warp's store
-            // instruction would touch 32 rows, 16 bytes each.  So the warp's 32 rows go through shared memory -- this tile's
-            // Q buffer, free since the last S product of this tile retired (o_ready of the last step implies it) -- and
-            // come back out with each store instruction covering whole
-            // rows: 16 lanes x 16 bytes = one 256-byte row at head_dim 128, 8 lanes per 128-byte row at 64.  Only the rows of
+            // instruction would touch 32 rows, 16 bytes each.  So the warp's 32 rows go through 4 KB of shared memory of its own, 64
+            // columns at a time, and come back out with each store instruction covering 128 bytes of four rows.  Only the rows of
             // this warp are exchanged, so a warp-level sync is all it takes; 16-byte units are XOR-swizzled by the row so
             // that both the row-wise writes and the row-wise reads spread over the banks.
-            constexpr int kUnits = D / 8;                       // 16-byte units per row
+            const int bh = w.bh;
             if constexpr (kMat) {
                 // feature-major matrices: the 32 rows of a warp are 128 contiguous bytes of every feature's row
+                const int b = bh / p.Hq, h = bh - b * p.Hq;
                 float* dst = p.o_mat + (long long)h * D * p.mat_stride + (long long)b * p.Sq + grow;
 #pragma unroll
                 for (int c = 0; c < D / 32; ++c) {
@@ -475,40 +551,39 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if (store)
                     p.lse_mat[(long long)h * p.mat_stride + (long long)b * p.Sq + grow] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
             } else {
-            uint8_t* stage = sQ + t * kTileBytes + (warp & 3) * 32 * (D * 2);
+            uint8_t* stage = sOut + warp * 4096;
+            const int sub = lane >> 3, unit0 = lane & 7, warp_row0 = grow - lane;      // (first row of this warp inside the slab)
+            __nv_bfloat16* dst = p.o + (size_t)bh * p.Sq * D;
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
-                uint32_t o[32];
-                tmem_ld32(tmem_O(t) + lane_off + (uint32_t)(c * 32), o);
-                tmem_ld_wait();
+            for (int half = 0; half < D / 64; ++half) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    uint4 w;
-                    w.x = pack_bf16(__uint_as_float(o[8 * i + 0]) * inv, __uint_as_float(o[8 * i + 1]) * inv);
-                    w.y = pack_bf16(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv);
-                    w.z = pack_bf16(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv);
-                    w.w = pack_bf16(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv);
-                    const int unit = c * 4 + i;
-                    *reinterpret_cast<uint4*>(stage + lane * (D * 2) + ((unit ^ (lane & (kUnits - 1) & 7)) << 4)) = w;
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(tmem_O(t) + lane_off + (uint32_t)(half * 64 + c * 32), o);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        uint4 v;
+                        v.x = pack_bf16(__uint_as_float(o[8 * i + 0]) * inv, __uint_as_float(o[8 * i + 1]) * inv);
+                        v.y = pack_bf16(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv);
+                        v.z = pack_bf16(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv);
+                        v.w = pack_bf16(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv);
+                        *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + i) ^ (lane & 7)) << 4)) = v;
+                    }
                 }
-            }
-            __syncwarp();
-            {
-                constexpr int kRowsPerStore = 32 / kUnits;       // rows one store instruction of the warp covers
-                const int sub = lane / kUnits, unit = lane % kUnits;
-                const int warp_row0 = grow - lane;                // first row of this warp inside the slab
-                const size_t part_base = (size_t)bh * p.Sq;
+                __syncwarp();
 #pragma unroll
-                for (int i = 0; i < 32 / kRowsPerStore; ++i) {
-                    const int r = i * kRowsPerStore + sub;        // row inside the warp's 32
-                    const uint4 w = *reinterpret_cast<const uint4*>(stage + r * (D * 2) + ((unit ^ (r & (kUnits - 1) & 7)) << 4));
-                    if (warp_row0 + r < p.Sq)
-                        *reinterpret_cast<uint4*>(p.o + (part_base + (size_t)(warp_row0 + r)) * D + unit * 8) = w;
+                for (int i = 0; i < 8; ++i) {
+                    const int r = i * 4 + sub;
+                    const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 128 + ((unit0 ^ (r & 7)) << 4));
+                    if (warp_row0 + r < p.Sq) *reinterpret_cast<uint4*>(dst + (size_t)(warp_row0 + r) * D + half * 64 + unit0 * 8) = v;
                 }
+                __syncwarp();
             }
             if (store)
                 p.lse[(size_t)bh * p.Sq + grow] = l > 0.0f ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
             }
+        }
         }
     }
 
@@ -566,6 +641,10 @@ int fwd_tiles_per_cta(const AttnShape& s)
     return t1 < 0.95 * t2 ? 1 : 2;
 }
 
+// Which kernels have a form that takes over blocks, for grids of more than one wave.  The plain one at head_dim 128 has not: its
+// softmax loop fills the registers, and with the bookkeeping it spills (B2 Hq28 Hkv4 S8192 737 -> 768 us).
+template <int D, int kMode> constexpr bool kTakesOver = D == 64 || kMode == kWindow;
+
 template <int D, int kMode, bool kMat>
 cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
 {
@@ -588,10 +667,16 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const long long ctas = (long long)p.n_qblk * s.B * s.Hq;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    const size_t smem = 6 * (size_t)(128 * D * 2) + sizeof(FwdBarriers) + 1024;
-    static std::atomic<unsigned long long> configured{0};   // per instantiation, one bit per device
-    if ((e = ensure_dynamic_smem(attn_fwd_tc_kernel<D, kMode, kMat>, smem, configured)) != cudaSuccess) return e;
-    return launch_kernel(attn_fwd_tc_kernel<D, kMode, kMat>, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p);
+    const size_t smem = 6 * (size_t)(128 * D * 2) + (kMat ? 0 : kOutBytes) + sizeof(FwdBarriers) + 1024;
+    auto launch = [&](auto kernel, std::atomic<unsigned long long>& configured) {
+        const cudaError_t err = ensure_dynamic_smem(kernel, smem, configured);
+        return err != cudaSuccess ? err : launch_kernel(kernel, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p);
+    };
+    static std::atomic<unsigned long long> configured_one{0}, configured_many{0};   // per instantiation, one bit per device
+    if constexpr (kTakesOver<D, kMode>) {
+        if (ctas > sm_count()) return launch(attn_fwd_tc_kernel<D, kMode, kMat, true>, configured_many);
+    }
+    return launch(attn_fwd_tc_kernel<D, kMode, kMat, false>, configured_one);
 }
 
 }  // namespace

@@ -178,6 +178,9 @@ __device__ __forceinline__ int clc_first_block(const void* response)
     return block;
 }
 
+// the same value in all lanes, and known to be: what depends on it stays in uniform registers and branches
+__device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 // barrier among a subset of the CTA's warps (id 1..15; `threads` a multiple of 32)
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads)
 {

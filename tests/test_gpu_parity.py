@@ -393,6 +393,20 @@ def test_forward_query_tiles_per_cta_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D,
     assert float((lse - lf).abs().max()) <= 1e-3
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,kw", [
+    (40, 8, 8, 100, 100, 64, {}),                                 # 320 blocks of one key tile, with rows in one query tile
+    (5, 40, 8, 300, 300, 64, {}),                                 # one, two and three key tiles; the second query tile ends early
+    (3, 36, 12, 1100, 1100, 64, {}),                              # rows long enough for the tiles to run half a pass apart
+    (20, 16, 8, 150, 260, 64, dict(causal=False)),
+    (4, 48, 16, 900, 900, 64, dict(window=200, global_tokens=5)),
+    (4, 48, 16, 900, 900, 128, dict(window=200, global_tokens=5)),
+    (6, 40, 8, 200, 200, 128, dict(window=1)),
+])
+def test_forward_blocks_taken_over_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, kw):
+    """More blocks than SMs, so that every CTA computes several in turn: bounds as for the query blocks above."""
+    test_forward_query_tiles_per_cta_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, kw)
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,S,D,kw", [
     (1, 2, 2, 1100, 128, {}),                                    # one head per group: tiles cut along the queries, ragged
     (1, 6, 2, 700, 64, dict(window=200, global_tokens=5)),       # pieces that end inside a head's query range

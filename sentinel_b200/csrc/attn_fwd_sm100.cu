@@ -221,11 +221,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     for (int c = 0; c < kChunks; ++c)
                         tma_load_3d(dst + ((c0 + j) & 1) * kTileBytes + c * kChunkBytes, map, bar, c * 64, w.key_tile(j) * kN, w.bh_kv);
                 };
-                // K_0 goes where the block before had its last K but one, which is free (its last pair has been loaded); Q once that
-                // block's last S product has read it
+                // Q and K_0 once the last S product of the block before has run: Q is free then, and K_0's stage and barrier were free
+                // before (the barrier must not be armed again while the K_0 before is on its way or unseen: rows of a single
+                // key tile get here that early)
+                if (u > 0 && !mbar_wait(&bars->q_empty, (uint32_t)((u - 1) & 1), abort_flag, kSiteQEmpty)) break;
                 mbar_arrive_expect_tx(&bars->k0_full, (uint32_t)kTileBytes);
                 load(sK, &tmap_k, &bars->k0_full, 0);
-                if (u > 0 && !mbar_wait(&bars->q_empty, (uint32_t)((u - 1) & 1), abort_flag, kSiteQEmpty)) break;
                 mbar_arrive_expect_tx(&bars->q_full, (uint32_t)((w.n1 > 0 ? 2 : 1) * kTileBytes));
                 for (int t = 0; t < (w.n1 > 0 ? 2 : 1); ++t)
                     for (int c = 0; c < kChunks; ++c)

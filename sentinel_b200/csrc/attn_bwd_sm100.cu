@@ -1006,8 +1006,9 @@ template <int D> constexpr int kPreRows = D == 64 ? 128 : 64;   // query rows pe
 
 // Per padded query row: the terms the main kernel wants (store_row_terms) from delta = rowsum(dO o O) and LSE, and the dQ
 // accumulator zeroed.  Bound by HBM: D/8 lanes per row with 16 bytes of O and of dO each and four rows per lane group in flight,
-// 8 warps x 8 (16 at head_dim 64) rows per block, whose part of the accumulator is contiguous.
-template <int D>
+// 8 warps x 8 (16 at head_dim 64) rows per block, whose part of the accumulator is contiguous.  kWide: O and dO start on 16-byte
+// boundaries; else on 8-byte ones (nothing else in the backward reads O, so it needs no more).
+template <int D, bool kWide>
 __global__ void __launch_bounds__(256) bwd_pre_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                                       const float* __restrict__ lse, const RowTerms terms, float* __restrict__ dq_accum, int Sq,
                                                       int Sq_pad, int acc_words_per_row)
@@ -1017,6 +1018,11 @@ __global__ void __launch_bounds__(256) bwd_pre_kernel(const __nv_bfloat16* __res
     static_assert(kRows == kPreRows<D>, "grid");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane % kLanes;
     const long long r0 = (long long)blockIdx.x * kRows;
+    auto load = [](const __nv_bfloat16* p) {
+        if constexpr (kWide) return __ldg(reinterpret_cast<const uint4*>(p));
+        const uint2 a = __ldg(reinterpret_cast<const uint2*>(p)), b = __ldg(reinterpret_cast<const uint2*>(p) + 1);
+        return make_uint4(a.x, a.y, b.x, b.y);
+    };
     uint4 x[kPer], y[kPer];
     int s[kPer];
     long long bh[kPer];
@@ -1027,8 +1033,8 @@ __global__ void __launch_bounds__(256) bwd_pre_kernel(const __nv_bfloat16* __res
         s[i] = (int)(r - bh[i] * Sq_pad);
         const bool live = s[i] < Sq;
         const size_t off = ((size_t)bh[i] * Sq + s[i]) * D + l * 8;
-        x[i] = live ? __ldg(reinterpret_cast<const uint4*>(o + off)) : make_uint4(0, 0, 0, 0);
-        y[i] = live ? __ldg(reinterpret_cast<const uint4*>(dout + off)) : make_uint4(0, 0, 0, 0);
+        x[i] = live ? load(o + off) : make_uint4(0, 0, 0, 0);
+        y[i] = live ? load(dout + off) : make_uint4(0, 0, 0, 0);
     }
     const int words = kRows * acc_words_per_row;       // (rows_padded is a multiple of 128: every block has all its rows)
     float4* z = reinterpret_cast<float4*>(dq_accum + r0 * acc_words_per_row);
@@ -1234,8 +1240,9 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     if (phases & kBwdPre) {
         const long long blocks = rows_padded / kPreRows<D>;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        if ((e = launch_kernel(bwd_pre_kernel<D>, (unsigned)blocks, 256, 0, st, 1, a.o, a.dout, a.lse, terms, a.dq_accum, s.Sq, Sq_pad,
-                               kDet ? 2 * D : D)) != cudaSuccess)
+        auto kernel = aligned(16, a.o, a.dout) ? bwd_pre_kernel<D, true> : bwd_pre_kernel<D, false>;
+        if ((e = launch_kernel(kernel, (unsigned)blocks, 256, 0, st, 1, a.o, a.dout, a.lse, terms, a.dq_accum, s.Sq, Sq_pad, kDet ? 2 * D : D)) !=
+            cudaSuccess)
             return e;
     }
     if (phases & kBwdMain) {
@@ -1345,6 +1352,14 @@ cudaError_t dispatch_bwd_out(const TcArgs& a, cudaStream_t st)
 
 cudaError_t tc_backward(const TcArgs& a, cudaStream_t st)
 {
+    // Every address is looked at before the first launch: operands go through tensor maps, the rest is accessed 16 bytes at a time
+    // (O and, by the pre-pass alone, dO 8).  Matrix results are stored element by element; unused pointers are null.
+    const int phases = a.phases ? a.phases : (kBwdPre | kBwdMain | kBwdPost);
+    bool ok = aligned(16, a.delta, a.dq_accum);
+    if (phases & kBwdPre) ok = ok && aligned(8, a.o, a.dout);
+    if (phases & kBwdMain) ok = ok && aligned(16, a.q, a.k, a.v, a.dout, a.dk, a.dv, a.dk_acc, a.dv_acc);
+    if (phases & kBwdPost) ok = ok && aligned(16, a.dq);
+    if (!ok) return cudaErrorMisalignedAddress;
     return a.s.D == 64 ? dispatch_bwd_out<64>(a, st) : dispatch_bwd_out<128>(a, st);
 }
 

@@ -763,6 +763,7 @@ cudaError_t dispatch_fwd(const TcArgs& a, cudaStream_t st)
 
 cudaError_t tc_forward(const TcArgs& a, cudaStream_t st)
 {
+    if (!aligned(16, a.q, a.k, a.v, a.o_out)) return cudaErrorMisalignedAddress;   // (matrix results go out element by element: o_out is null)
     return a.s.D == 64 ? dispatch_fwd<64>(a, st) : dispatch_fwd<128>(a, st);
 }
 

@@ -95,6 +95,9 @@ inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, si
     return e;
 }
 
+// What a kernel accesses `bytes` at a time has to start on such a boundary; a misaligned access would take the context down.
+template <typename... P> inline bool aligned(uintptr_t bytes, const P*... p) { return (((uintptr_t)p | ... | (uintptr_t)0) % bytes) == 0; }
+
 // SMs of the current device (148 on a B200), read once per device ordinal
 inline int sm_count()
 {

@@ -684,6 +684,8 @@ cudaError_t rope_unpack_f32(const __nv_bfloat16* src, float* dst, int B, int H, 
 
 cudaError_t stage_matrices(const MatrixStage& m, int B, int Hq, int S, int D, int stride_columns, int column_start, float scale, cudaStream_t st)
 {
+    // the bf16 tensors, the row terms and the accumulator are written 16 bytes at a time
+    if (!aligned(16, m.dst[0], m.dst[1], m.dst[2], m.dst[3], m.row_terms, m.dq_accum)) return cudaErrorMisalignedAddress;
     StagePlan p{};
     p.m = m;
     p.Hq = Hq; p.S = S; p.S_pad = (S + 127) / 128 * 128;

@@ -154,3 +154,66 @@ def test_deterministic_flag_makes_dq_bit_reproducible(sb):
         assert float(np.abs(got - wdq).max()) <= 2e-2
         assert float(np.linalg.norm(got - wdq) / np.linalg.norm(wdq)) <= 5e-3
     assert sb.poll_device_status() == 0
+
+
+def _offset(t, elements):
+    """The same values in a contiguous tensor that starts `elements` elements past an allocation."""
+    x = torch.empty(t.numel() + elements, dtype=t.dtype, device=t.device)[elements:].view(t.shape)
+    return x.copy_(t)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_backward_reads_o_from_any_8_byte_boundary(sb, D):
+    """O has no tensor map and is read by the pre-pass alone: a view 8 bytes past a 16-byte boundary gives the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, do = (torch.randn(2, 4, 201, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(2, 2, 201, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    o, lse = sb.attention_forward(q, k, v)
+    want = sb.attention_backward(q, k, v, o, lse, do, flags=4)
+    view = _offset(o, 4)
+    assert view.data_ptr() % 16 == 8
+    for got, ref in zip(sb.attention_backward(q, k, v, view, lse, do, flags=4), want):
+        assert torch.equal(got, ref)
+    # the backward in pieces reads dO that way too, before any product needs its tensor map
+    dk, dv = torch.zeros(k.shape, device="cuda"), torch.zeros(v.shape, device="cuda")
+    pieces = sb.BackwardPieces(q, view, lse, do)
+    pieces.block(k, v, dk, dv, causal=True)
+    assert float((pieces.end().float() - want[0].float()).norm() / want[0].float().norm()) <= 4e-3   # bf16 rounding of both
+    assert sb.poll_device_status() == 0
+
+
+def test_misaligned_tensors_are_refused_before_any_launch(sb):
+    """The tensor-core kernels access bf16 tensors and scratch 16 bytes at a time (O 8): other addresses are an error, and
+    nothing is launched.  (Only the refusal is tested: no kernel runs on such an address.)"""
+    import ctypes as C
+    from sentinel_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, do = (torch.randn(1, 4, 256, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(1, 2, 256, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    o, lse = sb.attention_forward(q, k, v)
+    sb.attention_backward(q, k, v, o, lse, do)
+    before = sb.launch_count()
+    args = dict(q=q, k=k, v=v, o=o, lse=lse, dout=do, dq=torch.empty_like(q), dk=torch.empty_like(k), dv=torch.empty_like(v))
+    for name in ("q", "k", "v", "dout", "dq", "dk", "dv", "o"):
+        with pytest.raises(RuntimeError):
+            sb.attention_backward(**{**args, name: _offset(args[name], 1 if name == "o" else 4)})
+    for name in ("q", "k", "v", "out"):
+        with pytest.raises(RuntimeError):
+            sb.attention_forward(**{**dict(q=q, k=k, v=v, out=torch.empty_like(q)), name: _offset(q if name in ("q", "out") else k, 4)})
+    with pytest.raises(RuntimeError):
+        sb.BackwardPieces(q, _offset(o, 1), lse, do)
+    with pytest.raises(RuntimeError):
+        sb.BackwardPieces(q, o, lse, _offset(do, 2))
+    # scratch, of the direct and of the staged calls
+    stream = torch.cuda.current_stream().cuda_stream
+    scratch = torch.empty(1 << 24, dtype=torch.uint8, device="cuda")
+    for dtype, layout, flags in ((_lib.DTYPE_BF16, _lib.LAYOUT_BHSD, 0), (_lib.DTYPE_F32, _lib.LAYOUT_SENTINEL, _lib.FLAG_ALLOW_BF16_COMPUTE)):
+        d = _lib.Desc(dtype, layout, 1, 4, 2, 256, 256, 64, 0.125, 1, 256, 0, flags)
+        m = [torch.empty(256 * 256 * 4, device="cuda") for _ in range(9)]
+        p = [t.data_ptr() for t in m]
+        assert lib.sntl_attn_bwd(C.byref(d), *p, scratch.data_ptr() + 8, 1 << 23, stream) == _lib.ERR_CUDA
+        if layout == _lib.LAYOUT_SENTINEL:
+            assert lib.sntl_attn_fwd(C.byref(d), *p[:5], scratch.data_ptr() + 8, 1 << 23, stream) == _lib.ERR_CUDA
+    assert sb.launch_count() == before
+    torch.cuda.synchronize()                 # no error is pending

@@ -445,10 +445,10 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 // Combines the partial results of a row: LSE = log sum_s exp(lse_s), O = sum_s exp(lse_s - LSE) * O_s; a part without a visible
 // key carries LSE = -inf and weighs nothing.  D/8 lanes hold one row, 16 bytes each, with the loads of four parts in flight.
 // kWide: the lane groups of a block share ONE row and take its parts in turn (decode of a few long sequences: dozens of parts
-// for a few dozen rows), else a row each.
+// for a few dozen rows), else a row each.  O is stored 16 bytes at a time where it starts on such a boundary.
 template <int D, bool kWide>
-__global__ void __launch_bounds__(256) cache_merge_kernel(const CacheParams p, int rows_per_unit, int parts_per_piece, __nv_bfloat16* __restrict__ o,
-                                                          float* __restrict__ lse)
+__global__ void __launch_bounds__(256) cache_merge_kernel(const CacheParams p, int rows_per_unit, int parts_per_piece, bool o_aligned,
+                                                          __nv_bfloat16* __restrict__ o, float* __restrict__ lse)
 {
     constexpr int kLanes = D / 8, kGroups = 256 / kLanes;
     __shared__ float s_acc[kWide ? kGroups : 1][kWide ? D : 1], s_m[kWide ? kGroups : 1], s_l[kWide ? kGroups : 1];
@@ -518,8 +518,14 @@ __global__ void __launch_bounds__(256) cache_merge_kernel(const CacheParams p, i
         }
     }
     const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
-    *reinterpret_cast<uint4*>(o + (size_t)r * D + l8) = make_uint4(pack_bf16(acc[0] * inv, acc[1] * inv), pack_bf16(acc[2] * inv, acc[3] * inv),
-                                                                   pack_bf16(acc[4] * inv, acc[5] * inv), pack_bf16(acc[6] * inv, acc[7] * inv));
+    __nv_bfloat16* dst = o + (size_t)r * D + l8;
+    if (o_aligned) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(acc[0] * inv, acc[1] * inv), pack_bf16(acc[2] * inv, acc[3] * inv),
+                                                    pack_bf16(acc[4] * inv, acc[5] * inv), pack_bf16(acc[6] * inv, acc[7] * inv));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dst[i] = __float2bfloat16_rn(acc[i] * inv);
+    }
     if (l8 == 0) lse[r] = sum > 0.0f ? m + __logf(sum) : -INFINITY;
 }
 
@@ -577,10 +583,11 @@ cudaError_t launch_cache(const TcArgs& a, const CachePlan& plan, int capacity, v
     if ((e = encode_tmap_bf16_3d(&tq, a.q, D, rows_per_slab, slabs, L::kQRows)) != cudaSuccess) return e;
     if ((e = encode_tmap_bf16_3d(&tk, a.k, D, s.Skv, slabs, 128, capacity)) != cudaSuccess) return e;
     if ((e = encode_tmap_bf16_3d(&tv, a.v, D, s.Skv, slabs, 128, capacity)) != cudaSuccess) return e;
+    if (!aligned(16, workspace)) return cudaErrorMisalignedAddress;   // the partial results are accessed 16 bytes at a time
     CacheParams p{};
     p.lse_part = reinterpret_cast<float*>(workspace);
     p.o_part = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<uint8_t*>(workspace) + lse_bytes(plan, rows));
-    const bool direct = plan.max_parts == 1;   // one part per unit: it is the result
+    const bool o_aligned = aligned(16, a.o_out), direct = plan.max_parts == 1 && o_aligned;   // one part per unit: it is the result
     if (direct) {
         p.o_part = a.o_out;
         p.lse_part = a.lse_out;
@@ -598,10 +605,10 @@ cudaError_t launch_cache(const TcArgs& a, const CachePlan& plan, int capacity, v
     const int per_piece = kMode == kPair ? 1 : 2;
     // more than eight parts a row: their loads want to be in flight at once
     if (plan.max_parts > 8 && rows <= 4096)
-        return launch_kernel(cache_merge_kernel<D, true>, (unsigned)rows, 256, 0, st, 1, p, unit_rows(kMode), per_piece, a.o_out, a.lse_out);
+        return launch_kernel(cache_merge_kernel<D, true>, (unsigned)rows, 256, 0, st, 1, p, unit_rows(kMode), per_piece, o_aligned, a.o_out, a.lse_out);
     constexpr int kRowsPerBlock = 256 / (D / 8);
     return launch_kernel(cache_merge_kernel<D, false>, (unsigned)((rows + kRowsPerBlock - 1) / kRowsPerBlock), 256, 0, st, 1, p,
-                         unit_rows(kMode), per_piece, a.o_out, a.lse_out);
+                         unit_rows(kMode), per_piece, o_aligned, a.o_out, a.lse_out);
 }
 
 }  // namespace

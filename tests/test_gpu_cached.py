@@ -179,3 +179,23 @@ def test_cached_forward_argument_errors(sb):
     q5 = torch.zeros(1, 4, 5, 64, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(ValueError):
         sb.attention_cached_forward(q5, kc, kc, 3)         # more new tokens than cached keys
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,T,L,D", [
+    (3, 8, 2, 1, 500, 64),            # merged, a row per lane group
+    (1, 4, 1, 1, 40000, 128),         # merged, a row per block
+    (3, 8, 2, 100, 900, 64),          # merged, 256 rows per unit
+    (74, 2, 2, 150, 150, 128),        # one partial result per unit: stored without a merge where the result is aligned
+])
+def test_cached_forward_writes_results_at_any_address(sb, B, Hq, Hkv, T, L, D):
+    """A result handed in by the caller may start on any element: the same bits as in a tensor of its own."""
+    g = torch.Generator(device="cuda").manual_seed(T + L)
+    q, kc, vc = (torch.randn(B, H, S, D, generator=g, device="cuda").to(torch.bfloat16) for H, S in ((Hq, T), (Hkv, L), (Hkv, L)))
+    o, lse = sb.attention_cached_forward(q, kc, vc, L)
+    for first in (1, 4):
+        block = torch.full((q.numel() + 16,), 9.0, dtype=torch.bfloat16, device="cuda")
+        out = block[first:first + q.numel()].view(q.shape)
+        got, got_lse = sb.attention_cached_forward(q, kc, vc, L, out=out)
+        assert got.data_ptr() == out.data_ptr() and torch.equal(got, o) and torch.equal(got_lse, lse)
+        assert bool((block[:first] == 9).all()) and bool((block[first + q.numel():] == 9).all())
+    assert sb.last_path() == "tcgen05_cache" and sb.poll_device_status() == 0

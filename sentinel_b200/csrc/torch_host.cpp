@@ -403,17 +403,6 @@ PyObject* unpack_heads(PyObject*, PyObject* const* a, Py_ssize_t n)
     });
 }
 
-// workspace(nbytes): the scratch of the current device and stream, for the callers that launch through ctypes
-PyObject* py_workspace(PyObject*, PyObject* arg)
-{
-    return guard([&]() -> PyObject* {
-        const int64_t bytes = as_int(arg);
-        want(bytes > 0);
-        const Where at_;
-        return THPVariable_Wrap(workspace((size_t)bytes, at_.device, at_.stream));
-    });
-}
-
 // bind(addresses): in the order of the pointers below
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n)
 {
@@ -440,7 +429,6 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n)
 
 PyMethodDef methods[] = {
     {"bind", (PyCFunction)(void (*)())bind, METH_FASTCALL, nullptr},
-    {"workspace", py_workspace, METH_O, nullptr},
     {"forward", (PyCFunction)(void (*)())forward, METH_FASTCALL, nullptr},
     {"backward", (PyCFunction)(void (*)())backward, METH_FASTCALL, nullptr},
     {"cached_forward", (PyCFunction)(void (*)())cached_forward, METH_FASTCALL, nullptr},

@@ -13,7 +13,7 @@ the current stream.
 
 The calls below hand their arguments to the native module first (``csrc/torch_host.cpp``: checks, allocation and the C ABI
 call in native code, about 20 us less per call).  It declines with ``None`` when anything is not as it expects; the Python
-code that follows then names the error, or makes the call for arguments it alone accepts.
+code that follows then names the error, raises torch's own (out of memory), or makes the call for arguments it alone accepts.
 """
 from __future__ import annotations
 
@@ -28,12 +28,9 @@ def _stream_ptr() -> int:
 
 
 def _workspace(nbytes: int, device) -> torch.Tensor | None:
-    """Grow-only scratch per (device, stream) (the reference grows its buffers the same way, CudaMatmul.cu:119-136).
-    Calls on different streams may overlap on the GPU, so each stream gets scratch of its own."""
-    if nbytes == 0:
-        return None
-    with torch.cuda.device(device):
-        return _lib.host().workspace(nbytes)
+    """Scratch of one call made from here: from torch's allocator, which hands it on in stream order and raises
+    ``torch.OutOfMemoryError`` when there is none.  (Calls through the native module keep scratch per stream.)"""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
 
 
 def _dtype_code(t: torch.Tensor) -> int:

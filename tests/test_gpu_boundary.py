@@ -217,3 +217,28 @@ def test_misaligned_tensors_are_refused_before_any_launch(sb):
             assert lib.sntl_attn_fwd(C.byref(d), *p[:5], scratch.data_ptr() + 8, 1 << 23, stream) == _lib.ERR_CUDA
     assert sb.launch_count() == before
     torch.cuda.synchronize()                 # no error is pending
+
+
+def test_out_of_memory_for_scratch_is_torchs_own_error(sb):
+    """A call whose scratch cannot be allocated raises torch.OutOfMemoryError (what retry and batch-shrinking code catches), and
+    the same call works once there is memory.  The process's own limit is lowered; the GPU's memory is not exhausted."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, do = (torch.randn(2, 16, 8192, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(2, 4, 8192, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    o, lse = sb.attention_forward(q, k, v)
+    out = dict(dq=torch.empty_like(q), dk=torch.empty_like(k), dv=torch.empty_like(v))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+    try:
+        with torch.cuda.stream(stream), pytest.raises(torch.OutOfMemoryError):
+            sb.attention_backward(q, k, v, o, lse, do, flags=4, **out)      # 270 MB of 64-bit dQ words and more
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    with torch.cuda.stream(stream):
+        sb.attention_backward(q, k, v, o, lse, do, flags=4, **out)
+    torch.cuda.synchronize()
+    assert sb.poll_device_status() == 0 and bool(torch.isfinite(out["dq"]).all())

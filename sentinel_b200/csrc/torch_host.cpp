@@ -25,6 +25,7 @@
 
 #include <cmath>
 #include <map>
+#include <mutex>
 #include <utility>
 
 #include "sntl_attn.h"
@@ -120,38 +121,49 @@ PyObject* guard(F&& f)
     }
 }
 
-// the launches themselves run without the interpreter lock, as they do through ctypes
-template <typename F>
-int unlocked(F&& f)
-{
-    PyThreadState* s = PyEval_SaveThread();
-    const int rc = f();
-    PyEval_RestoreThread(s);
-    return rc;
-}
-
 // ---- scratch ----
 // Grow-only, one buffer per (device, stream): calls on different streams may overlap on the GPU.  torch hands out streams
-// from pools of 32 per device and priority, which bounds the number of entries.  Guarded by the interpreter lock; a call
-// keeps its own reference while it launches, and a buffer that was replaced goes back to torch's allocator in stream order.
+// from pools of 32 per device and priority, which bounds the number of entries.  The interpreter lock guards the map; it is given
+// up during the launches, and the kernels of one call hand data to one another through the buffer, so calls of several threads on
+// one stream are kept apart by the entry's own lock (taken without the interpreter lock: nothing waits for both).  A call keeps its
+// own reference to the buffer while it launches; one that was replaced goes back to torch's allocator in stream order.
 using WsKey = std::pair<int, void*>;
-std::map<WsKey, at::Tensor>& ws_cache()
+struct Scratch {
+    at::Tensor buffer;
+    std::mutex launching;
+};
+Scratch& scratch(const WsKey& key)
 {
-    static auto* m = new std::map<WsKey, at::Tensor>;   // never destroyed: torch's allocator may be gone by then
-    return *m;
-}
-at::Tensor workspace(size_t bytes, c10::DeviceIndex device, void* stream)
-{
-    at::Tensor& t = ws_cache()[WsKey(device, stream)];
-    if (!t.defined() || (size_t)t.numel() < bytes)
-        t = at::Tensor(at::detail::empty_cuda({(int64_t)bytes}, at::kByte, at::Device(at::kCUDA, device), std::nullopt));
-    return t;
+    static auto* m = new std::map<WsKey, Scratch>;   // never destroyed: torch's allocator may be gone by then
+    return (*m)[key];
 }
 
 struct Where {
     c10::DeviceIndex device = c10::cuda::current_device();
     void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
 };
+
+// call(pointer to `bytes` of scratch, null for none), without the interpreter lock, as through ctypes
+template <typename F>
+int launch(const Where& at_, size_t bytes, F&& call)
+{
+    at::Tensor buffer;
+    std::unique_lock<std::mutex> alone;
+    if (bytes) {
+        Scratch& s = scratch(WsKey(at_.device, at_.stream));
+        if (!s.buffer.defined() || (size_t)s.buffer.numel() < bytes)
+            s.buffer = at::Tensor(at::detail::empty_cuda({(int64_t)bytes}, at::kByte, at::Device(at::kCUDA, at_.device), std::nullopt));
+        buffer = s.buffer;
+        alone = std::unique_lock<std::mutex>(s.launching, std::defer_lock);
+    }
+    void* const p = bytes ? buffer.mutable_data_ptr() : nullptr;
+    PyThreadState* state = PyEval_SaveThread();
+    if (bytes) alone.lock();
+    const int rc = call(p);
+    if (bytes) alone.unlock();
+    PyEval_RestoreThread(state);
+    return rc;
+}
 
 int32_t dtype_code(const at::Tensor& t)
 {
@@ -199,11 +211,9 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n)
         const at::Tensor o = result(a[6], q.sizes(), q.scalar_type(), at_.device);
         const at::Tensor lse = result(a[7], q.sizes().slice(0, 3), at::kFloat, at_.device);
         const size_t bytes = p_fwd_ws(&d);
-        at::Tensor ws;
-        if (bytes) ws = workspace(bytes, at_.device, at_.stream);
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, bytes, [&](void* ws) {
             return p_fwd(&d, q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), o.mutable_data_ptr(), (float*)lse.mutable_data_ptr(),
-                         bytes ? ws.mutable_data_ptr() : nullptr, bytes, at_.stream);
+                         ws, bytes, at_.stream);
         });
         return rc == SNTL_OK ? pack_tuple(o, lse) : PyLong_FromLong(rc);
     });
@@ -225,12 +235,10 @@ PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n)
         const at::Tensor dq = result(a[9], q.sizes(), type, at_.device), dk = result(a[10], k.sizes(), type, at_.device);
         const at::Tensor dv = result(a[11], v.sizes(), type, at_.device);
         const size_t bytes = p_bwd_ws(&d);
-        at::Tensor ws;
-        if (bytes) ws = workspace(bytes, at_.device, at_.stream);
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, bytes, [&](void* ws) {
             return p_bwd(&d, q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), o.const_data_ptr(), (const float*)lse.const_data_ptr(),
                          dout.const_data_ptr(), dq.mutable_data_ptr(), dk.mutable_data_ptr(), dv.mutable_data_ptr(),
-                         bytes ? ws.mutable_data_ptr() : nullptr, bytes, at_.stream);
+                         ws, bytes, at_.stream);
         });
         return rc == SNTL_OK ? pack_tuple(dq, dk, dv) : PyLong_FromLong(rc);
     });
@@ -250,11 +258,9 @@ PyObject* cached_forward(PyObject*, PyObject* const* a, Py_ssize_t n)
         const at::Tensor o = result(a[6], q.sizes(), q.scalar_type(), at_.device);
         const at::Tensor lse = result(a[7], q.sizes().slice(0, 3), at::kFloat, at_.device);
         const size_t bytes = p_cached_ws(&d, capacity);
-        at::Tensor ws;
-        if (bytes) ws = workspace(bytes, at_.device, at_.stream);
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, bytes, [&](void* ws) {
             return p_cached(&d, q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), capacity, o.mutable_data_ptr(),
-                            (float*)lse.mutable_data_ptr(), bytes ? ws.mutable_data_ptr() : nullptr, bytes, at_.stream);
+                            (float*)lse.mutable_data_ptr(), ws, bytes, at_.stream);
         });
         return rc == SNTL_OK ? pack_tuple(o, lse) : PyLong_FromLong(rc);
     });
@@ -310,11 +316,9 @@ PyObject* matrix_forward(PyObject*, PyObject* const* a, Py_ssize_t n)
         const sntl_attn_desc d = matrix_desc(q, k, a + 5);
         want(k.sizes() == v.sizes() && o.sizes() == q.sizes() && lse.size(0) == d.q_heads && lse.size(1) == d.stride_columns);
         const size_t bytes = p_fwd_ws(&d);
-        at::Tensor ws;
-        if (bytes) ws = workspace(bytes, at_.device, at_.stream);
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, bytes, [&](void* ws) {
             return p_fwd(&d, q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), o.mutable_data_ptr(), (float*)lse.mutable_data_ptr(),
-                         bytes ? ws.mutable_data_ptr() : nullptr, bytes, at_.stream);
+                         ws, bytes, at_.stream);
         });
         return rc == SNTL_OK ? pack_tuple(o, lse) : PyLong_FromLong(rc);
     });
@@ -333,12 +337,10 @@ PyObject* matrix_backward(PyObject*, PyObject* const* a, Py_ssize_t n)
         want(k.sizes() == v.sizes() && o.sizes() == q.sizes() && g.sizes() == q.sizes() && dq.sizes() == q.sizes());
         want(dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && lse.size(0) == d.q_heads && lse.size(1) == d.stride_columns);
         const size_t bytes = p_bwd_ws(&d);
-        at::Tensor ws;
-        if (bytes) ws = workspace(bytes, at_.device, at_.stream);
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, bytes, [&](void* ws) {
             return p_bwd(&d, q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), o.const_data_ptr(), (const float*)lse.const_data_ptr(),
                          g.const_data_ptr(), dq.mutable_data_ptr(), dk.mutable_data_ptr(), dv.mutable_data_ptr(),
-                         bytes ? ws.mutable_data_ptr() : nullptr, bytes, at_.stream);
+                         ws, bytes, at_.stream);
         });
         return rc == SNTL_OK ? pack_tuple(dq, dk, dv) : PyLong_FromLong(rc);
     });
@@ -374,7 +376,7 @@ PyObject* pack_heads(PyObject*, PyObject* const* a, Py_ssize_t n)
         const int32_t start = as_i32(a[5]), offset = as_i32(a[8]);
         const int64_t shape[4] = {batch, heads, seq, dim};
         const at::Tensor out = result(a[9], shape, at::kBFloat16, at_.device);
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, 0, [&](void*) {
             return p_pack((const float*)m.const_data_ptr(), out.mutable_data_ptr(), batch, heads, seq, dim, (int32_t)m.size(1), start, t.cos,
                           t.sin, offset, t.positions, at_.stream);
         });
@@ -393,7 +395,7 @@ PyObject* unpack_heads(PyObject*, PyObject* const* a, Py_ssize_t n)
         for (int i = 0; i < 4; ++i) want(x.size(i) <= INT32_MAX);
         const Tables t = as_tables(a[3], a[4], x.size(3), at_.device);
         const int32_t start = as_i32(a[2]), offset = as_i32(a[5]), inverse = as_bool(a[6]) ? 1 : 0;
-        const int rc = unlocked([&] {
+        const int rc = launch(at_, 0, [&](void*) {
             return p_unpack(x.const_data_ptr(), (float*)m.mutable_data_ptr(), (int32_t)x.size(0), (int32_t)x.size(1), (int32_t)x.size(2),
                             (int32_t)x.size(3), (int32_t)m.size(1), start, t.cos, t.sin, offset, t.positions, inverse, at_.stream);
         });

@@ -242,3 +242,36 @@ def test_out_of_memory_for_scratch_is_torchs_own_error(sb):
         sb.attention_backward(q, k, v, o, lse, do, flags=4, **out)
     torch.cuda.synchronize()
     assert sb.poll_device_status() == 0 and bool(torch.isfinite(out["dq"]).all())
+
+
+def test_threads_on_one_stream_keep_their_scratch_apart(sb):
+    """Python threads share the default stream, and the interpreter lock is given up while a call launches its kernels: the kernels
+    of two calls must not alternate on one buffer.  Different problems in each thread, every result as when called alone."""
+    import sys
+    import threading
+    cases = []
+    for seed, (H, S, D) in enumerate(((8, 384, 64), (3, 640, 128), (12, 200, 64))):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        q, do, k, v = (torch.randn(1, H, S, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+        o, lse = sb.attention_forward(q, k, v)
+        cases.append(((q, k, v, o, lse, do), [t.clone() for t in sb.attention_backward(q, k, v, o, lse, do, flags=4)]))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(args, want):
+        for _ in range(150):
+            got = sb.attention_backward(*args, flags=4)
+            if not all(torch.equal(x, y) for x, y in zip(got, want)):
+                wrong.append(args[0].shape)
+
+    switch = sys.getswitchinterval()
+    sys.setswitchinterval(1e-5)
+    try:
+        threads = [threading.Thread(target=work, args=c) for c in cases for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(switch)
+    assert not wrong and sb.poll_device_status() == 0

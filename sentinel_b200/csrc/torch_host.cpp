@@ -20,6 +20,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -27,6 +28,7 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include "sntl_attn.h"
 
@@ -127,10 +129,15 @@ PyObject* guard(F&& f)
 // up during the launches, and the kernels of one call hand data to one another through the buffer, so calls of several threads on
 // one stream are kept apart by the entry's own lock (taken without the interpreter lock: nothing waits for both).  A call keeps its
 // own reference to the buffer while it launches; one that was replaced goes back to torch's allocator in stream order.
+// A graph replays with the address it recorded.  A call that is being captured uses the buffer that is there (after a warm-up on
+// this stream), which is then kept when a later call outgrows it; where there is none that is large enough it takes one of its
+// own, which torch's allocator keeps for as long as the graph.
 using WsKey = std::pair<int, void*>;
 struct Scratch {
     at::Tensor buffer;
     std::mutex launching;
+    bool recorded = false;            // a graph may hold the address of `buffer`
+    std::vector<at::Tensor> kept;     // outgrown buffers of which that is true (one per growth at most)
 };
 Scratch& scratch(const WsKey& key)
 {
@@ -149,18 +156,30 @@ int launch(const Where& at_, size_t bytes, F&& call)
 {
     at::Tensor buffer;
     std::unique_lock<std::mutex> alone;
+    auto allocate = [&] { return at::Tensor(at::detail::empty_cuda({(int64_t)bytes}, at::kByte, at::Device(at::kCUDA, at_.device), std::nullopt)); };
     if (bytes) {
         Scratch& s = scratch(WsKey(at_.device, at_.stream));
-        if (!s.buffer.defined() || (size_t)s.buffer.numel() < bytes)
-            s.buffer = at::Tensor(at::detail::empty_cuda({(int64_t)bytes}, at::kByte, at::Device(at::kCUDA, at_.device), std::nullopt));
-        buffer = s.buffer;
-        alone = std::unique_lock<std::mutex>(s.launching, std::defer_lock);
+        const bool captured = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+        const bool fits = s.buffer.defined() && (size_t)s.buffer.numel() >= bytes;
+        if (captured && !fits) {
+            buffer = allocate();
+        } else {
+            if (!fits) {
+                at::Tensor larger = allocate();
+                if (s.recorded) s.kept.push_back(s.buffer);
+                s.buffer = larger;
+                s.recorded = false;
+            }
+            s.recorded = s.recorded || captured;
+            buffer = s.buffer;
+            alone = std::unique_lock<std::mutex>(s.launching, std::defer_lock);
+        }
     }
     void* const p = bytes ? buffer.mutable_data_ptr() : nullptr;
     PyThreadState* state = PyEval_SaveThread();
-    if (bytes) alone.lock();
+    if (alone.mutex()) alone.lock();
     const int rc = call(p);
-    if (bytes) alone.unlock();
+    if (alone.owns_lock()) alone.unlock();
     PyEval_RestoreThread(state);
     return rc;
 }

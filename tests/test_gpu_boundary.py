@@ -275,3 +275,34 @@ def test_threads_on_one_stream_keep_their_scratch_apart(sb):
     finally:
         sys.setswitchinterval(switch)
     assert not wrong and sb.poll_device_status() == 0
+
+
+@pytest.mark.parametrize("warm", [True, False])
+def test_scratch_of_a_captured_call_stays_with_its_graph(sb, warm):
+    """A call is captured on a stream that has made the same call before, or has not; a larger call then replaces that stream's
+    scratch, and other tensors take its place.  A replay gives the same results and leaves those tensors alone."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, do, k, v = (torch.randn(1, 4, 512, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    big = [torch.randn(2, 8, 2048, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    o, lse = sb.attention_forward(q, k, v)
+    big_o, big_lse = sb.attention_forward(*big[:3])
+    grads = dict(dq=torch.empty_like(q), dk=torch.empty_like(k), dv=torch.empty_like(v))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream if warm else torch.cuda.current_stream()):
+        want = [t.clone() for t in sb.attention_backward(q, k, v, o, lse, do, flags=4, **grads)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        sb.attention_backward(q, k, v, o, lse, do, flags=4, **grads)
+    with torch.cuda.stream(stream):
+        sb.attention_backward(*big[:3], big_o, big_lse, big[3], flags=4)
+        others = [torch.full((1 << n,), 3.0, device="cuda") for n in range(10, 21) for _ in range(4)]
+    stream.synchronize()
+    for t in grads.values():
+        t.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    for got, ref in zip(grads.values(), want):
+        assert torch.equal(got, ref)
+    assert all(bool((t == 3).all()) for t in others) and sb.poll_device_status() == 0

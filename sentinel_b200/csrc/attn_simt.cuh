@@ -10,6 +10,9 @@
 //   outputs  acc[i][c] += sum_k W[k][ty + 8i] * B[k][c]            W (probabilities) is stored [k][ty*TM + i]: the order in which
 //                                                                  the thread that owns the rows reads them back
 // W is written and read by the 16 threads of one ty, which are half a warp: no CTA barrier between the two products.
+// A hidden (query, key) pair has weight 0, which adds nothing unless the other factor is not finite (0 * inf).  Tiles that the mask
+// cuts through are looked at for that, V while it is staged and the backward's operands by their scores; where a value is not
+// finite the products leave the hidden pairs out one by one (outputs_visible).
 #pragma once
 
 #include "common.cuh"
@@ -73,9 +76,17 @@ __device__ __forceinline__ void unit_of(int u, bool rows_contiguous, int& r, int
     else { d = (u / ROWS) * 4; r = u % ROWS; }                                // feature-major: tokens are
 }
 
-template <typename T, int DP, int ROWS>
-__device__ __forceinline__ void stage(float* dst, const T* base, const Slab& m, int row0)
+// 0, or NaN once a value was not finite
+__device__ __forceinline__ float zero_if_finite(float z, const float4& x)
 {
+    return fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, fmaf(x.w, 0.f, z))));
+}
+
+// Returns zero_if_finite of what this thread has staged.
+template <typename T, int DP, int ROWS>
+__device__ __forceinline__ float stage(float* dst, const T* base, const Slab& m, int row0)
+{
+    float z = 0.f;
     constexpr int kUnits = ROWS * DP / 4, kPer = (kUnits + kThreads - 1) / kThreads, kBatch = kPer < 4 ? kPer : 4;
 #pragma unroll
     for (int k0 = 0; k0 < kPer; k0 += kBatch) {
@@ -92,9 +103,13 @@ __device__ __forceinline__ void stage(float* dst, const T* base, const Slab& m, 
             const int u = (k0 + k) * kThreads + (int)threadIdx.x;
             int r, d;
             unit_of<DP, ROWS>(u, m.sd != 1, r, d);
-            if (u < kUnits) *reinterpret_cast<float4*>(dst + r * (DP + 4) + d) = x[k];
+            if (u < kUnits) {
+                *reinterpret_cast<float4*>(dst + r * (DP + 4) + d) = x[k];
+                z = zero_if_finite(z, x[k]);
+            }
         }
     }
+    return z;
 }
 
 // dO rows as above and, for delta = rowsum(dO o O), one partial sum per 16-byte unit: part[row][unit]
@@ -180,6 +195,24 @@ __device__ __forceinline__ void scores(float (&out)[TM][TN], const float* A, con
         for (int j = 0; j < TN; ++j) out[i][j] = acc[i][j].x + acc[i][j].y;
 }
 
+// Whether one of the warp's scores (all scores of a row are not finite if one of its values is not) or of the terms of their columns
+// (in shared memory, or null) is not finite.
+template <int TM, int TN>
+__device__ __forceinline__ bool not_finite(const float (&a)[TM][TN], const float (&b)[TM][TN], const float* terms)
+{
+    float z = 0.f, y = 0.f;     // (two chains: one would be 2 * TM * TN long)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+        if (terms) z = fmaf(terms[(threadIdx.x & 15) + 16 * j], 0.f, z);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            z = fmaf(a[i][j], 0.f, z);
+            y = fmaf(b[i][j], 0.f, y);
+        }
+    }
+    return __any_sync(0xffffffffu, z + y != 0.f);
+}
+
 // columns of the outputs a thread owns: NV vectors of VW, starting at tx*VW + 16*VW*c
 template <int DP> struct OutMap {
     static constexpr int VW = DP % 64 == 0 ? 4 : DP % 32 == 0 ? 2 : 1;
@@ -221,6 +254,25 @@ __device__ __forceinline__ void outputs(float2 (&acc)[TM / 2][OutMap<DP>::N], co
         for (int n = 0; n < M::N; ++n)
 #pragma unroll
             for (int i = 0; i < TM / 2; ++i) acc[i][n] = ffma2(make_float2(w[2 * i], w[2 * i + 1]), make_float2(b[n], b[n]), acc[i][n]);
+    }
+}
+// The same for a tile that holds values that are not finite and pairs that are hidden: visible(i, k), of the thread's row ty + 8*i.
+template <int TM, int DP, int K, typename F>
+__device__ __forceinline__ void outputs_visible(float2 (&acc)[TM / 2][OutMap<DP>::N], const float* W, const float* B, F&& visible)
+{
+    using M = OutMap<DP>;
+#pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            if (!visible(i, k)) continue;
+            const float w = W[k * (8 * TM + 4) + (threadIdx.x >> 4) * TM + i];
+#pragma unroll
+            for (int n = 0; n < M::N; ++n) {
+                float& a = i & 1 ? acc[i / 2][n].y : acc[i / 2][n].x;
+                a = fmaf(w, B[k * (DP + 4) + M::col(n)], a);
+            }
+        }
     }
 }
 template <int TM, int N> __device__ __forceinline__ void clear(float2 (&acc)[TM][N])

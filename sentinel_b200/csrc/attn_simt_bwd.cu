@@ -26,6 +26,33 @@ template <int TM, int TN, int DP> struct BwdSmem {
     static constexpr size_t bytes = (delta + kDeltaRows) * sizeof(float);
 };
 
+// outputs_visible as a function of its own, with the sums handed over in memory: inlined, it costs the kernel registers where it never
+// runs (B8 H12 S512 D64 410 us without it, 447 inlined, 412 so).
+template <int TM, int DP, int K, typename F>
+__device__ __noinline__ void outputs_visible_call(float2* sums, const float* W, const float* B, F visible)
+{
+    using M = OutMap<DP>;
+    for (int i = 0; i < TM; ++i)
+        for (int n = 0; n < M::N; ++n) {
+            float2& sum = sums[i / 2 * M::N + n];
+            float a = i & 1 ? sum.y : sum.x;
+            for (int k = 0; k < K; ++k)
+                if (visible(i, k)) a = fmaf(W[k * (8 * TM + 4) + (threadIdx.x >> 4) * TM + i], B[k * (DP + 4) + M::col(n)], a);
+            (i & 1 ? sum.y : sum.x) = a;
+        }
+}
+template <int TM, int DP, int K, typename F>
+__device__ __forceinline__ void outputs_visible_apart(float2 (&acc)[TM / 2][OutMap<DP>::N], const float* W, const float* B, F visible)
+{
+    constexpr int N = OutMap<DP>::N;
+    float2 sums[TM / 2 * N];
+#pragma unroll
+    for (int i = 0; i < TM / 2 * N; ++i) sums[i] = acc[i / N][i % N];
+    outputs_visible_call<TM, DP, K>(sums, W, B, visible);
+#pragma unroll
+    for (int i = 0; i < TM / 2 * N; ++i) acc[i / N][i % N] = sums[i];
+}
+
 template <typename T, int TM, int TN, int DP>
 __device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* smem)
 {
@@ -66,6 +93,7 @@ __device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* sme
             __syncthreads();
             // every (query, key) pair of the tile is visible: no masks
             const bool cut = (s.causal && q0 + shift < key0 + L::kRows - 1) || s.window > 0 || key0 + L::kRows > s.Skv;
+            const bool odd = cut && not_finite(p, ds, smem + L::delta);
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
                 const int q = q0 + tx + 16 * j;
@@ -82,8 +110,17 @@ __device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* sme
                 put_weights<TM>(smem + L::w1, tx + 16 * j, ws);
             }
             __syncwarp();
-            outputs<TM, DP, L::kLoop>(dv, smem + L::w0, smem + L::in1);
-            outputs<TM, DP, L::kLoop>(dk, smem + L::w1, smem + L::in0);
+            if (!odd) {
+                outputs<TM, DP, L::kLoop>(dv, smem + L::w0, smem + L::in1);
+                outputs<TM, DP, L::kLoop>(dk, smem + L::w1, smem + L::in0);
+            } else {
+                auto visible = [=](int i, int k) {
+                    const int key = key0 + ty + 8 * i, q = q0 + k;
+                    return q < s.Sq && (!s.causal || key <= q + shift) && window_allows(s, q + shift, key);
+                };
+                outputs_visible_apart<TM, DP, L::kLoop>(dv, smem + L::w0, smem + L::in1, visible);
+                outputs_visible_apart<TM, DP, L::kLoop>(dk, smem + L::w1, smem + L::in0, visible);
+            }
         }
     }
     __syncthreads();
@@ -128,7 +165,7 @@ __device__ __forceinline__ void dq_role(const SimtArgs& a, int tile, int n_qt, f
         float p[TM][TN], ds[TM][TN];
         scores<TM, TN, DP>(p, smem + L::own0, smem + L::in0);
         scores<TM, TN, DP>(ds, smem + L::own1, smem + L::in1);
-        const bool cut = k0 + L::kLoop > visible_keys(s, row0) || s.window > 0;
+        const bool cut = k0 + L::kLoop > visible_keys(s, row0) || s.window > 0, odd = cut && not_finite(p, ds, nullptr);
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int key = k0 + tx + 16 * j;
@@ -143,14 +180,25 @@ __device__ __forceinline__ void dq_role(const SimtArgs& a, int tile, int n_qt, f
             put_weights<TM>(smem + L::w0, tx + 16 * j, w);
         }
         __syncwarp();
-        outputs<TM, DP, L::kLoop>(dq, smem + L::w0, smem + L::in0);
+        if (!odd) {
+            outputs<TM, DP, L::kLoop>(dq, smem + L::w0, smem + L::in0);
+        } else {
+            outputs_visible_apart<TM, DP, L::kLoop>(dq, smem + L::w0, smem + L::in0, [=](int i, int k) {
+                const int row = row0 + ty + 8 * i, key = k0 + k;
+                return key < visible_keys(s, row) && window_allows(s, row + shift, key);
+            });
+        }
     }
     __syncthreads();
     store_rows<T, TM, DP>((T*)a.dq + qoff, mq, row0, dq, smem + L::own0);
 }
 
+// CTAs beside each other that shared memory allows and registers can follow without spilling (left to the compiler, 16-row tiles at
+// head_dim 128 take 254 registers and run two beside each other: B4 H8 S256 119 -> 143 us)
+template <int TM, int DP> constexpr int kMinCtas = TM == 2 ? (DP == 16 ? 4 : DP <= 128 ? 3 : 1) : TM == 4 && (DP <= 32 || DP == 96) ? 3 : 1;
+
 template <typename T, int TM, int TN, int DP>
-__global__ void __launch_bounds__(kThreads) simt_bwd_kernel(const SimtArgs a, int n_dkv, int n_qt)
+__global__ void __launch_bounds__(kThreads, kMinCtas<TM, DP>) simt_bwd_kernel(const SimtArgs a, int n_dkv, int n_qt)
 {
     extern __shared__ __align__(16) float smem[];
     wait_for_stream();

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
         // ---- one key per thread ----
         const int key = k0 + (int)threadIdx.x;
         float sc[R];
+        bool visible[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) sc[r] = 0.f;
         if ((int)threadIdx.x < n) {
@@ -114,7 +115,8 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int pos = first_pos + r % s.Sq;
-            sc[r] = ((int)threadIdx.x < n && r < rows && key <= pos && window_allows(s, pos, key)) ? sc[r] * s.scale : -INFINITY;
+            visible[r] = (int)threadIdx.x < n && r < rows && key <= pos && window_allows(s, pos, key);
+            sc[r] = visible[r] ? sc[r] * s.scale : -INFINITY;
             float mx = sc[r];
 #pragma unroll
             for (int x = 16; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
@@ -131,7 +133,8 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
             corr[r] = expf(m[r] - ref);
             m[r] = mx;
             const float p = expf(sc[r] - ref);
-            smem[L::p + r * kChunk + threadIdx.x] = p;
+            smem[L::p + r * kChunk + threadIdx.x] = visible[r] ? p : -1.f;   // hidden: V is left out below, whatever it holds (rows past
+                                                                             // the last: never stored)
             float sum = p;
 #pragma unroll
             for (int x = 16; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
             for (int r = 0; r < R; ++r) {
                 const float p = smem[L::p + r * kChunk + j];
 #pragma unroll
-                for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p, v[c], acc[r][c]);
+                for (int c = 0; c < kCols; ++c) acc[r][c] = p < 0.f ? acc[r][c] : fmaf(p, v[c], acc[r][c]);
             }
         }
         __syncthreads();                                      // the buffers are refilled

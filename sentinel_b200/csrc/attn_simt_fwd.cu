@@ -57,11 +57,13 @@ __global__ void __launch_bounds__(kThreads, DP <= 64 ? 3 : 2) simt_fwd_kernel(co
         if (s.window > 0 && k0 >= s.global_tokens && k0 + L::kKeys - 1 < row0 + shift - s.window + 1) continue;
         __syncthreads();
         stage<T, DP, L::kKeys>(smem + L::k, kb, mk, k0);
-        stage<T, DP, L::kKeys>(smem + L::v, vb, mk, k0);
-        __syncthreads();
+        const float z = stage<T, DP, L::kKeys>(smem + L::v, vb, mk, k0);
+        const bool cut = k0 + L::kKeys > visible_keys(s, row0) || s.window > 0;   // some (row, key) pair may be hidden
+        bool odd = false;                                     // ... and V holds values that are not finite
+        if (cut) odd = __syncthreads_or(z != 0.f);
+        else __syncthreads();
         float sc[TM][TN];
         scores<TM, TN, DP>(sc, smem + L::q, smem + L::k);
-        const bool cut = k0 + L::kKeys > visible_keys(s, row0) || s.window > 0;   // some (row, key) pair may be hidden
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
             const int row = row0 + ty + 8 * i, n_row = cut ? visible_keys(s, row) : 0;
@@ -94,7 +96,14 @@ __global__ void __launch_bounds__(kThreads, DP <= 64 ? 3 : 2) simt_fwd_kernel(co
             put_weights<TM>(smem + L::w, tx + 16 * j, w);
         }
         __syncwarp();
-        outputs<TM, DP, L::kKeys>(o, smem + L::w, smem + L::v);
+        if (!odd) {
+            outputs<TM, DP, L::kKeys>(o, smem + L::w, smem + L::v);
+        } else {
+            outputs_visible<TM, DP, L::kKeys>(o, smem + L::w, smem + L::v, [&](int i, int k) {
+                const int row = row0 + ty + 8 * i, key = k0 + k;
+                return key < visible_keys(s, row) && window_allows(s, row + shift, key);
+            });
+        }
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i)

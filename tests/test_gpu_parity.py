@@ -739,3 +739,59 @@ def test_full_size_sliding_window_sampled_oracle(sb, oracle):
     assert torch.equal(o_wide, o_plain) and torch.equal(lse_wide, lse_plain)
     # the first W rows see every earlier key, so they match plain causal attention exactly
     assert torch.equal(o[:, :, :W], o_plain[:, :, :W])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,window,dtype", [
+    (1, 4, 2, 200, 64, 0, torch.float32),      # tiles of 16 query rows, keys split over a cluster
+    (2, 24, 24, 300, 64, 40, torch.float32),   # 32 rows
+    (4, 48, 48, 200, 32, 0, torch.float32),    # 64 rows
+    (1, 3, 1, 150, 128, 30, torch.float32),    # 32 keys per tile
+    (1, 2, 2, 70, 256, 0, torch.bfloat16),
+])
+def test_exact_kernels_keep_hidden_tokens_apart(sb, B, Hq, Hkv, S, D, window, dtype, bad):
+    """Tokens that a row does not see may hold anything (padding, a cache's unused slots): results whose visible tokens are all
+    finite are the bits they are without such values, also where a tile of the kernel holds both."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, do, k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").to(dtype) for H in (Hq, Hq, Hkv, Hkv))
+    kw = dict(window=window, global_tokens=0, flags=2)
+    first = S - 37                              # from here on: in the middle of a tile of any height
+    q2, do2, k2, v2 = (t.clone() for t in (q, do, k, v))
+    for t in (q2, do2, k2, v2):
+        t[:, :, first::2] = bad
+    o, lse = sb.attention_forward(q, k, v, **kw)
+    o2, lse2 = sb.attention_forward(q2, k2, v2, **kw)
+    assert sb.last_path() in ("simt_f32", "simt_bf16")
+    assert torch.equal(o[:, :, :first], o2[:, :, :first]) and torch.equal(lse[:, :, :first], lse2[:, :, :first])
+    want, got = sb.attention_backward(q, k, v, o, lse, do, **kw), sb.attention_backward(q2, k2, v2, o2, lse2, do2, **kw)
+    assert torch.equal(want[0][:, :, :first], got[0][:, :, :first])
+    if window:                                  # keys that no query from `first` on sees
+        keys = first - window + 1
+        assert all(torch.equal(x[:, :, :keys], y[:, :, :keys]) for x, y in zip(want[1:], got[1:]))
+    # the other side: the first tokens, hidden from every row behind their window
+    if window:
+        for t, src in ((q2, q), (do2, do), (k2, k), (v2, v)):
+            t.copy_(src)
+            t[:, :, :9] = bad
+        o2, lse2 = sb.attention_forward(q2, k2, v2, **kw)
+        rows = 9 + window - 1
+        assert torch.equal(o[:, :, rows:], o2[:, :, rows:]) and torch.equal(lse[:, :, rows:], lse2[:, :, rows:])
+        got = sb.attention_backward(q2, k2, v2, o2, lse2, do2, **kw)
+        assert all(torch.equal(x[:, :, rows:], y[:, :, rows:]) for x, y in zip(want, got))
+
+
+@pytest.mark.parametrize("Hq,Hkv,T,L,D,window", [(4, 4, 1, 300, 64, 60), (2, 2, 3, 260, 128, 0), (8, 4, 4, 500, 32, 100)])
+def test_exact_decode_keeps_hidden_tokens_apart(sb, Hq, Hkv, T, L, D, window):
+    """The same for new tokens behind a cache: slots below the window, and later new tokens."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    q, k, v = (torch.randn(1, H, S, D, generator=g, device="cuda") for H, S in ((Hq, T), (Hkv, L), (Hkv, L)))
+    kw = dict(window=window)
+    o, lse = sb.attention_cached_forward(q, k, v, L, **kw)
+    k2, v2 = k.clone(), v.clone()
+    if T > 1:
+        k2[:, :, L - 1] = v2[:, :, L - 1] = float("inf")       # the last new token: hidden from the others
+    if window:
+        k2[:, :, :L - T - window + 1] = v2[:, :, :L - T - window + 1] = float("nan")
+    o2, lse2 = sb.attention_cached_forward(q, k2, v2, L, **kw)
+    n = max(1, T - 1)
+    assert torch.equal(o[:, :, :n], o2[:, :, :n]) and torch.equal(lse[:, :, :n], lse2[:, :, :n])

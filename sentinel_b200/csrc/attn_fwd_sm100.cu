@@ -433,7 +433,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             uint32_t pk[32];
             float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
             RowMax mx;
-            float neg_m = -m_ref;
+            auto shift = [&]() { return m_ref == -INFINITY ? 0.0f : -m_ref; };   // (no finite score so far: -inf + inf would be NaN)
+            float neg_m = shift();
             // whether some row of the warp has outgrown its reference (false when both are -inf: NaN compare)
             auto outgrown = [&](float m_new) { return j > 0 && __any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold); };
             auto s_read = [&]() {       // nothing reads S_j any more: the next S of this tile may overwrite it
@@ -464,7 +465,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     tmem_st32(tmem_O(t) + lane_off + (uint32_t)(c * 32), o);
                 }
                 tmem_st_wait();
-                neg_m = -m_ref;
+                neg_m = shift();
             };
             if (ahead) {
                 exp_half<0, true>(s, p.scale_log2, neg_m, pk, sum, mx);
@@ -502,7 +503,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if (!ok) break;
                 if (j == 0) m_ref = m_new;
                 else if (again) rescale(m_new);
-                neg_m = (m_ref == -INFINITY) ? 0.0f : -m_ref;
+                neg_m = shift();
                 SNTL_TRACE_EV(tw, 1 + t, tn, 4);
                 exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
             }

@@ -795,3 +795,34 @@ def test_exact_decode_keeps_hidden_tokens_apart(sb, Hq, Hkv, T, L, D, window):
     o2, lse2 = sb.attention_cached_forward(q, k2, v2, L, **kw)
     n = max(1, T - 1)
     assert torch.equal(o[:, :, :n], o2[:, :, :n]) and torch.equal(lse[:, :, :n], lse2[:, :, :n])
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,D,window", [
+    (1, 2, 1, 64, 0),
+    (1, 2, 1, 128, 0),
+    (6, 40, 8, 64, 0),           # more blocks than SMs
+    (1, 4, 2, 64, 160),          # rows 31 of a warp see nothing of the window's first tile
+])
+def test_forward_with_scores_of_minus_infinity(sb, B, Hq, Hkv, D, window):
+    """Keys whose scores overflow to -inf (masking by the type's lowest value) weigh nothing, also where they are all that a row
+    has seen for several tiles; a row that sees nothing else gets O = 0 and LSE = -inf."""
+    S, first = 900, 384
+    g = torch.Generator(device="cuda").manual_seed(D + window)
+    q, k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").to(torch.bfloat16) for H in (Hq, Hkv, Hkv))
+    q[..., 0] = 4.0
+    k[..., 0] = 0.0
+    k[:, :, :first, 0] = -3.0e38
+    o, lse = sb.attention_forward(q, k, v, window=window)
+    assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+    assert bool((o[:, :, :first] == 0).all()) and bool((lse[:, :, :first] == -float("inf")).all())
+    kf, vf = (t.float().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+    s = (q.float() @ kf.transpose(2, 3)) * D ** -0.5
+    i, j = torch.arange(S, device="cuda")[:, None], torch.arange(S, device="cuda")[None]
+    hidden = j > i
+    if window:
+        hidden = hidden | (j < i - window + 1)
+    s = s.masked_fill(hidden, -float("inf"))[:, :, first:]
+    want = torch.softmax(s, -1) @ vf
+    got = o[:, :, first:].float()
+    assert float((got - want).norm() / want.norm()) <= 4e-3                    # P and O rounded to bf16
+    assert float((lse[:, :, first:] - torch.logsumexp(s, -1)).abs().max()) <= 1e-3

@@ -84,7 +84,11 @@ enum {
      * 2*world-1-r (results come back in the same order).  A host that keeps its activations in this order for the whole
      * model -- the usual arrangement of causal sequence parallelism -- saves the redistribution round before and after
      * every call: the deal becomes a local copy. */
-    SNTL_FLAG_RING_ZIGZAG = 8
+    SNTL_FLAG_RING_ZIGZAG = 8,
+    /* Backward: the dK and dV of a key tile are summed in one run.  Without it the tensor-core kernel cuts the long key tiles of a
+     * small grid into pieces, whose sums are added in a fixed order: reproducible from run to run too, but in the last bits
+     * another sum, so that dK and dV of a sequence can depend on what else is in the call.  With it they do not. */
+    SNTL_FLAG_WHOLE_KEY_TILES = 16
 };
 
 typedef struct sntl_attn_desc {

@@ -44,12 +44,13 @@ int validate(const sntl_attn_desc* d)
     return SNTL_OK;
 }
 
-AttnShape shape_of(const sntl_attn_desc* d, bool whole_tiles = false)
+AttnShape shape_of(const sntl_attn_desc* d)
 {
     // a window that already covers the sequence is plain causal attention
     const int window = (d->window_size > 0 && d->window_size < d->seq_kv) ? d->window_size : 0;
     return AttnShape{d->batch, d->q_heads, d->kv_heads, d->seq_q, d->seq_kv, d->head_dim, d->scale, d->causal ? 1 : 0,
-                     window, window > 0 ? d->global_tokens : 0, (d->flags & SNTL_FLAG_DETERMINISTIC) ? 1 : 0, whole_tiles ? 1 : 0};
+                     window, window > 0 ? d->global_tokens : 0, (d->flags & SNTL_FLAG_DETERMINISTIC) ? 1 : 0,
+                     (d->flags & SNTL_FLAG_WHOLE_KEY_TILES) ? 1 : 0};
 }
 
 // tensor-core path is taken for bf16 tensors, or fp32 tensors when the caller allows bf16 operands
@@ -167,24 +168,18 @@ size_t sntl_attn_fwd_workspace_bytes(const sntl_attn_desc* d)
     return align_up(2 * nq_elems(d)) * (d->layout == SNTL_LAYOUT_SENTINEL ? 1 : 2) + align_up(2 * nkv_elems(d)) * 2;
 }
 
-size_t sntl_attn_bwd_workspace_bytes(const sntl_attn_desc* d) { return bwd_workspace_bytes(d, false); }
-
-}  // extern "C"
-
-size_t sntl::bwd_workspace_bytes(const sntl_attn_desc* d, bool whole_tiles)
+size_t sntl_attn_bwd_workspace_bytes(const sntl_attn_desc* d)
 {
     if (validate(d) != SNTL_OK) return 0;
-    size_t bytes = align_up(4 * nlse(d));  // delta (exact path) -- the tensor-core path sizes its own below
+    size_t bytes = align_up(4 * nlse(d));  // exact path: room for delta, which its kernel no longer needs; what callers bring is unchanged
     if (!wants_tc(d, true)) return bytes;
-    bytes = align_up(tc_backward_workspace_bytes(shape_of(d, whole_tiles)));
+    bytes = align_up(tc_backward_workspace_bytes(shape_of(d)));
     if (d->layout == SNTL_LAYOUT_SENTINEL)   // bf16 Q, dO, K, V
         bytes += align_up(2 * nq_elems(d)) * 2 + align_up(2 * nkv_elems(d)) * 2;
     else if (needs_staging(d))               // bf16 Q, O, dO, dQ, K, V, dK, dV
         bytes += align_up(2 * nq_elems(d)) * 4 + align_up(2 * nkv_elems(d)) * 4;
     return bytes;
 }
-
-extern "C" {
 
 int sntl_attn_fwd(const sntl_attn_desc* d, const void* q, const void* k, const void* v, void* o, float* lse,
                   void* workspace, size_t workspace_bytes, void* stream)
@@ -328,20 +323,12 @@ int sntl_attn_bwd(const sntl_attn_desc* d, const void* q, const void* k, const v
                   const float* lse, const void* dout, void* dq, void* dk, void* dv, void* workspace,
                   size_t workspace_bytes, void* stream)
 {
-    return bwd_run(d, q, k, v, o, lse, dout, dq, dk, dv, workspace, workspace_bytes, stream, false);
-}
-
-}  // extern "C"
-
-int sntl::bwd_run(const sntl_attn_desc* d, const void* q, const void* k, const void* v, const void* o, const float* lse, const void* dout,
-                  void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, void* stream, bool whole_tiles)
-{
     int rc = validate(d);
     if (rc != SNTL_OK) return rc;
     if (!q || !k || !v || !o || !lse || !dout || !dq || !dk || !dv) return SNTL_ERR_BAD_ARGUMENT;
     if (!device_ok()) return SNTL_ERR_NO_DEVICE;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t need = bwd_workspace_bytes(d, whole_tiles);
+    const size_t need = sntl_attn_bwd_workspace_bytes(d);
     if (!workspace || workspace_bytes < need) return SNTL_ERR_WORKSPACE;
     Carve c{(char*)workspace, workspace_bytes};
 
@@ -361,7 +348,7 @@ int sntl::bwd_run(const sntl_attn_desc* d, const void* q, const void* k, const v
     }
 
     TcArgs t{};
-    t.s = shape_of(d, whole_tiles);
+    t.s = shape_of(d);
     char* tcws = (char*)c.take(tc_backward_workspace_bytes(t.s));
     if (!c.ok) return SNTL_ERR_WORKSPACE;
     const size_t sq_pad = ((size_t)d->seq_q + 127) / 128 * 128;
@@ -444,8 +431,6 @@ void pieces_args(const sntl_attn_desc* d, void* workspace, TcArgs& t)
 }
 }  // namespace
 }  // namespace sntl
-
-extern "C" {
 
 size_t sntl_attn_bwd_pieces_workspace_bytes(const sntl_attn_desc* d)
 {

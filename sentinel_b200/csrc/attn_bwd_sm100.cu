@@ -131,9 +131,12 @@ BwdCut bwd_cut_uncached(const AttnShape& s)
     BwdCut cut;
     if (s.whole_tiles) return cut;
     if (s.deterministic) {
-        // dK and dV must not depend on how a caller cuts the batch (their partials are summed in another order than whole tiles):
-        // the rule looks at the tile alone.  At most four pieces of 24 steps or so cost a large grid little.
-        if (longest < 24) return cut;
+        // Steps take longer here (twice the bytes of dQ) and a piece costs about four of them, so only a grid that is clearly out of
+        // balance is cut (by the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
+        // D128, 100-key window, 4 global tokens), 0.45 194 -> 144 (B3 Hq16 Hkv4 S1237 D128), 0.53 206 -> 165 (B6 Hq14 Hkv2 S1500 D64), 0.57
+        // 271 -> 261; but 0.65 134 -> 134, 0.85 101 -> 114, 0.97 421 -> 482 (B8 Hq28 Hkv4 S1024 D128), 1.84 644 -> 714.  How a tile is cut
+        // depends on the tile alone: a part of a batch that is cut gives the same bits as the whole.  Two to five pieces.
+        if (longest < 24 || total * slabs / sms > 0.6 * longest) return cut;
         cut.steps = (longest + 1) / std::max(2, std::min(4, longest / 32));
         cut.pieces = bwd_piece_count(longest, cut.steps);
         while (cut.tiles < n_kt && steps(cut.tiles) * 4 > cut.steps * 5) ++cut.tiles;

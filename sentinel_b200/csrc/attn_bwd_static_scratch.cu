@@ -65,19 +65,19 @@ int sntl_attn_bwd_static_scratch(const sntl_attn_desc* desc, const void* q, cons
 {
     if (!desc) return SNTL_ERR_BAD_ARGUMENT;
     // key tiles stay whole where the partials of cut ones would not fit
-    bool whole = false;
-    size_t need = sntl_attn_bwd_workspace_bytes(desc);
+    sntl_attn_desc d = *desc;
+    size_t need = sntl_attn_bwd_workspace_bytes(&d);
     if (need > kStaticScratchBytes) {
-        whole = true;
-        need = sntl::bwd_workspace_bytes(desc, true);
+        d.flags |= SNTL_FLAG_WHOLE_KEY_TILES;
+        need = sntl_attn_bwd_workspace_bytes(&d);
     }
     if (need == 0)  // the descriptor does not validate: let the normal entry point name the reason (it launches nothing)
-        return sntl_attn_bwd(desc, q, k, v, o, lse, dout, dq, dk, dv, nullptr, 0, stream);
+        return sntl_attn_bwd(&d, q, k, v, o, lse, dout, dq, dk, dv, nullptr, 0, stream);
     if (need > kStaticScratchBytes) return SNTL_ERR_SCRATCH_LIMIT;
     void* scratch = nullptr;
     const int rc = static_scratch_pointer(&scratch);
     if (rc != SNTL_OK) return rc;
-    return sntl::bwd_run(desc, q, k, v, o, lse, dout, dq, dk, dv, scratch, kStaticScratchBytes, stream, whole);
+    return sntl_attn_bwd(&d, q, k, v, o, lse, dout, dq, dk, dv, scratch, kStaticScratchBytes, stream);
 }
 
 }  // extern "C"

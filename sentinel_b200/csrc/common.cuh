@@ -12,11 +12,6 @@
 
 namespace sntl {
 
-// sntl_attn_bwd_workspace_bytes / sntl_attn_bwd (attn_api.cu) with AttnShape::whole_tiles
-size_t bwd_workspace_bytes(const sntl_attn_desc* desc, bool whole_tiles);
-int bwd_run(const sntl_attn_desc* desc, const void* q, const void* k, const void* v, const void* o, const float* lse, const void* dout,
-            void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, void* stream, bool whole_tiles);
-
 // Launch accounting (attn_api.cu).
 void count_launch(int n = 1);
 
@@ -36,7 +31,7 @@ struct AttnShape {
     int window;         // sliding window (keys a query sees counting itself); <= 0: unlimited.  Needs causal.
     int global_tokens;  // the first global_tokens keys stay visible to every later query
     int deterministic;  // backward: dQ summed in 64-bit fixed point, so the result does not depend on the order of arrival
-    int whole_tiles;    // tensor-core backward: never cut key tiles into pieces (saves the scratch of their partials)
+    int whole_tiles;    // tensor-core backward: never cut key tiles into pieces
 };
 
 // The window part of the reference's CausalSelfAttention::allowsKey (CausalSelfAttention.cpp:95-100); the causal part

@@ -18,8 +18,11 @@ Host tensors should be pinned (``tensor.pin_memory()``); pageable memory works b
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
+from . import _lib
 from . import flash_attention as fa
 
 _cache: dict = {}
@@ -89,6 +92,15 @@ def forward_backward_host(q, k, v, dout, *, causal=True, scale=None, flags=0, de
         for t, like in ((h_o, buf["h_o"]), (h_lse, buf["h_lse"]), (h_dq, buf["h_dq"]), (h_dk, buf["h_dk"]), (h_dv, buf["h_dv"])):
             if t.shape != like.shape or t.dtype != like.dtype or t.is_cuda:
                 raise ValueError("out must be host tensors shaped (O, LSE, dQ, dK, dV)")
+    if flags & _lib.FLAG_DETERMINISTIC:
+        # the same bits as one call on everything: where that leaves its long key tiles whole, so does every chunk (where it
+        # cuts them, a chunk cuts them in the same way)
+        d = fa._bhsd_desc(q, k, causal, scale, flags, window, global_tokens)
+        whole = fa._bhsd_desc(q, k, causal, scale, flags | _lib.FLAG_WHOLE_KEY_TILES, window, global_tokens)
+        size = _lib.load().sntl_attn_bwd_workspace_bytes
+        with torch.cuda.device(dev):
+            if size(C.byref(d)) == size(C.byref(whole)):
+                flags |= _lib.FLAG_WHOLE_KEY_TILES
     caller = torch.cuda.current_stream(dev)
     up, down, down_g, lanes = buf["up"], buf["down"], buf["down_grads"], buf["compute"]
     for st in (up, down, down_g, *lanes):

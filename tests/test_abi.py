@@ -295,3 +295,30 @@ def test_native_ring_binding_refuses_tensors_it_cannot_hand_to_the_library():
     q = torch.zeros(1, 4, 128, 64, dtype=torch.bfloat16)
     with pytest.raises(ValueError, match="CUDA tensor"):      # host memory: there is no CPU path
         NativeRing._check(q, q[:, :2], q[:, :2])
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,window,cuts", [
+    (3, 16, 4, 1237, 128, 0, True),        # 120 tiles of up to 40 steps on 148 SMs
+    (2, 28, 4, 8192, 128, 1024, True),     # one tile, with the global tokens, is six times as long as the others
+    (8, 28, 4, 1024, 128, 0, False),       # balanced: an SM's load is about the longest tile
+    (2, 28, 4, 8192, 128, 0, False),
+    (8, 16, 4, 2048, 64, 0, False),
+    (1, 4, 4, 1024, 64, 0, False),         # short tiles
+])
+def test_reproducible_backward_cuts_key_tiles_of_unbalanced_grids_only(lib, B, Hq, Hkv, S, D, window, cuts):
+    """Cut tiles show in the scratch, by their partials; SNTL_FLAG_WHOLE_KEY_TILES keeps every tile whole."""
+    size = lambda flags: lib.sntl_attn_bwd_workspace_bytes(C.byref(_lib.Desc(_lib.DTYPE_BF16, _lib.LAYOUT_BHSD, B, Hq, Hkv, S, S, D, 0.1, 1, 0, 0, flags,
+                                                                           window, 64 if window else 0)))
+    rows = B * Hq * (-(-S // 128) * 128)
+    whole = size(_lib.FLAG_DETERMINISTIC | _lib.FLAG_WHOLE_KEY_TILES)
+    assert whole == -(-32 * rows // 256) * 256 + 8 * rows * D                       # row terms and the 64-bit dQ accumulator
+    assert (size(_lib.FLAG_DETERMINISTIC) > whole) == cuts
+    assert size(_lib.FLAG_WHOLE_KEY_TILES) == -(-32 * rows // 256) * 256 + 4 * rows * D
+
+
+def test_reproducible_cut_depends_on_the_tile_alone(lib):
+    """Calls on fewer sequences of a call that is cut are cut in the same way: the partials per sequence have the same size."""
+    def partials(B):
+        size = lambda flags: lib.sntl_attn_bwd_workspace_bytes(C.byref(_lib.Desc(_lib.DTYPE_BF16, _lib.LAYOUT_BHSD, B, 16, 4, 1237, 1237, 128, 0.1, 1, 0, 0, flags, 0, 0)))
+        return size(_lib.FLAG_DETERMINISTIC) - size(_lib.FLAG_DETERMINISTIC | _lib.FLAG_WHOLE_KEY_TILES)
+    assert partials(1) > 0 and partials(2) == 2 * partials(1) and partials(3) == 3 * partials(1) and partials(32) == 0

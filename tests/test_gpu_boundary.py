@@ -306,3 +306,24 @@ def test_scratch_of_a_captured_call_stays_with_its_graph(sb, warm):
     for got, ref in zip(grads.values(), want):
         assert torch.equal(got, ref)
     assert all(bool((t == 3).all()) for t in others) and sb.poll_device_status() == 0
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,S,D", [(24, 14, 2, 1024, 64), (3, 16, 4, 1237, 128)])
+def test_reproducible_gradients_do_not_depend_on_the_chunks_of_the_host_call(sb, B, Hq, Hkv, S, D):
+    """The first call is balanced with whole key tiles and its chunks are not; in the second the call and its chunks cut them."""
+    from sentinel_b200 import _lib
+    from sentinel_b200.host_pipeline import forward_backward_host
+    g = torch.Generator().manual_seed(S)
+    q, do, k, v = ((torch.randn(B, H, S, D, generator=g) * 0.5).to(torch.bfloat16).pin_memory() for H in (Hq, Hq, Hkv, Hkv))
+    qd, dod, kd, vd = (t.cuda() for t in (q, do, k, v))
+    o, lse = sb.attention_forward(qd, kd, vd)
+    want = sb.attention_backward(qd, kd, vd, o, lse, dod, flags=_lib.FLAG_DETERMINISTIC)
+    for got, ref in zip(forward_backward_host(q, k, v, do, flags=_lib.FLAG_DETERMINISTIC)[2:], want):
+        assert torch.equal(got, ref.cpu())
+    # with whole key tiles a sequence's gradients are the same bits whatever else is in the call
+    flags = _lib.FLAG_DETERMINISTIC | _lib.FLAG_WHOLE_KEY_TILES
+    want = sb.attention_backward(qd, kd, vd, o, lse, dod, flags=flags)
+    alone = sb.attention_backward(*(t[1:2].contiguous() for t in (qd, kd, vd, o, lse, dod)), flags=flags)
+    for got, ref in zip(alone, want):
+        assert torch.equal(got, ref[1:2])
+    assert sb.poll_device_status() == 0

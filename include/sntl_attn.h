@@ -182,8 +182,10 @@ int sntl_attn_bwd_end(const sntl_attn_desc* desc, void* dq, void* workspace, siz
 /* The same backward for callers that cannot allocate device memory and so cannot bring a workspace (a plugin
  * running inside another component's stream capture, a host that bans cudaMalloc in its hot loop, a binding with
  * no allocator to lend).  The scratch is a fixed array inside the library image, sntl_attn_static_scratch_capacity()
- * bytes (32 MiB) on every GPU that loads the library; a problem whose sntl_attn_bwd_workspace_bytes() exceeds it
- * returns SNTL_ERR_SCRATCH_LIMIT and launches nothing.  The first call on a device resolves the array's device
+ * bytes (32 MiB) on every GPU that loads the library.  A problem whose sntl_attn_bwd_workspace_bytes() exceeds it is
+ * computed as with SNTL_FLAG_WHOLE_KEY_TILES (no partial sums of dK and dV in the scratch; their last bits can so differ from
+ * sntl_attn_bwd without that flag); one that exceeds it even then returns SNTL_ERR_SCRATCH_LIMIT and launches nothing.
+ * The first call on a device resolves the array's device
  * address and should be made before any stream capture.  All calls on a device share the array (each call rewrites
  * what it reads, so nothing needs clearing), hence calls that can overlap on one GPU race and must be ordered by
  * the caller.  Allocates nothing.  This entry point has no counterpart in the reference. */

@@ -6,16 +6,17 @@
 // control, or a binding that simply has no allocator to lend.  The normal entry point, sntl_attn_bwd, needs the
 // caller to bring a scratch buffer; this one brings its own.
 //
-// How: the scratch (delta, LSE*log2e and the fp32 dQ accumulator, or just delta on the exact-fp32 route) lives in
-// a fixed array in device global memory that is part of the library image.  Its size, kStaticScratchBytes, is the
-// limit: a problem whose sntl_attn_bwd_workspace_bytes() is larger is refused with SNTL_ERR_SCRATCH_LIMIT and
-// nothing is launched.  Every GPU on which this library is loaded carries the array until the process exits.
+// How: the scratch (the per-row terms, the dQ accumulator and the partial sums of cut key tiles) lives in a fixed array in
+// device global memory that is part of the library image.  Its size, kStaticScratchBytes, is the limit: a problem whose
+// sntl_attn_bwd_workspace_bytes() is larger keeps its key tiles whole (SNTL_FLAG_WHOLE_KEY_TILES: no partial sums), and
+// one that is larger even then is refused with SNTL_ERR_SCRATCH_LIMIT and nothing is launched.  Every GPU on which this
+// library is loaded carries the array until the process exits.
 //
 // Rules of use
 //   * The first call on each device looks up the device address of the array (cudaGetSymbolAddress, once per
 //     device, with that device current).  Make that first call eagerly, before any stream capture begins.
 //   * All calls on one device share the one array, and it still holds whatever the previous call left there.  The
-//     backward itself rewrites every word it later reads (its first pass stores delta and LSE*log2e and clears the
+//     backward itself rewrites every word it later reads (its first pass stores the per-row terms and clears the
 //     dQ accumulator), so nothing has to be cleared by the caller.
 //   * For the same reason two calls whose kernels can be in flight together on one GPU (different streams, or two
 //     host threads) race on the array and corrupt each other's gradients.  Keep such calls on one stream, or order

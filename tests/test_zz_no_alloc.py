@@ -98,3 +98,26 @@ def test_static_scratch_refuses_problems_beyond_its_capacity():
     bad = sb._lib.Desc(sb._lib.DTYPE_BF16, sb._lib.LAYOUT_BHSD, 1, 7, 2, 128, 128, 128, 0.088, 1, 0, 0, 0)
     rc = lib.sntl_attn_bwd_static_scratch(C.byref(bad), dummy, dummy, dummy, dummy, dummy, dummy, dummy, dummy, dummy, None)
     assert rc == sb._lib.ERR_BAD_ARGUMENT
+
+
+@pytest.mark.parametrize("flags", [0, 4])
+def test_static_scratch_keeps_key_tiles_whole_where_their_partials_would_not_fit(flags):
+    """A problem that exceeds the built-in scratch only by the partial sums of cut key tiles: the bits of the ordinary backward with
+    SNTL_FLAG_WHOLE_KEY_TILES."""
+    import sentinel_b200 as sb
+    lib = sb._lib.load()
+    w = sb.WORKLOADS["gqa7b_d128"]
+    q, k, v, do = (t.cuda() for t in sb.make_inputs(w, batch=1, q_heads=8, kv_heads=4, seq=3300))
+    o, lse = sb.attention_forward(q, k, v)
+    d, whole = (sb._lib.Desc(sb._lib.DTYPE_BF16, sb._lib.LAYOUT_BHSD, 1, 8, 4, 3300, 3300, 128, 128 ** -0.5, 1, 0, 0, f)
+                for f in (flags, flags | sb._lib.FLAG_WHOLE_KEY_TILES))
+    cap = lib.sntl_attn_static_scratch_capacity()
+    assert lib.sntl_attn_bwd_workspace_bytes(C.byref(d)) > cap >= lib.sntl_attn_bwd_workspace_bytes(C.byref(whole))
+    got = [torch.empty_like(t) for t in (q, k, v)]
+    rc = lib.sntl_attn_bwd_static_scratch(C.byref(d), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
+                                          do.data_ptr(), *(t.data_ptr() for t in got), torch.cuda.current_stream().cuda_stream)
+    assert rc == sb._lib.OK
+    want = sb.attention_backward(q, k, v, o, lse, do, flags=flags | sb._lib.FLAG_WHOLE_KEY_TILES)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    _close(got[0], want[0], "dQ")
+    assert sb.poll_device_status() == 0

@@ -54,7 +54,10 @@ def host():
         if not os.path.exists(HOST_MODULE_PATH):
             raise LibraryMissing(f"{HOST_MODULE_PATH} is missing: run `python -m sentinel_b200.build`.")
         spec = importlib.util.spec_from_file_location("_sntl_host", HOST_MODULE_PATH)
-        module = importlib.util.module_from_spec(spec)
+        try:
+            module = importlib.util.module_from_spec(spec)
+        except ImportError as e:      # another torch than it was built for, or one that it does not even link with
+            raise LibraryMissing(f"{HOST_MODULE_PATH} does not fit the installed torch ({e}): run `python -m sentinel_b200.build`.") from e
         spec.loader.exec_module(module)
         module.bind(*(C.cast(getattr(lib, n), C.c_void_p).value for n in
                       ("sntl_attn_fwd", "sntl_attn_bwd", "sntl_attn_cached_fwd", "sntl_attn_fwd_workspace_bytes",

@@ -19,6 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libsntl_attn.so")
 HOST_MODULE = os.path.join(LIB_DIR, "_sntl_host.so")
+HOST_STAMP = os.path.join(LIB_DIR, "_sntl_host.built_for")   # the torch and the Python that the module was built for
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = ["attn_api.cu", "attn_simt_fwd.cu", "attn_simt_bwd.cu", "attn_simt_decode.cu", "layout_convert.cu", "attn_fwd_sm100.cu", "attn_cache_sm100.cu", "attn_bwd_sm100.cu",
@@ -41,10 +42,22 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def host_module_stale() -> bool:
+    """Whether the module is older than its source, or was built for another torch or Python than those that run now."""
+    import torch
+    try:
+        with open(HOST_STAMP) as f:
+            built_for = f.read()
+    except OSError:
+        return True
+    return built_for != f"{torch.__version__} {sys.version}" or _stale(
+        HOST_MODULE, [os.path.join(CSRC, "torch_host.cpp"), os.path.join(ROOT, "include", "sntl_attn.h")])
+
+
 def build_host_module(force: bool = False) -> str:
     """The CPython module of csrc/torch_host.cpp, against the headers and libraries of the torch that is installed."""
     src = os.path.join(CSRC, "torch_host.cpp")
-    if not force and not _stale(HOST_MODULE, [src, os.path.join(ROOT, "include", "sntl_attn.h")]):
+    if not force and not host_module_stale():
         return HOST_MODULE
     import torch
     from torch.utils import cpp_extension
@@ -52,12 +65,15 @@ def build_host_module(force: bool = False) -> str:
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc()))), "include")
     includes = cpp_extension.include_paths() + [sysconfig.get_path("include"), cuda, os.path.join(ROOT, "include")]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DSNTL_TORCH_VERSION="{torch.__version__}"',
            src, "-o", HOST_MODULE] + [x for d in includes for x in ("-isystem", d)]
     cmd += ["-L" + libs, "-Wl,-rpath," + libs, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("g++ failed on torch_host.cpp")
+    with open(HOST_STAMP, "w") as f:
+        f.write(f"{torch.__version__} {sys.version}")
     return HOST_MODULE
 
 

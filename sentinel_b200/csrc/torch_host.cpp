@@ -25,6 +25,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -462,4 +463,22 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_sntl_host", nullptr, -1, methods,
 
 }  // namespace
 
-extern "C" __attribute__((visibility("default"))) PyObject* PyInit__sntl_host() { return PyModule_Create(&module); }
+// Nothing else notices when torch has been exchanged since the build: its C++ interface is not stable from version to version.
+bool torch_is_the_one_built_for()
+{
+    PyObject* torch = PyImport_ImportModule("torch");
+    PyObject* version = torch ? PyObject_GetAttrString(torch, "__version__") : nullptr;
+    PyObject* text = version ? PyObject_Str(version) : nullptr;
+    const char* running = text ? PyUnicode_AsUTF8(text) : nullptr;
+    const bool same = running && std::strcmp(running, SNTL_TORCH_VERSION) == 0;
+    if (running && !same) PyErr_Format(PyExc_ImportError, "built for torch %s, running with %s", SNTL_TORCH_VERSION, running);
+    Py_XDECREF(text);
+    Py_XDECREF(version);
+    Py_XDECREF(torch);
+    return same;
+}
+
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit__sntl_host()
+{
+    return torch_is_the_one_built_for() ? PyModule_Create(&module) : nullptr;
+}

@@ -322,3 +322,21 @@ def test_reproducible_cut_depends_on_the_tile_alone(lib):
         size = lambda flags: lib.sntl_attn_bwd_workspace_bytes(C.byref(_lib.Desc(_lib.DTYPE_BF16, _lib.LAYOUT_BHSD, B, 16, 4, 1237, 1237, 128, 0.1, 1, 0, 0, flags, 0, 0)))
         return size(_lib.FLAG_DETERMINISTIC) - size(_lib.FLAG_DETERMINISTIC | _lib.FLAG_WHOLE_KEY_TILES)
     assert partials(1) > 0 and partials(2) == 2 * partials(1) and partials(3) == 3 * partials(1) and partials(32) == 0
+
+
+def test_host_module_is_rebuilt_and_refused_for_another_torch(lib, monkeypatch):
+    """The native module is bound to the C++ interface of the torch it was built for: with another one the build sees it as stale,
+    and loading it says so instead of running on a changed interface."""
+    import subprocess
+    import sys
+    import torch
+    from sentinel_b200 import build
+    _lib.host()
+    assert not build.host_module_stale()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.host_module_stale()
+    code = ("import torch; torch.__version__ = '0.0.1'\n"
+            "from sentinel_b200 import _lib\n"
+            "try:\n    _lib.host()\nexcept _lib.LibraryMissing as e:\n    print(e)\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=300)
+    assert "running with 0.0.1" in r.stdout and "sentinel_b200.build" in r.stdout, (r.stdout, r.stderr)

@@ -194,7 +194,7 @@ def test_pieces_ring_and_selftest_entry_points_validate_without_a_gpu(lib):
     assert lib.sntl_attn_bwd_block(C.byref(d), dummy, dummy, dummy, dummy, None, dummy, dummy, need, None) == _lib.ERR_BAD_ARGUMENT
     assert lib.sntl_attn_bwd_end(C.byref(d), None, dummy, need, None) == _lib.ERR_BAD_ARGUMENT
     # deterministic flag: the backward scratch doubles its dQ accumulator
-    # (kv_heads == q_heads: no key tiles cut by query head, whose partials the default form would add to its scratch)
+    # (short key tiles, which neither form cuts: the partials of cut ones would add to the scratch)
     plain = lib.sntl_attn_bwd_workspace_bytes(C.byref(_desc(kv_heads=8)))
     det = lib.sntl_attn_bwd_workspace_bytes(C.byref(_desc(kv_heads=8, flags=_lib.FLAG_DETERMINISTIC)))
     assert det - plain == 4 * 2 * 8 * 256 * 128

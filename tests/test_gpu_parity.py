@@ -242,7 +242,7 @@ def test_bf16_tensor_core_noncausal_rectangular(sb, oracle):
 
 @pytest.mark.parametrize("B,Hq,Hkv,S,D,col0,tail,window", [
     (1, 2, 2, 1, 64, 0, 0, 0),         # one token
-    (2, 4, 2, 129, 64, 3, 5, 0),       # unaligned window: 4-byte accesses; key tiles cut by query head
+    (2, 4, 2, 129, 64, 3, 5, 0),       # unaligned window: 4-byte accesses
     (3, 6, 1, 384, 128, 32, 0, 0),     # head_dim 128: fp32 row-term columns, two feature tiles per head
     (5, 3, 3, 300, 64, 0, 4, 70),      # sliding window, 16-byte accesses, ragged tiles
 ])
@@ -320,8 +320,8 @@ def test_staged_fp32_sentinel_layout_on_tensor_cores(sb, oracle):
 
 def test_forward_is_deterministic_and_recompute_stable(sb):
     """Activation checkpointing re-runs the forward inside backward (CudaTransformerBlock.cu:277-284): two runs
-    must agree bit for bit, and so must two backward runs of dK/dV (each key tile is owned by one CTA, or by one CTA
-    per query head whose partials are added in a fixed order)."""
+    must agree bit for bit, and so must two backward runs of dK/dV (each key tile is owned by one CTA, or cut into pieces
+    whose partials are added in a fixed order)."""
     w = sb.WORKLOADS["gqa7b_d128"]
     q, k, v, do = (t.cuda() for t in _bf16_case(w, batch=1, q_heads=4, kv_heads=1, seq=512))
     o1, l1 = sb.attention_forward(q, k, v)
@@ -335,16 +335,16 @@ def test_forward_is_deterministic_and_recompute_stable(sb):
     dq1, dk3, dv3 = sb.attention_backward(q, k, v, o1, l1, do, flags=_lib.FLAG_DETERMINISTIC)
     dq2, dk4, dv4 = sb.attention_backward(q, k, v, o1, l1, do, flags=_lib.FLAG_DETERMINISTIC)
     assert torch.equal(dq1, dq2) and torch.equal(dk3, dk4) and torch.equal(dv3, dv4)
-    # (on this small grid the default path cuts its long key tiles by query head and the flagged one does not, so their
-    # dK/dV are two different fixed summation orders of the same terms: close, not identical)
+    # (on this small grid the default path cuts its long key tiles and the flagged one does not, so their dK/dV are two
+    # different fixed summation orders of the same terms: close, not identical)
     assert float((dk3.float() - dk1.float()).abs().max()) <= 2e-2 * float(dk1.float().abs().max())
 
 
 def test_backward_long_key_tiles_cut_by_query_head(sb, oracle):
-    """On a small grid the backward cuts the key tiles whose CTA would outlast an SM's average load into one CTA per
-    query head of the group and adds their fp32 dK/dV partials in head order.  B4 / Hq28 / Hkv4 / S768 mixes cut tiles
-    (the first four) with uncut ones (the last two): dK/dV of both kinds against fp64-oracle columns and against the
-    exact kernels on a whole slice, dQ rows against the oracle, and two runs bit-identical."""
+    """On a small grid the backward cuts key tiles whose CTA would outlast an SM's average load into pieces, one CTA each, and
+    adds their fp32 dK/dV partials in piece order.  B4 / Hq28 / Hkv4 / S768 mixes cut tiles (the first three, two pieces each)
+    with uncut ones: dK/dV of both kinds against fp64-oracle columns and against the exact kernels on a whole slice, dQ rows
+    against the oracle, and two runs bit-identical."""
     w = sb.WORKLOADS["gqa7b_d128"]
     q, k, v, do = _bf16_case(w, batch=4, q_heads=28, kv_heads=4, seq=768)
     qd, kd, vd, dod = (t.cuda() for t in (q, k, v, do))
@@ -354,7 +354,7 @@ def test_backward_long_key_tiles_cut_by_query_head(sb, oracle):
     dq2, dk2, dv2 = sb.attention_backward(qd, kd, vd, o, lse, dod)
     assert torch.equal(dk, dk2) and torch.equal(dv, dv2)
     qf, kf, vf, dof = (t.to(torch.float32).numpy() for t in (q, k, v, do))
-    cols = np.array([0, 100, 383, 511, 512, 767])       # key tiles 0, 0, 2, 3 (cut) and 4, 5 (uncut)
+    cols = np.array([0, 100, 383, 511, 512, 767])       # key tiles 0, 0, 2 (cut) and 3, 4, 5 (uncut)
     for (b, hk) in ((0, 0), (3, 3)):
         wdk, wdv = oracle.attn_cols(qf, kf, vf, dof, b, hk, cols)
         _check_bf16(_np(dk[b, hk, cols]), wdk, "dk cols")
@@ -407,6 +407,16 @@ def test_forward_blocks_taken_over_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, k
     test_forward_query_tiles_per_cta_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, kw)
 
 
+def _cuts_key_tiles(B, Hq, Hkv, S, D, kw):
+    """Whether the backward cuts key tiles into pieces: their partial sums show in the scratch."""
+    import ctypes as C
+    from sentinel_b200 import _lib
+    size = [_lib.load().sntl_attn_bwd_workspace_bytes(C.byref(_lib.Desc(
+        _lib.DTYPE_BF16, _lib.LAYOUT_BHSD, B, Hq, Hkv, S, S, D, 0.1, 1, 0, 0, kw.get("flags", 0) | f, kw.get("window", 0), kw.get("global_tokens", 0))))
+        for f in (0, _lib.FLAG_WHOLE_KEY_TILES)]
+    return size[0] > size[1]
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,S,D,kw", [
     (1, 2, 2, 1100, 128, {}),                                    # one head per group: tiles cut along the queries, ragged
     (1, 6, 2, 700, 64, dict(window=200, global_tokens=5)),       # pieces that end inside a head's query range
@@ -417,6 +427,7 @@ def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
     """Key tiles cut into pieces against the exact kernels on the same bf16 values.  P, dS and the operands are bf16 (2^-9 each,
     independent): dQ, dK within 8e-3 relative L2, dV within 4e-3; dK, dV bit-identical from run to run."""
     w = sb.WORKLOADS["gqa7b_d128"]
+    assert _cuts_key_tiles(B, Hq, Hkv, S, D, kw)
     g = torch.Generator(device="cuda").manual_seed(S)
     q, k, v, do = ((torch.randn(B, H, S, D, generator=g, device="cuda") * std).to(torch.bfloat16)
                    for H, std in ((Hq, 0.5), (Hkv, 0.5), (Hkv, 1.0), (Hq, w.do_std)))
@@ -436,13 +447,19 @@ def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
     (40, 8, 8, 100, 100, 64, {}),                                 # 320 blocks of one step each
     (30, 6, 6, 129, 129, 128, {}),                                # one- and two-step blocks, the last with one query
     (9, 12, 6, 700, 700, 64, dict(window=150, global_tokens=3)),
-    (3, 36, 12, 640, 640, 128, dict(flags=4)),                    # cut tiles among whole ones
+    (3, 36, 12, 640, 640, 128, dict(flags=4)),                    # reproducible dQ, whole tiles
     (20, 8, 8, 150, 260, 64, dict(causal=False)),
+    (3, 16, 4, 1237, 1237, 128, dict(flags=4)),                   # from here on: pieces of cut tiles among whole ones
+    (4, 28, 4, 1400, 1400, 128, {}),
+    (5, 16, 4, 1100, 1100, 128, dict(window=100, global_tokens=5)),
+    (4, 28, 4, 1400, 1400, 64, dict(window=200, global_tokens=130, flags=4)),
 ])
 def test_backward_blocks_taken_over_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, kw):
     """More blocks than SMs, so that every CTA computes several in turn, of equal and of different lengths, against the exact
     kernels on the same bf16 values (bounds as for the cut pieces above); dK, dV do not depend on which CTA took which block."""
     w = sb.WORKLOADS["gqa7b_d128"]
+    if Sq >= 1100:
+        assert _cuts_key_tiles(B, Hq, Hkv, Sq, D, kw)
     g = torch.Generator(device="cuda").manual_seed(Sq + B)
     q, k, v, do = ((torch.randn(B, H, S, D, generator=g, device="cuda") * std).to(torch.bfloat16)
                    for H, S, std in ((Hq, Sq, 0.5), (Hkv, Sk, 0.5), (Hkv, Sk, 1.0), (Hq, Sq, w.do_std)))
@@ -461,7 +478,7 @@ def test_backward_blocks_taken_over_vs_exact_kernels(sb, B, Hq, Hkv, Sq, Sk, D, 
 def test_backward_head_dim_64_buffers_and_cut_tiles_vs_oracle(sb, oracle):
     """head_dim 64 takes a path of its own inside the backward kernel (LSE and delta folded into the S^T / dP^T products,
     two S^T buffers, three Q stages, two dS tiles).  B1 / Hq8 / Hkv2 / S1400 is a grid small enough that every key tile is
-    cut by query head, with more steps per CTA than there are buffers of any kind and a ragged last tile: whole tensors
+    cut into pieces, with more steps per CTA than there are buffers of any kind and a ragged last tile: whole tensors
     against the fp64 oracle, two runs bit-identical in dK/dV; then a single-tile case (fewer steps than buffers)."""
     w = sb.WORKLOADS["llama1b_gqa"]
     q, k, v, do = _bf16_case(w, batch=1, q_heads=8, kv_heads=2, seq=1400)

@@ -5,8 +5,8 @@
 // pushes dK/dV out with global atomics after scalar FMA loops; here all five products run on tcgen05 tensor
 // cores and the loop is key-tile-outer:
 //
-//   * one CTA owns one 128-key tile of one (batch, KV head) and walks every 128-query tile that can see it,
-//     for every query head of the group, so dK and dV accumulate in TMEM for the whole CTA lifetime and are
+//   * one block is one 128-key tile of one (batch, KV head), or a piece of one (BwdCut): it walks the 128-query tiles that can
+//     see it, for every query head of the group, so dK and dV accumulate in TMEM for the whole block and are
 //     written exactly once: deterministic, no atomics, grouped-query sums done in place (the reference
 //     materialises repeated K/V and reduces afterwards, CudaCausalSelfAttention.cu:27-44);
 //   * everything is computed transposed (rows = keys) so that both P^T and dS^T are consumed by the next MMA
@@ -30,9 +30,8 @@
 //     (setmaxnreg).  Q (with its LSE records) has two stages and dO (with its delta records) one at D=128
 //     (shared-memory capacity); three and two at D=64.
 //
-// A pre-pass computes the per-query records (delta = rowsum(dO o O) and LSE/scale, each split in two bf16; padded rows get a
-// huge LSE so they produce P = 0) and zeroes the dQ accumulator; a post-pass converts the accumulator to bf16 dQ (times
-// scale).
+// A pre-pass computes the per-query terms (row_terms.cuh: from delta = rowsum(dO o O) and LSE; padded rows get a term that makes
+// P = 0) and zeroes the dQ accumulator; a post-pass converts the accumulator to bf16 dQ (times scale).
 //
 // Long key tiles are cut into pieces (BwdCut): one CTA per (key tile, KV head, piece), each leaving its dK/dV as an fp32
 // partial in scratch, and a small kernel adds the partials in piece order (deterministic) and writes the result.
@@ -103,7 +102,7 @@ __host__ __device__ inline int bwd_piece_count(int steps, int split_steps) { ret
 // Which key tiles to cut, and how fine.  The CTA of key tile 0 visits every query tile of every head of its group; on a small
 // grid (few sequences x KV heads, one layer's strong-scaling share, short batches) or where a window leaves only the tiles with
 // global tokens long, that one CTA outlasts the average SM's whole load.  Cutting balances the grid and costs each piece its
-// set-up and an fp32 partial of dK and dV: about two steps for a CTA, four for a piece.  The estimate below weighs the
+// set-up and an fp32 partial of dK and dV: about one and a half steps for a CTA, four for a piece.  The estimate below weighs the
 // two for a few piece lengths (a CTA's cost counts once per block, although blocks that follow one another in a CTA hide part of
 // it).  B3 Hq16 Hkv4 S1237 D128 with reproducible dQ: 120 CTAs of up to 40 steps on 148 SMs took
 // 158 us, 108 us cut.
@@ -447,7 +446,7 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
     }
 }
 
-// kSplit: the grid may hold key tiles cut by query head (a separate instantiation, so that the plain kernel carries none
+// kSplit: the grid may hold pieces of cut key tiles (a separate instantiation, so that the plain kernel carries none
 // of that bookkeeping)
 // kDet: dQ contributions leave as 64-bit fixed point (see the drain warpgroup)
 // kMat: dK and dV leave as feature-major fp32 matrices (an instantiation of its own: with that store in the common kernel it is

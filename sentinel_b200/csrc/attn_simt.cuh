@@ -151,18 +151,8 @@ __device__ __forceinline__ float delta_of(const float* part, int r)
     return s;
 }
 
-// Two fp32 FMAs in one instruction, each rounded as the scalar one.  The products below use nothing else: three-operand
-// scalar FMAs stall in dispatch on their register reads (forward B8 H12 S512 D64: 129 us with them, the FMA pipes 45 % busy).
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
-{
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-
+// The products below use nothing but packed FMAs (ffma2): three-operand scalar ones stall in dispatch on their register reads (forward
+// B8 H12 S512 D64: 129 us with them, the FMA pipes 45 % busy).
 // (the two halves of an accumulator take the even and the odd features)
 template <int TM, int TN, int DP>
 __device__ __forceinline__ void scores(float (&out)[TM][TN], const float* A, const float* B)

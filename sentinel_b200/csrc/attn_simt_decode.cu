@@ -28,15 +28,6 @@ template <int DP, int R> struct DecodeSmem {
     static_assert(kWarps * R * DP <= kChunk * P, "the warps' partial outputs reuse the K buffer");
 };
 
-__device__ __forceinline__ void copy16(float* dst, const float* src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-template <int N> __device__ __forceinline__ void copies_left()
-{
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // rows [k0, k0 + n) of K or V
 template <int DP>
 __device__ __forceinline__ void stage_async(float* dst, const float* base, long long ss, int k0, int n)
@@ -47,7 +38,7 @@ __device__ __forceinline__ void stage_async(float* dst, const float* base, long 
         const int r = u / kUnits, d = (u % kUnits) * 4;
         if (r < n) copy16(dst + r * (DP + 4) + d, base + (k0 + r) * ss + d);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    copies_commit();
 }
 
 template <int DP, int R>

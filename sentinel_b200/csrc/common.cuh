@@ -93,6 +93,25 @@ inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, si
 // What a kernel accesses `bytes` at a time has to start on such a boundary; a misaligned access would take the context down.
 template <typename... P> inline bool aligned(uintptr_t bytes, const P*... p) { return (((uintptr_t)p | ... | (uintptr_t)0) % bytes) == 0; }
 
+// Asynchronous copies of 16 bytes, global -> shared (both on 16-byte boundaries), in groups per thread
+__device__ __forceinline__ void copy16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_left() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Two fp32 FMAs in one instruction, each rounded as the scalar one
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+          "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
+}
+
 // SMs of the current device (148 on a B200), read once per device ordinal
 inline int sm_count()
 {
@@ -174,10 +193,6 @@ cudaError_t rope_pack_bf16(const float* src, __nv_bfloat16* dst, int B, int H, i
 cudaError_t rope_unpack_f32(const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
                             int column_start, const float* cos_t, const float* sin_t, int position_offset, bool inverse,
                             cudaStream_t st);
-cudaError_t sentinel_to_bhsd_bf16(const float* src, __nv_bfloat16* dst, int B, int H, int S, int D, int stride_columns,
-                                  int column_start, cudaStream_t st);
-cudaError_t bhsd_bf16_to_sentinel(const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
-                                  int column_start, cudaStream_t st);
 // Everything a tensor-core call needs from feature-major fp32 matrices, in one launch: up to four of them converted to bf16
 // [B][H][S][D], and for the backward (o_mat non-null) the per-query terms from O, dO and LSE, and the dQ accumulator zeroed.
 struct MatrixStage {

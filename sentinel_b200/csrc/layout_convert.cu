@@ -290,13 +290,6 @@ __global__ void __launch_bounds__(256, 4) unpack64_kernel(const __nv_bfloat16* _
 // buffers) while this one is converted.  Bound by HBM: 6 bytes per element; B2 H28 S8192 D128 (352 MB): rotated 95 us with the
 // tile loaded, converted and stored in turn, 62 us here (0.87 of the copy rate), plain 63 and 60.  The tile lies in shared memory as it came; its 16-byte units are XOR-permuted
 // by row so that the reads across the grain (eight tokens x four units, or eight quads of tokens x four pairs) hit all banks.
-__device__ __forceinline__ void copy16(void* dst, const void* src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copies_left() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 template <int kRot, int DT>
 __global__ void __launch_bounds__(256, 3) pack64_pipe_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int H, int S, int D,
                                                           int stride_columns, int column_start, const float* __restrict__ cos_t,
@@ -438,28 +431,29 @@ cudaError_t launch_convert64(Kernel kernel, size_t smem, std::atomic<unsigned lo
         return launch_convert64(KERNEL<ROT, 64>, SMEM, configured, src, dst, B, H, S, D, stride_columns, column_start, cos_t, sin_t,      \
                                 position_offset, HEADS, st);                                                                              \
     } while (0)
-#define SNTL_CONVERT_ROT(KERNEL, SMEM, HEADS)                   \
-    do {                                                        \
-        if (rot == 0) SNTL_CONVERT(KERNEL, 0, SMEM, HEADS);            \
-        else if (rot == 1) SNTL_CONVERT(KERNEL, 1, SMEM, HEADS);       \
-        else SNTL_CONVERT(KERNEL, 2, SMEM, HEADS);                     \
-    } while (0)
 
 constexpr size_t kTileBytes = (size_t)kTok * 65 * sizeof(float);
 
-cudaError_t launch_pack64(int rot, bool vec, const float* src, __nv_bfloat16* dst, int B, int H, int S, int D, int stride_columns,
+cudaError_t launch_pack64(bool rot, bool vec, const float* src, __nv_bfloat16* dst, int B, int H, int S, int D, int stride_columns,
                           int column_start, const float* cos_t, const float* sin_t, int position_offset, cudaStream_t st)
 {
-    if (vec) SNTL_CONVERT_ROT(pack64_pipe_kernel, 2 * kTok * 64 * sizeof(float), kHeadsPerCta);
-    SNTL_CONVERT_ROT(pack64_kernel, kTileBytes, kHeadsPerCtaScalar);
+    constexpr size_t pipe = 2 * kTok * 64 * sizeof(float);
+    if (vec && rot) SNTL_CONVERT(pack64_pipe_kernel, 1, pipe, kHeadsPerCta);
+    if (vec) SNTL_CONVERT(pack64_pipe_kernel, 0, pipe, kHeadsPerCta);
+    if (rot) SNTL_CONVERT(pack64_kernel, 1, kTileBytes, kHeadsPerCtaScalar);
+    SNTL_CONVERT(pack64_kernel, 0, kTileBytes, kHeadsPerCtaScalar);
 }
 cudaError_t launch_unpack64(int rot, bool vec, const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
                             int column_start, const float* cos_t, const float* sin_t, int position_offset, cudaStream_t st)
 {
-    if (vec) SNTL_CONVERT_ROT(unpack64_pipe_kernel, 2 * kTok * 64 * sizeof(__nv_bfloat16), kHeadsPerCta);
-    SNTL_CONVERT_ROT(unpack64_kernel, kTileBytes, kHeadsPerCtaScalar);
+    constexpr size_t pipe = 2 * kTok * 64 * sizeof(__nv_bfloat16);
+    if (vec && rot == 2) SNTL_CONVERT(unpack64_pipe_kernel, 2, pipe, kHeadsPerCta);
+    if (vec && rot == 1) SNTL_CONVERT(unpack64_pipe_kernel, 1, pipe, kHeadsPerCta);
+    if (vec) SNTL_CONVERT(unpack64_pipe_kernel, 0, pipe, kHeadsPerCta);
+    if (rot == 2) SNTL_CONVERT(unpack64_kernel, 2, kTileBytes, kHeadsPerCtaScalar);
+    if (rot == 1) SNTL_CONVERT(unpack64_kernel, 1, kTileBytes, kHeadsPerCtaScalar);
+    SNTL_CONVERT(unpack64_kernel, 0, kTileBytes, kHeadsPerCtaScalar);
 }
-#undef SNTL_CONVERT_ROT
 #undef SNTL_CONVERT
 
 // ---- everything a tensor-core call needs from feature-major matrices (see MatrixStage) ----
@@ -619,21 +613,18 @@ inline int blocks_for(size_t n, int threads)
 
 }  // namespace
 
-cudaError_t sentinel_to_bhsd_bf16(const float* src, __nv_bfloat16* dst, int B, int H, int S, int D, int stride_columns,
+static cudaError_t sentinel_to_bhsd_bf16(const float* src, __nv_bfloat16* dst, int B, int H, int S, int D, int stride_columns,
                                   int column_start, cudaStream_t st)
 {
-    if (D % 64 == 0 && (long long)B * H <= 65535) return rope_pack_bf16(src, dst, B, H, S, D, stride_columns, column_start, nullptr, nullptr, 0, st);
     dim3 grid((S + 31) / 32, (D + 31) / 32, B * H), block(32, 8);
     sentinel_to_bhsd_kernel<<<grid, block, 0, st>>>(src, dst, H, S, D, stride_columns, column_start);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t bhsd_bf16_to_sentinel(const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
+static cudaError_t bhsd_bf16_to_sentinel(const __nv_bfloat16* src, float* dst, int B, int H, int S, int D, int stride_columns,
                                   int column_start, cudaStream_t st)
 {
-    if (D % 64 == 0 && (long long)B * H <= 65535)
-        return rope_unpack_f32(src, dst, B, H, S, D, stride_columns, column_start, nullptr, nullptr, 0, false, st);
     dim3 grid((S + 31) / 32, (D + 31) / 32, B * H), block(32, 8);
     bhsd_to_sentinel_kernel<<<grid, block, 0, st>>>(src, dst, H, S, D, stride_columns, column_start);
     count_launch();
@@ -653,7 +644,7 @@ cudaError_t rope_pack_bf16(const float* src, __nv_bfloat16* dst, int B, int H, i
     if (D % 64 == 0) {
         // the bf16 side and the angle tables are accessed 16 bytes at a time (as are all bf16 tensors of the tensor-core kernels)
         if (((uintptr_t)dst & 15u) != 0 || (cos_t && !tables_aligned(cos_t, sin_t))) return cudaErrorMisalignedAddress;
-        return launch_pack64(cos_t ? 1 : 0, f32_rows_aligned(src, S, stride_columns, column_start), src, dst, B, H, S, D, stride_columns,
+        return launch_pack64(cos_t != nullptr, f32_rows_aligned(src, S, stride_columns, column_start), src, dst, B, H, S, D, stride_columns,
                              column_start, cos_t, sin_t, position_offset, st);
     }
     if (!cos_t) return sentinel_to_bhsd_bf16(src, dst, B, H, S, D, stride_columns, column_start, st);

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace sntl {
 namespace ptx {
 
@@ -192,15 +194,7 @@ template <int N> __device__ __forceinline__ void setmaxnreg_inc() { asm volatile
 template <int N> __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // packed fp32x2 arithmetic (two independent fp32 lanes in one 64-bit register)
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
-{
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
+using ::sntl::ffma2;
 __device__ __forceinline__ float2 fmul2(float2 a, float2 b)
 {
     float2 d;

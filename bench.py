@@ -32,9 +32,8 @@ FALLBACK_PEAKS = {"bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0, "hbm_g
 # DRAM bytes (read + write) of one launch of the dominant kernel per batch element, from an ncu capture on the full workload (batch 2)
 # that predates the kernel taking over blocks; traffic grows in proportion to the batch
 NCU_DRAM_BYTES_PER_BATCH = {"gqa7b_d128": (1823.955e6 + 987.866e6) / 2}
-# the same for a KV-cache forward, one new token, no window, batch 16: K and V once and a few per cent, of the kernel before the
-# present persistent one, which reads the same bytes
-NCU_CACHED_DRAM_BYTES_PER_BATCH = {"gqa7b_d128": (268640768 + 5306880) / 16.0}
+# the same for the KV-cache kernel, one new token, no window (captured at batch 16)
+NCU_CACHED_DRAM_BYTES_PER_BATCH = {"gqa7b_d128": (268734208 + 3560960) / 16.0}
 
 
 class stdout_to_stderr:

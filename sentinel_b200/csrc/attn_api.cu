@@ -92,6 +92,33 @@ void set_vector_access(SimtArgs& a)
     a.vec_kv = rows_of_four(a.vkv, a.s.D, a.is_bf16, {a.k, a.v, a.dk, a.dv});
 }
 
+size_t nq_elems(const sntl_attn_desc* d) { return (size_t)d->batch * d->q_heads * d->seq_q * d->head_dim; }
+size_t nkv_elems(const sntl_attn_desc* d) { return (size_t)d->batch * d->kv_heads * d->seq_kv * d->head_dim; }
+size_t nlse(const sntl_attn_desc* d) { return (size_t)d->batch * d->q_heads * d->seq_q; }
+
+// The exact kernels: split products on the tensor cores where those take the call, with the FMA kernels behind them for the blocks
+// that they leave; the FMA kernels alone otherwise.
+cudaError_t exact_forward(SimtArgs& a, const sntl_attn_desc* d, cudaStream_t st)
+{
+    g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
+    if (!(d->flags & SNTL_FLAG_FORCE_SIMT) && f32_tc_forward_supported(a)) {
+        const cudaError_t e = f32_tc_forward(a, st);
+        if (e != cudaSuccess) return e;
+        a.only_odd = true;
+    }
+    return simt_forward(a, st);
+}
+cudaError_t exact_backward(SimtArgs& a, const sntl_attn_desc* d, void* workspace, cudaStream_t st)
+{
+    g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
+    if (!(d->flags & SNTL_FLAG_FORCE_SIMT) && aligned(4, workspace) && f32_tc_backward_supported(a, 4 * nlse(d))) {
+        a.odd_marks = (uint32_t*)workspace;
+        const cudaError_t e = f32_tc_backward(a, st);
+        if (e != cudaSuccess) return e;
+    }
+    return simt_backward(a, st);
+}
+
 struct Carve {
     char* p;
     size_t left;
@@ -106,10 +133,6 @@ struct Carve {
         return r;
     }
 };
-
-size_t nq_elems(const sntl_attn_desc* d) { return (size_t)d->batch * d->q_heads * d->seq_q * d->head_dim; }
-size_t nkv_elems(const sntl_attn_desc* d) { return (size_t)d->batch * d->kv_heads * d->seq_kv * d->head_dim; }
-size_t nlse(const sntl_attn_desc* d) { return (size_t)d->batch * d->q_heads * d->seq_q; }
 
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? SNTL_OK : SNTL_ERR_CUDA; }
 
@@ -171,7 +194,7 @@ size_t sntl_attn_fwd_workspace_bytes(const sntl_attn_desc* d)
 size_t sntl_attn_bwd_workspace_bytes(const sntl_attn_desc* d)
 {
     if (validate(d) != SNTL_OK) return 0;
-    size_t bytes = align_up(4 * nlse(d));  // exact path: room for delta, which its kernel no longer needs; what callers bring is unchanged
+    size_t bytes = align_up(4 * nlse(d));  // exact path: marks of blocks of 128 rows (a word per row is what callers bring)
     if (!wants_tc(d, true)) return bytes;
     bytes = align_up(tc_backward_workspace_bytes(shape_of(d)));
     if (d->layout == SNTL_LAYOUT_SENTINEL)   // bf16 Q, dO, K, V
@@ -203,8 +226,7 @@ int sntl_attn_fwd(const sntl_attn_desc* d, const void* q, const void* k, const v
         a.o_out = (char*)o + off; a.lse_out = (float*)((char*)lse + off);
         views(d, a.vq, a.vkv, a.vlse);
         set_vector_access(a);
-        g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
-        return cuda_status(simt_forward(a, st));
+        return cuda_status(exact_forward(a, d, st));
     }
 
     TcArgs t{};
@@ -315,8 +337,7 @@ int sntl_attn_cached_fwd(const sntl_attn_desc* d, const void* q, const void* k_c
     const long long D = d->head_dim, C = cache_capacity;
     a.vkv = d->layout == SNTL_LAYOUT_BHSD ? View4{(long long)d->kv_heads * C * D, C * D, D, 1} : View4{0, D * C, 1, C};
     set_vector_access(a);
-    g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
-    return cuda_status(simt_forward(a, st));
+    return cuda_status(exact_forward(a, d, st));
 }
 
 int sntl_attn_bwd(const sntl_attn_desc* d, const void* q, const void* k, const void* v, const void* o,
@@ -343,8 +364,7 @@ int sntl_attn_bwd(const sntl_attn_desc* d, const void* q, const void* k, const v
         a.dq = (char*)dq + off; a.dk = (char*)dk + off; a.dv = (char*)dv + off;
         views(d, a.vq, a.vkv, a.vlse);
         set_vector_access(a);
-        g_last_path = a.is_bf16 ? "simt_bf16" : "simt_f32";
-        return cuda_status(simt_backward(a, st));
+        return cuda_status(exact_backward(a, d, workspace, st));
     }
 
     TcArgs t{};

@@ -1384,7 +1384,9 @@ cudaError_t read_and_clear_bwd_status(cudaStream_t st, uint32_t* word)
     unsigned int w = 0, zero = 0;
     if ((e = cudaMemcpyFromSymbol(&w, ptx::g_device_status, sizeof(w))) != cudaSuccess) return e;
     if (w != 0 && (e = cudaMemcpyToSymbol(ptx::g_device_status, &zero, sizeof(zero))) != cudaSuccess) return e;
-    *word = w;
+    uint32_t f32 = 0;
+    if ((e = read_and_clear_f32_bwd_status(&f32)) != cudaSuccess) return e;
+    *word = w ? w : f32;
     return cudaSuccess;
 }
 

@@ -814,7 +814,9 @@ cudaError_t read_and_clear_fwd_status(cudaStream_t st, uint32_t* word)
     if (w != 0 && (e = cudaMemcpyToSymbol(ptx::g_device_status, &zero, sizeof(zero))) != cudaSuccess) return e;
     uint32_t cache = 0;
     if ((e = read_and_clear_cache_status(&cache)) != cudaSuccess) return e;
-    *word = w ? w : cache;
+    uint32_t f32 = 0;
+    if ((e = read_and_clear_f32_fwd_status(&f32)) != cudaSuccess) return e;
+    *word = w ? w : cache ? cache : f32;
     return cudaSuccess;
 }
 

@@ -62,6 +62,7 @@ __device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* sme
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, group = s.Hq / s.Hkv;
     const int slabs = s.B * s.Hkv, slab = tile % slabs, b = slab / s.Hkv, hk = slab - b * s.Hkv;
     const int key0 = (tile / slabs) * L::kRows;               // causal: the first key tiles are seen by the most queries
+    if (a.odd_marks && a.odd_marks[key0 / 128 * slabs + slab] == 0) return;
     const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
     const long long kvoff = b * a.vkv.sb + hk * a.vkv.sh;
     stage<T, DP, L::kRows>(smem + L::own0, (const T*)a.k + kvoff, mk, key0);
@@ -137,6 +138,7 @@ __device__ __forceinline__ void dq_role(const SimtArgs& a, int tile, int n_qt, f
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int slabs = s.B * s.Hq, bh = tile % slabs, b = bh / s.Hq, h = bh - b * s.Hq, hk = h / (s.Hq / s.Hkv);
     const int row0 = (n_qt - 1 - tile / slabs) * L::kRows;    // longest query tiles first
+    if (a.odd_marks && a.odd_marks[(s.Skv + 127) / 128 * (s.B * s.Hkv) + row0 / 128 * slabs + bh] == 0) return;
     const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
     const long long qoff = b * a.vq.sb + h * a.vq.sh;
     const T* kb = (const T*)a.k + b * a.vkv.sb + hk * a.vkv.sh;

@@ -37,6 +37,8 @@ __global__ void __launch_bounds__(kThreads, DP <= 64 ? 3 : 2) simt_fwd_kernel(co
     const int slabs = s.B * s.Hq, bh = tile % slabs, b = bh / s.Hq, h = bh - b * s.Hq, hk = h / (s.Hq / s.Hkv);
     const int qt = n_qt - 1 - tile / slabs;                   // longest query tiles first
     const int row0 = qt * L::kRows;
+    // (every row carries the mark, and only its tile's CTA or cluster overwrites it, after all of that have looked)
+    if (a.only_odd && __float_as_uint(a.lse_out[b * a.vlse.sb + h * a.vlse.sh + (long long)row0 * a.vlse.ss]) != kOddLse) return;
     const T* kb = (const T*)a.k + b * a.vkv.sb + hk * a.vkv.sh;
     const T* vb = (const T*)a.v + b * a.vkv.sb + hk * a.vkv.sh;
     const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
@@ -207,7 +209,7 @@ cudaError_t dispatch_dim(const SimtArgs& a, cudaStream_t st)
 
 cudaError_t simt_forward(const SimtArgs& a, cudaStream_t st)
 {
-    if (simt_decode_supported(a)) return simt_decode(a, st);
+    if (!a.only_odd && simt_decode_supported(a)) return simt_decode(a, st);
     return a.is_bf16 ? dispatch_dim<__nv_bfloat16>(a, st) : dispatch_dim<float>(a, st);
 }
 

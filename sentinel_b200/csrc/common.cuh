@@ -137,12 +137,23 @@ struct SimtArgs {
     View4 vq, vkv;     // q-like tensors (Q, O, dO, dQ) and kv-like tensors (K, V, dK, dV)
     View3 vlse;
     bool vec_q, vec_kv;   // every row of all q-like / kv-like tensors can be accessed four elements at a time
+    // The FMA kernels behind the tensor-core ones compute only what those left (blocks of 128 rows with values that their products do
+    // not take): forward, query tiles whose LSE rows hold kOddLse; backward, tiles whose word of odd_marks is not 0 (null: all tiles).
+    bool only_odd;
+    uint32_t* odd_marks;  // backward: one word per 128 keys of every (batch, KV head), then one per 128 queries of every (batch, head)
 };
+constexpr uint32_t kOddLse = 0x7fc0dd5au;   // a NaN that no computation returns
 cudaError_t simt_forward(const SimtArgs& a, cudaStream_t st);
 // few query rows per KV head (decode): simt_forward takes this path by itself where it applies
 bool simt_decode_supported(const SimtArgs& a);
 cudaError_t simt_decode(const SimtArgs& a, cudaStream_t st);
 cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st);  // one launch
+// The same results from split products on the tensor cores (attn_f32_fwd_sm100.cu, attn_f32_bwd_sm100.cu): fp32, head_dim up to 64, where
+// there is enough work.  They leave odd blocks to simt_forward / simt_backward with the marks.
+bool f32_tc_forward_supported(const SimtArgs& a);
+cudaError_t f32_tc_forward(const SimtArgs& a, cudaStream_t st);
+bool f32_tc_backward_supported(const SimtArgs& a, size_t marks_bytes);
+cudaError_t f32_tc_backward(const SimtArgs& a, cudaStream_t st);
 
 // Results in the reference's feature-major layout: element (b, h, s, d) at ((h*D + d)*stride + b*S + s), LSE (b, h, s) at
 // (h*stride + b*S + s); the pointers include the first column of the window.
@@ -216,9 +227,12 @@ cudaError_t merge_partials(int acc_dtype, int part_dtype, long long rows, int D,
 // give-up path of the bounded waits without hanging or faulting anything.  *gave_up (device memory, optional) <- 1.
 cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned int* gave_up, cudaStream_t st);
 
-// Device status words written by bounded waits (one per tensor-core translation unit; the first reports the KV-cache kernel's too).
+// Device status words written by bounded waits (one per tensor-core translation unit; the first reports the KV-cache kernel's and the fp32 forward's too, the second the
+// fp32 backward's).
 cudaError_t read_and_clear_fwd_status(cudaStream_t st, uint32_t* word);
 cudaError_t read_and_clear_cache_status(uint32_t* word);   // after a synchronisation of the stream
+cudaError_t read_and_clear_f32_fwd_status(uint32_t* word);
+cudaError_t read_and_clear_f32_bwd_status(uint32_t* word);
 cudaError_t read_and_clear_bwd_status(cudaStream_t st, uint32_t* word);
 
 }  // namespace sntl

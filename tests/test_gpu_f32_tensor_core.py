@@ -1,0 +1,155 @@
+"""Exact fp32 through split products on the tensor cores (csrc/attn_f32_fwd_sm100.cu, attn_f32_bwd_sm100.cu): calls with enough work
+and head_dim up to 64 take them by themselves, flags=FORCE_SIMT keeps the FMA kernels.
+
+Bound against the fp64 oracle: a product of parts is within 2^-23 of its terms' size (the tensor core cuts off below 2^-24, the parts
+left out are below 2^-25), the exponential and the sums of up to a few thousand such products add a few units of 2^-24 of the
+result's size: 1e-6 relative L2 covers them (measured 1e-7 to 4e-7; the FMA kernels 1e-7 to 1.1e-6).
+"""
+import numpy as np
+import pytest
+import torch
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+FORCE_SIMT = 2
+REL = 1e-6
+
+
+@pytest.fixture(scope="module")
+def sb():
+    import sentinel_b200
+    sentinel_b200._lib.load()
+    assert torch.cuda.is_available()
+    return sentinel_b200
+
+
+def _inputs(seed, B, Hq, Hkv, S, D, Skv=None):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    Skv = Skv or S
+    return [torch.randn(B, H, n, D, generator=g, device="cuda") for H, n in ((Hq, S), (Hkv, Skv), (Hkv, Skv), (Hq, S))]
+
+
+def _launches(sb, f):
+    n = sb.launch_count()
+    r = f()
+    return r, sb.launch_count() - n
+
+
+def _both(sb, q, k, v, do, **kw):
+    (o, lse), nf = _launches(sb, lambda: sb.attention_forward(q, k, v, **kw))
+    g, nb = _launches(sb, lambda: sb.attention_backward(q, k, v, o, lse, do, **kw))
+    assert sb.last_path() == "simt_f32" and sb.poll_device_status() == 0
+    return (o, lse) + tuple(g), (nf, nb)
+
+
+NAMES = ("o", "lse", "dq", "dk", "dv")
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,window,global_tokens,causal", [
+    (8, 12, 12, 129, 64, 0, 0, True),       # a row more than a block, a KV tile with one token
+    (4, 16, 16, 192, 64, 0, 0, True),       # half a block
+    (2, 12, 4, 301, 62, 0, 0, True),        # ragged, head_dim not a multiple of 4, grouped heads
+    (6, 24, 24, 128, 30, 0, 0, True),       # features filled up to 64; exactly one block
+    (8, 40, 40, 191, 16, 0, 0, True),
+    (2, 6, 2, 700, 64, 130, 5, True),       # window edges inside tiles, global tokens
+    (3, 6, 6, 640, 64, 64, 130, True),      # global tokens beyond one tile of keys
+    (2, 8, 4, 257, 64, 0, 0, False),
+    (1, 12, 4, 1153, 48, 0, 0, True),       # many tiles
+])
+def test_against_the_oracle(sb, oracle, B, Hq, Hkv, S, D, window, global_tokens, causal):
+    q, k, v, do = _inputs(S + D, B, Hq, Hkv, S, D)
+    kw = dict(window=window, global_tokens=global_tokens, causal=causal)
+    got, launches = _both(sb, q, k, v, do, **kw)
+    assert launches == (2, 2)               # the tensor-core kernel and the FMA kernel for what it leaves
+    a = [t.cpu().numpy() for t in (q, k, v, do)]
+    want = oracle.attn_fwd(*a[:3], **kw) + tuple(oracle.attn_bwd(*a, **kw)[:3])
+    for x, w, name in zip(got, want, NAMES):
+        assert rel_l2(x.cpu().numpy(), w) <= REL, (name, rel_l2(x.cpu().numpy(), w))
+    again, _ = _both(sb, q, k, v, do, **kw)
+    assert all(torch.equal(x, y) for x, y in zip(got, again))
+
+
+def test_keys_longer_than_queries(sb):
+    """New tokens behind a fp32 cache, and a rectangular call without a causal mask."""
+    q, k, v, do = _inputs(3, 2, 12, 6, 150, 64, 1000)
+    o, n = _launches(sb, lambda: sb.attention_cached_forward(q, k, v, 900))
+    o2, _ = sb.attention_cached_forward(q, k, v, 900, flags=FORCE_SIMT), 0
+    assert n == 2 and all(rel_l2(x.cpu().numpy(), y.cpu().numpy()) <= REL for x, y in zip(o, o2))
+    got, launches = _both(sb, q, k, v, do, causal=False)
+    want, _ = _both(sb, q, k, v, do, causal=False, flags=FORCE_SIMT)
+    assert launches == (2, 2)
+    for x, w, name in zip(got, want, NAMES):
+        assert rel_l2(x.cpu().numpy(), w.cpu().numpy()) <= 2 * REL, name
+
+
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_matrices_and_unaligned_tensors(sb, offset):
+    """Feature-major matrices with a column offset, and token-major tensors that start anywhere."""
+    from sentinel_b200.flash_attention import CudaFlashAttention as F
+    B, H, S, D = 4, 12, 160, 64
+    q, k, v, do = _inputs(offset, B, H, H, S, D)
+    want, _ = _both(sb, q, k, v, do)
+    C = 5 + B * S + 2
+    mats = []
+    for t in (q, k, v, do):
+        m = torch.full((H * D, C), float("nan"), device="cuda")
+        m[:, 5:5 + B * S] = t.permute(1, 3, 0, 2).reshape(H * D, B * S)
+        mats.append(m)
+    out = {n: torch.zeros(H * D if n != "lse" else H, C, device="cuda") for n in NAMES}
+    F.allow_reduced_precision = False
+    shape = (H, D, D ** -0.5, True, 5, S, B)
+    F.forwardMultiHead(*mats[:3], out["o"], out["lse"], *shape)
+    F.backwardMultiHead(*mats[:3], out["o"], out["lse"], mats[3], out["dq"], out["dk"], out["dv"], None, *shape)
+    for w, name in zip(want, NAMES):
+        rows = 1 if name == "lse" else D
+        x = out[name][:, 5:5 + B * S].reshape(H, rows, B, S).permute(2, 0, 3, 1).reshape(w.shape)
+        assert torch.equal(x, w), name       # the same products in the same order
+        assert not out[name][:, :5].any() and not out[name][:, 5 + B * S:].any()
+    moved = []
+    for t in (q, k, v, do):
+        flat = torch.empty(t.numel() + offset, device="cuda")
+        flat[offset:] = t.reshape(-1)
+        moved.append(flat[offset:].view(t.shape))
+    got, _ = _both(sb, *moved)
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -3.0e38, 2.0 ** 31, 1e-37])
+def test_blocks_with_odd_values_are_the_fma_kernels(sb, bad, window):
+    """A block that meets a value that its products do not take is computed by the FMA kernels, bit for bit; the others stay."""
+    B, H, S, D = 2, 24, 300, 64
+    q, k, v, do = _inputs(7, B, H, H, S, D)
+    kw = dict(window=window)
+    clean, _ = _both(sb, q, k, v, do, **kw)
+    for t in (q, do, k, v):
+        t[1, 3, 170::2, 5] = bad              # query and key tile 1 on of one head
+    fma, _ = _both(sb, q, k, v, do, flags=FORCE_SIMT, **kw)
+    o, lse = sb.attention_forward(q, k, v, **kw)
+    # the backward of both from the same forward results
+    got = (o, lse) + tuple(sb.attention_backward(q, k, v, fma[0], fma[1], do, **kw))
+    want = fma[:2] + tuple(sb.attention_backward(q, k, v, fma[0], fma[1], do, flags=FORCE_SIMT, **kw))
+    assert sb.poll_device_status() == 0
+    same = lambda x, y: torch.equal(x.nan_to_num(7.0), y.nan_to_num(7.0)) and torch.equal(x.isnan(), y.isnan())
+    for x, w, c, name in zip(got, want, clean, NAMES):
+        assert same(x[1, 3, 128:], w[1, 3, 128:]), name
+        if name in ("o", "lse", "dq"):
+            assert torch.equal(x[1, 3, :128], c[1, 3, :128]) or name == "dq", name      # sees no such token
+        if name in ("o", "lse"):
+            assert torch.equal(x[0], c[0]) and torch.equal(x[1, :3], c[1, :3]) and torch.equal(x[1, 4:], c[1, 4:]), name
+
+
+def test_inconsistent_lse_is_the_fma_kernels(sb):
+    """Weights far above 1 (an LSE that is not this call's) would overflow in parts: the FMA kernels' results, infinities included."""
+    q, k, v, do = _inputs(11, 2, 24, 24, 256, 64)
+    o, lse = sb.attention_forward(q, k, v)
+    lse[0, 1, 200] = -120.0
+    lse[1, 0, 3] = float("nan")
+    lse[1, 1, 4] = float("inf")
+    got = sb.attention_backward(q, k, v, o, lse, do)
+    want = sb.attention_backward(q, k, v, o, lse, do, flags=FORCE_SIMT)
+    for x, w in zip(got, want):
+        assert torch.equal(x.isfinite(), w.isfinite())
+        fin = w.isfinite()
+        assert float((x - w)[fin].norm() / w[fin].norm()) <= 2 * REL

@@ -25,18 +25,11 @@ constexpr int kRowBytes = kDim * 2;      // a row of one part: 128 bytes, 128-by
 constexpr int kOwnRows = 128;            // rows of a block: the TMEM lanes
 constexpr int kFetchRows = 64;           // rows that are staged at a time
 // warps 0-7 sums, 8-13 stage, 14 issues the products, 15 idle; the first two warpgroups take registers from the others
-constexpr int kSumThreads = 256, kStageThreads = 192, kThreads = 512, kIssueWarp = 14, kSumRegs = 160, kOtherRegs = 96;
-static_assert(kSumThreads * kSumRegs + (kThreads - kSumThreads) * kOtherRegs <= kThreads * 128, "what the block is launched with");
+constexpr int kSumThreads = 256, kStageThreads = 192, kThreads = 512, kIssueWarp = 14;
+// (128 registers a thread at launch.  Nothing in the loops may be spilled: next to the streamed rows local memory does not stay in L1.)
+__host__ __device__ constexpr int other_regs(int sum_regs) { return (kThreads * 128 - kSumThreads * sum_regs) / (kThreads - kSumThreads) / 8 * 8; }
 constexpr float kLargest = 1073741824.0f;                 // 2^30: products of two such, summed, stay far from overflow
 constexpr float kLargestWeight = 1.152921504606847e18f;   // 2^60, for what the kernels compute themselves
-
-// rows [.., S) of a slab of D features with element strides ss, sd
-struct Rows {
-    const float* base;
-    long long ss, sd;
-    int S, D;
-    bool vec;       // sd == 1, D % 4 == 0 and every row on a 16-byte boundary
-};
 
 // What a thread has seen of the values that it staged.
 struct Check {
@@ -60,63 +53,92 @@ __device__ __forceinline__ void split2(float2 x, uint32_t& h, uint32_t& m, uint3
     lost |= a | b;
 }
 
-// eight features of a row, from feature d
-__device__ __forceinline__ void load8(float (&x)[8], const Rows& m, int row, int d)
-{
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = 0.f;
-    if (row >= m.S || d >= m.D) return;
-    const float* p = m.base + row * m.ss + d * m.sd;
-    if (m.vec) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-        if (d + 4 < m.D) {
-            const float4 b = __ldg(reinterpret_cast<const float4*>(p + 4));
-            x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (d + i < m.D) x[i] = __ldg(p + i * m.sd);
+// Rows that are to be staged: the address of the first, and how many there are from it on (the others read as zero).
+struct Source {
+    const float* at;
+    int left;
+};
+
+// A staging thread's share of a half tile: units of eight features of a row, numbered along the contiguous direction of the tensors so
+// that a warp's loads coalesce.  (kStageThreads is a multiple of the 8 units of a row and of kFetchRows: from one unit of a thread to
+// its next either the row or the features change, by a constant.)
+// kVec: all rows lie on 16-byte boundaries with features side by side, head_dim a multiple of 4.
+template <bool kVec> struct Share {
+    static constexpr int kUnits = kFetchRows * 8, kPer = (kUnits + kStageThreads - 1) / kStageThreads;
+    static_assert(kStageThreads % kFetchRows == 0 && kStageThreads % 64 == 0, "");
+    int t, row0, chunk0, off0, step, sd, D;
+    bool rows_contiguous;        // (feature-major matrices)
+
+    __device__ __forceinline__ Share(int t_, int ss, int sd_, int D_) : t(t_), sd(sd_), D(D_), rows_contiguous(sd_ != 1)
+    {
+        row0 = matrix() ? t % kFetchRows : t >> 3;
+        chunk0 = matrix() ? t / kFetchRows : t & 7;
+        off0 = row0 * ss + chunk0 * 8 * sd;
+        step = kStageThreads / 8 * (matrix() ? sd : ss);
     }
+    __device__ __forceinline__ bool matrix() const { return !kVec && rows_contiguous; }
+    __device__ __forceinline__ bool valid(int k) const { return k + 1 < kPer || t < kUnits - (kPer - 1) * kStageThreads; }
+    __device__ __forceinline__ int row(int k) const { return matrix() ? row0 : row0 + k * (kStageThreads / 8); }
+    __device__ __forceinline__ int chunk(int k) const { return matrix() ? chunk0 + k * (kStageThreads / kFetchRows) : chunk0; }
+    // where the unit goes inside a part: rows of 128 bytes, 128-byte swizzle (the rows of a thread's units differ by multiples of 8)
+    __device__ __forceinline__ int place(int k) const
+    {
+        return matrix() ? row0 * kRowBytes + ((chunk(k) ^ (row0 & 7)) << 4)
+                        : row0 * kRowBytes + ((chunk0 ^ (row0 & 7)) << 4) + k * (kStageThreads / 8) * kRowBytes;
+    }
+};
+
+// Loads of rows that pass once: they go first when L1 (28 KB beside this shared memory) is full, not what the other warps have there.
+// x stays what it is where `in` is false.  (Predicated, into place: behind a branch the compiler copies the values where the paths
+// meet, and the copy waits for the load; the staging warps then spent two thirds of their time on the latency of L2.)
+__device__ __forceinline__ void load_once4(float* x, const float* p, bool in)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.global.nc.L1::evict_first.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "+f"(x[0]), "+f"(x[1]), "+f"(x[2]), "+f"(x[3]) : "l"(p), "r"((uint32_t)in));
+}
+__device__ __forceinline__ void load_once(float& x, const float* p, bool in)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.nc.L1::evict_first.f32 %0, [%1];\n\t}" : "+f"(x) : "l"(p), "r"((uint32_t)in));
 }
 
-// kFetchRows rows on their way from global memory to shared memory, in the registers of kStageThreads threads numbered t: loaded ahead
-// of the wait for the place that they go to.  A unit is eight features of a row, numbered along the contiguous direction of the
-// source so that a warp's loads coalesce.
-struct Fetch {
-    static constexpr int kUnits = kFetchRows * 8, kPer = (kUnits + kStageThreads - 1) / kStageThreads;
-    float x[kPer][8];
+// Half a tile on its way from global memory to shared memory, in registers: loaded ahead of the wait for the place that it goes to.
+template <bool kVec> struct Fetch {
+    using Share = f32tc::Share<kVec>;
+    float x[Share::kPer][8];
 
-    static __device__ __forceinline__ bool unit(int k, int t, bool rows_contiguous, int& r, int& c)
-    {
-        const int u = k * kStageThreads + t;
-        r = rows_contiguous ? u % kFetchRows : u >> 3;
-        c = rows_contiguous ? u / kFetchRows : u & 7;
-        return kUnits % kStageThreads == 0 || k + 1 < kPer || u < kUnits;
-    }
-    __device__ __forceinline__ void load(const Rows& m, int row0, int t)
+    __device__ __forceinline__ void load(const Source& m, const Share& w)
     {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            int r, c;
-            if (unit(k, t, m.sd != 1, r, c)) load8(x[k], m, row0 + r, c * 8);
+        for (int k = 0; k < Share::kPer; ++k) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[k][i] = 0.f;
+            int sd = w.sd;
+            if (!kVec) asm volatile("" : "+r"(sd));      // (or its multiples, 64 bits each, would be kept in registers)
+            const int d = w.chunk(k) * 8;
+            const bool in = w.valid(k) && w.row(k) < m.left;
+            const float* p = m.at + w.off0 + k * w.step;
+            if constexpr (kVec) {
+                load_once4(x[k], p, in && d < w.D);
+                load_once4(x[k] + 4, p + 4, in && d + 4 < w.D);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i, p += sd) load_once(x[k][i], p, in && d + i < w.D);
+            }
         }
     }
     // -> the three parts, `pitch` bytes apart, each kFetchRows x 128 bytes.  (The 16-byte stores of eight lanes fall into different
     // banks in either order of the units: rows are swizzled.)
-    __device__ __forceinline__ void put(uint8_t* dst, int pitch, bool rows_contiguous, int t, Check& check) const
+    __device__ __forceinline__ void put(uint8_t* dst, int pitch, const Share& w, Check& check) const
     {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            int r, c;
-            if (!unit(k, t, rows_contiguous, r, c)) continue;
+        for (int k = 0; k < Share::kPer; ++k) {
+            if (!w.valid(k)) continue;
             uint4 h, m, l;
             split2(make_float2(x[k][0], x[k][1]), h.x, m.x, l.x, check.lost);
             split2(make_float2(x[k][2], x[k][3]), h.y, m.y, l.y, check.lost);
             split2(make_float2(x[k][4], x[k][5]), h.z, m.z, l.z, check.lost);
             split2(make_float2(x[k][6], x[k][7]), h.w, m.w, l.w, check.lost);
-            uint8_t* at = dst + r * kRowBytes + ((c ^ (r & 7)) << 4);
+            uint8_t* at = dst + w.place(k);
             *reinterpret_cast<uint4*>(at) = h;
             *reinterpret_cast<uint4*>(at + pitch) = m;
             *reinterpret_cast<uint4*>(at + 2 * pitch) = l;
@@ -125,16 +147,15 @@ struct Fetch {
         }
     }
     // sums of products with the same units of `other`, to part[row * 9 + unit]
-    __device__ __forceinline__ void dots(bool rows_contiguous, int t, const Fetch& other, float* part) const
+    __device__ __forceinline__ void dots(const Share& w, const Fetch& other, float* part) const
     {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            int r, c;
-            if (!unit(k, t, rows_contiguous, r, c)) continue;
+        for (int k = 0; k < Share::kPer; ++k) {
+            if (!w.valid(k)) continue;
             float sum = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) sum = fmaf(x[k][i], other.x[k][i], sum);
-            part[r * 9 + c] = sum;
+            part[w.row(k) * 9 + w.chunk(k)] = sum;
         }
     }
 };
@@ -183,26 +204,73 @@ template <bool kSwap = false, typename F> __device__ __forceinline__ void six(F&
     f(0, 0, 1u);
 }
 
-// kN columns of the parts of kN pairs of values, part p at taddr + p * kPitch; what is left in x is the last part.
+// kN columns of each of the parts of kN pairs of values, part p at taddr + p * kPitch; what is left in x is the last part.
 template <int kN, int kPitch> __device__ __forceinline__ void put_parts(uint32_t taddr, float2 (&x)[kN])
 {
+    constexpr int kC = kN == 16 ? 16 : 8;      // (as registers allow)
     const float2 minus = make_float2(-1.f, -1.f);
-    uint32_t w[kN];
 #pragma unroll
-    for (int p = 0; p < 3; ++p) {
+    for (int c = 0; c < kN; c += kC) {
 #pragma unroll
-        for (int i = 0; i < kN; ++i) {
-            if (p < 2) {
-                w[i] = ptx::pack_bf16(x[i].x, x[i].y);
-                x[i] = ffma2(unpack2(w[i]), minus, x[i]);
-            } else {
-                w[i] = __byte_perm(__float_as_uint(x[i].x), __float_as_uint(x[i].y), 0x7632);
+        for (int p = 0; p < 3; ++p) {
+            uint32_t w[kC];
+#pragma unroll
+            for (int i = 0; i < kC; ++i) {
+                float2& y = x[c + i];
+                if (p < 2) {
+                    w[i] = ptx::pack_bf16(y.x, y.y);
+                    y = ffma2(unpack2(w[i]), minus, y);
+                } else {
+                    w[i] = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x7632);
+                }
             }
+            if constexpr (kC == 8) ptx::tmem_st8(taddr + p * kPitch + c, w);
+            else ptx::tmem_st16(taddr + p * kPitch + c, w);
         }
-        if constexpr (kN == 32) ptx::tmem_st32(taddr + p * kPitch, w);
-        else ptx::tmem_st16(taddr + p * kPitch, w);
     }
 }
+
+// The blocks that a CTA computes one after the other: its own, then blocks of the grid that have not started, which the block scheduler
+// hands over on request (one is asked for when the last tile of a block is being staged).  Set-up, first loads and first products of
+// a block so run under the end of the one before, and its code has been fetched.  Block number u of a CTA; every warp that works
+// reads the answer for it.
+constexpr int kWorkWarps = kIssueWarp + 1;
+struct BlockQueue {
+    alignas(16) uint4 answer[2];
+    uint64_t full[2], empty[2];
+
+    __device__ __forceinline__ void init()
+    {
+        for (int i = 0; i < 2; ++i) {
+            ptx::mbar_init(&full[i], 1);
+            ptx::mbar_init(&empty[i], kWorkWarps);
+        }
+    }
+    // by one thread; false: a wait gave up
+    __device__ __forceinline__ bool ask(int u, volatile uint32_t* abort_flag)
+    {
+        if (u > 2 && !ptx::mbar_wait(&empty[u & 1], (((u - 1) >> 1) - 1) & 1, abort_flag, 20)) return false;
+        ptx::mbar_arrive_expect_tx(&full[u & 1], 16);
+        ptx::clc_try_cancel(&answer[u & 1], &full[u & 1]);
+        return true;
+    }
+    // by a whole warp: block number u, or -1 where there is none
+    __device__ __forceinline__ int get(int u, volatile uint32_t* abort_flag)
+    {
+        if (!ptx::mbar_wait_warp(&full[u & 1], ((u - 1) >> 1) & 1, abort_flag, 21)) return -1;
+        const int block = ptx::warp_uniform(ptx::clc_first_block(&answer[u & 1]));
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(&empty[u & 1]);
+        return block;
+    }
+};
+// Which block (u + 1) of the last four was found odd
+struct OddBlocks {
+    volatile int number[4];
+    __device__ __forceinline__ void set(int u) { number[u & 3] = u + 1; }
+    __device__ __forceinline__ bool get(int u) const { return number[u & 3] == u + 1; }
+};
 
 // Whether the call has the work that the blocks' set-up and their chains of tiles are worth: visible pairs x features.  Below, the FMA
 // kernels' small tiles and their split of the keys over clusters are faster (B4 H8 S128 D64 forward 12.1 us against 13.3, S256 D32
@@ -216,22 +284,28 @@ inline bool enough_work(const AttnShape& s)
 // Scales that keep the scores of values below kLargest, and those that stand for hidden pairs, apart from each other and in range
 inline bool scale_supported(float scale) { return scale >= 1.0f / 65536 && scale <= 65536.0f; }
 
-// 32 features of a row times f, from feature d0 on, to global memory
-__device__ __forceinline__ void store_row(float* base, const Rows& m, int row, int d0, const float2 (&y)[16], float f)
+// One pair of strides for all tensors, and offsets inside a tile that fit 32 bits
+inline bool strides_supported(const SimtArgs& a)
 {
-    if (row >= m.S) return;
-    float* p = base + row * m.ss + d0 * m.sd;
+    return a.vq.ss == a.vkv.ss && a.vq.sd == a.vkv.sd && a.vq.ss <= (1 << 24) && a.vq.sd <= (1 << 24);
+}
+
+// 32 features of row `row` times f, from feature d0 on, to a slab of S rows with strides ss, sd (vec: stores of four features)
+__device__ __forceinline__ void store_row(float* base, long long ss, long long sd, int S, int D, bool vec, int row, int d0, const float2 (&y)[16], float f)
+{
+    if (row >= S) return;
+    float* p = base + row * ss + d0 * sd;
     float x[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) x[i] = (i & 1 ? y[i / 2].y : y[i / 2].x) * f;
-    if (m.vec) {
+    if (vec) {
 #pragma unroll
         for (int i = 0; i < 32; i += 4)
-            if (d0 + i < m.D) *reinterpret_cast<float4*>(p + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+            if (d0 + i < D) *reinterpret_cast<float4*>(p + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
     } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-            if (d0 + i < m.D) p[i * m.sd] = x[i];
+            if (d0 + i < D) p[i * sd] = x[i];
     }
 }
 

@@ -1,0 +1,318 @@
+// dQ with one owner per element: the backward's third product for SNTL_FLAG_DETERMINISTIC.  A block owns 128 query rows of one
+// (batch, head) and visits the key tiles that they see: S = Q K^T, dP = dO V^T, dS = P o (dP - delta), dQ += dS K.  The sum stays in
+// TMEM, in the order of the keys, so the bits depend on nothing but the block's own rows and keys, and no scratch is needed; the kernel
+// for dK and dV (attn_bwd_sm100.cu) then leaves dQ out.  Seven products instead of five, against reductions of 64-bit words that
+// outlasted the five: 128 KB per step at the 25.5 bytes per clock that an SM gets through to L2.
+//
+//   warps 0-7  sums: thread = one query row and half of a tile's 128 keys
+//   warp 8     loads (TMA), warp 9 issues the products, 10 and 11 idle
+// TMEM: S [0, 128), dP [128, 256), dS (bf16, two buffers of 64 columns) [256, 384), dQ [384, 384 + D).
+#include "block_queue.cuh"
+#include "row_terms.cuh"
+
+namespace sntl {
+using namespace ptx;
+namespace {
+
+constexpr int kT = 128, kThreads = 384, kSumThreads = 256, kChunkBytes = kT * 128;
+constexpr uint32_t kColS = 0, kColDp = 128, kColDs = 256, kColDq = 384;
+
+struct Bars {
+    BlockQueue<10> queue;
+    uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], scores_full, scores_free, ds_full[2], dq_done[2];
+    uint32_t tmem_base, abort_flag;
+};
+template <int D> struct Smem {
+    static constexpr int kTile = kT * D * 2, q = 0, dout = kTile, k = 2 * kTile, v = 4 * kTile, bars = 6 * kTile;
+    static constexpr int bytes = bars + (int)sizeof(Bars) + 1024;
+};
+static_assert(Smem<128>::bytes <= 227 * 1024, "");
+
+struct Params {
+    AttnShape s;
+    const void *lse, *delta;          // terms of the padded query rows (store_row_terms)
+    __nv_bfloat16* dq;
+    float* dq_mat;                    // or an fp32 feature-major matrix (MatrixOut)
+    long long mat_stride;
+    int n_qt;
+};
+
+struct Block {
+    int b, h, bh, bh_kv, qt, n_keys;
+
+    __device__ __forceinline__ Block(const Params& p, int block)
+    {
+        const AttnShape& s = p.s;
+        bh = block % (s.B * s.Hq);
+        b = bh / s.Hq;
+        h = bh - b * s.Hq;
+        bh_kv = b * s.Hkv + h / (s.Hq / s.Hkv);
+        qt = p.n_qt - 1 - block / (s.B * s.Hq);             // longest query tiles first
+        n_keys = s.causal ? min((qt + 1) * kT, s.Skv) : s.Skv;
+    }
+    // k0, or the first key tile after it that some row sees (those between the global tokens and the window of the first row: none)
+    __device__ __forceinline__ int tile(const AttnShape& s, int k0) const
+    {
+        while (s.window > 0 && k0 < n_keys && k0 >= s.global_tokens && k0 + kT - 1 < qt * kT - s.window + 1) k0 += kT;
+        return k0;
+    }
+};
+
+template <int D, bool kMat>
+__global__ void __launch_bounds__(kThreads, 1)
+    attn_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                      const __grid_constant__ CUtensorMap tmap_do, const Params p)
+{
+    using L = Smem<D>;
+    constexpr int kChunks = D / 64;
+    extern __shared__ uint8_t raw[];
+    uint8_t* smem = raw + (1024 - (smem_u32(raw) & 1023)) % 1024;
+    Bars* bars = reinterpret_cast<Bars*>(smem + L::bars);
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        bars->queue.init();
+        mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->q_free, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->k_full[i], 1);
+            mbar_init(&bars->k_free[i], 1);
+            mbar_init(&bars->v_full[i], 1);
+            mbar_init(&bars->v_free[i], 1);
+            mbar_init(&bars->ds_full[i], kSumThreads);
+            mbar_init(&bars->dq_done[i], 1);
+        }
+        mbar_init(&bars->scores_full, 1);
+        mbar_init(&bars->scores_free, kSumThreads);
+        bars->abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == 9) {
+        tmem_alloc(&bars->tmem_base, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    volatile uint32_t* abort_flag = &bars->abort_flag;
+    wait_for_stream();
+
+    // Counters of key tiles run on over the blocks: c for this block's tile.
+    const AttnShape& s = p.s;
+    if (warp < 8) {
+        const int half = warp >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t lanes = tmem + ((uint32_t)(warp & 3) << 21);
+        const float2 scale2 = make_float2(s.scale * 1.4426950408889634f, s.scale * 1.4426950408889634f);
+        int c = 0;
+        for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
+            const Block w(p, block);
+            const int row = w.qt * kT + r, n_row = s.causal ? min(row + 1, s.Skv) : s.Skv;
+            const size_t padded = (size_t)w.bh * p.n_qt * kT + row;
+            float lse, delta;      // -LSE (log2) and -delta; at head_dim 64 the record of -LSE / scale is the sum of three bf16
+            if constexpr (bwd_folds_row_terms(D)) {
+                auto sum = [&](const void* records) {
+                    const uint2 x = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint4*>(records) + padded));
+                    return __uint_as_float(x.x << 16) + (__uint_as_float(x.x & 0xffff0000u) + __uint_as_float(x.y << 16));
+                };
+                lse = sum(p.lse) * scale2.x;
+                delta = sum(p.delta);
+            } else {
+                lse = __ldg(static_cast<const float*>(p.lse) + padded);
+                delta = __ldg(static_cast<const float*>(p.delta) + padded);
+            }
+            bool ok = true;
+            for (int k0 = w.tile(s, 0); k0 < w.n_keys; k0 = w.tile(s, k0 + kT), ++c) {
+                if (!(ok = mbar_wait_warp(&bars->scores_full, c & 1, abort_flag, 0x61))) break;
+                tc_fence_after();
+                uint32_t x[64], y[64];
+                tmem_ld32(lanes + kColS + half * 64, x);
+                tmem_ld32(lanes + kColS + half * 64 + 32, x + 32);
+                tmem_ld32(lanes + kColDp + half * 64, y);
+                tmem_ld32(lanes + kColDp + half * 64 + 32, y + 32);
+                tmem_ld_wait();
+                tc_fence_before();
+                mbar_arrive(&bars->scores_free);
+                // every pair of the tile is visible, or a mask per 32 keys
+                const bool cut = k0 + kT > (s.causal ? w.qt * kT + 1 : s.Skv) || s.window > 0;
+                uint32_t ds[32];
+                auto weights = [&](auto&& seen) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const float2 e = ffma2(make_float2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), scale2, make_float2(lse, lse));
+                        float2 w2 = make_float2(seen(2 * i) ? ex2(e.x) : 0.f, seen(2 * i + 1) ? ex2(e.y) : 0.f);
+                        if constexpr (D == 64) {      // as the P that dV and dK are made of, whose dS is rounded three times there
+                            const uint32_t rounded = pack_bf16(w2.x, w2.y);
+                            w2 = make_float2(__uint_as_float(rounded << 16), __uint_as_float(rounded & 0xffff0000u));
+                        }
+                        const float2 d = fmul2(w2, fadd2(make_float2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1])), make_float2(delta, delta)));
+                        ds[i] = pack_bf16(d.x, d.y);
+                    }
+                };
+                if (!cut) {
+                    weights([](int) { return true; });
+                } else {
+                    const uint32_t seen0 = keys_seen(s, row, n_row, k0 + half * 64), seen1 = keys_seen(s, row, n_row, k0 + half * 64 + 32);
+                    weights([&](int i) { return ((i < 32 ? seen0 : seen1) >> (i & 31) & 1u) != 0; });
+                }
+                // (the buffer is free once the product before last has read it)
+                if (c >= 2 && !(ok = mbar_wait_warp(&bars->dq_done[c & 1], ((c >> 1) - 1) & 1, abort_flag, 0x62))) break;
+                tc_fence_after();
+                tmem_st32(lanes + kColDs + (c & 1) * 64 + half * 32, ds);
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(&bars->ds_full[c & 1]);
+            }
+            if (!ok || !mbar_wait_warp(&bars->dq_done[(c - 1) & 1], ((c - 1) >> 1) & 1, abort_flag, 0x63)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int i = 0; i < D / 64; ++i) {
+                const int d0 = half * (D / 2) + i * 32;
+                uint32_t x[32];
+                tmem_ld32(lanes + kColDq + d0, x);
+                tmem_ld_wait();
+                if (row >= s.Sq) continue;
+                if constexpr (kMat) {
+                    float* dst = p.dq_mat + ((long long)w.h * D + d0) * p.mat_stride + (long long)w.b * s.Sq + row;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) dst[j * p.mat_stride] = __uint_as_float(x[j]) * s.scale;
+                } else {
+                    uint4* dst = reinterpret_cast<uint4*>(p.dq + ((size_t)w.bh * s.Sq + row) * D + d0);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint32_t v[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            v[e] = pack_bf16(__uint_as_float(x[8 * j + 2 * e]) * s.scale, __uint_as_float(x[8 * j + 2 * e + 1]) * s.scale);
+                        dst[j] = make_uint4(v[0], v[1], v[2], v[3]);
+                    }
+                }
+            }
+            tc_fence_before();
+        }
+    } else if (warp == 8) {
+        int c = 0;
+        for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
+            const Block w(p, block);
+            bool ok = true;
+            if (lane == 0) {
+                auto load = [&](int dst, const CUtensorMap* map, uint64_t* bar, int row, int slab) {
+                    for (int i = 0; i < kChunks; ++i) tma_load_3d(smem + dst + i * kChunkBytes, map, bar, i * 64, row, slab);
+                };
+                // Q and dO once the last scores of the block before have been computed
+                ok = u == 0 || mbar_wait(&bars->q_free, (u - 1) & 1, abort_flag, 0x64);
+                if (ok) {
+                    mbar_arrive_expect_tx(&bars->q_full, 2 * L::kTile);
+                    load(L::q, &tmap_q, &bars->q_full, w.qt * kT, w.bh);
+                    load(L::dout, &tmap_do, &bars->q_full, w.qt * kT, w.bh);
+                }
+                for (int k0 = w.tile(s, 0); ok && k0 < w.n_keys; ++c) {
+                    const int st = c & 1, next = w.tile(s, k0 + kT);
+                    if (c >= 2 && !(ok = mbar_wait(&bars->k_free[st], ((c >> 1) - 1) & 1, abort_flag, 0x65))) break;
+                    mbar_arrive_expect_tx(&bars->k_full[st], L::kTile);
+                    load(L::k + st * L::kTile, &tmap_k, &bars->k_full[st], k0, w.bh_kv);
+                    if (c >= 2 && !(ok = mbar_wait(&bars->v_free[st], ((c >> 1) - 1) & 1, abort_flag, 0x66))) break;
+                    mbar_arrive_expect_tx(&bars->v_full[st], L::kTile);
+                    load(L::v + st * L::kTile, &tmap_v, &bars->v_full[st], k0, w.bh_kv);
+                    k0 = next;
+                }
+                if (ok) ok = bars->queue.ask(u + 1, abort_flag);
+            }
+            c = warp_uniform(c);
+            if (!__all_sync(0xffffffffu, ok)) break;
+        }
+    } else if (warp == 9) {
+        constexpr uint32_t idesc_s = make_idesc(kT, kT, false, false), idesc_dq = make_idesc(kT, D, false, true);
+        const uint64_t q = make_sdesc(smem_u32(smem + L::q), 16, 1024), dout = make_sdesc(smem_u32(smem + L::dout), 16, 1024);
+        const uint64_t k = make_sdesc(smem_u32(smem + L::k), 16, 1024), v = make_sdesc(smem_u32(smem + L::v), 16, 1024);
+        const uint64_t k_mn = make_sdesc(smem_u32(smem + L::k), kChunkBytes, 1024);
+        auto wait = [&](uint64_t* bar, int parity, uint32_t site) { return mbar_wait_warp(bar, parity & 1, abort_flag, site); };
+        auto product = [&](uint32_t d, uint64_t a, uint64_t b) {
+#pragma unroll
+            for (int i = 0; i < kChunks; ++i) mma_ss_4<2, 2>(d, sdesc_advance(a, i * kChunkBytes), sdesc_advance(b, i * kChunkBytes), idesc_s, i > 0);
+        };
+        // scores of tile number n, `last` of its block
+        auto scores = [&](int n, bool last) {
+            const int st = n & 1;
+            if (!wait(&bars->k_full[st], n >> 1, 0x67) || !wait(&bars->v_full[st], n >> 1, 0x68)) return false;
+            if (n > 0 && !wait(&bars->scores_free, n - 1, 0x69)) return false;
+            tc_fence_after();
+            product(tmem + kColS, q, sdesc_advance(k, st * L::kTile));
+            product(tmem + kColDp, dout, sdesc_advance(v, st * L::kTile));
+            tc_commit_p(&bars->scores_full);
+            tc_commit_p(&bars->v_free[st]);
+            if (last) tc_commit_p(&bars->q_free);
+            return true;
+        };
+        int c = 0;
+        for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
+            const Block w(p, block);
+            int k0 = w.tile(s, 0);
+            bool ok = wait(&bars->q_full, u, 0x6a) && scores(c, w.tile(s, k0 + kT) >= w.n_keys), accumulate = false;
+            for (; ok && k0 < w.n_keys; ++c) {
+                const int st = c & 1;
+                k0 = w.tile(s, k0 + kT);
+                if (k0 < w.n_keys && !(ok = scores(c + 1, w.tile(s, k0 + kT) >= w.n_keys))) break;
+                if (!(ok = wait(&bars->ds_full[st], c >> 1, 0x6b))) break;
+                tc_fence_after();
+                const uint32_t ds = tmem + kColDs + st * 64;
+                const uint64_t b = sdesc_advance(k_mn, st * L::kTile);
+                mma_ts_4<8, 128>(tmem + kColDq, ds, b, idesc_dq, accumulate);
+                mma_ts_4<8, 128>(tmem + kColDq, ds + 32, sdesc_advance(b, 4 * 2048), idesc_dq, 1);
+                tc_commit_p(&bars->dq_done[st]);
+                tc_commit_p(&bars->k_free[st]);
+                accumulate = true;
+            }
+            if (!ok) break;
+        }
+    }
+    if (*abort_flag) {
+        for (int i = 0; i < 64; ++i) __nanosleep(2000);      // a wait gave up: copies and products in flight end before the block does
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+template <int D, bool kMat> cudaError_t launch(const TcArgs& a, const RowTerms& terms, cudaStream_t st)
+{
+    const AttnShape& s = a.s;
+    CUtensorMap tq, tk, tv, tdo;
+    cudaError_t e;
+    if ((e = encode_tmap_bf16_3d(&tq, a.q, D, s.Sq, s.B * s.Hq, 128)) != cudaSuccess) return e;
+    if ((e = encode_tmap_bf16_3d(&tdo, a.dout, D, s.Sq, s.B * s.Hq, 128)) != cudaSuccess) return e;
+    if ((e = encode_tmap_bf16_3d(&tk, a.k, D, s.Skv, s.B * s.Hkv, 128)) != cudaSuccess) return e;
+    if ((e = encode_tmap_bf16_3d(&tv, a.v, D, s.Skv, s.B * s.Hkv, 128)) != cudaSuccess) return e;
+    static std::atomic<unsigned long long> configured{0};
+    if ((e = ensure_dynamic_smem(attn_dq_tc_kernel<D, kMat>, Smem<D>::bytes, configured)) != cudaSuccess) return e;
+    const int n_qt = (s.Sq + kT - 1) / kT;
+    const long long blocks = (long long)n_qt * s.B * s.Hq;
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    Params p{s, terms.lse, terms.delta, a.dq, a.mat.dq, a.mat.stride, n_qt};
+    if (!s.causal) p.s.window = 0;
+    return launch_kernel(attn_dq_tc_kernel<D, kMat>, (unsigned)blocks, kThreads, Smem<D>::bytes, st, 1, tq, tk, tv, tdo, p);
+}
+
+}  // namespace
+
+cudaError_t tc_backward_dq(const TcArgs& a, cudaStream_t st)
+{
+    const AttnShape& s = a.s;
+    const RowTerms terms = row_terms_of(a.delta, (long long)s.B * s.Hq * ((s.Sq + kT - 1) / kT) * kT, s.D, s.scale);
+    if (a.mat.dq) return s.D == 64 ? launch<64, true>(a, terms, st) : launch<128, true>(a, terms, st);
+    return s.D == 64 ? launch<64, false>(a, terms, st) : launch<128, false>(a, terms, st);
+}
+
+cudaError_t read_and_clear_dq_status(uint32_t* word)
+{
+    uint32_t w = 0, zero = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(&w, g_device_status, sizeof(w));
+    if (e != cudaSuccess) return e;
+    if (w != 0 && (e = cudaMemcpyToSymbol(g_device_status, &zero, sizeof(zero))) != cudaSuccess) return e;
+    *word = w;
+    return cudaSuccess;
+}
+
+}  // namespace sntl

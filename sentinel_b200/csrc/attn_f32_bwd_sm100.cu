@@ -26,7 +26,7 @@ constexpr uint32_t kColS = 0, kColDp = 64, kColP = 128, kColDs = 224, kColDv = 3
 constexpr int kSumRegs = 152;
 
 struct Bars {
-    BlockQueue queue;
+    Queue queue;
     uint64_t own_free, in0_full[2], in0_free[2], in1_full[2], in1_free[2], scores_full, scores_free, weights_full, out_full, dots_full, block_done;
     uint32_t tmem_base, abort_flag;
     OddBlocks odd;

@@ -25,7 +25,7 @@ constexpr uint32_t kColS = 0, kColP = 128, kColO = 320;
 constexpr int kSumRegs = 144;
 
 struct Bars {
-    BlockQueue queue;
+    Queue queue;
     uint64_t q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full, s_free, p_full, o_full, pair[4];   // (V: its two halves)
     uint32_t tmem_base, abort_flag;
     OddBlocks odd;

@@ -192,6 +192,7 @@ size_t tc_cache_workspace_bytes(const AttnShape& s);
 bool tc_cache_supported(const AttnShape& s);
 cudaError_t tc_cache_forward(const TcArgs& a, int capacity, void* workspace, cudaStream_t st);
 cudaError_t tc_backward(const TcArgs& a, cudaStream_t st);
+cudaError_t tc_backward_dq(const TcArgs& a, cudaStream_t st);   // dQ alone, one owner per element (attn_dq_sm100.cu); a.delta holds the row terms
 size_t tc_backward_workspace_bytes(const AttnShape& s);
 // Bytes per padded query row at the head of the tensor-core backward workspace: two 16-byte records (the extra
 // contraction-step operands that carry -delta and -LSE/scale into the dP^T and S^T products)
@@ -233,6 +234,7 @@ cudaError_t read_and_clear_fwd_status(cudaStream_t st, uint32_t* word);
 cudaError_t read_and_clear_cache_status(uint32_t* word);   // after a synchronisation of the stream
 cudaError_t read_and_clear_f32_fwd_status(uint32_t* word);
 cudaError_t read_and_clear_f32_bwd_status(uint32_t* word);
+cudaError_t read_and_clear_dq_status(uint32_t* word);
 cudaError_t read_and_clear_bwd_status(cudaStream_t st, uint32_t* word);
 
 }  // namespace sntl

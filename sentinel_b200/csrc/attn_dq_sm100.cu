@@ -4,8 +4,12 @@
 // for dK and dV (attn_bwd_sm100.cu) then leaves dQ out.  Seven products instead of five, against reductions of 64-bit words that
 // outlasted the five: 128 KB per step at the 25.5 bytes per clock that an SM gets through to L2.
 //
-//   warps 0-7  sums: thread = one query row and half of a tile's 128 keys
-//   warp 8     loads (TMA), warp 9 issues the products, 10 and 11 idle
+// Backward, us, against the 64-bit reductions: B3 Hq16 Hkv4 S1237 D128 132 -> 97; B8 Hq28 Hkv4 S1024 D128 412 -> 240; B1 Hq28 Hkv4 S8192
+// D128 1910 -> 1320; B4 Hq32 Hkv8 S4096 D64 1036 -> 970; a 300-key window over B4 Hq12 S4096 D64 161 -> 157 to 165.  At head_dim 64 a tile
+// takes 2000 cycles of this kernel for 1000 of products and 1024 of exponentials: all warps load, compute and store a tile together.
+//
+//   warps 0-15  sums: thread = one query row and a quarter of a tile's 128 keys
+//   warp 16     loads (TMA), warp 17 issues the products
 // TMEM: S [0, 128), dP [128, 256), dS (bf16, two buffers of 64 columns) [256, 384), dQ [384, 384 + D).
 #include "block_queue.cuh"
 #include "row_terms.cuh"
@@ -14,16 +18,19 @@ namespace sntl {
 using namespace ptx;
 namespace {
 
-constexpr int kT = 128, kThreads = 384, kSumThreads = 256, kChunkBytes = kT * 128;
+constexpr int kT = 128, kSumThreads = 512, kLoadWarp = 16, kIssueWarp = 17, kThreads = 576, kChunkBytes = kT * 128;
 constexpr uint32_t kColS = 0, kColDp = 128, kColDs = 256, kColDq = 384;
 
 struct Bars {
-    BlockQueue<10> queue;
-    uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], scores_full, scores_free, ds_full[2], dq_done[2];
+    BlockQueue<18> queue;
+    uint64_t q_full[2], q_free[2], k_full[4], k_free[4], v_full[4], v_free[4], scores_full, scores_free, ds_full[2], dq_done[2];
     uint32_t tmem_base, abort_flag;
 };
 template <int D> struct Smem {
-    static constexpr int kTile = kT * D * 2, q = 0, dout = kTile, k = 2 * kTile, v = 4 * kTile, bars = 6 * kTile;
+    // A K tile is read last by its tile's dQ product, so the loop from its release over the next load, scores and sums to the next
+    // release spans as many tiles as there are stages: two are too few.
+    static constexpr int kKStages = D == 64 ? 4 : 3, kVStages = D == 64 ? 4 : 2, kQStages = D == 64 ? 2 : 1;
+    static constexpr int kTile = kT * D * 2, q = 0, dout = kQStages * kTile, k = 2 * kQStages * kTile, v = k + kKStages * kTile, bars = v + kVStages * kTile;
     static constexpr int bytes = bars + (int)sizeof(Bars) + 1024;
 };
 static_assert(Smem<128>::bytes <= 227 * 1024, "");
@@ -71,13 +78,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         bars->queue.init();
-        mbar_init(&bars->q_full, 1);
-        mbar_init(&bars->q_free, 1);
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             mbar_init(&bars->k_full[i], 1);
             mbar_init(&bars->k_free[i], 1);
             mbar_init(&bars->v_full[i], 1);
             mbar_init(&bars->v_free[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->q_full[i], 1);
+            mbar_init(&bars->q_free[i], 1);
             mbar_init(&bars->ds_full[i], kSumThreads);
             mbar_init(&bars->dq_done[i], 1);
         }
@@ -86,7 +95,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         bars->abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 9) {
+    if (warp == kIssueWarp) {
         tmem_alloc(&bars->tmem_base, 512);
         tmem_relinquish();
     }
@@ -99,8 +108,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     // Counters of key tiles run on over the blocks: c for this block's tile.
     const AttnShape& s = p.s;
-    if (warp < 8) {
-        const int half = warp >> 2, r = (warp & 3) * 32 + lane;
+    if (warp < kLoadWarp) {
+        const int quarter = warp >> 2, r = (warp & 3) * 32 + lane;
         const uint32_t lanes = tmem + ((uint32_t)(warp & 3) << 21);
         const float2 scale2 = make_float2(s.scale * 1.4426950408889634f, s.scale * 1.4426950408889634f);
         int c = 0;
@@ -124,20 +133,18 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int k0 = w.tile(s, 0); k0 < w.n_keys; k0 = w.tile(s, k0 + kT), ++c) {
                 if (!(ok = mbar_wait_warp(&bars->scores_full, c & 1, abort_flag, 0x61))) break;
                 tc_fence_after();
-                uint32_t x[64], y[64];
-                tmem_ld32(lanes + kColS + half * 64, x);
-                tmem_ld32(lanes + kColS + half * 64 + 32, x + 32);
-                tmem_ld32(lanes + kColDp + half * 64, y);
-                tmem_ld32(lanes + kColDp + half * 64 + 32, y + 32);
+                uint32_t x[32], y[32];
+                tmem_ld32(lanes + kColS + quarter * 32, x);
+                tmem_ld32(lanes + kColDp + quarter * 32, y);
                 tmem_ld_wait();
                 tc_fence_before();
                 mbar_arrive(&bars->scores_free);
-                // every pair of the tile is visible, or a mask per 32 keys
+                // every pair of the tile is visible, or a mask
                 const bool cut = k0 + kT > (s.causal ? w.qt * kT + 1 : s.Skv) || s.window > 0;
-                uint32_t ds[32];
+                uint32_t ds[16];
                 auto weights = [&](auto&& seen) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
+                    for (int i = 0; i < 16; ++i) {
                         const float2 e = ffma2(make_float2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), scale2, make_float2(lse, lse));
                         float2 w2 = make_float2(seen(2 * i) ? ex2(e.x) : 0.f, seen(2 * i + 1) ? ex2(e.y) : 0.f);
                         if constexpr (D == 64) {      // as the P that dV and dK are made of, whose dS is rounded three times there
@@ -151,13 +158,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!cut) {
                     weights([](int) { return true; });
                 } else {
-                    const uint32_t seen0 = keys_seen(s, row, n_row, k0 + half * 64), seen1 = keys_seen(s, row, n_row, k0 + half * 64 + 32);
-                    weights([&](int i) { return ((i < 32 ? seen0 : seen1) >> (i & 31) & 1u) != 0; });
+                    const uint32_t mask = keys_seen(s, row, n_row, k0 + quarter * 32);
+                    weights([&](int i) { return (mask >> i & 1u) != 0; });
                 }
                 // (the buffer is free once the product before last has read it)
                 if (c >= 2 && !(ok = mbar_wait_warp(&bars->dq_done[c & 1], ((c >> 1) - 1) & 1, abort_flag, 0x62))) break;
                 tc_fence_after();
-                tmem_st32(lanes + kColDs + (c & 1) * 64 + half * 32, ds);
+                tmem_st16(lanes + kColDs + (c & 1) * 64 + quarter * 16, ds);
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&bars->ds_full[c & 1]);
@@ -166,19 +173,20 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_fence_after();
 #pragma unroll
             for (int i = 0; i < D / 64; ++i) {
-                const int d0 = half * (D / 2) + i * 32;
-                uint32_t x[32];
-                tmem_ld32(lanes + kColDq + d0, x);
+                const int d0 = quarter * (D / 4) + i * 16;
+                uint32_t x[16];
+                tmem_ld8(lanes + kColDq + d0, x);
+                tmem_ld8(lanes + kColDq + d0 + 8, x + 8);
                 tmem_ld_wait();
                 if (row >= s.Sq) continue;
                 if constexpr (kMat) {
                     float* dst = p.dq_mat + ((long long)w.h * D + d0) * p.mat_stride + (long long)w.b * s.Sq + row;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) dst[j * p.mat_stride] = __uint_as_float(x[j]) * s.scale;
+                    for (int j = 0; j < 16; ++j) dst[j * p.mat_stride] = __uint_as_float(x[j]) * s.scale;
                 } else {
                     uint4* dst = reinterpret_cast<uint4*>(p.dq + ((size_t)w.bh * s.Sq + row) * D + d0);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < 2; ++j) {
                         uint32_t v[4];
 #pragma unroll
                         for (int e = 0; e < 4; ++e)
@@ -189,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_before();
         }
-    } else if (warp == 8) {
+    } else if (warp == kLoadWarp) {
         int c = 0;
         for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
             const Block w(p, block);
@@ -198,21 +206,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                 auto load = [&](int dst, const CUtensorMap* map, uint64_t* bar, int row, int slab) {
                     for (int i = 0; i < kChunks; ++i) tma_load_3d(smem + dst + i * kChunkBytes, map, bar, i * 64, row, slab);
                 };
-                // Q and dO once the last scores of the block before have been computed
-                ok = u == 0 || mbar_wait(&bars->q_free, (u - 1) & 1, abort_flag, 0x64);
+                // Q and dO once the last scores of the block before (head_dim 64: of the one before that) have been computed
+                const int sq = u % L::kQStages;
+                ok = u < L::kQStages || mbar_wait(&bars->q_free[sq], (u / L::kQStages - 1) & 1, abort_flag, 0x64);
                 if (ok) {
-                    mbar_arrive_expect_tx(&bars->q_full, 2 * L::kTile);
-                    load(L::q, &tmap_q, &bars->q_full, w.qt * kT, w.bh);
-                    load(L::dout, &tmap_do, &bars->q_full, w.qt * kT, w.bh);
+                    mbar_arrive_expect_tx(&bars->q_full[sq], 2 * L::kTile);
+                    load(L::q + sq * L::kTile, &tmap_q, &bars->q_full[sq], w.qt * kT, w.bh);
+                    load(L::dout + sq * L::kTile, &tmap_do, &bars->q_full[sq], w.qt * kT, w.bh);
                 }
                 for (int k0 = w.tile(s, 0); ok && k0 < w.n_keys; ++c) {
-                    const int st = c & 1, next = w.tile(s, k0 + kT);
-                    if (c >= 2 && !(ok = mbar_wait(&bars->k_free[st], ((c >> 1) - 1) & 1, abort_flag, 0x65))) break;
-                    mbar_arrive_expect_tx(&bars->k_full[st], L::kTile);
-                    load(L::k + st * L::kTile, &tmap_k, &bars->k_full[st], k0, w.bh_kv);
-                    if (c >= 2 && !(ok = mbar_wait(&bars->v_free[st], ((c >> 1) - 1) & 1, abort_flag, 0x66))) break;
-                    mbar_arrive_expect_tx(&bars->v_full[st], L::kTile);
-                    load(L::v + st * L::kTile, &tmap_v, &bars->v_full[st], k0, w.bh_kv);
+                    const int sk = c % L::kKStages, sv = c % L::kVStages, next = w.tile(s, k0 + kT);
+                    if (c >= L::kKStages && !(ok = mbar_wait(&bars->k_free[sk], (c / L::kKStages - 1) & 1, abort_flag, 0x65))) break;
+                    mbar_arrive_expect_tx(&bars->k_full[sk], L::kTile);
+                    load(L::k + sk * L::kTile, &tmap_k, &bars->k_full[sk], k0, w.bh_kv);
+                    if (c >= L::kVStages && !(ok = mbar_wait(&bars->v_free[sv], (c / L::kVStages - 1) & 1, abort_flag, 0x66))) break;
+                    mbar_arrive_expect_tx(&bars->v_full[sv], L::kTile);
+                    load(L::v + sv * L::kTile, &tmap_v, &bars->v_full[sv], k0, w.bh_kv);
                     k0 = next;
                 }
                 if (ok) ok = bars->queue.ask(u + 1, abort_flag);
@@ -220,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             c = warp_uniform(c);
             if (!__all_sync(0xffffffffu, ok)) break;
         }
-    } else if (warp == 9) {
+    } else if (warp == kIssueWarp) {
         constexpr uint32_t idesc_s = make_idesc(kT, kT, false, false), idesc_dq = make_idesc(kT, D, false, true);
         const uint64_t q = make_sdesc(smem_u32(smem + L::q), 16, 1024), dout = make_sdesc(smem_u32(smem + L::dout), 16, 1024);
         const uint64_t k = make_sdesc(smem_u32(smem + L::k), 16, 1024), v = make_sdesc(smem_u32(smem + L::v), 16, 1024);
@@ -231,35 +240,36 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int i = 0; i < kChunks; ++i) mma_ss_4<2, 2>(d, sdesc_advance(a, i * kChunkBytes), sdesc_advance(b, i * kChunkBytes), idesc_s, i > 0);
         };
         // scores of tile number n, `last` of its block
-        auto scores = [&](int n, bool last) {
-            const int st = n & 1;
-            if (!wait(&bars->k_full[st], n >> 1, 0x67) || !wait(&bars->v_full[st], n >> 1, 0x68)) return false;
+        auto scores = [&](int n, int sq, bool last) {
+            const int sk = n % L::kKStages, sv = n % L::kVStages;
+            if (!wait(&bars->k_full[sk], n / L::kKStages, 0x67) || !wait(&bars->v_full[sv], n / L::kVStages, 0x68)) return false;
             if (n > 0 && !wait(&bars->scores_free, n - 1, 0x69)) return false;
             tc_fence_after();
-            product(tmem + kColS, q, sdesc_advance(k, st * L::kTile));
-            product(tmem + kColDp, dout, sdesc_advance(v, st * L::kTile));
+            product(tmem + kColS, sdesc_advance(q, sq * L::kTile), sdesc_advance(k, sk * L::kTile));
+            product(tmem + kColDp, sdesc_advance(dout, sq * L::kTile), sdesc_advance(v, sv * L::kTile));
             tc_commit_p(&bars->scores_full);
-            tc_commit_p(&bars->v_free[st]);
-            if (last) tc_commit_p(&bars->q_free);
+            tc_commit_p(&bars->v_free[sv]);
+            if (last) tc_commit_p(&bars->q_free[sq]);
             return true;
         };
         int c = 0;
         for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
             const Block w(p, block);
+            const int sq = u % L::kQStages;
             int k0 = w.tile(s, 0);
-            bool ok = wait(&bars->q_full, u, 0x6a) && scores(c, w.tile(s, k0 + kT) >= w.n_keys), accumulate = false;
+            bool ok = wait(&bars->q_full[sq], u / L::kQStages, 0x6a) && scores(c, sq, w.tile(s, k0 + kT) >= w.n_keys), accumulate = false;
             for (; ok && k0 < w.n_keys; ++c) {
-                const int st = c & 1;
+                const int st = c & 1, sk = c % L::kKStages;
                 k0 = w.tile(s, k0 + kT);
-                if (k0 < w.n_keys && !(ok = scores(c + 1, w.tile(s, k0 + kT) >= w.n_keys))) break;
+                if (k0 < w.n_keys && !(ok = scores(c + 1, sq, w.tile(s, k0 + kT) >= w.n_keys))) break;
                 if (!(ok = wait(&bars->ds_full[st], c >> 1, 0x6b))) break;
                 tc_fence_after();
                 const uint32_t ds = tmem + kColDs + st * 64;
-                const uint64_t b = sdesc_advance(k_mn, st * L::kTile);
+                const uint64_t b = sdesc_advance(k_mn, sk * L::kTile);
                 mma_ts_4<8, 128>(tmem + kColDq, ds, b, idesc_dq, accumulate);
                 mma_ts_4<8, 128>(tmem + kColDq, ds + 32, sdesc_advance(b, 4 * 2048), idesc_dq, 1);
                 tc_commit_p(&bars->dq_done[st]);
-                tc_commit_p(&bars->k_free[st]);
+                tc_commit_p(&bars->k_free[sk]);
                 accumulate = true;
             }
             if (!ok) break;
@@ -270,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == kIssueWarp) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }

@@ -1,0 +1,86 @@
+"""dQ of the deterministic backward (csrc/attn_dq_sm100.cu): one owner per element, so its bits depend on the block's own rows and keys
+alone.  Bounds as for the other tensor-core kernels (bf16 operands, dS rounded to bf16): 2e-2 absolute, 5e-3 relative L2."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import max_abs, rel_l2
+
+pytestmark = pytest.mark.gpu
+DETERMINISTIC = 4
+
+
+@pytest.fixture(scope="module")
+def sb():
+    import sentinel_b200
+    sentinel_b200._lib.load()
+    assert torch.cuda.is_available()
+    return sentinel_b200
+
+
+def _inputs(B, Hq, Hkv, S, D, Skv=None):
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    make = lambda H, n, std: (torch.randn(B, H, n, D, generator=g, device="cuda") * std).to(torch.bfloat16)
+    return make(Hq, S, 0.5), make(Hkv, Skv or S, 0.5), make(Hkv, Skv or S, 1.0), make(Hq, S, 1.0)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,S,Skv,window,global_tokens,causal", [
+    (1, 2, 1, 1, 1, 0, 0, True),
+    (1, 2, 2, 128, 128, 0, 0, True),          # exactly one tile
+    (2, 6, 2, 129, 129, 0, 0, True),          # one row and one key more
+    (1, 4, 1, 1100, 1100, 0, 0, True),        # more tiles than stages
+    (7, 24, 8, 200, 200, 0, 0, True),         # more blocks than SMs: blocks taken over
+    (1, 2, 1, 700, 700, 130, 5, True),        # window edges inside tiles, global tokens
+    (1, 2, 1, 900, 900, 64, 260, True),       # tiles skipped between the global tokens and the window
+    (2, 4, 2, 150, 1000, 0, 0, False),        # rectangular, a ragged last key tile
+])
+def test_dq_against_the_oracle(sb, oracle, B, Hq, Hkv, S, Skv, window, global_tokens, causal, D):
+    q, k, v, do = _inputs(B, Hq, Hkv, S, D, Skv)
+    kw = dict(window=window, global_tokens=global_tokens, causal=causal)
+    o, lse = sb.attention_forward(q, k, v, **kw)
+    got = sb.attention_backward(q, k, v, o, lse, do, flags=DETERMINISTIC, **kw)
+    assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+    a = [t.float().cpu().numpy() for t in (q, k, v, do)]
+    want = oracle.attn_bwd(*a, **kw)[:3]
+    for x, w, name in zip(got, want, ("dq", "dk", "dv")):
+        x = x.float().cpu().numpy()
+        assert np.isfinite(x).all() and max_abs(x, w) <= 2e-2 * max(1.0, float(np.abs(w).max())), (name, max_abs(x, w))
+        if float(np.abs(w).max()) > 1e-6:
+            assert rel_l2(x, w) <= 5e-3, (name, rel_l2(x, w))
+    # a part of the call gives the bits of the whole
+    last = [t[B - 1:].contiguous() for t in (q, k, v, o, lse, do)]
+    part = sb.attention_backward(*last, flags=DETERMINISTIC, **kw)
+    assert torch.equal(part[0], got[0][B - 1:])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_dq_as_a_matrix_is_the_same(sb, D):
+    """Feature-major fp32 matrices with bf16 operands allowed, against the token-major call on the rounded operands."""
+    from sentinel_b200.flash_attention import CudaFlashAttention as F
+    from sentinel_b200 import _lib
+    B, H, S = 3, 4, 200
+    q, k, v, do = _inputs(B, H, H, S, D)
+    mats = [t.float().permute(1, 3, 0, 2).reshape(H * D, B * S).contiguous() for t in (q, k, v, do)]
+    out = [torch.zeros(H * D, B * S, device="cuda") for _ in range(4)]
+    lse = torch.zeros(H, B * S, device="cuda")
+    shape = (H, D, D ** -0.5, True, 0, S, B)
+    old = F.allow_reduced_precision
+    F.allow_reduced_precision = True
+    try:
+        F.forwardMultiHead(*mats[:3], out[0], lse, *shape)
+        d = F._desc(mats[0], mats[1], H, D, D ** -0.5, True, 0, S, B)
+        d.flags |= _lib.FLAG_DETERMINISTIC
+        import ctypes as C
+        lib = _lib.load()
+        ws = torch.empty(lib.sntl_attn_bwd_workspace_bytes(C.byref(d)), dtype=torch.uint8, device="cuda")
+        rc = lib.sntl_attn_bwd(C.byref(d), *(t.data_ptr() for t in mats[:3]), out[0].data_ptr(), lse.data_ptr(), mats[3].data_ptr(),
+                               *(t.data_ptr() for t in out[1:]), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    finally:
+        F.allow_reduced_precision = old
+    assert rc == 0 and sb.poll_device_status() == 0
+    back = lambda m: m.reshape(H, D, B, S).permute(2, 0, 3, 1)
+    o = back(out[0]).contiguous()
+    ref = sb.attention_backward(q, k, v, o.to(torch.bfloat16), lse.reshape(H, B, S).permute(1, 0, 2).contiguous(), do, flags=DETERMINISTIC)
+    # delta from O in fp32 there, from O rounded to bf16 here: as far apart as the rounding of O
+    assert rel_l2(back(out[1]).cpu().numpy(), ref[0].float().cpu().numpy()) <= 5e-3

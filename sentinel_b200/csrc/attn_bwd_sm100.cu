@@ -1182,6 +1182,16 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
             cudaSuccess)
             return e;
     }
+    // dQ before dK and dV, which may lie where K and V lie; and where dQ lies on an input itself, it waits in the unused accumulator
+    [[maybe_unused]] const size_t q_bytes = 2 * (size_t)s.B * s.Hq * s.Sq * D, kv_bytes = 2 * (size_t)s.B * s.Hkv * s.Skv * D;
+    [[maybe_unused]] bool apart = true;
+    if constexpr (kDet) {
+        auto clear_of = [&](const void* x, size_t bytes) { return (uintptr_t)x + bytes <= (uintptr_t)a.dq || (uintptr_t)a.dq + q_bytes <= (uintptr_t)x; };
+        apart = kMat || (clear_of(a.q, q_bytes) && clear_of(a.dout, q_bytes) && clear_of(a.k, kv_bytes) && clear_of(a.v, kv_bytes));
+        TcArgs b = a;
+        if (!apart) b.dq = reinterpret_cast<__nv_bfloat16*>(a.dq_accum);
+        if ((e = tc_backward_dq(b, st)) != cudaSuccess) return e;
+    }
     if (phases & kBwdMain) {
     CUtensorMap tq, tk, tv, tdo;
     if ((e = encode_tmap_bf16_3d(&tq, a.q, D, s.Sq, s.B * s.Hq, 128)) != cudaSuccess) return e;
@@ -1244,7 +1254,7 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     }   // kBwdMain
     if (!(phases & kBwdPost)) return cudaSuccess;
     const unsigned tiles = (unsigned)((long long)s.B * s.Hq * n_qt);
-    if constexpr (kDet) return tc_backward_dq(a, st);
+    if constexpr (kDet) return apart ? cudaSuccess : cudaMemcpyAsync(a.dq, a.dq_accum, q_bytes, cudaMemcpyDeviceToDevice, st);
     if constexpr (kMat)
         return launch_kernel(bwd_post_matrix_kernel<D>, tiles, 256, 0, st, 1, a.dq_accum, a.mat.dq, a.mat.stride, s.Hq, s.Sq, n_qt, s.scale);
     else

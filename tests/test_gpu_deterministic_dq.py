@@ -54,6 +54,22 @@ def test_dq_against_the_oracle(sb, oracle, B, Hq, Hkv, S, Skv, window, global_to
     assert torch.equal(part[0], got[0][B - 1:])
 
 
+@pytest.mark.parametrize("flags", [0, DETERMINISTIC])
+@pytest.mark.parametrize("D", [64, 128])
+def test_gradients_in_the_place_of_the_operands(sb, D, flags):
+    """dQ, dK and dV may lie where Q (or dO), K and V lie."""
+    q, k, v, do = _inputs(2, 4, 4, 300, D)
+    o, lse = sb.attention_forward(q, k, v)
+    want = sb.attention_backward(q, k, v, o, lse, do, flags=flags)
+    for outs in (lambda q, k, v, do: (q, k, v), lambda q, k, v, do: (do, k, v), lambda q, k, v, do: (torch.empty_like(q), k, v)):
+        c = [t.clone() for t in (q, k, v, do)]
+        dq, dk, dv = outs(*c)
+        got = sb.attention_backward(*c[:3], o, lse, c[3], flags=flags, dq=dq, dk=dk, dv=dv)
+        assert got[0].data_ptr() == dq.data_ptr()
+        for x, w in zip(got, want):
+            assert torch.equal(x, w) if flags or x is not got[0] else rel_l2(x.float().cpu().numpy(), w.float().cpu().numpy()) <= 1e-3
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_dq_as_a_matrix_is_the_same(sb, D):
     """Feature-major fp32 matrices with bf16 operands allowed, against the token-major call on the rounded operands."""

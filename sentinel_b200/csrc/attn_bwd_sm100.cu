@@ -35,6 +35,8 @@
 //
 // Long key tiles are cut into pieces (BwdCut): one CTA per (key tile, KV head, piece), each leaving its dK/dV as an fp32
 // partial in scratch, and a small kernel adds the partials in piece order (deterministic) and writes the result.
+//
+// Under SNTL_FLAG_DETERMINISTIC (kDet) this kernel leaves dQ out and attn_dq_sm100.cu computes it.
 // TMEM map (512 columns): S^T/P^T [0,128)  dP^T/dQ [128,256)  then dV [256,384) dK [384,512) at head_dim 128, and
 // dV [256,320) dK [320,384) plus a second S^T/P^T buffer [384,512) at head_dim 64.
 #include "common.cuh"
@@ -130,8 +132,9 @@ BwdCut bwd_cut_uncached(const AttnShape& s)
     BwdCut cut;
     if (s.whole_tiles) return cut;
     if (s.deterministic) {
-        // Steps take longer here (twice the bytes of dQ) and a piece costs about four of them, so only a grid that is clearly out of
-        // balance is cut (by the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
+        // Only a grid that is clearly out of balance is cut.  The rule is older than the kernel that dQ has here, and its figures (with
+        // dQ as 64-bit reductions, a piece at about four steps) too; it stays as it is because how a tile is cut decides the last bits
+        // of dK and dV (by the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
         // D128, 100-key window, 4 global tokens), 0.45 194 -> 144 (B3 Hq16 Hkv4 S1237 D128), 0.53 206 -> 165 (B6 Hq14 Hkv2 S1500 D64), 0.57
         // 271 -> 261; but 0.65 134 -> 134, 0.85 101 -> 114, 0.97 421 -> 482 (B8 Hq28 Hkv4 S1024 D128), 1.84 644 -> 714.  How a tile is cut
         // depends on the tile alone: a part of a batch that is cut gives the same bits as the whole.  Two to five pieces.
@@ -1288,7 +1291,7 @@ cudaError_t dispatch_bwd(const TcArgs& a, cudaStream_t st)
 template <int D>
 cudaError_t dispatch_bwd_out(const TcArgs& a, cudaStream_t st)
 {
-    // the accumulate form (backward in pieces) has no window, no fixed-point dQ and no cut key tiles: their fp32 partials
+    // the accumulate form (backward in pieces) has no window, no dQ of its own and no cut key tiles: their fp32 partials
     // would need a second adding pass
     if (a.dk_acc) return launch_bwd<D, false, false, false, false>(a, st);
     return a.mat.dk ? dispatch_bwd<D, true>(a, st) : dispatch_bwd<D, false>(a, st);

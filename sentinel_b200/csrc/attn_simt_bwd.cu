@@ -6,6 +6,9 @@
 // delta = rowsum(dO o O) from the O rows that are read along with dO: 1/64 of a tile's FMAs instead of a launch of its own.
 // Seven products where a backward with dQ reductions needs five, but dQ stays reproducible without scratch.
 //
+// With odd_marks it computes the blocks that the split products on the tensor cores leave (attn_f32_bwd_sm100.cu), and alone the calls
+// that are too small for those, head_dim above 64 and bf16 tensors without a tensor-core kernel.
+//
 // Bound by the fp32 FMA pipes (B8 H12 S512 D64: 424 us against 195 us of packed FMAs at the 112 lanes per clock that they
 // reach in isolation; staging and exponentials are 10 % each, the rest is shared-memory latency at eight warps per SM; 2740 us
 // with one warp per row).  Twice the warps with half the rows each take as long: they load twice as much per FMA.  The dK/dV CTAs come first: they are the longer ones (four products per pair against three,

@@ -2,6 +2,9 @@
 // (same math as sentinel/NeuralNet/Layers/CausalSelfAttention.cpp:232-254, tiled like
 // sentinel/NeuralNet/Cuda/CudaFlashAttention.cu:337-438).
 //
+// With only_odd it computes the blocks that the split products on the tensor cores leave (attn_f32_fwd_sm100.cu), and alone the calls
+// that are too small for those, head_dim above 64 and bf16 tensors without a tensor-core kernel.
+//
 // Bound by the fp32 FMA pipes: 2*D FMAs per visible (query, key) pair.  B8 H12 S512 D64: 125 us, 1000 us with one warp per
 // row.  Small grids (few heads, few
 // new tokens behind a long cache) take smaller query tiles first and then a cluster of up to eight CTAs per query tile, each

@@ -30,7 +30,7 @@ struct AttnShape {
     int causal;
     int window;         // sliding window (keys a query sees counting itself); <= 0: unlimited.  Needs causal.
     int global_tokens;  // the first global_tokens keys stay visible to every later query
-    int deterministic;  // backward: dQ summed in 64-bit fixed point, so the result does not depend on the order of arrival
+    int deterministic;  // backward: dQ with one owner per element (attn_dq_sm100.cu), so the result does not depend on an order of arrival
     int whole_tiles;    // tensor-core backward: never cut key tiles into pieces
 };
 

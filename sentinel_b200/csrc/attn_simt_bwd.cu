@@ -65,7 +65,6 @@ __device__ __forceinline__ void dkv_role(const SimtArgs& a, int tile, float* sme
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, group = s.Hq / s.Hkv;
     const int slabs = s.B * s.Hkv, slab = tile % slabs, b = slab / s.Hkv, hk = slab - b * s.Hkv;
     const int key0 = (tile / slabs) * L::kRows;               // causal: the first key tiles are seen by the most queries
-    if (a.odd_marks && a.odd_marks[key0 / 128 * slabs + slab] == 0) return;
     const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
     const long long kvoff = b * a.vkv.sb + hk * a.vkv.sh;
     stage<T, DP, L::kRows>(smem + L::own0, (const T*)a.k + kvoff, mk, key0);
@@ -141,7 +140,6 @@ __device__ __forceinline__ void dq_role(const SimtArgs& a, int tile, int n_qt, f
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int slabs = s.B * s.Hq, bh = tile % slabs, b = bh / s.Hq, h = bh - b * s.Hq, hk = h / (s.Hq / s.Hkv);
     const int row0 = (n_qt - 1 - tile / slabs) * L::kRows;    // longest query tiles first
-    if (a.odd_marks && a.odd_marks[(s.Skv + 127) / 128 * (s.B * s.Hkv) + row0 / 128 * slabs + bh] == 0) return;
     const Slab mq{a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q}, mk{a.vkv.ss, a.vkv.sd, s.Skv, s.D, a.vec_kv};
     const long long qoff = b * a.vq.sb + h * a.vq.sh;
     const T* kb = (const T*)a.k + b * a.vkv.sb + hk * a.vkv.sh;
@@ -207,6 +205,13 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<TM, DP>) simt_bwd_kernel(co
 {
     extern __shared__ __align__(16) float smem[];
     wait_for_stream();
+    if (a.odd_marks) {      // (here and not in the roles, whose loops it would cost registers: B1 Hq8 Hkv2 S512 D128 461 -> 466 us)
+        const AttnShape& s = a.s;
+        const bool dkv = (int)blockIdx.x < n_dkv;
+        const int slabs = s.B * (dkv ? s.Hkv : s.Hq), tile = dkv ? blockIdx.x : blockIdx.x - n_dkv;
+        const int row0 = (dkv ? tile / slabs : n_qt - 1 - tile / slabs) * 8 * TM, first = dkv ? 0 : (s.Skv + 127) / 128 * (s.B * s.Hkv);
+        if (a.odd_marks[first + row0 / 128 * slabs + tile % slabs] == 0) return;
+    }
     if ((int)blockIdx.x < n_dkv) dkv_role<T, TM, TN, DP>(a, blockIdx.x, smem);
     else dq_role<T, TM, TN, DP>(a, blockIdx.x - n_dkv, n_qt, smem);
 }

@@ -396,7 +396,7 @@ int sntl_attn_bwd(const sntl_attn_desc* d, const void* q, const void* k, const v
         m.o_mat = (const float*)o; m.do_mat = (const float*)dout; m.lse_mat = lse;
         m.row_terms = t.delta;
         m.dq_accum = t.dq_accum;
-        m.accum_bytes = t.s.deterministic ? 0 : 4 * (size_t)d->batch * d->q_heads * sq_pad * d->head_dim;
+        m.accum_bytes = (!t.s.deterministic ? 4 : bwd_dq_has_kernel(d->head_dim) ? 0 : 8) * (size_t)d->batch * d->q_heads * sq_pad * d->head_dim;
         if (stage_matrices(m, d->batch, d->q_heads, d->seq_q, d->head_dim, d->stride_columns, d->column_start, d->scale, st) != cudaSuccess)
             return SNTL_ERR_CUDA;
         t.mat.dq = (float*)dq + d->column_start;

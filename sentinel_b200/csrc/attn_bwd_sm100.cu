@@ -36,7 +36,8 @@
 // Long key tiles are cut into pieces (BwdCut): one CTA per (key tile, KV head, piece), each leaving its dK/dV as an fp32
 // partial in scratch, and a small kernel adds the partials in piece order (deterministic) and writes the result.
 //
-// Under SNTL_FLAG_DETERMINISTIC (kDet) this kernel leaves dQ out and attn_dq_sm100.cu computes it.
+// Under SNTL_FLAG_DETERMINISTIC (kDet) the dQ contributions of the key tiles are summed as 64-bit integers, which no order can change:
+// at head_dim 64 the drain warpgroup pushes them as such; at 128 this kernel leaves dQ out and attn_dq_sm100.cu sums them (kOwnDq).
 // TMEM map (512 columns): S^T/P^T [0,128)  dP^T/dQ [128,256)  then dV [256,384) dK [384,512) at head_dim 128, and
 // dV [256,320) dK [320,384) plus a second S^T/P^T buffer [384,512) at head_dim 64.
 #include "common.cuh"
@@ -132,9 +133,8 @@ BwdCut bwd_cut_uncached(const AttnShape& s)
     BwdCut cut;
     if (s.whole_tiles) return cut;
     if (s.deterministic) {
-        // Only a grid that is clearly out of balance is cut.  The rule is older than the kernel that dQ has here, and its figures (with
-        // dQ as 64-bit reductions, a piece at about four steps) too; it stays as it is because how a tile is cut decides the last bits
-        // of dK and dV (by the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
+        // Steps take longer here (twice the bytes of dQ) and a piece costs about four of them, so only a grid that is clearly out of
+        // balance is cut (by the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
         // D128, 100-key window, 4 global tokens), 0.45 194 -> 144 (B3 Hq16 Hkv4 S1237 D128), 0.53 206 -> 165 (B6 Hq14 Hkv2 S1500 D64), 0.57
         // 271 -> 261; but 0.65 134 -> 134, 0.85 101 -> 114, 0.97 421 -> 482 (B8 Hq28 Hkv4 S1024 D128), 1.84 644 -> 714.  How a tile is cut
         // depends on the tile alone: a part of a batch that is cut gives the same bits as the whole.  Two to five pieces.
@@ -281,26 +281,54 @@ __device__ __forceinline__ uint64_t make_sdesc_plain(uint32_t smem_addr, uint32_
 // one thread that owns the bulk groups.  kStagingBytes of staging in all; `piece` counts pieces over the CTA's lifetime, so
 // that the rotation carries on from tile to tile (a buffer is rewritten only after the kStages - 1 groups issued since
 // its last use are all that may still be reading).
-template <int D, int kStageCols, int kStagingBytes>
+template <int D, bool kDet, int kStageCols, int kStagingBytes>
 __device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile, uint8_t* sStage, int row, bool elected, uint32_t& piece)
 {
     constexpr int kStageBytes = kStageCols * kT * 4;
     constexpr int kStages = kStagingBytes / kStageBytes;
     static_assert(kStages >= 2 && kStages * kStageBytes == kStagingBytes, "staging must hold whole pieces");
+    if constexpr (!kDet) {
 #pragma unroll
-    for (int c = 0; c < D / kStageCols; ++c) {
-        uint8_t* stage = sStage + (piece++ % kStages) * kStageBytes;
-        if (elected) bulk_wait_read<kStages - 1>();
-        named_barrier_sync(1, 128);
+        for (int c = 0; c < D / kStageCols; ++c) {
+            uint8_t* stage = sStage + (piece++ % kStages) * kStageBytes;
+            if (elected) bulk_wait_read<kStages - 1>();
+            named_barrier_sync(1, 128);
 #pragma unroll
-        for (int v = 0; v < kStageCols / 4; ++v)
-            *reinterpret_cast<uint4*>(stage + ((size_t)v * kT + row) * 16) =
-                make_uint4(r[c * kStageCols + 4 * v], r[c * kStageCols + 4 * v + 1], r[c * kStageCols + 4 * v + 2], r[c * kStageCols + 4 * v + 3]);
-        fence_proxy_async_smem();
-        named_barrier_sync(1, 128);
-        if (elected) {
-            bulk_reduce_add_f32(tile + (size_t)c * kStageCols * kT, stage, (uint32_t)kStageBytes);
-            bulk_commit();
+            for (int v = 0; v < kStageCols / 4; ++v)
+                *reinterpret_cast<uint4*>(stage + ((size_t)v * kT + row) * 16) =
+                    make_uint4(r[c * kStageCols + 4 * v], r[c * kStageCols + 4 * v + 1], r[c * kStageCols + 4 * v + 2], r[c * kStageCols + 4 * v + 3]);
+            fence_proxy_async_smem();
+            named_barrier_sync(1, 128);
+            if (elected) {
+                bulk_reduce_add_f32(tile + (size_t)c * kStageCols * kT, stage, (uint32_t)kStageBytes);
+                bulk_commit();
+            }
+        }
+    } else {
+        // Order-independent form: each fp32 value times 2^32 is an integer that fits 64 bits exactly (24-bit
+        // mantissa, |value| < 2^31), and integer addition is associative, so the accumulated sum is the same
+        // whatever order the key tiles arrive in.  Same staging buffers, half as many columns per piece; the
+        // accumulator tile is [d/2][row][2] 64-bit words, so a piece is still one contiguous block.
+        constexpr int kDetCols = kStageCols / 2;
+        unsigned long long* tile64 = reinterpret_cast<unsigned long long*>(tile);
+#pragma unroll
+        for (int c = 0; c < D / kDetCols; ++c) {
+            uint8_t* stage = sStage + (piece++ % kStages) * kStageBytes;
+            if (elected) bulk_wait_read<kStages - 1>();
+            named_barrier_sync(1, 128);
+#pragma unroll
+            for (int v = 0; v < kDetCols / 2; ++v) {
+                const long long a = __float2ll_rn(__uint_as_float(r[c * kDetCols + 2 * v]) * 4294967296.0f);
+                const long long b2 = __float2ll_rn(__uint_as_float(r[c * kDetCols + 2 * v + 1]) * 4294967296.0f);
+                *reinterpret_cast<ulonglong2*>(stage + ((size_t)v * kT + row) * 16) =
+                    make_ulonglong2((unsigned long long)a, (unsigned long long)b2);
+            }
+            fence_proxy_async_smem();
+            named_barrier_sync(1, 128);
+            if (elected) {
+                bulk_reduce_add_u64(tile64 + (size_t)c * kDetCols * kT, stage, (uint32_t)kStageBytes);
+                bulk_commit();
+            }
         }
     }
 }
@@ -423,7 +451,8 @@ __device__ __forceinline__ void write_dkv(const BwdParams& p, bool ok, bool spli
 
 // kSplit: the grid may hold pieces of cut key tiles (a separate instantiation, so that the plain kernel carries none
 // of that bookkeeping)
-// kDet: dQ is left to attn_dq_sm100.cu: no dQ product, nothing to drain
+// kDet: dQ contributions leave as 64-bit fixed point (see the drain warpgroup), or dQ is left to attn_dq_sm100.cu (kOwnDq): no dQ
+// product then, nothing to drain
 // kMat: dK and dV leave as feature-major fp32 matrices (an instantiation of its own: with that store in the common kernel it is
 // 3 % slower at head_dim 128; the accumulate form, in contrast, is better left in: without it the kernel is 3 % slower too)
 template <int D, bool kWin, bool kSplit, bool kDet, bool kMat>
@@ -457,6 +486,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // P^T = exp2(scale*log2e * that) and dS^T = P^T o that.  One column block (8 bf16) per operand is real; the second
     // block of the constant operand is zeros, so the second block of the record operand may alias the first (LBO 0).
     constexpr bool kAug = bwd_folds_row_terms(D);
+    constexpr bool kOwnDq = kDet && bwd_dq_has_kernel(D);
     constexpr int kAugBytes = kT * 16;             // 128 records
     constexpr int kDsBytes = kT * kT * 2;          // dS^T tile: [128 keys][128 queries] bf16 as two 64-query chunks
     // The layout uses every byte of the 227 KB a CTA may have (D = 128), so there is no room for an alignment
@@ -731,8 +761,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 // dP^T of step n, into the columns that dQ of the step before has left
                 auto issue_dp = [&](int n) {
                     const int nd = n % kDoStages;
-                    // (kDet: dP^T of the step before has been read, this warp has seen ds_ready)
-                    if (!kDet && n > 0 && !wait(&bars->dq_drained, (uint32_t)((n - 1) & 1), kSiteDrained)) return false;
+                    // (kOwnDq: dP^T of the step before has been read, this warp has seen ds_ready)
+                    if (!kOwnDq && n > 0 && !wait(&bars->dq_drained, (uint32_t)((n - 1) & 1), kSiteDrained)) return false;
                     SNTL_TRACE_EV(tl14, 4, tn, 5);
                     if (!wait(&bars->do_full[nd], (uint32_t)((n / kDoStages) & 1), kSiteDoFull)) return false;
                     tc_fence_after();
@@ -753,7 +783,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     // dQ first: it gates the drain and with it the next dP^T
                     const uint32_t ds_off = (uint32_t)((n % kDsBufs) * kDsBytes);
                     const uint64_t ds_mn = sdesc_advance(dDs_mn, ds_off);
-                    if constexpr (!kDet) {
+                    if constexpr (!kOwnDq) {
                         mma_ss_4<128, 128>(tm_dP, ds_mn, dK_mn, idesc_dq, 0);
                         mma_ss_4<128, 128>(tm_dP, sdesc_advance(ds_mn, 4 * 2048), sdesc_advance(dK_mn, 4 * 2048), idesc_dq, 1);
                         tc_commit_p(&bars->dq_ready);
@@ -800,10 +830,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const BwdWork w = bars->work[u & 1];
         const int bh0 = w.slab * group;      // b * Hq + hk * group
         int g = w.g_first, tile_r = w.r_first;
-        for (const int end = n + (kDet ? 0 : w.n_iter); n < end; ++n) {
+        for (const int end = n + (kOwnDq ? 0 : w.n_iter); n < end; ++n) {
             const int qt = w.qt_first + tile_r, bh = bh0 + g;
             if (++tile_r == w.per_head) { tile_r = 0; ++g; }
-            float* tile = p.dq_accum + ((size_t)bh * p.n_qt + qt) * (size_t)(kT * D);
+            // fp32 accumulator: kT*D words per tile; fixed-point accumulator: kT*D 64-bit words per tile
+            float* tile = p.dq_accum + ((size_t)bh * p.n_qt + qt) * (size_t)(kT * D) * (kDet ? 2 : 1);
             ok = __all_sync(0xffffffffu, mbar_wait(&bars->dq_ready, (uint32_t)(n & 1), abort_flag, kSiteDQ));
             SNTL_TRACE_EV(tw, 3, tn, 1);
             if (!ok) break;
@@ -823,7 +854,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             tc_fence_before();
             mbar_arrive(&bars->dq_drained);
             SNTL_TRACE_EV(tw, 3, tn, 2);
-            push_dq_tile<D, kStageCols, kStagingBytes>(r, tile, sStage, row, elected, piece);
+            push_dq_tile<D, kDet, kStageCols, kStagingBytes>(r, tile, sStage, row, elected, piece);
             SNTL_TRACE_EV(tw, 3, tn, 3);
         }
         }
@@ -1067,6 +1098,34 @@ __global__ void __launch_bounds__(256, 2) bwd_post_kernel(const float* __restric
     }
 }
 
+// The same for the 64-bit fixed-point accumulator (tiles of [d/2][row][2] words in units of 2^-32): the one rounding
+// of the exact integer sum happens here.
+template <int D>
+__global__ void __launch_bounds__(256) bwd_post_det_kernel(const unsigned long long* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq,
+                                                           int Sq, int n_qt, float scale)
+{
+    wait_for_stream();
+    const size_t t = blockIdx.x, bh = t / n_qt;
+    const int qt = (int)(t - bh * n_qt), row = threadIdx.x & 127, half = threadIdx.x >> 7, s = qt * kT + row;
+    if (s >= Sq) return;
+    const longlong2* src = reinterpret_cast<const longlong2*>(dq_accum + t * (size_t)(kT * D)) + row;
+    __nv_bfloat16* dst = dq + (bh * Sq + s) * D;
+#pragma unroll 2
+    for (int g = half; g < D / 16; g += 2) {
+        longlong2 x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = src[(size_t)(g * 8 + i) * kT];
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            w[i] = pack_bf16((float)((double)x[i].x * (1.0 / 4294967296.0)) * scale, (float)((double)x[i].y * (1.0 / 4294967296.0)) * scale);
+        uint4* out = reinterpret_cast<uint4*>(dst + g * 16);
+        out[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        out[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+
 // How many partials each cut key tile has.
 struct BwdPieces {
     int n_qt, causal, window, global_tokens, group, steps, stride;
@@ -1144,8 +1203,8 @@ __global__ void __launch_bounds__(256) bwd_dkv_reduce_matrix_kernel(const float*
 }
 
 // dQ as an fp32 feature-major matrix = scale * accumulator: four features of one query per thread, consecutive threads on
-// consecutive queries.
-template <int D>
+// consecutive queries, in either form of the accumulator (fp32 [d/4][row][4] or 2^-32 fixed point [d/2][row][2]).
+template <int D, bool kDet>
 __global__ void __launch_bounds__(256) bwd_post_matrix_kernel(const float* __restrict__ dq_accum, float* __restrict__ dq, long long stride, int Hq,
                                                               int Sq, int n_qt, float scale)
 {
@@ -1154,12 +1213,23 @@ __global__ void __launch_bounds__(256) bwd_post_matrix_kernel(const float* __res
     const int bh = (int)(t / n_qt), qt = (int)(t - (size_t)bh * n_qt), b = bh / Hq, h = bh - b * Hq;
     const int row = threadIdx.x & 127, s = qt * kT + row;
     if (s >= Sq) return;
-    const float* src = dq_accum + t * (size_t)(kT * D);
+    const float* src = dq_accum + t * (size_t)(kT * D) * (kDet ? 2 : 1);
     float* dst = dq + (long long)h * D * stride + (long long)b * Sq + s;
 #pragma unroll 4
     for (int c = threadIdx.x >> 7; c < D / 4; c += 2) {
-        const float4 v = *reinterpret_cast<const float4*>(src + ((size_t)c * kT + row) * 4);
-        const float x[4] = {v.x, v.y, v.z, v.w};
+        float x[4];
+        if constexpr (!kDet) {
+            const float4 v = *reinterpret_cast<const float4*>(src + ((size_t)c * kT + row) * 4);
+            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+        } else {
+            const longlong2* w = reinterpret_cast<const longlong2*>(src);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const longlong2 v = w[(size_t)(2 * c + i) * kT + row];
+                x[2 * i] = (float)((double)v.x * (1.0 / 4294967296.0));
+                x[2 * i + 1] = (float)((double)v.y * (1.0 / 4294967296.0));
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) dst[(4 * c + i) * stride] = x[i] * scale;
     }
@@ -1173,7 +1243,7 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     const int Sq_pad = n_qt * kT;
     const long long rows_padded = (long long)s.B * s.Hq * Sq_pad;
     // workspace: [delta records | LSE records] then the accumulator (see tc_backward_workspace_bytes)
-    constexpr bool kAug = bwd_folds_row_terms(D);
+    constexpr bool kAug = bwd_folds_row_terms(D), kOwnDq = kDet && bwd_dq_has_kernel(D);
     const RowTerms terms = row_terms_of(a.delta, rows_padded, D, s.scale);
     cudaError_t e;
     const int phases = a.phases ? a.phases : (kBwdPre | kBwdMain | kBwdPost);
@@ -1181,14 +1251,14 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
         const long long blocks = rows_padded / kPreRows<D>;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
         auto kernel = aligned(16, a.o, a.dout) ? bwd_pre_kernel<D, true> : bwd_pre_kernel<D, false>;
-        if ((e = launch_kernel(kernel, (unsigned)blocks, 256, 0, st, 1, a.o, a.dout, a.lse, terms, a.dq_accum, s.Sq, Sq_pad, kDet ? 0 : D)) !=
+        if ((e = launch_kernel(kernel, (unsigned)blocks, 256, 0, st, 1, a.o, a.dout, a.lse, terms, a.dq_accum, s.Sq, Sq_pad, kOwnDq ? 0 : kDet ? 2 * D : D)) !=
             cudaSuccess)
             return e;
     }
     // dQ before dK and dV, which may lie where K and V lie; and where dQ lies on an input itself, it waits in the unused accumulator
     [[maybe_unused]] const size_t q_bytes = 2 * (size_t)s.B * s.Hq * s.Sq * D, kv_bytes = 2 * (size_t)s.B * s.Hkv * s.Skv * D;
     [[maybe_unused]] bool apart = true;
-    if constexpr (kDet) {
+    if constexpr (kOwnDq) {
         auto clear_of = [&](const void* x, size_t bytes) { return (uintptr_t)x + bytes <= (uintptr_t)a.dq || (uintptr_t)a.dq + q_bytes <= (uintptr_t)x; };
         apart = kMat || (clear_of(a.q, q_bytes) && clear_of(a.dout, q_bytes) && clear_of(a.k, kv_bytes) && clear_of(a.v, kv_bytes));
         TcArgs b = a;
@@ -1257,9 +1327,13 @@ cudaError_t launch_bwd(const TcArgs& a, cudaStream_t st)
     }   // kBwdMain
     if (!(phases & kBwdPost)) return cudaSuccess;
     const unsigned tiles = (unsigned)((long long)s.B * s.Hq * n_qt);
-    if constexpr (kDet) return apart ? cudaSuccess : cudaMemcpyAsync(a.dq, a.dq_accum, q_bytes, cudaMemcpyDeviceToDevice, st);
-    if constexpr (kMat)
-        return launch_kernel(bwd_post_matrix_kernel<D>, tiles, 256, 0, st, 1, a.dq_accum, a.mat.dq, a.mat.stride, s.Hq, s.Sq, n_qt, s.scale);
+    if constexpr (kOwnDq)
+        return apart ? cudaSuccess : cudaMemcpyAsync(a.dq, a.dq_accum, q_bytes, cudaMemcpyDeviceToDevice, st);
+    else if constexpr (kMat)
+        return launch_kernel(bwd_post_matrix_kernel<D, kDet>, tiles, 256, 0, st, 1, a.dq_accum, a.mat.dq, a.mat.stride, s.Hq, s.Sq, n_qt, s.scale);
+    else if constexpr (kDet)
+        return launch_kernel(bwd_post_det_kernel<D>, tiles, 256, 0, st, 1, reinterpret_cast<const unsigned long long*>(a.dq_accum), a.dq, s.Sq,
+                             n_qt, s.scale);
     else
         return launch_kernel(bwd_post_kernel<D>, tiles, 256, 0, st, 1, a.dq_accum, a.dq, s.Sq, n_qt, s.scale);
 }
@@ -1291,7 +1365,7 @@ cudaError_t dispatch_bwd(const TcArgs& a, cudaStream_t st)
 template <int D>
 cudaError_t dispatch_bwd_out(const TcArgs& a, cudaStream_t st)
 {
-    // the accumulate form (backward in pieces) has no window, no dQ of its own and no cut key tiles: their fp32 partials
+    // the accumulate form (backward in pieces) has no window, no fixed-point dQ and no cut key tiles: their fp32 partials
     // would need a second adding pass
     if (a.dk_acc) return launch_bwd<D, false, false, false, false>(a, st);
     return a.mat.dk ? dispatch_bwd<D, true>(a, st) : dispatch_bwd<D, false>(a, st);

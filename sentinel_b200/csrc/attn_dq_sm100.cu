@@ -5,8 +5,7 @@
 // outlasted the five: 128 KB per step at the 25.5 bytes per clock that an SM gets through to L2.
 //
 // Backward, us, against the 64-bit reductions: B3 Hq16 Hkv4 S1237 D128 132 -> 97; B8 Hq28 Hkv4 S1024 D128 412 -> 240; B1 Hq28 Hkv4 S8192
-// D128 1910 -> 1320; B4 Hq32 Hkv8 S4096 D64 1036 -> 970; a 300-key window over B4 Hq12 S4096 D64 161 -> 157 to 165.  At head_dim 64 a tile
-// takes 2000 cycles of this kernel for 1000 of products and 1024 of exponentials: all warps load, compute and store a tile together.
+// D128 1910 -> 1320.  Head_dim 64 stays with the reductions (bwd_dq_has_kernel).
 //
 //   warps 0-15  sums: thread = one query row and a quarter of a tile's 128 keys
 //   warp 16     loads (TMA), warp 17 issues the products
@@ -311,8 +310,7 @@ cudaError_t tc_backward_dq(const TcArgs& a, cudaStream_t st)
 {
     const AttnShape& s = a.s;
     const RowTerms terms = row_terms_of(a.delta, (long long)s.B * s.Hq * ((s.Sq + kT - 1) / kT) * kT, s.D, s.scale);
-    if (a.mat.dq) return s.D == 64 ? launch<64, true>(a, terms, st) : launch<128, true>(a, terms, st);
-    return s.D == 64 ? launch<64, false>(a, terms, st) : launch<128, false>(a, terms, st);
+    return a.mat.dq ? launch<128, true>(a, terms, st) : launch<128, false>(a, terms, st);
 }
 
 cudaError_t read_and_clear_dq_status(uint32_t* word)

@@ -30,7 +30,7 @@ struct AttnShape {
     int causal;
     int window;         // sliding window (keys a query sees counting itself); <= 0: unlimited.  Needs causal.
     int global_tokens;  // the first global_tokens keys stay visible to every later query
-    int deterministic;  // backward: dQ with one owner per element (attn_dq_sm100.cu), so the result does not depend on an order of arrival
+    int deterministic;  // backward: dQ summed in 64-bit fixed point, so the result does not depend on the order of arrival
     int whole_tiles;    // tensor-core backward: never cut key tiles into pieces
 };
 
@@ -192,7 +192,11 @@ size_t tc_cache_workspace_bytes(const AttnShape& s);
 bool tc_cache_supported(const AttnShape& s);
 cudaError_t tc_cache_forward(const TcArgs& a, int capacity, void* workspace, cudaStream_t st);
 cudaError_t tc_backward(const TcArgs& a, cudaStream_t st);
-cudaError_t tc_backward_dq(const TcArgs& a, cudaStream_t st);   // dQ alone, one owner per element (attn_dq_sm100.cu); a.delta holds the row terms
+// Deterministic backward: whether dQ comes from a kernel with one owner per element (attn_dq_sm100.cu); else the main kernel reduces 64-bit
+// words, whose traffic costs less at head_dim 64 than computing S and dP twice (backward, us, reductions against such a kernel: B4 Hq32
+// Hkv8 S4096 1056 against 977 with fewer roundings, B8 H8 S2048 57 against 59, one head of 8192 tokens 88 against 106).
+__host__ __device__ constexpr bool bwd_dq_has_kernel(int D) { return D == 128; }
+cudaError_t tc_backward_dq(const TcArgs& a, cudaStream_t st);   // dQ alone; a.delta holds the row terms
 size_t tc_backward_workspace_bytes(const AttnShape& s);
 // Bytes per padded query row at the head of the tensor-core backward workspace: two 16-byte records (the extra
 // contraction-step operands that carry -delta and -LSE/scale into the dP^T and S^T products)

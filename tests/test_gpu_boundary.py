@@ -120,9 +120,9 @@ def test_bounded_wait_runs_out_reports_and_leaves_the_context_usable(sb):
 
 
 def test_deterministic_flag_makes_dq_bit_reproducible(sb):
-    """SNTL_FLAG_DETERMINISTIC: dQ has one owner per element, so it is bit-identical from run to run, between the
+    """SNTL_FLAG_DETERMINISTIC: dQ is summed in 64-bit fixed point, so it is bit-identical from run to run, between the
     one-stream and two-stream variants and through the chunked host-buffer pipeline -- and it meets the same oracle
-    bounds as the default path."""
+    bounds as the default path (it is the exact sum of the same fp32 contributions, rounded once)."""
     import numpy as np
     from oracle import cpu
     from sentinel_b200 import _lib

@@ -1,5 +1,8 @@
-"""dQ of the deterministic backward (csrc/attn_dq_sm100.cu): one owner per element, so its bits depend on the block's own rows and keys
-alone.  Bounds as for the other tensor-core kernels (bf16 operands, dS rounded to bf16): 2e-2 absolute, 5e-3 relative L2."""
+"""dQ of the deterministic backward: the exact sum of the fp32 contributions of its key tiles (64-bit fixed point), rounded once, so no
+order of arrival and no other row changes its bits.  Bounds against the oracle as for the other tensor-core kernels (bf16 operands, dS
+rounded to bf16): 2e-2 absolute, 5e-3 relative L2."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -100,3 +103,58 @@ def test_dq_as_a_matrix_is_the_same(sb, D):
     ref = sb.attention_backward(q, k, v, o.to(torch.bfloat16), lse.reshape(H, B, S).permute(1, 0, 2).contiguous(), do, flags=DETERMINISTIC)
     # delta from O in fp32 there, from O rounded to bf16 here: as far apart as the rounding of O
     assert rel_l2(back(out[1]).cpu().numpy(), ref[0].float().cpu().numpy()) <= 5e-3
+
+
+def _matrix_backward(sb, q, k, v, do, flags):
+    """dQ of the feature-major call (fp32 matrices, bf16 operands allowed), as [B, H, S, D]: not rounded to bf16 at the end."""
+    from sentinel_b200.flash_attention import CudaFlashAttention as F
+    from sentinel_b200 import _lib
+    B, H, S, D = q.shape
+    mats = [t.float().permute(1, 3, 0, 2).reshape(H * D, B * S).contiguous() for t in (q, k, v, do)]
+    out = [torch.zeros(H * D, B * S, device="cuda") for _ in range(4)]
+    lse = torch.zeros(H, B * S, device="cuda")
+    lib = _lib.load()
+    d = F._desc(mats[0], mats[1], H, D, D ** -0.5, True, 0, S, B)
+    d.flags |= flags | _lib.FLAG_ALLOW_BF16_COMPUTE
+    size = max(lib.sntl_attn_fwd_workspace_bytes(C.byref(d)), lib.sntl_attn_bwd_workspace_bytes(C.byref(d)))
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    p = lambda *ts: [t.data_ptr() for t in ts]
+    assert lib.sntl_attn_fwd(C.byref(d), *p(*mats[:3], out[0], lse, ws), size, stream) == 0
+    assert lib.sntl_attn_bwd(C.byref(d), *p(*mats[:3], out[0], lse, mats[3], *out[1:], ws), size, stream) == 0
+    assert sb.last_path() == "tcgen05_staged" and sb.poll_device_status() == 0
+    return out[1].reshape(H, D, B, S).permute(2, 0, 3, 1)
+
+
+EXACT_SUMS = [64]      # head_dim
+
+
+@pytest.mark.parametrize("D", EXACT_SUMS)
+@pytest.mark.parametrize("B,H,S", [(2, 3, 129), (1, 2, 1000), (3, 4, 200)])
+def test_dq_sums_the_contributions_of_the_call_without_the_flag(sb, B, H, S, D):
+    """The two calls differ by the rounding of fp32 sums of up to 8 contributions: below 8 x 2^-24 of a row's largest partial sum."""
+    q, k, v, do = _inputs(B, H, H, S, D)
+    plain, exact = (_matrix_backward(sb, q, k, v, do, f).cpu().numpy() for f in (0, DETERMINISTIC))
+    assert rel_l2(exact, plain) <= 2e-6
+
+
+@pytest.mark.parametrize("D", EXACT_SUMS)
+@pytest.mark.parametrize("S", [3 * 128, 3 * 128 + 40])
+def test_large_contributions_that_cancel_leave_the_bits_of_the_others(sb, S, D):
+    """Keys 0-127 and 256-383 agree in V and in the first half of their features, are of opposite sign and 2^10 times as large in the second, where Q
+    is zero: their contributions to dQ there cancel exactly, and what the other keys give must come out as if they were zero there."""
+    q, k, v, do = _inputs(1, 2, 2, S, D)
+    q[..., D // 2:] = 0
+    k[:, :, 256:384, :D // 2] = k[:, :, :128, :D // 2]
+    v[:, :, 256:384] = v[:, :, :128]
+    k[:, :, 256:384, D // 2:] = -1024 * k[:, :, :128, D // 2:]
+    k[:, :, :128, D // 2:] *= 1024
+    zeros = k.clone()
+    zeros[:, :, :128, D // 2:] = 0
+    zeros[:, :, 256:384, D // 2:] = 0
+    kw = dict(causal=False)
+    o, lse = sb.attention_forward(q, k, v, **kw)
+    got, want = (sb.attention_backward(q, x, v, o, lse, do, flags=DETERMINISTIC, **kw)[0] for x in (k, zeros))
+    assert sb.poll_device_status() == 0
+    assert float(want[..., D // 2:].float().abs().max()) > 1e-3
+    assert torch.equal(got, want)

@@ -71,11 +71,12 @@ enum {
     /* Backward: make dQ bit-reproducible from run to run.  The tensor-core kernel sums the dQ contributions of the
      * key tiles in global memory in their order of arrival; fp32 addition is not associative, so without this flag
      * the last bits of dQ vary between runs (dK, dV and the forward are always reproducible: each of their elements
-     * has one owner).  With it, at head_dim 64, every contribution is converted exactly to 64-bit fixed point (2^-32
-     * units) and summed as integers, which no order can change; the sum is rounded once at the end, so it is also slightly
-     * more accurate; |dQ / scale| must stay below 2^31.  At head_dim 128 dQ comes from a kernel of its own in which every
-     * element has one owner too.  The scratch holds 8 bytes per element of dQ (sntl_attn_bwd_workspace_bytes accounts for
-     * it).  The reference's
+     * has one owner).  With it every contribution is converted exactly to 64-bit fixed point (2^-32 units) and
+     * summed as integers, which no order can change; the sum is rounded once at the end, so it is also slightly
+     * more accurate; |dQ / scale| must stay below 2^31.  Cost: at head_dim 64 the dQ accumulator in the workspace and its
+     * reduction traffic double; at 128 dQ comes from a kernel of its own, which computes S and dP once more, and the
+     * accumulator is used only where dQ lies on one of the inputs (sntl_attn_bwd_workspace_bytes asks for it at both).  The
+     * reference's
      * head_dim-64 backward has an exclusive dQ store (sentinel/NeuralNet/Cuda/CudaFlashAttention.cu:1434-1455);
      * a caller that relies on bit-stable input gradients sets this flag.  Ignored by the exact kernels, whose
      * dQ is reproducible already. */

@@ -318,6 +318,20 @@ __device__ __forceinline__ void mma_ts_4(uint32_t d_tmem, uint32_t a_tmem, uint6
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(first), "n"(kA), "n"(2 * kA), "n"(3 * kA), "n"(kB), "n"(2 * kB), "n"(3 * kB)
         : "memory");
 }
+// two steps, likewise
+template <int kA, int kB>
+__device__ __forceinline__ void mma_ts_2(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t first)
+{
+    asm volatile(
+        "{\n\t.reg .pred e, f, t;\n\t.reg .b32 a1;\n\t.reg .b64 b1;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.u32 f, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+        "add.u32 a1, %1, %5;\n\tadd.u64 b1, %2, %6;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, f;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(first), "n"(kA), "n"(kB)
+        : "memory");
+}
 // one accumulating step, likewise
 __device__ __forceinline__ void mma_ss_1(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
 {

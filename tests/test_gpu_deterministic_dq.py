@@ -126,35 +126,37 @@ def _matrix_backward(sb, q, k, v, do, flags):
     return out[1].reshape(H, D, B, S).permute(2, 0, 3, 1)
 
 
-EXACT_SUMS = [64]      # head_dim
-
-
-@pytest.mark.parametrize("D", EXACT_SUMS)
-@pytest.mark.parametrize("B,H,S", [(2, 3, 129), (1, 2, 1000), (3, 4, 200)])
-def test_dq_sums_the_contributions_of_the_call_without_the_flag(sb, B, H, S, D):
-    """The two calls differ by the rounding of fp32 sums of up to 8 contributions: below 8 x 2^-24 of a row's largest partial sum."""
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,S,big", [(2, 3, 129, 1), (1, 2, 1000, 1), (3, 4, 200, 1), (2, 3, 300, 3e3)])
+def test_dq_sums_the_contributions_of_the_call_without_the_flag(sb, B, H, S, big, D):
+    """The two calls differ by the rounding of fp32 sums of up to 8 contributions: below 8 x 2^-24 of a row's largest partial sum.  (big: contributions beyond
+    2^13 on both sides of the call's own.)"""
     q, k, v, do = _inputs(B, H, H, S, D)
+    v, do = v * big, do * big
     plain, exact = (_matrix_backward(sb, q, k, v, do, f).cpu().numpy() for f in (0, DETERMINISTIC))
     assert rel_l2(exact, plain) <= 2e-6
 
 
-@pytest.mark.parametrize("D", EXACT_SUMS)
-@pytest.mark.parametrize("S", [3 * 128, 3 * 128 + 40])
-def test_large_contributions_that_cancel_leave_the_bits_of_the_others(sb, S, D):
-    """Keys 0-127 and 256-383 agree in V and in the first half of their features, are of opposite sign and 2^10 times as large in the second, where Q
-    is zero: their contributions to dQ there cancel exactly, and what the other keys give must come out as if they were zero there."""
-    q, k, v, do = _inputs(1, 2, 2, S, D)
-    q[..., D // 2:] = 0
-    k[:, :, 256:384, :D // 2] = k[:, :, :128, :D // 2]
-    v[:, :, 256:384] = v[:, :, :128]
-    k[:, :, 256:384, D // 2:] = -1024 * k[:, :, :128, D // 2:]
-    k[:, :, :128, D // 2:] *= 1024
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S,at,big", [(3 * 128, 2, 1), (3 * 128 + 40, 2, 1), (3 * 128, 2, 1024), (260 * 128 + 40, 258, 1), (260 * 128, 258, 1024)])
+def test_large_contributions_that_cancel_leave_the_bits_of_the_others(sb, S, at, big, D):
+    """The keys of tiles 0 and `at` agree in V and in the first half of their features, are of opposite sign and 2^10 times as large in the second, where Q
+    is zero: their contributions to dQ there cancel exactly, and what the other keys give must come out as if they were zero there.  (More than 256
+    tiles, and with `big` contributions beyond 2^13, are summed in another way on the way.)"""
+    q, k, v, do = _inputs(1, 2, 2, 150, D, S)
+    v, do = v * big, do * big
+    h, a, b = D // 2, slice(0, 128), slice(at * 128, at * 128 + 128)
+    q[..., h:] = 0
+    k[:, :, b, :h] = k[:, :, a, :h]
+    v[:, :, b] = v[:, :, a]
+    k[:, :, b, h:] = -1024 * k[:, :, a, h:]
+    k[:, :, a, h:] *= 1024
     zeros = k.clone()
-    zeros[:, :, :128, D // 2:] = 0
-    zeros[:, :, 256:384, D // 2:] = 0
+    zeros[:, :, a, h:] = 0
+    zeros[:, :, b, h:] = 0
     kw = dict(causal=False)
     o, lse = sb.attention_forward(q, k, v, **kw)
     got, want = (sb.attention_backward(q, x, v, o, lse, do, flags=DETERMINISTIC, **kw)[0] for x in (k, zeros))
     assert sb.poll_device_status() == 0
-    assert float(want[..., D // 2:].float().abs().max()) > 1e-3
+    assert float(want[..., h:].float().abs().max()) > 1e-4
     assert torch.equal(got, want)

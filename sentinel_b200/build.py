@@ -22,7 +22,7 @@ HOST_MODULE = os.path.join(LIB_DIR, "_sntl_host.so")
 HOST_STAMP = os.path.join(LIB_DIR, "_sntl_host.built_for")   # the torch and the Python that the module was built for
 OBJ_DIR = os.path.join(HERE, "build")
 
-SOURCES = ["attn_api.cu", "attn_simt_fwd.cu", "attn_simt_bwd.cu", "attn_simt_decode.cu", "attn_f32_fwd_sm100.cu", "attn_f32_bwd_sm100.cu", "layout_convert.cu", "attn_fwd_sm100.cu", "attn_cache_sm100.cu", "attn_bwd_sm100.cu", "attn_dq_sm100.cu",
+SOURCES = ["attn_api.cu", "attn_simt_fwd.cu", "attn_simt_bwd.cu", "attn_simt_decode.cu", "attn_f32_fwd_sm100.cu", "attn_f32_bwd_sm100.cu", "attn_f32_route.cu", "layout_convert.cu", "attn_fwd_sm100.cu", "attn_cache_sm100.cu", "attn_bwd_sm100.cu", "attn_dq_sm100.cu",
            "sentinel_compat.cu", "attn_bwd_static_scratch.cu", "ring_nccl.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "include"), "-I", CSRC]

@@ -405,7 +405,8 @@ bool f32_tc_backward_supported(const SimtArgs& a, size_t marks_bytes)
 {
     const AttnShape& s = a.s;
     const long long n = blocks(s.Skv, s.B * s.Hkv) + blocks(s.Sq, s.B * s.Hq);
-    return !a.is_bf16 && s.D <= kDim && strides_supported(a) && scale_supported(s.scale) && enough_work(s, kBackwardTiles) && n <= 0x7fffffffLL && (size_t)n * sizeof(uint32_t) <= marks_bytes;
+    return !a.is_bf16 && s.D <= kDim && strides_supported(a) && scale_supported(s.scale) && enough_work(s, kBackwardTiles) && n <= 0x7fffffffLL &&
+           (size_t)n * sizeof(uint32_t) <= marks_bytes && f32_tc_backward_pays(s);
 }
 
 template <bool kVec> static cudaError_t launch(const SimtArgs& a, cudaStream_t st)

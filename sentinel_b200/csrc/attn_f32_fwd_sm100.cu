@@ -322,7 +322,8 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_fwd_kern
 bool f32_tc_forward_supported(const SimtArgs& a)
 {
     const AttnShape& s = a.s;
-    return !a.is_bf16 && s.D <= kDim && strides_supported(a) && scale_supported(s.scale) && enough_work(s, kForwardTiles) && (long long)s.B * s.Hq * ((s.Sq + kOwnRows - 1) / kOwnRows) <= 0x7fffffffLL;
+    return !a.is_bf16 && s.D <= kDim && strides_supported(a) && scale_supported(s.scale) && enough_work(s, kForwardTiles) &&
+           (long long)s.B * s.Hq * ((s.Sq + kOwnRows - 1) / kOwnRows) <= 0x7fffffffLL && f32_tc_forward_pays(s);
 }
 
 template <bool kVec> static cudaError_t launch(const SimtArgs& a, cudaStream_t st)

@@ -220,10 +220,9 @@ struct OddBlocks {
     __device__ __forceinline__ bool get(int u) const { return number[u & 3] == u + 1; }
 };
 
-// Whether the call has the work that the blocks' set-up and their chains of tiles are worth: visible pairs x features, in tiles of 128 x
-// 128 x 64.  Below, the FMA kernels' small tiles and their split of the keys over clusters are faster.  Measured, FMA -> here: forward
-// B4 H8 S128 D64 (16 tiles) 12.1 -> 13.3 us, B2 H2 S512 D64 (32) 22.5 -> 21.5, B4 H8 S256 D32 (32) 16.7 -> 15.1; backward B8 H12 S64
-// D64 (12) 26 -> 29, B4 H8 S128 D64 (16) 25 -> 20, B1 H8 S256 D64 (16) 36 -> 28.
+// A lower bound for what is worth the blocks' set-up: pairs x features, in tiles of 128 x 128 x 64.  Measured, FMA -> here: forward B4 H8 S128
+// D64 (16 tiles) 12.1 -> 13.3 us, B2 H2 S512 D64 (32) 22.5 -> 21.5, B4 H8 S256 D32 (32) 16.7 -> 15.1; backward B8 H12 S64 D64 (12) 26 ->
+// 29, B4 H8 S128 D64 (16) 25 -> 20, B1 H8 S256 D64 (16) 36 -> 28.  Above it the estimates of attn_f32_route.cu decide.
 constexpr int kForwardTiles = 32, kBackwardTiles = 16;
 inline bool enough_work(const AttnShape& s, int tiles)
 {

@@ -230,18 +230,13 @@ cudaError_t launch(const SimtArgs& a, cudaStream_t st)
     return launch_kernel(kernel, (unsigned)(n_dkv + n_dq), kThreads, L::bytes, st, 1, a, (int)n_dkv, n_qt);
 }
 
-// Tile height as in the forward: the largest whose grid still gives every SM its two resident CTAs.
 template <typename T, int DP>
 cudaError_t dispatch(const SimtArgs& a, cudaStream_t st)
 {
     constexpr int TN = DP <= 64 ? 4 : 2, kTop = DP <= 64 ? 8 : 4;
-    auto ctas = [&](int rows) {
-        return ((a.s.Sq + rows - 1) / rows * (long long)a.s.Hq + (a.s.Skv + rows - 1) / rows * (long long)a.s.Hkv) * a.s.B;
-    };
-    const int sms = sm_count();
-    if (kTop == 8 && ctas(64) >= 4 * sms) return launch<T, kTop, TN, DP>(a, st);
-    if (ctas(32) >= 4 * sms) return launch<T, 4, TN, DP>(a, st);
-    return launch<T, 2, TN, DP>(a, st);
+    const int rows = simt_backward_rows(a.s);
+    if (kTop == 8 && rows == 64) return launch<T, kTop, TN, DP>(a, st);
+    return rows == 32 ? launch<T, 4, TN, DP>(a, st) : launch<T, 2, TN, DP>(a, st);
 }
 
 template <typename T>
@@ -256,6 +251,15 @@ cudaError_t dispatch_dim(const SimtArgs& a, cudaStream_t st)
 }
 
 }  // namespace
+
+// Tile height as in the forward: the largest whose grid still gives every SM its two resident CTAs.
+int simt_backward_rows(const AttnShape& s)
+{
+    auto ctas = [&](int rows) { return ((s.Sq + rows - 1) / rows * (long long)s.Hq + (s.Skv + rows - 1) / rows * (long long)s.Hkv) * s.B; };
+    const int sms = sm_count();
+    if (s.D <= 64 && ctas(64) >= 4 * sms) return 64;
+    return ctas(32) >= 4 * sms ? 32 : 16;
+}
 
 cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st)
 {

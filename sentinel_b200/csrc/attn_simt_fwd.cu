@@ -179,22 +179,15 @@ cudaError_t launch(const SimtArgs& a, int n_qt, int n_split, cudaStream_t st)
     return launch_kernel(kernel, (unsigned)ctas, kThreads, smem, st, kSplit ? n_split : 1, a, n_qt, n_split);
 }
 
-// Tile height: 64 rows keep the FMA pipes busiest, but a grid that does not give every SM a CTA or two loses more than the
-// smaller tiles cost.  After the smallest tile, the keys are split as well.
 template <typename T, int DP>
 cudaError_t dispatch(const SimtArgs& a, cudaStream_t st)
 {
     constexpr int TN = DP <= 64 ? 4 : 2, kTop = DP <= 64 ? 8 : 4;
-    const long long slabs = (long long)a.s.B * a.s.Hq;
-    auto tiles = [&](int rows) { return (a.s.Sq + rows - 1) / rows; };
-    const int sms = sm_count();
-    if (kTop == 8 && tiles(64) * slabs >= 2 * sms) return launch<T, kTop, TN, DP, false>(a, tiles(64), 1, st);
-    if (tiles(32) * slabs >= 2 * sms) return launch<T, 4, TN, DP, false>(a, tiles(32), 1, st);
-    const long long ctas = tiles(16) * slabs;
-    const int key_tiles = (a.s.Skv + 16 * TN - 1) / (16 * TN);
-    int split = 1;
-    while (split < 8 && ctas * split * 2 <= 3 * sms && split * 2 <= key_tiles) split *= 2;
-    return split > 1 ? launch<T, 2, TN, DP, true>(a, tiles(16), split, st) : launch<T, 2, TN, DP, false>(a, tiles(16), 1, st);
+    const SimtTiles t = simt_forward_tiles(a.s);
+    const int n_qt = (a.s.Sq + t.rows - 1) / t.rows;
+    if (kTop == 8 && t.rows == 64) return launch<T, kTop, TN, DP, false>(a, n_qt, 1, st);
+    if (t.rows == 32) return launch<T, 4, TN, DP, false>(a, n_qt, 1, st);
+    return t.split > 1 ? launch<T, 2, TN, DP, true>(a, n_qt, t.split, st) : launch<T, 2, TN, DP, false>(a, n_qt, 1, st);
 }
 
 template <typename T>
@@ -209,6 +202,23 @@ cudaError_t dispatch_dim(const SimtArgs& a, cudaStream_t st)
 }
 
 }  // namespace
+
+// Tile height: 64 rows keep the FMA pipes busiest, but a grid that does not give every SM a CTA or two loses more than the
+// smaller tiles cost.  After the smallest tile, the keys are split as well.
+SimtTiles simt_forward_tiles(const AttnShape& s)
+{
+    const bool tall = s.D <= 64;
+    const long long slabs = (long long)s.B * s.Hq;
+    auto tiles = [&](int rows) { return (s.Sq + rows - 1) / rows; };
+    const int sms = sm_count(), keys = tall ? 64 : 32;
+    if (tall && tiles(64) * slabs >= 2 * sms) return SimtTiles{64, 1};
+    if (tiles(32) * slabs >= 2 * sms) return SimtTiles{32, 1};
+    const long long ctas = tiles(16) * slabs;
+    const int key_tiles = (s.Skv + keys - 1) / keys;
+    int split = 1;
+    while (split < 8 && ctas * split * 2 <= 3 * sms && split * 2 <= key_tiles) split *= 2;
+    return SimtTiles{16, split};
+}
 
 cudaError_t simt_forward(const SimtArgs& a, cudaStream_t st)
 {

@@ -150,6 +150,14 @@ cudaError_t simt_decode(const SimtArgs& a, cudaStream_t st);
 cudaError_t simt_backward(const SimtArgs& a, cudaStream_t st);  // one launch
 // The same results from split products on the tensor cores (attn_f32_fwd_sm100.cu, attn_f32_bwd_sm100.cu): fp32, head_dim up to 64, where
 // there is enough work.  They leave odd blocks to simt_forward / simt_backward with the marks.
+// Where that pays by the estimates of attn_f32_route.cu, from the tiles that the FMA kernels would take (head_dim up to 64).
+struct SimtTiles {
+    int rows, split;      // query rows of a tile, CTAs that share its keys
+};
+SimtTiles simt_forward_tiles(const AttnShape& s);
+int simt_backward_rows(const AttnShape& s);
+bool f32_tc_forward_pays(const AttnShape& s);
+bool f32_tc_backward_pays(const AttnShape& s);
 bool f32_tc_forward_supported(const SimtArgs& a);
 cudaError_t f32_tc_forward(const SimtArgs& a, cudaStream_t st);
 bool f32_tc_backward_supported(const SimtArgs& a, size_t marks_bytes);

@@ -153,3 +153,21 @@ def test_inconsistent_lse_is_the_fma_kernels(sb):
         assert torch.equal(x.isfinite(), w.isfinite())
         fin = w.isfinite()
         assert float((x - w)[fin].norm() / w[fin].norm()) <= 2 * REL
+
+
+@pytest.mark.parametrize("Hq,Hkv,T,L,D,window,launches", [
+    (4, 4, 64, 8192, 64, 0, 1),       # 64 tiles of 128 keys in one chain on four SMs (200 us; the FMA kernels over clusters: 85)
+    (1, 1, 1024, 1024, 64, 0, 1),     # 33 / 22
+    (2, 1, 154, 1996, 64, 0, 1),      # 57 / 25
+    (12, 12, 256, 2048, 64, 0, 2),    # 57 / 100
+    (4, 4, 512, 2048, 64, 0, 2),      # 57 / 82
+    (12, 12, 1024, 1024, 32, 16, 1),  # hidden pairs are no work: 15.6 / 14.4
+    (12, 12, 1024, 1024, 32, 256, 2), # 19 / 29
+])
+def test_route_follows_the_chains_and_the_mask(sb, Hq, Hkv, T, L, D, window, launches):
+    """The tensor-core kernel (a second launch looks for its marks) takes a call where its chains of tiles are shorter than the FMA kernels'."""
+    q, k, v, _ = _inputs(19, 1, Hq, Hkv, T, D, L)
+    (o, lse), n = _launches(sb, lambda: sb.attention_cached_forward(q, k, v, L, window=window))
+    assert n == launches and sb.last_path() == "simt_f32" and sb.poll_device_status() == 0
+    for x, y in zip((o, lse), sb.attention_cached_forward(q, k, v, L, window=window, flags=FORCE_SIMT)):
+        assert rel_l2(x.cpu().numpy(), y.cpu().numpy()) <= REL

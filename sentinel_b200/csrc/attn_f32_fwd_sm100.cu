@@ -118,8 +118,10 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_fwd_kern
             const Block w(s, block, n_qt);
             const int row = w.row0 + r, n_row = s.causal ? min(row + w.shift + 1, s.Skv) : s.Skv;
             const int n_first = s.causal ? min(w.row0 + w.shift + 1, s.Skv) : s.Skv;
-            // largest score before scaling; what weights are relative to: that times scale (kHidden: no key seen yet)
-            float top = kHidden, ref = kHidden, l = 0.f, corr = 1.f;
+            // Largest score before scaling (kHidden: no key seen yet).  It is subtracted before scaling: the largest weight is 1 whatever the
+            // size of the scores.  (Subtracted afterwards, with one FMA, it left exp of the rounding error of the scaled score, half a unit in
+            // its last place: infinity or 0 from 2^31 on.)
+            float top = kHidden, l = 0.f, corr = 1.f;
             float2 o[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) o[i] = make_float2(0.f, 0.f);
@@ -164,15 +166,14 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_fwd_kern
                 for (int i = 0; i < 32; ++i) mx[i & 1] = fmax3(mx[i & 1], x[i].x, x[i].y);
                 float other;
                 if (!(ok = other_half(bars, exchange, exchanges++, half, r, fmaxf(mx[0], mx[1]), other))) break;
+                const float before = top;
                 top = fmax3(mx[0], mx[1], other);
-                const bool none = top <= 0.5f * kHidden;
-                const float next_ref = none ? kHidden : top * s.scale, sub = none ? 0.f : -next_ref;
-                const float next_corr = exp_pair(make_float2(ref - next_ref, 0.f)).x;
-                ref = next_ref;
+                const float sub = top <= 0.5f * kHidden ? 0.f : -top;
+                const float next_corr = exp_pair(make_float2((before - top) * s.scale, 0.f)).x;
                 float2 sum[4] = {};
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
-                    x[i] = exp_pair(ffma2(x[i], scale, make_float2(sub, sub)));
+                    x[i] = exp_pair(fmul2(fadd2(x[i], make_float2(sub, sub)), scale));
                     sum[i % 4] = fadd2(sum[i % 4], x[i]);
                 }
                 const float2 all = fadd2(fadd2(sum[0], sum[1]), fadd2(sum[2], sum[3]));
@@ -201,7 +202,7 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_fwd_kern
                 store_row((float*)a.o_out + w.b * a.vq.sb + w.h * a.vq.sh, a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q, row, half * 32, o, l > 0.f ? 1.f / l : 0.f);
             if (half == 0 && row < s.Sq)
                 a.lse_out[w.b * a.vlse.sb + w.h * a.vlse.sh + (long long)row * a.vlse.ss] =
-                    odd ? __uint_as_float(kOddLse) : l > 0.f ? ref + logf(l) : -INFINITY;
+                    odd ? __uint_as_float(kOddLse) : l > 0.f ? fmaf(top, s.scale, logf(l)) : -INFINITY;
         }
     } else if (warp < kIssueWarp) {
         setmaxnreg_dec<other_regs(kSumRegs)>();

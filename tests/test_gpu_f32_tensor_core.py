@@ -171,3 +171,23 @@ def test_route_follows_the_chains_and_the_mask(sb, Hq, Hkv, T, L, D, window, lau
     assert n == launches and sb.last_path() == "simt_f32" and sb.poll_device_status() == 0
     for x, y in zip((o, lse), sb.attention_cached_forward(q, k, v, L, window=window, flags=FORCE_SIMT)):
         assert rel_l2(x.cpu().numpy(), y.cpu().numpy()) <= REL
+
+
+@pytest.mark.parametrize("exponent", [10, 16, 24, 31, 40])
+@pytest.mark.parametrize("D", [32, 48, 64])
+def test_large_scores_of_rows_with_one_key(sb, D, exponent):
+    """Scores around 2^exponent, each row's own far above its others: the weight is 1, not exp of the rounding error of its scaled score (half a unit
+    in the last place of the score; at D 32 and 48, whose scale is no power of two).  O is V and the LSE the score."""
+    B, H, S = 2, 24, 256
+    _, _, v, _ = _inputs(17, B, H, H, S, D)
+    g = torch.Generator(device="cuda").manual_seed(18)
+    rand = lambda *shape: torch.rand(*shape, generator=g, device="cuda")
+    k = torch.where(rand(B, H, S, D) < 0.5, -1.0, 1.0) * (0.9 + 0.2 * rand(B, H, 1, D)) * 2.0 ** (exponent / 2)
+    q = k * (1 + rand(B, H, S, 1)) * D ** -0.5
+    x = torch.einsum("bhqd,bhkd->bhqk", q.double(), k.double()) * float(np.float32(D ** -0.5))
+    own = x.diagonal(dim1=-2, dim2=-1)
+    assert float((own - x.masked_fill(torch.eye(S, device="cuda").bool(), -float("inf")).amax(-1)).min()) > 20
+    (o, lse), launches = _launches(sb, lambda: sb.attention_forward(q, k, v))
+    assert launches == 2 and sb.poll_device_status() == 0
+    for x, w in ((o, v), (lse, own)):
+        assert rel_l2(x.cpu().numpy(), w.cpu().numpy()) <= REL

@@ -141,7 +141,7 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_bwd_kern
         for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
             const Block w(s, block, n_dkv);
             const int row = w.row0 + r;
-            float2 out0[16], out1[16];                             // dK and dV, or dQ; dK and dQ without the factor `scale`
+            float2 out0[16], out1[16];                             // dK and dV, or dQ, times kUp; dK and dQ without the factor `scale`
             uint32_t largest_p = 0;                                // (as bits: also NaN and what should not be negative)
             float largest_ds = 0.f;
 #pragma unroll
@@ -194,7 +194,7 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_bwd_kern
                     }
                 }
                 auto weights = [&](int i, float2 lse, float2 delta) {
-                    p[i] = exp_pair(ffma2(p[i], scale, lse));
+                    p[i] = exp_pair<true>(ffma2(p[i], scale, lse));
                     ds[i] = fmul2(p[i], fadd2(ds[i], delta));
                     largest_p = max(largest_p, max(__float_as_uint(p[i].x), __float_as_uint(p[i].y)));
                     largest_ds = fmax3(largest_ds, fabsf(ds[i].x), fabsf(ds[i].y));
@@ -232,8 +232,8 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_bwd_kern
                 const long long off = w.dkv ? w.b * a.vkv.sb + w.hk * a.vkv.sh : w.b * a.vq.sb + w.h0 * a.vq.sh;
                 const int S = w.dkv ? s.Skv : s.Sq;
                 const bool vec = w.dkv ? a.vec_kv : a.vec_q;
-                store_row((float*)(w.dkv ? a.dk : a.dq) + off, a.vq.ss, a.vq.sd, S, s.D, vec, row, half * 32, out0, s.scale);
-                if (w.dkv) store_row((float*)a.dv + off, a.vq.ss, a.vq.sd, S, s.D, vec, row, half * 32, out1, 1.f);
+                store_row((float*)(w.dkv ? a.dk : a.dq) + off, a.vq.ss, a.vq.sd, S, s.D, vec, row, half * 32, out0, s.scale * kDown);
+                if (w.dkv) store_row((float*)a.dv + off, a.vq.ss, a.vq.sd, S, s.D, vec, row, half * 32, out1, kDown);
             }
         }
     } else if (warp < kIssueWarp) {
@@ -287,7 +287,7 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_bwd_kern
                         const float lse = q < s.Sq ? a.lse[w.b * a.vlse.sb + h * a.vlse.sh + (long long)q * a.vlse.ss] : -INFINITY;
                         float2* dst = n < 0 ? own_terms + (u & 1) * kOwnRows + st * kLoop : terms + st * kLoop;
                         dst[t] = make_float2(lse > -INFINITY && lse < -kHidden ? -lse : kHidden, -delta);
-                        if (!(fabsf(delta) < kLargestWeight)) bars->odd.set(u);
+                        if (!(fabsf(delta) < kLargestDelta)) bars->odd.set(u);
                     }
                 }
                 if (n >= 0) {

@@ -173,7 +173,7 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_fwd_kern
                 float2 sum[4] = {};
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
-                    x[i] = exp_pair(fmul2(fadd2(x[i], make_float2(sub, sub)), scale));
+                    x[i] = exp_pair<true>(fmul2(fadd2(x[i], make_float2(sub, sub)), scale));
                     sum[i % 4] = fadd2(sum[i % 4], x[i]);
                 }
                 const float2 all = fadd2(fadd2(sum[0], sum[1]), fadd2(sum[2], sum[3]));
@@ -202,7 +202,7 @@ template <bool kVec> __global__ void __launch_bounds__(kThreads, 1) f32_fwd_kern
                 store_row((float*)a.o_out + w.b * a.vq.sb + w.h * a.vq.sh, a.vq.ss, a.vq.sd, s.Sq, s.D, a.vec_q, row, half * 32, o, l > 0.f ? 1.f / l : 0.f);
             if (half == 0 && row < s.Sq)
                 a.lse_out[w.b * a.vlse.sb + w.h * a.vlse.sh + (long long)row * a.vlse.ss] =
-                    odd ? __uint_as_float(kOddLse) : l > 0.f ? fmaf(top, s.scale, logf(l)) : -INFINITY;
+                    odd ? __uint_as_float(kOddLse) : l > 0.f ? fmaf(top, s.scale, logf(l * kDown)) : -INFINITY;
         }
     } else if (warp < kIssueWarp) {
         setmaxnreg_dec<other_regs(kSumRegs)>();

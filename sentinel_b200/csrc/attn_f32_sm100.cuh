@@ -30,7 +30,12 @@ constexpr int kSumThreads = 256, kStageThreads = 192, kThreads = 512, kIssueWarp
 // (128 registers a thread at launch.  Nothing in the loops may be spilled: next to the streamed rows local memory does not stay in L1.)
 __host__ __device__ constexpr int other_regs(int sum_regs) { return (kThreads * 128 - kSumThreads * sum_regs) / (kThreads - kSumThreads) / 8 * 8; }
 constexpr float kLargest = 1073741824.0f;                 // 2^30: products of two such, summed, stay far from overflow
-constexpr float kLargestWeight = 1.152921504606847e18f;   // 2^60, for what the kernels compute themselves
+// The kernels compute weights and dS times kUp: parts add up to a value from 2^-110 on (below, the last ones have no room in bf16), and so
+// they do for all of these from 2^-134 on; the results are divided again, which costs no bits.  (Weights below 2^-126, which fp32
+// holds with fewer bits anyway, are 0: ex2.)
+constexpr float kUp = 16777216.0f, kDown = 1.0f / kUp;    // 2^24
+constexpr float kLargestWeight = 7.555786372591432e22f;   // 2^76 = kUp 2^52, for these
+constexpr float kLargestDelta = 1.152921504606847e18f;    // 2^60
 
 // What a thread has seen of the values that it staged.
 struct Check {
@@ -165,12 +170,13 @@ template <bool kVec> struct Fetch {
 // 5e-8 on average for arguments below -1 (2e-8 between -1/2 and 0), which the correction gives back: 4.0e-8 relative (rms), as
 // expf; 6.4e-8 without.  kHidden gives 0.
 constexpr float kHidden = -1e30f;
-__device__ __forceinline__ float2 exp_pair(float2 x)
+template <bool kTimesUp = false> __device__ __forceinline__ float2 exp_pair(float2 x)
 {
     const float2 t = ptx::fmul2(x, make_float2(1.44269504f, 1.44269504f));
     float2 e = ffma2(t, make_float2(-0.693147182f, -0.693147182f), x);
     e = ptx::fadd2(ffma2(t, make_float2(1.90465421e-9f, 1.90465421e-9f), e), make_float2(5e-8f, 5e-8f));
-    const float2 p = make_float2(ptx::ex2(t.x), ptx::ex2(t.y));
+    float2 p = make_float2(ptx::ex2(t.x), ptx::ex2(t.y));
+    if (kTimesUp) p = ptx::fmul2(p, make_float2(kUp, kUp));
     return ffma2(p, e, p);
 }
 

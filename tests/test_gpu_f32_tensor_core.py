@@ -191,3 +191,40 @@ def test_large_scores_of_rows_with_one_key(sb, D, exponent):
     assert launches == 2 and sb.poll_device_status() == 0
     for x, w in ((o, v), (lse, own)):
         assert rel_l2(x.cpu().numpy(), w.cpu().numpy()) <= REL
+
+
+def _exact(q, k, v, do):
+    q, k, v, do = (t.double() for t in (q, k, v, do))
+    scale = float(np.float32(q.shape[-1] ** -0.5))
+    p = torch.softmax(q @ k.transpose(-1, -2) * scale, -1)
+    o = p @ v
+    ds = p * (do @ v.transpose(-1, -2) - (do * o).sum(-1, keepdim=True)) * scale
+    return p, o, ds @ k, ds.transpose(-1, -2) @ q, p.transpose(-1, -2) @ do
+
+
+@pytest.mark.parametrize("D", [48, 64])
+def test_weights_near_the_smallest(sb, D):
+    """A token that every row gives a weight of about 2^-124, whose V is all that is not zero in some features: the parts of such weights have no room
+    in bf16.  Bound: scores of size 86 are known to 2^-23 of it, so their exponentials to 1e-5."""
+    q, k, v, do = _inputs(23, 1, 24, 24, 300, D)
+    q[..., 0], k[..., 0] = 8.0, 0.0
+    k[:, :, 0] = 0.0
+    k[:, :, 0, 0] = -80.0 / 8 * D ** 0.5
+    v[:, :, 1:, :5] = 0.0
+    got, launches = _both(sb, q, k, v, do, causal=False)
+    assert launches == (2, 2)
+    p, o, dq, dk, dv = _exact(q, k, v, do)
+    assert 2.0 ** -126 < float(p[..., 0].min()) and float(p[..., 0].max()) < 2.0 ** -112
+    for x, w in ((got[0][..., :5], o[..., :5]), (got[4][:, :, 0], dv[:, :, 0]), (got[3][:, :, 0], dk[:, :, 0])):
+        assert rel_l2(x.double().cpu().numpy() * 2.0 ** 120, w.cpu().numpy() * 2.0 ** 120) <= 1e-5
+
+
+@pytest.mark.parametrize("D", [48, 64])
+def test_gradients_near_the_smallest(sb, D):
+    """dO around 2^-114, of so few bits that its parts add up to it: dS around 2^-122 and below has to keep its bits."""
+    q, k, v, do = _inputs(29, 1, 24, 24, 300, D)
+    do = (do.sign() * do.abs().clamp(0.25, 4.0)).to(torch.bfloat16).float() * 2.0 ** -114
+    got, launches = _both(sb, q, k, v, do, causal=False)
+    assert launches == (2, 2)
+    for x, w in zip(got[2:], _exact(q, k, v, do)[2:]):
+        assert rel_l2(x.double().cpu().numpy() * 2.0 ** 110, w.cpu().numpy() * 2.0 ** 110) <= 2 * REL

@@ -89,7 +89,8 @@ enum {
     SNTL_FLAG_RING_ZIGZAG = 8,
     /* Backward: the dK and dV of a key tile are summed in one run.  Without it the tensor-core kernel cuts the long key tiles of a
      * small grid into pieces, whose sums are added in a fixed order: reproducible from run to run too, but in the last bits
-     * another sum, so that dK and dV of a sequence can depend on what else is in the call.  With it they do not. */
+     * another sum, so that dK and dV of a sequence can depend on what else is in the call.  With it they do not.  (Exact fp32: the
+     * kernel that a backward call takes depends on its size; with this flag or SNTL_FLAG_DETERMINISTIC on the rows and head_dim alone.) */
     SNTL_FLAG_WHOLE_KEY_TILES = 16
 };
 

@@ -405,8 +405,12 @@ bool f32_tc_backward_supported(const SimtArgs& a, size_t marks_bytes)
 {
     const AttnShape& s = a.s;
     const long long n = blocks(s.Skv, s.B * s.Hkv) + blocks(s.Sq, s.B * s.Hq);
-    return !a.is_bf16 && s.D <= kDim && strides_supported(a) && scale_supported(s.scale) && enough_work(s, kBackwardTiles) && n <= 0x7fffffffLL &&
-           (size_t)n * sizeof(uint32_t) <= marks_bytes && f32_tc_backward_pays(s);
+    if (a.is_bf16 || s.D > kDim || !strides_supported(a) || !scale_supported(s.scale) || n > 0x7fffffffLL || (size_t)n * sizeof(uint32_t) > marks_bytes)
+        return false;
+    // With either flag the bits must not depend on what else is in the call, so the rows alone decide (FMA -> here at the edge: B4 H8 S128 D64
+    // 24 -> 20 us, B1 H8 S256 D32 24 -> 26).
+    if (s.deterministic || s.whole_tiles) return s.Sq >= 64 && (long long)s.Sq * s.D >= 8192;
+    return enough_work(s, kBackwardTiles) && f32_tc_backward_pays(s);
 }
 
 template <bool kVec> static cudaError_t launch(const SimtArgs& a, cudaStream_t st)

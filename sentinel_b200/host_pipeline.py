@@ -71,10 +71,17 @@ def _chunk_slices(B, Hq, Hkv, chunks):
     return out
 
 
+def _exact(q, flags):
+    """Whether the exact kernels compute the call, not those with bf16 tensor-core operands."""
+    bf16 = q.dtype == torch.bfloat16 or bool(flags & _lib.FLAG_ALLOW_BF16_COMPUTE)
+    return not bf16 or bool(flags & _lib.FLAG_FORCE_SIMT) or q.shape[-1] not in (64, 128)
+
+
 def forward_backward_host(q, k, v, dout, *, causal=True, scale=None, flags=0, device="cuda", chunks=None, window=0,
                           global_tokens=0, out=None):
     """Returns host tensors (O, LSE, dQ, dK, dV).  ``chunks`` = number of pipeline chunks (default: up to 8, cut along
-    batch elements first and KV groups second; every chunk is a complete attention problem).
+    batch elements first and KV groups second; every chunk is a complete attention problem).  With FLAG_DETERMINISTIC the results have
+    the bits of one call on everything, for which fp32 tensors (without FLAG_ALLOW_BF16_COMPUTE) are one chunk.
 
     Without ``out`` the five returned tensors are this module's cached pinned staging buffers: they stay valid only
     until the next call (which overwrites them, or drops them when the shape changes) -- copy what must be kept.
@@ -101,6 +108,8 @@ def forward_backward_host(q, k, v, dout, *, causal=True, scale=None, flags=0, de
         with torch.cuda.device(dev):
             if size(C.byref(d)) == size(C.byref(whole)):
                 flags |= _lib.FLAG_WHOLE_KEY_TILES
+        if _exact(q, flags):
+            chunks = 1      # the exact forward chooses its kernel, and how it splits the keys, by the size of the call
     caller = torch.cuda.current_stream(dev)
     up, down, down_g, lanes = buf["up"], buf["down"], buf["down_grads"], buf["compute"]
     for st in (up, down, down_g, *lanes):

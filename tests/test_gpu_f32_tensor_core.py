@@ -228,3 +228,32 @@ def test_gradients_near_the_smallest(sb, D):
     assert launches == (2, 2)
     for x, w in zip(got[2:], _exact(q, k, v, do)[2:]):
         assert rel_l2(x.double().cpu().numpy() * 2.0 ** 110, w.cpu().numpy() * 2.0 ** 110) <= 2 * REL
+<<<<<<< Updated upstream
+=======
+
+
+@pytest.mark.parametrize("flags", [4, 16])       # SNTL_FLAG_DETERMINISTIC, SNTL_FLAG_WHOLE_KEY_TILES
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,window", [(8, 4, 4, 256, 64, 0), (8, 6, 2, 100, 64, 0), (8, 4, 2, 300, 32, 0), (8, 8, 8, 640, 16, 70)])
+def test_gradients_of_a_part_have_the_bits_of_the_whole(sb, flags, B, Hq, Hkv, S, D, window):
+    q, k, v, do = _inputs(31, B, Hq, Hkv, S, D)
+    o, lse = sb.attention_forward(q, k, v, window=window)
+    kw = dict(flags=flags, window=window)
+    whole, n = _launches(sb, lambda: sb.attention_backward(q, k, v, o, lse, do, **kw))
+    assert n == (2 if S * D >= 8192 else 1)
+    for b, h in ((3, slice(0, Hkv)), (5, slice(Hkv - 1, Hkv))):
+        g = slice(h.start * Hq // Hkv, h.stop * Hq // Hkv)
+        part = [t[b:b + 1, g].contiguous() for t in (q, o, lse, do)]
+        kv = [t[b:b + 1, h].contiguous() for t in (k, v)]
+        got = sb.attention_backward(part[0], *kv, *part[1:], **kw)
+        assert all(torch.equal(x, y[b:b + 1, s]) for x, y, s in zip(got, whole, (g, h, h)))
+
+
+@pytest.mark.parametrize("B,H,S,D", [(8, 16, 224, 64), (4, 4, 256, 64), (2, 4, 300, 96)])
+def test_deterministic_host_pipeline_has_the_bits_of_one_call(sb, B, H, S, D):
+    from sentinel_b200.host_pipeline import forward_backward_host
+    q, k, v, do = _inputs(37, B, H, H, S, D)
+    o, lse = sb.attention_forward(q, k, v, flags=4)
+    want = (o, lse) + tuple(sb.attention_backward(q, k, v, o, lse, do, flags=4))
+    got = forward_backward_host(*(t.cpu().pin_memory() for t in (q, k, v, do)), flags=4)
+    assert all(torch.equal(x, y.cpu()) for x, y in zip(got, want))
+>>>>>>> Stashed changes

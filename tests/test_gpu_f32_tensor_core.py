@@ -228,8 +228,6 @@ def test_gradients_near_the_smallest(sb, D):
     assert launches == (2, 2)
     for x, w in zip(got[2:], _exact(q, k, v, do)[2:]):
         assert rel_l2(x.double().cpu().numpy() * 2.0 ** 110, w.cpu().numpy() * 2.0 ** 110) <= 2 * REL
-<<<<<<< Updated upstream
-=======
 
 
 @pytest.mark.parametrize("flags", [4, 16])       # SNTL_FLAG_DETERMINISTIC, SNTL_FLAG_WHOLE_KEY_TILES
@@ -256,4 +254,3 @@ def test_deterministic_host_pipeline_has_the_bits_of_one_call(sb, B, H, S, D):
     want = (o, lse) + tuple(sb.attention_backward(q, k, v, o, lse, do, flags=4))
     got = forward_backward_host(*(t.cpu().pin_memory() for t in (q, k, v, do)), flags=4)
     assert all(torch.equal(x, y.cpu()) for x, y in zip(got, want))
->>>>>>> Stashed changes

@@ -126,8 +126,9 @@ const char* sntl_status_string(int status);
 /* Scratch bytes sntl_attn_fwd needs for this descriptor (0 unless a layout/dtype staging copy is needed). */
 size_t sntl_attn_fwd_workspace_bytes(const sntl_attn_desc* desc);
 
-/* Scratch bytes sntl_attn_bwd needs: delta [B][Hq][Sq] fp32, the fp32 dQ accumulator of the tensor-core
- * kernel, and staging copies when the layout/dtype is converted. */
+/* Scratch bytes sntl_attn_bwd needs.  Tensor-core kernels: 32 bytes per padded query row, the dQ accumulator, the partial sums of cut
+ * key tiles, and staging copies when the layout/dtype is converted.  Exact kernels: a word per query row, of which those with
+ * tensor-core products use one per block of 128 rows. */
 size_t sntl_attn_bwd_workspace_bytes(const sntl_attn_desc* desc);
 
 /* O = softmax(scale * Q K^T + mask) V and LSE = m + ln(sum exp(s - m)) (natural log) per (b, head, query).

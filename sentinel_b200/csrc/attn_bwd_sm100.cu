@@ -135,7 +135,8 @@ BwdCut bwd_cut_uncached(const AttnShape& s)
     if (s.deterministic) {
         // Measured with reductions of 64-bit words at either head size: steps take longer then (twice the bytes of dQ) and a piece costs
         // about four of them, so only a grid that is clearly out of balance is cut.  (At 128, where dQ has a kernel of its own now, the rule
-        // stays because the cut decides the last bits of dK and dV.)  (By the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
+        // stays because the cut decides the last bits of dK and dV; what it cuts still gains: 126 -> 110 for B3 Hq16 Hkv4 S1237, 256 -> 227 for
+        // B6 Hq14 Hkv2 S1500, 145 -> 113 for B2 Hq28 Hkv4 S1024, 867 -> 301 for the windowed call.)  (By the SMs' average load over the longest tile; backward uncut -> cut, us): 0.08 1938 -> 526 (B1 Hq28 Hkv4 S8000
         // D128, 100-key window, 4 global tokens), 0.45 194 -> 144 (B3 Hq16 Hkv4 S1237 D128), 0.53 206 -> 165 (B6 Hq14 Hkv2 S1500 D64), 0.57
         // 271 -> 261; but 0.65 134 -> 134, 0.85 101 -> 114, 0.97 421 -> 482 (B8 Hq28 Hkv4 S1024 D128), 1.84 644 -> 714.  How a tile is cut
         // depends on the tile alone: a part of a batch that is cut gives the same bits as the whole.  Two to five pieces.

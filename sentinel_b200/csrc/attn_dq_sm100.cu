@@ -7,8 +7,9 @@
 //
 // Backward, us, against the 64-bit reductions: B3 Hq16 Hkv4 S1237 D128 133 -> 110; B8 Hq28 Hkv4 S1024 417 -> 259; B1 Hq28 Hkv4 S8192 2140 ->
 // 1575; B1 Hq28 Hkv4 S256 66 -> 42; one head of 2048 tokens 73 -> 64, of 16384 (a chain of 128 tiles on most SMs) 298 -> 320.  (The exact
-// sums cost 12 % of this: with fp32 sums in TMEM, which cut off towards zero, B3 S1237 took 98, B8 S1024 240.)  A tile takes about 2400
-// cycles for 1536 of products, 1024 of exponentials and 1024 of fp32 additions; a block's set-up, Q and dO loads and last sums about 4000.
+// sums cost 12 % of this: with fp32 sums in TMEM, which cut off towards zero, B3 S1237 took 98, B8 S1024 240.)  A tile takes about 2750
+// cycles for 1536 of products, 1024 of exponentials and 1024 of fp32 additions: dP goes where dS was, so from dS of a tile over its dQ
+// product and the next dP to the next dS is one loop.  A block costs about 7500 more (loads of Q and dO, the first scores, the last sums).
 //
 //   warps 0-15   weights: thread = one query row and a quarter of a tile's 128 keys
 //   warps 16-23  sums: thread = one query row and half of the features, 64 integers in registers (128 of its 160)

@@ -2,7 +2,7 @@
 //
 // An fp32 value is the exact sum of three bf16 values, x = h + m + l (8 + 8 + 8 significant bits; each is the rounding of what the
 // ones before leave).  A product of two matrices is taken as six bf16 products over these parts, hh, hm, mh, mm, hl, lh; what is
-// left out is below 2^-26 of a term.  The tensor core adds in fp32 and cuts off below 2^-24 of the largest addend, towards zero, so
+// left out is at most 2^-24 of a term, 2^-27 rms (operands between 1 and 1.03: 2^-26).  The tensor core adds in fp32 and cuts off below 2^-24 of the largest addend, towards zero, so
 //   * the small parts are added first: an accumulator is large only in the last few steps (the hh part);
 //   * every product starts from zero and is at most 128 terms long; longer sums are made of such products in registers, rounded
 //     to nearest.
@@ -27,7 +27,9 @@ constexpr int kOwnRows = 128;            // rows of a block: the TMEM lanes
 constexpr int kFetchRows = 64;           // rows that are staged at a time
 // warps 0-7 sums, 8-13 stage, 14 issues the products, 15 idle; the first two warpgroups take registers from the others
 constexpr int kSumThreads = 256, kStageThreads = 192, kThreads = 512, kIssueWarp = 14;
-// (128 registers a thread at launch.  Nothing in the loops may be spilled: next to the streamed rows local memory does not stay in L1.)
+// (128 registers a thread at launch.  A spill in the staging loop is read from L2: next to the streamed rows local memory does not stay in
+// L1.  The split between the groups is the one that spills least: 28 bytes in the forward, 96 and 100 in the backward; more on either side
+// of it.)
 __host__ __device__ constexpr int other_regs(int sum_regs) { return (kThreads * 128 - kSumThreads * sum_regs) / (kThreads - kSumThreads) / 8 * 8; }
 constexpr float kLargest = 1073741824.0f;                 // 2^30: products of two such, summed, stay far from overflow
 // The kernels compute weights and dS times kUp: parts add up to a value from 2^-110 on (below, the last ones have no room in bf16), and so

@@ -9,7 +9,7 @@
 // With odd_marks it computes the blocks that the split products on the tensor cores leave (attn_f32_bwd_sm100.cu), and alone the calls
 // that are too small for those, head_dim above 64 and bf16 tensors without a tensor-core kernel.
 //
-// Bound by the fp32 FMA pipes (B8 H12 S512 D64: 424 us against 195 us of packed FMAs at the 112 lanes per clock that they
+// Bound by the fp32 FMA pipes (B8 H12 S512 D64: 404 us against 195 us of packed FMAs at the 112 lanes per clock that they
 // reach in isolation; staging and exponentials are 10 % each, the rest is shared-memory latency at eight warps per SM; 2740 us
 // with one warp per row).  Twice the warps with half the rows each take as long: they load twice as much per FMA.  The dK/dV CTAs come first: they are the longer ones (four products per pair against three,
 // times the heads of the group).
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<TM, DP>) simt_bwd_kernel(co
 {
     extern __shared__ __align__(16) float smem[];
     wait_for_stream();
-    if (a.odd_marks) {      // (here and not in the roles, whose loops it would cost registers: B1 Hq8 Hkv2 S512 D128 461 -> 466 us)
+    if (a.odd_marks) {      // (here and not in the roles, whose loops it would cost registers: B1 Hq8 Hkv2 S512 D128 465 us, as without marks, and 470)
         const AttnShape& s = a.s;
         const bool dkv = (int)blockIdx.x < n_dkv;
         const int slabs = s.B * (dkv ? s.Hkv : s.Hq), tile = dkv ? blockIdx.x : blockIdx.x - n_dkv;

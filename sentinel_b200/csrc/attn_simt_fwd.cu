@@ -5,7 +5,7 @@
 // With only_odd it computes the blocks that the split products on the tensor cores leave (attn_f32_fwd_sm100.cu), and alone the calls
 // that are too small for those, head_dim above 64 and bf16 tensors without a tensor-core kernel.
 //
-// Bound by the fp32 FMA pipes: 2*D FMAs per visible (query, key) pair.  B8 H12 S512 D64: 125 us, 1000 us with one warp per
+// Bound by the fp32 FMA pipes: 2*D FMAs per visible (query, key) pair.  B8 H12 S512 D64: 118 us, 1000 us with one warp per
 // row.  Small grids (few heads, few
 // new tokens behind a long cache) take smaller query tiles first and then a cluster of up to eight CTAs per query tile, each
 // with every eighth key tile; their partial (m, l, O) are merged through distributed shared memory, without scratch or a

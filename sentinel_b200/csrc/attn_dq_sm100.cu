@@ -83,9 +83,9 @@ struct Block {
 // be another), infinities and NaN are converted and go to `wide`, which is in local memory; so do the sums of every 256 tiles, before
 // they could leave 32 bits.
 constexpr uint32_t kHighBits = 0x46c00000u, kLowBits = 0x3b400000u;     // 1.5 2^14, 1.5 2^-9
-struct Wide {
+struct Wide {      // (with the rest of a thread's stack below 1 KB, which every context has; more would be allocated by the first launch)
     volatile long long sum[64];
-    volatile uint32_t stage[2][64];      // on the way to the sums: loops over registers would be unrolled, with all their conversions
+    volatile uint32_t stage[64];         // on the way to the sums: loops over registers would be unrolled, with all their conversions
 };
 struct Sums {
     uint32_t high[64], low[64];
@@ -137,33 +137,36 @@ struct Sums {
         for (int i = 0; i < 16; i += 2) {
             float2 t, u;
             split(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), t, u);
-            wide.stage[0][i] = x[i];
-            wide.stage[0][i + 1] = x[i + 1];
+            wide.stage[i] = x[i];
+            wide.stage[i + 1] = x[i + 1];
             high[i0 + i] -= __float_as_uint(t.x) - kHighBits;
             high[i0 + i + 1] -= __float_as_uint(t.y) - kHighBits;
             low[i0 + i] -= __float_as_uint(u.x) - kLowBits;
             low[i0 + i + 1] -= __float_as_uint(u.y) - kLowBits;
         }
 #pragma unroll 1
-        for (int i = 0; i < 16; ++i) wide.sum[i0 + i] = wide.sum[i0 + i] + __float2ll_rn(__uint_as_float(wide.stage[0][i]) * 4294967296.0f);
+        for (int i = 0; i < 16; ++i) wide.sum[i0 + i] = wide.sum[i0 + i] + __float2ll_rn(__uint_as_float(wide.stage[i]) * 4294967296.0f);
+    }
+    // `high` and `low` added to `wide`
+    __device__ __forceinline__ void widen()
+    {
+        use_wide();
+#pragma unroll
+        for (int i = 0; i < 64; ++i) wide.stage[i] = high[i];
+#pragma unroll 1
+        for (int i = 0; i < 64; ++i) wide.sum[i] = wide.sum[i] + (long long)(int)(wide.stage[i] - n * kHighBits) * (1 << 23);
+#pragma unroll
+        for (int i = 0; i < 64; ++i) wide.stage[i] = low[i];
+#pragma unroll 1
+        for (int i = 0; i < 64; ++i) wide.sum[i] = wide.sum[i] + (int)(wide.stage[i] - n * kLowBits);
     }
     // (|high| grows by up to 2^22 per tile, |low| too)
-    __device__ __forceinline__ long long value(uint32_t h, uint32_t l) const
-    {
-        return (long long)(int)(h - n * kHighBits) * (1 << 23) + (int)(l - n * kLowBits);
-    }
     __device__ __forceinline__ void tile_done()
     {
         if (++n < 256) return;
+        widen();
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-            wide.stage[0][i] = high[i];
-            wide.stage[1][i] = low[i];
-            high[i] = low[i] = 0;
-        }
-        use_wide();
-#pragma unroll 1
-        for (int i = 0; i < 64; ++i) wide.sum[i] = wide.sum[i] + value(wide.stage[0][i], wide.stage[1][i]);
+        for (int i = 0; i < 64; ++i) high[i] = low[i] = 0;
         n = 0;
     }
     // scale times the sums, as fp32 in the place of `high`: the integers rounded to fp32, to nearest even.  Usually by one FMA of two that
@@ -194,17 +197,11 @@ struct Sums {
                 high[i + 1] = __float_as_uint(y.y);
             }
         } else {
-            use_wide();
-#pragma unroll
-            for (int i = 0; i < 64; ++i) {
-                wide.stage[0][i] = high[i];
-                wide.stage[1][i] = low[i];
-            }
+            widen();
 #pragma unroll 1
-            for (int i = 0; i < 64; ++i)
-                wide.stage[0][i] = __float_as_uint((float)(double)(wide.sum[i] + value(wide.stage[0][i], wide.stage[1][i])) * 2.3283064365386963e-10f * scale);
+            for (int i = 0; i < 64; ++i) wide.stage[i] = __float_as_uint((float)(double)wide.sum[i] * 2.3283064365386963e-10f * scale);
 #pragma unroll
-            for (int i = 0; i < 64; ++i) high[i] = wide.stage[0][i];
+            for (int i = 0; i < 64; ++i) high[i] = wide.stage[i];
         }
     }
 };

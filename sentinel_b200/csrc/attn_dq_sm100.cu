@@ -5,11 +5,12 @@
 // end.  dQ so has the bits that reductions of 64-bit words give, and no scratch is needed.  Seven products instead of five, against
 // reductions that outlasted the five: 128 KB per step at the 25.5 bytes per clock that an SM gets through to L2.
 //
-// Backward, us, against the 64-bit reductions: B3 Hq16 Hkv4 S1237 D128 133 -> 110; B8 Hq28 Hkv4 S1024 417 -> 259; B1 Hq28 Hkv4 S8192 2140 ->
-// 1575; B1 Hq28 Hkv4 S256 66 -> 42; one head of 2048 tokens 73 -> 64, of 16384 (a chain of 128 tiles on most SMs) 298 -> 320.  (The exact
-// sums cost 12 % of this: with fp32 sums in TMEM, which cut off towards zero, B3 S1237 took 98, B8 S1024 240.)  A tile takes about 2750
-// cycles for 1536 of products, 1024 of exponentials and 1024 of fp32 additions: dP goes where dS was, so from dS of a tile over its dQ
-// product and the next dP to the next dS is one loop.  A block costs about 7500 more (loads of Q and dO, the first scores, the last sums).
+// Backward, us, against the 64-bit reductions: B3 Hq16 Hkv4 S1237 D128 133 -> 110; B8 Hq28 Hkv4 S1024 417 -> 255 (336 and 294 for gradients
+// 10^3 and 10^5 times as large, WideSums); B1 Hq28 Hkv4 S8192 2140 -> 1575; B1 Hq28 Hkv4 S256 66 -> 42; one head of 2048 tokens 73 -> 64, of
+// 16384 (a chain of 128 tiles on most SMs) 298 -> 320.  (The exact sums cost 6 to 13 % of this: with fp32 sums in TMEM, which cut off towards
+// zero, B3 S1237 took 98, B8 S1024 240.)  A tile takes about 2750 cycles for 1536 of products, 1024 of exponentials and 1024 of fp32
+// additions: dP goes where dS was, so from dS of a tile over its dQ product and the next dP to the next dS is one loop.  A block costs
+// about 7500 more (loads of Q and dO, the first scores, the last sums).
 //
 //   warps 0-15   weights: thread = one query row and a quarter of a tile's 128 keys
 //   warps 16-23  sums: thread = one query row and half of the features, 64 integers in registers (128 of its 160)
@@ -79,35 +80,18 @@ struct Block {
 // A thread's sums of 64 elements in units of 2^-32; every contribution is rounded to such a unit to nearest even, as __float2ll_rn(2^32 x)
 // does.  That conversion has the rate of the exponentials and would share their pipe, and 64-bit additions take as long again, so the usual
 // case is done in 32 bits: x + 1.5 2^14 has its last bit at 2^-9, what that leaves of x plus 1.5 2^-9 at 2^-32, and the bits of the two
-// are integers in these units but for constants, which are subtracted at the end.  |x| from 2^13 on (the exponent of the first sum would
-// be another), infinities and NaN are converted and go to `wide`, which is in local memory; so do the sums of every 256 tiles, before
-// they could leave 32 bits.
+// are integers in these units but for constants, which are subtracted at the end.  Once |x| reaches 2^13 (the exponent of the first sum
+// would be another) or is not finite, the warp goes on with conversions and 64-bit sums for the rest of the block (WideSums).
 constexpr uint32_t kHighBits = 0x46c00000u, kLowBits = 0x3b400000u;     // 1.5 2^14, 1.5 2^-9
-struct Wide {      // (with the rest of a thread's stack below 1 KB, which every context has; more would be allocated by the first launch)
-    volatile long long sum[64];
-    volatile uint32_t stage[64];         // on the way to the sums: loops over registers would be unrolled, with all their conversions
-};
+constexpr float kUnit = 2.3283064365386963e-10f;                        // 2^-32
 struct Sums {
     uint32_t high[64], low[64];
-    int n;             // contributions in them
-    bool wide_used;
-    // (a reference, or the other members would be in local memory too)
-    Wide& wide;
+    int n = 0;         // contributions in them
 
-    __device__ __forceinline__ explicit Sums(Wide& w) : wide(w) {}
-    __device__ __forceinline__ void clear()
+    __device__ __forceinline__ Sums()
     {
 #pragma unroll
         for (int i = 0; i < 64; ++i) high[i] = low[i] = 0;
-        n = 0;
-        wide_used = false;
-    }
-    __device__ __forceinline__ void use_wide()
-    {
-        if (wide_used) return;
-#pragma unroll 1
-        for (int i = 0; i < 64; ++i) wide.sum[i] = 0;
-        wide_used = true;
     }
     static __device__ __forceinline__ void split(float2 y, float2& t, float2& u)
     {
@@ -115,95 +99,88 @@ struct Sums {
         t = fadd2(y, h);
         u = fadd2(ffma2(fadd2(t, make_float2(-h.x, -h.y)), make_float2(-1.f, -1.f), y), l);
     }
-    // contributions to the elements from i0 on, and the sum of their squares
-    template <int i0> __device__ __forceinline__ void add(const uint32_t (&x)[16], float2& squares)
+    // contributions to the elements from i0 on, and the sum of their squares; kTakeOut: taken out again
+    template <int i0, bool kTakeOut> __device__ __forceinline__ void add(const uint32_t (&x)[16], float2& squares)
     {
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
             const float2 y = make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1]));
             float2 t, u;
             split(y, t, u);
-            high[i0 + i] += __float_as_uint(t.x);
-            high[i0 + i + 1] += __float_as_uint(t.y);
-            low[i0 + i] += __float_as_uint(u.x);
-            low[i0 + i + 1] += __float_as_uint(u.y);
-            squares = ffma2(y, y, squares);
+            if constexpr (kTakeOut) {
+                high[i0 + i] -= __float_as_uint(t.x);
+                high[i0 + i + 1] -= __float_as_uint(t.y);
+                low[i0 + i] -= __float_as_uint(u.x);
+                low[i0 + i + 1] -= __float_as_uint(u.y);
+            } else {
+                high[i0 + i] += __float_as_uint(t.x);
+                high[i0 + i + 1] += __float_as_uint(t.y);
+                low[i0 + i] += __float_as_uint(u.x);
+                low[i0 + i + 1] += __float_as_uint(u.y);
+                squares = ffma2(y, y, squares);
+            }
         }
     }
-    // takes them out again, to `wide`
-    template <int i0> __device__ __forceinline__ void move(const uint32_t (&x)[16])
+    // |high| grows by up to 2^22 per tile, |low| too: every 256 tiles `low` is carried over.  False: `high` may not have room for as many more.
+    __device__ __forceinline__ bool carry_over()
     {
+        const uint32_t h0 = n * kHighBits, l0 = n * kLowBits;
+        uint32_t large = 0;
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-            float2 t, u;
-            split(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), t, u);
-            wide.stage[i] = x[i];
-            wide.stage[i + 1] = x[i + 1];
-            high[i0 + i] -= __float_as_uint(t.x) - kHighBits;
-            high[i0 + i + 1] -= __float_as_uint(t.y) - kHighBits;
-            low[i0 + i] -= __float_as_uint(u.x) - kLowBits;
-            low[i0 + i + 1] -= __float_as_uint(u.y) - kLowBits;
+        for (int i = 0; i < 64; ++i) {
+            const uint32_t l = low[i] - l0;
+            high[i] = high[i] - h0 + (uint32_t)((int)l >> 23);
+            low[i] = l & 0x7fffffu;
+            large |= high[i] + (1u << 29);
         }
-#pragma unroll 1
-        for (int i = 0; i < 16; ++i) wide.sum[i0 + i] = wide.sum[i0 + i] + __float2ll_rn(__uint_as_float(wide.stage[i]) * 4294967296.0f);
-    }
-    // `high` and `low` added to `wide`
-    __device__ __forceinline__ void widen()
-    {
-        use_wide();
-#pragma unroll
-        for (int i = 0; i < 64; ++i) wide.stage[i] = high[i];
-#pragma unroll 1
-        for (int i = 0; i < 64; ++i) wide.sum[i] = wide.sum[i] + (long long)(int)(wide.stage[i] - n * kHighBits) * (1 << 23);
-#pragma unroll
-        for (int i = 0; i < 64; ++i) wide.stage[i] = low[i];
-#pragma unroll 1
-        for (int i = 0; i < 64; ++i) wide.sum[i] = wide.sum[i] + (int)(wide.stage[i] - n * kLowBits);
-    }
-    // (|high| grows by up to 2^22 per tile, |low| too)
-    __device__ __forceinline__ void tile_done()
-    {
-        if (++n < 256) return;
-        widen();
-#pragma unroll
-        for (int i = 0; i < 64; ++i) high[i] = low[i] = 0;
         n = 0;
+        return __all_sync(0xffffffffu, large >> 30 == 0);
     }
-    // scale times the sums, as fp32 in the place of `high`: the integers rounded to fp32, to nearest even.  Usually by one FMA of two that
-    // fp32 holds, high + carry and the low 23 bits (signed): conversions, with the rate of the exponentials again, took 3300 cycles of a
-    // block, 7200 beside them.
-    __device__ __forceinline__ void finish(float scale)
+    // Scale times the sums, as fp32 in the place of `high`: the integers rounded to fp32, to nearest even, by one FMA of two that fp32 holds,
+    // high + carry and the low 23 bits (signed).  (Conversions, with the rate of the exponentials again, took 3300 cycles of a block, 7200
+    // beside them.)  False, and nothing done: some |high| is 2^21 or more (with the carry it has to be below 2^22).
+    __device__ __forceinline__ bool finish(float scale)
     {
         const uint32_t h0 = n * kHighBits, l0 = n * kLowBits - (1u << 22);
         uint32_t large = 0;
 #pragma unroll
         for (int i = 0; i < 64; ++i) large |= high[i] - (h0 - (1u << 21));
-        if (!wide_used && large >> 22 == 0) {         // |high| < 2^21, so with the carry < 2^22
-            constexpr uint32_t kTwo23 = 0x4b000000u;  // 2^23 in fp32, whose last bit is 1
-            const float2 h1 = make_float2(-12582912.f, -12582912.f), unit = make_float2(2.3283064365386963e-10f, 2.3283064365386963e-10f);
+        if (__any_sync(0xffffffffu, large >> 22 != 0)) return false;
+        constexpr uint32_t kTwo23 = 0x4b000000u;      // 2^23 in fp32, whose last bit is 1
+        const float2 h1 = make_float2(-12582912.f, -12582912.f), unit = make_float2(kUnit, kUnit);
 #pragma unroll
-            for (int i = 0; i < 64; i += 2) {
-                float2 h, l;
-                auto split = [&](int j, float& hf, float& lf) {
-                    const uint32_t low_up = low[j] - l0;       // low + 2^22
-                    hf = __uint_as_float(high[j] - (h0 - kTwo23 - (1u << 22)) + (uint32_t)((int)low_up >> 23));
-                    lf = __uint_as_float((low_up & 0x7fffffu) | kTwo23);
-                };
-                split(i, h.x, l.x);
-                split(i + 1, h.y, l.y);
-                const float2 sum = ffma2(fadd2(h, h1), make_float2(8388608.f, 8388608.f), fadd2(l, h1));
-                const float2 y = fmul2(fmul2(sum, unit), make_float2(scale, scale));
-                high[i] = __float_as_uint(y.x);
-                high[i + 1] = __float_as_uint(y.y);
-            }
-        } else {
-            widen();
-#pragma unroll 1
-            for (int i = 0; i < 64; ++i) wide.stage[i] = __float_as_uint((float)(double)wide.sum[i] * 2.3283064365386963e-10f * scale);
-#pragma unroll
-            for (int i = 0; i < 64; ++i) high[i] = wide.stage[i];
+        for (int i = 0; i < 64; i += 2) {
+            float2 h, l;
+            auto parts = [&](int j, float& hf, float& lf) {
+                const uint32_t low_up = low[j] - l0;       // low + 2^22
+                hf = __uint_as_float(high[j] - (h0 - kTwo23 - (1u << 22)) + (uint32_t)((int)low_up >> 23));
+                lf = __uint_as_float((low_up & 0x7fffffu) | kTwo23);
+            };
+            parts(i, h.x, l.x);
+            parts(i + 1, h.y, l.y);
+            const float2 sum = ffma2(fadd2(h, h1), make_float2(8388608.f, 8388608.f), fadd2(l, h1));
+            const float2 y = fmul2(fmul2(sum, unit), make_float2(scale, scale));
+            high[i] = __float_as_uint(y.x);
+            high[i + 1] = __float_as_uint(y.y);
         }
+        return true;
     }
+};
+struct WideSums {
+    long long sum[64];
+
+    __device__ __forceinline__ explicit WideSums(const Sums& s)
+    {
+        const uint32_t h0 = s.n * kHighBits, l0 = s.n * kLowBits;
+#pragma unroll
+        for (int i = 0; i < 64; ++i) sum[i] = (long long)(int)(s.high[i] - h0) * (1 << 23) + (int)(s.low[i] - l0);
+    }
+    template <int i0> __device__ __forceinline__ void add(const uint32_t (&x)[16])
+    {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[i0 + i] += __float2ll_rn(__uint_as_float(x[i]) * 4294967296.0f);
+    }
+    __device__ __forceinline__ float result(int i, float scale) const { return (float)(double)sum[i] * kUnit * scale; }
 };
 
 template <bool kMat>
@@ -323,16 +300,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int u = 0, block = blockIdx.x; block >= 0; block = bars->queue.get(++u, abort_flag)) {
             const Block w(p, block);
             const int row = w.qt * kT + r;
-            Wide wide;
-            Sums sums(wide);
-            sums.clear();
             bool ok = true;
-            for (int k0 = w.tile(s, 0); k0 < w.n_keys; k0 = w.tile(s, k0 + kT), ++c) {
-                if (!(ok = mbar_wait_warp(&bars->dq_full[c & 1], (c >> 1) & 1, abort_flag, 0x63))) break;
-                tc_fence_after();
+            int k0 = w.tile(s, 0);
+            auto next_tile = [&]() {
+                tc_fence_before();
+                mbar_arrive(&bars->dq_free[c & 1]);
+                k0 = w.tile(s, k0 + kT);
+                ++c;
+            };
+            // f(first column, sixteen values) for a thread's 64 columns of the contribution
+            auto all = [&](auto&& f) {
                 const uint32_t dq = lanes + kColDq + (c & 1) * 128 + half * 64;
-                float2 squares = make_float2(0.f, 0.f);
-                auto sixteen = [&](auto j_, auto&& f) {
+                auto sixteen = [&](auto j_) {
                     constexpr int j = decltype(j_)::value;
                     uint32_t x[16];
                     tmem_ld8(dq + j * 16, x);
@@ -340,30 +319,54 @@ __global__ void __launch_bounds__(kThreads, 1)
                     tmem_ld_wait();
                     f(Int<j * 16>{}, x);
                 };
-                auto all = [&](auto&& f) { sixteen(Int<0>{}, f); sixteen(Int<1>{}, f); sixteen(Int<2>{}, f); sixteen(Int<3>{}, f); };
-                all([&](auto i0, const uint32_t (&x)[16]) { sums.template add<decltype(i0)::value>(x, squares); });
-                // all |x| are below 2^13; if not (a whole warp: it loads them again)
-                if (__any_sync(0xffffffffu, !(squares.x + squares.y < 67108864.0f))) {
-                    sums.use_wide();
-                    all([&](auto i0, const uint32_t (&x)[16]) { sums.template move<decltype(i0)::value>(x); });
+                sixteen(Int<0>{}); sixteen(Int<1>{}); sixteen(Int<2>{}); sixteen(Int<3>{});
+            };
+            auto store = [&](auto&& result) {
+                if (row < s.Sq && kMat) {
+                    float* dst = p.dq_mat + ((long long)w.h * kD + half * 64) * p.mat_stride + (long long)w.b * s.Sq + row;
+#pragma unroll
+                    for (int i = 0; i < 64; ++i, dst += p.mat_stride) *dst = result(i);
+                } else if (row < s.Sq) {
+                    uint4* dst = reinterpret_cast<uint4*>(p.dq + ((size_t)w.bh * s.Sq + row) * kD + half * 64);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        auto two = [&](int i) { return pack_bf16(result(8 * j + i), result(8 * j + i + 1)); };
+                        dst[j] = make_uint4(two(0), two(2), two(4), two(6));
+                    }
                 }
-                tc_fence_before();
-                mbar_arrive(&bars->dq_free[c & 1]);
-                sums.tile_done();
+            };
+            Sums sums;
+            bool wide = false, have = false;      // (the same in all lanes; have: the tile that is waited for already)
+            while (k0 < w.n_keys) {
+                if (!(ok = mbar_wait_warp(&bars->dq_full[c & 1], (c >> 1) & 1, abort_flag, 0x63))) break;
+                tc_fence_after();
+                float2 squares = make_float2(0.f, 0.f);
+                all([&](auto i0, const uint32_t (&x)[16]) { sums.template add<decltype(i0)::value, false>(x, squares); });
+                // below 2^26 all |x| are below 2^13
+                if (__any_sync(0xffffffffu, !(squares.x + squares.y < 67108864.0f))) {
+                    all([&](auto i0, const uint32_t (&x)[16]) { sums.template add<decltype(i0)::value, true>(x, squares); });
+                    wide = have = true;
+                    break;
+                }
+                next_tile();
+                if (++sums.n == 256 && !sums.carry_over()) {
+                    wide = true;
+                    break;
+                }
             }
             if (!ok) break;
-            sums.finish(s.scale);
-            if (row < s.Sq && kMat) {
-                float* dst = p.dq_mat + ((long long)w.h * kD + half * 64) * p.mat_stride + (long long)w.b * s.Sq + row;
-#pragma unroll
-                for (int i = 0; i < 64; ++i, dst += p.mat_stride) *dst = __uint_as_float(sums.high[i]);
-            } else if (row < s.Sq) {
-                uint4* dst = reinterpret_cast<uint4*>(p.dq + ((size_t)w.bh * s.Sq + row) * kD + half * 64);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    auto two = [&](int i) { return pack_bf16(__uint_as_float(sums.high[8 * j + i]), __uint_as_float(sums.high[8 * j + i + 1])); };
-                    dst[j] = make_uint4(two(0), two(2), two(4), two(6));
+            if (!wide && sums.finish(s.scale)) {
+                store([&](int i) { return __uint_as_float(sums.high[i]); });
+            } else {
+                WideSums sums64(sums);
+                for (; k0 < w.n_keys; have = false) {
+                    if (!have && !(ok = mbar_wait_warp(&bars->dq_full[c & 1], (c >> 1) & 1, abort_flag, 0x63))) break;
+                    tc_fence_after();
+                    all([&](auto i0, const uint32_t (&x)[16]) { sums64.template add<decltype(i0)::value>(x); });
+                    next_tile();
                 }
+                if (!ok) break;
+                store([&](int i) { return sums64.result(i, s.scale); });
             }
             __syncwarp();
         }

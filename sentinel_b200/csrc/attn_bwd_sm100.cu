@@ -579,7 +579,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     auto next = [&](int u) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->work_empty[u & 1]);
-        return mbar_wait_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && bars->work[(u + 1) & 1].n_iter >= 0;
+        return mbar_wait_prompt_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && bars->work[(u + 1) & 1].n_iter >= 0;
     };
 
     if (warp == 15) {
@@ -594,7 +594,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             for (int u = 0, block = 0; block >= 0; ++u) {
                 // K and V: once every product of the block before has read them
                 if (w.n_iter > 0) {
-                    ok = blocks == 0 || mbar_wait(&bars->final_bar, (uint32_t)((blocks - 1) & 1), abort_flag, kSiteFinal);
+                    ok = blocks == 0 || mbar_wait_prompt(&bars->final_bar, (uint32_t)((blocks - 1) & 1), abort_flag, kSiteFinal);
                     if (!ok) break;
                     mbar_arrive_expect_tx(&bars->k_full, (uint32_t)kTileBytes);
                     for (int c = 0; c < kChunks; ++c) tma_load_3d(sK + c * kChunkBytes, &tmap_k, &bars->k_full, c * 64, w.kt * kT, w.slab);
@@ -606,7 +606,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     const int qt = w.qt_first + r, bh = bh0 + g, n = n0 + i;
                     if (++r == w.per_head) { r = 0; ++g; }
                     const int sq = n % kQStages;
-                    if (n >= kQStages && !(ok = mbar_wait(&bars->q_empty[sq], (uint32_t)(((n / kQStages) - 1) & 1), abort_flag, kSiteQEmpty))) break;
+                    if (n >= kQStages && !(ok = mbar_wait_prompt(&bars->q_empty[sq], (uint32_t)(((n / kQStages) - 1) & 1), abort_flag, kSiteQEmpty))) break;
                     mbar_arrive_expect_tx(&bars->q_full[sq], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 2 * kT * 4)));
                     for (int c = 0; c < kChunks; ++c)
                         tma_load_3d(sQ + sq * kTileBytes + c * kChunkBytes, &tmap_q, &bars->q_full[sq], c * 64, qt * kT, bh);
@@ -622,7 +622,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     }
                     const int sd = n % kDoStages;
                     if (n >= kDoStages &&
-                        !(ok = mbar_wait(&bars->do_empty[sd], (uint32_t)(((n / kDoStages) - 1) & 1), abort_flag, kSiteDoEmpty)))
+                        !(ok = mbar_wait_prompt(&bars->do_empty[sd], (uint32_t)(((n / kDoStages) - 1) & 1), abort_flag, kSiteDoEmpty)))
                         break;
                     mbar_arrive_expect_tx(&bars->do_full[sd], (uint32_t)(kTileBytes + (kAug ? kAugBytes : 0)));
                     if constexpr (kAug)
@@ -639,13 +639,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if (p.several_waves) {
                     mbar_arrive_expect_tx(&bars->response_full, 16);
                     clc_try_cancel(&bars->response, &bars->response_full);
-                    if (!mbar_wait(&bars->response_full, (uint32_t)(u & 1), abort_flag, kSiteNext)) break;
+                    if (!mbar_wait_prompt(&bars->response_full, (uint32_t)(u & 1), abort_flag, kSiteNext)) break;
                     block = clc_first_block(&bars->response);
                     fence_proxy_async_smem();
                 }
                 w.n_iter = -1;
                 if (block >= 0) w.decode<kWin, kSplit>(p, block);
-                if (u >= 1 && !mbar_wait(&bars->work_empty[(u + 1) & 1], (uint32_t)(((u - 1) >> 1) & 1), abort_flag, kSiteNext)) break;
+                if (u >= 1 && !mbar_wait_prompt(&bars->work_empty[(u + 1) & 1], (uint32_t)(((u - 1) >> 1) & 1), abort_flag, kSiteNext)) break;
                 bars->work[(u + 1) & 1] = w;
                 mbar_arrive(&bars->work_full[(u + 1) & 1]);
             }
@@ -672,7 +672,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             (void)tl;
             constexpr uint32_t idesc_st = make_idesc(kT, kT, false, false);
             constexpr uint32_t idesc_kv = make_idesc(kT, D, false, true);
-            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_warp(bar, parity, abort_flag, site); };
+            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_prompt_warp(bar, parity, abort_flag, site); };
             const uint64_t d_ones = make_sdesc_plain(smem_u32(sOnes), kAugBytes), d_qaug0 = make_sdesc_plain(smem_u32(sQaug), 0);
             // the D/16 steps over the head dimension, then the extra step that subtracts LSE/scale (see kAugBytes)
             auto issue_kmajor = [&](uint32_t d_tmem, uint64_t a, uint64_t b, uint64_t aug) {
@@ -736,7 +736,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             // dS side, in the same form
             const bool tl14 = lane == 0;
             (void)tl14;
-            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_warp(bar, parity, abort_flag, site); };
+            auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_prompt_warp(bar, parity, abort_flag, site); };
             SNTL_TRACE_DECL(tn);
             constexpr uint32_t idesc_st = make_idesc(kT, kT, false, false);   // S^T, dP^T
             constexpr uint32_t idesc_kv = make_idesc(kT, D, false, true);     // dV, dK: A in TMEM, B MN-major
@@ -837,7 +837,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             if (++tile_r == w.per_head) { tile_r = 0; ++g; }
             // fp32 accumulator: kT*D words per tile; fixed-point accumulator: kT*D 64-bit words per tile
             float* tile = p.dq_accum + ((size_t)bh * p.n_qt + qt) * (size_t)(kT * D) * (kDet ? 2 : 1);
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->dq_ready, (uint32_t)(n & 1), abort_flag, kSiteDQ));
+            ok = mbar_wait_prompt_warp(&bars->dq_ready, (uint32_t)(n & 1), abort_flag, kSiteDQ);
             SNTL_TRACE_EV(tw, 3, tn, 1);
             if (!ok) break;
             tc_fence_after();
@@ -887,8 +887,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             // ---- P^T ----
             const uint32_t tm_Si = tm_S + (uint32_t)(n % kSBufs) * kSBufStride;
             // (the Q stage's barrier also covers the LSE and delta columns this warp reads when they come as plain columns)
-            ok = __all_sync(0xffffffffu, (kAug || mbar_wait(&bars->q_full[n % kQStages], (uint32_t)((n / kQStages) & 1), abort_flag, kSiteQFull)) &&
-                                             mbar_wait(&bars->s_ready[n % kSBufs], (uint32_t)((n / kSBufs) & 1), abort_flag, kSiteS));
+            ok = (kAug || mbar_wait_prompt_warp(&bars->q_full[n % kQStages], (uint32_t)((n / kQStages) & 1), abort_flag, kSiteQFull)) &&
+                 mbar_wait_prompt_warp(&bars->s_ready[n % kSBufs], (uint32_t)((n / kSBufs) & 1), abort_flag, kSiteS);
             SNTL_TRACE_EV(tw, 1 + wg, tn, 1);
             if (!ok) break;
             tc_fence_after();
@@ -951,7 +951,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             mbar_arrive(&bars->p_ready[n % kSBufs]);
             SNTL_TRACE_EV(tw, 1 + wg, tn, 4);
             // ---- dS^T ----
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_ready, ph, abort_flag, kSiteDP));
+            ok = mbar_wait_prompt_warp(&bars->dp_ready, ph, abort_flag, kSiteDP);
             SNTL_TRACE_EV(tw, 1 + wg, tn, 5);
             if (!ok) break;
             tc_fence_after();
@@ -992,7 +992,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             SNTL_TRACE_EV(tw, 1 + wg, tn, 8);
         }
         // ---- epilogue: dV (warpgroup 0) and dK (warpgroup 1) ----
-        const bool done = __all_sync(0xffffffffu, ok && n_iter > 0 && mbar_wait(&bars->final_bar, (uint32_t)(blocks & 1), abort_flag, kSiteFinal));
+        const bool done = ok && n_iter > 0 && mbar_wait_prompt_warp(&bars->final_bar, (uint32_t)(blocks & 1), abort_flag, kSiteFinal);
         if (n_iter > 0) {
             ok = done;
             ++blocks;

@@ -199,7 +199,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         if (!kMany) return false;
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->work_empty[u & 1]);
-        return mbar_wait_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && warp_uniform(bars->work[(u + 1) & 1].n0) >= 0;
+        return mbar_wait_prompt_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && warp_uniform(bars->work[(u + 1) & 1].n0) >= 0;
     };
 
     auto work = [&](int u) -> const FwdWork& { return kMany ? bars->work[u & 1] : own; };
@@ -224,7 +224,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 // Q and K_0 once the last S product of the block before has run: Q is free then, and K_0's stage and barrier were free
                 // before (the barrier must not be armed again while the K_0 before is on its way or unseen: rows of a single
                 // key tile get here that early)
-                if (u > 0 && !mbar_wait(&bars->q_empty, (uint32_t)((u - 1) & 1), abort_flag, kSiteQEmpty)) break;
+                if (u > 0 && !mbar_wait_prompt(&bars->q_empty, (uint32_t)((u - 1) & 1), abort_flag, kSiteQEmpty)) break;
                 mbar_arrive_expect_tx(&bars->k0_full, (uint32_t)kTileBytes);
                 load(sK, &tmap_k, &bars->k0_full, 0);
                 mbar_arrive_expect_tx(&bars->q_full, (uint32_t)((w.n1 > 0 ? 2 : 1) * kTileBytes));
@@ -235,7 +235,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     // K_{c+1} and V_c go where K_{c-1} and V_{c-2} were: pair c - 2, the (c >> 1)-th release of this barrier for odd c
                     // (pair -1 was the first), the one before for even c
                     const int c = c0 + j;
-                    if (c >= 1 && !(ok = mbar_wait(&bars->pair_empty[c & 1], (uint32_t)((c >> 1) - (c & 1 ? 0 : 1)) & 1u, abort_flag, kSitePairEmpty))) break;
+                    if (c >= 1 && !(ok = mbar_wait_prompt(&bars->pair_empty[c & 1], (uint32_t)((c >> 1) - (c & 1 ? 0 : 1)) & 1u, abort_flag, kSitePairEmpty))) break;
                     const bool k_too = j + 1 < n_max;
                     mbar_arrive_expect_tx(&bars->pair_full[c & 1], (uint32_t)(k_too ? 2 * kTileBytes : kTileBytes));
                     if (k_too) load(sK, &tmap_k, &bars->pair_full[c & 1], j + 1);
@@ -249,12 +249,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 if constexpr (kMany) {
                     mbar_arrive_expect_tx(&bars->response_full, 16);
                     clc_try_cancel(&bars->response, &bars->response_full);
-                    if (!mbar_wait(&bars->response_full, (uint32_t)(u & 1), abort_flag, kSiteNext)) break;
+                    if (!mbar_wait_prompt(&bars->response_full, (uint32_t)(u & 1), abort_flag, kSiteNext)) break;
                     block = clc_first_block(&bars->response);
                     fence_proxy_async_smem();
                     w.n0 = -1;
                     if (block >= 0) w.decode<kWin>(p, block);
-                    if (u >= 1 && !mbar_wait(&bars->work_empty[(u + 1) & 1], (uint32_t)(((u - 1) >> 1) & 1), abort_flag, kSiteNext)) break;
+                    if (u >= 1 && !mbar_wait_prompt(&bars->work_empty[(u + 1) & 1], (uint32_t)(((u - 1) >> 1) & 1), abort_flag, kSiteNext)) break;
                     bars->work[(u + 1) & 1] = w;
                     mbar_arrive(&bars->work_full[(u + 1) & 1]);
                 }
@@ -269,7 +269,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         // the issue order below makes this warp's pace count; no change at 128).
         {
             auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
-                return mbar_wait_warp(bar, parity, abort_flag, site);
+                return mbar_wait_prompt_warp(bar, parity, abort_flag, site);
             };
             const bool tl8 = lane == 0;
             (void)tl8;
@@ -411,7 +411,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         bool s_seen = false;
         const int row_lo = q0 + t * kM + (warp & 3) * 32;      // first row of the warp
         for (int j = 0; j < n_mine; ++j, phase = kMany ? phase ^ 1u : (uint32_t)(j & 1)) {
-            if (!(ok = __all_sync(0xffffffffu, s_seen || mbar_wait(&bars->s_ready[t], phase, abort_flag, kSiteSReady)))) break;
+            if (!(ok = (s_seen || mbar_wait_prompt_warp(&bars->s_ready[t], phase, abort_flag, kSiteSReady)))) break;
             SNTL_TRACE_EV(tw, 1 + t, tn, 1);
             tc_fence_after();
             uint32_t s[128];
@@ -446,7 +446,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             bool o_seen = false;
             auto o_done = [&]() {       // P_{j-1} has been consumed and O holds its product (head_dim 128: S_j was issued behind it)
                 if constexpr (kOwnP) {
-                    ok = __all_sync(0xffffffffu, o_seen || mbar_wait(&bars->o_ready[t], phase ^ 1u, abort_flag, kSiteOReady));
+                    ok = o_seen || mbar_wait_prompt_warp(&bars->o_ready[t], phase ^ 1u, abort_flag, kSiteOReady);
                     tc_fence_after();
                 }
             };
@@ -470,7 +470,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             if (ahead) {
                 exp_half<0, true>(s, p.scale_log2, neg_m, pk, sum, mx);
                 SNTL_TRACE_EV(tw, 1 + t, tn, 3);
-                if (kOwnP) o_seen = mbar_try_wait(&bars->o_ready[t], phase ^ 1u);
+                if (kOwnP) o_seen = __all_sync(0xffffffffu, mbar_try_wait(&bars->o_ready[t], phase ^ 1u));
                 const float m_new = fmaxf(m_ref, mx.value() * p.scale_log2);
                 const bool again = outgrown(m_new);
                 if (!again) s_read();
@@ -514,7 +514,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 mbar_arrive(&bars->p_half[t]);
             }
             exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, mx);
-            if (kOwnP) s_seen = j + 1 < n_mine && mbar_try_wait(&bars->s_ready[t], phase ^ 1u);
+            if (kOwnP) s_seen = j + 1 < n_mine && __all_sync(0xffffffffu, mbar_try_wait(&bars->s_ready[t], phase ^ 1u));
             tmem_st32(tmem_S(t) + kPOff + lane_off + 32u, pk);
             l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             SNTL_TRACE_EV(tw, 1 + t, tn, 5);
@@ -524,7 +524,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             SNTL_TRACE_EV(tw, 1 + t, tn, 6);
         }
         if (ok && n_mine > 0)
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_ready[t], kOwnP ? phase ^ 1u : blocks & 1u, abort_flag, kSiteOReady));
+            ok = mbar_wait_prompt_warp(&bars->o_ready[t], kOwnP ? phase ^ 1u : blocks & 1u, abort_flag, kSiteOReady);
         if (ok && n_mine > 0) {
             ++blocks;
             tc_fence_after();

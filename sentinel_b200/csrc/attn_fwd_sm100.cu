@@ -5,15 +5,15 @@
 // (sentinel/NeuralNet/Cuda/CudaFlashAttention.cu:1105-1266): same math -- S = scale*Q K^T, causal mask,
 // online softmax, O = P V, LSE = m + ln(l) -- re-designed for Blackwell:
 //
-//   * one CTA owns 256 (small grids: 128) consecutive query rows of one (batch, head) as two 128-row tiles; each tile has its
-//     own softmax warpgroup (one thread per query row: tcgen05.ld's 32x32b shape hands thread i row i, so the
-//     row max / row sum need no shuffles) while a single MMA-issuing warp (one elected lane) feeds the tensor core for both,
-//     so one tile's softmax overlaps the other tile's MMAs;
-//   * S (fp32, 128 columns) and O (fp32, D columns) live in TMEM; P is written back as packed bf16 -- over S at
-//     head_dim 128, into 64 columns of its own at head_dim 64, where the next S of the tile is then issued as soon as
-//     the softmax warps have read the current one -- and consumed by the PV MMA straight from TMEM (A operand in
-//     TMEM), V is consumed from shared memory as an MN-major operand, so nothing is transposed and P never touches
-//     shared memory;
+//   * head_dim 128 (attn_fwd_tc_kernel): one CTA owns 256 (small grids: 128) consecutive query rows of one (batch, head) as two
+//     128-row tiles; each tile has its own softmax warpgroup (one thread per query row: tcgen05.ld's 32x32b shape hands thread i
+//     row i, so the row max / row sum need no shuffles) while a single MMA-issuing warp (one elected lane) feeds the tensor core
+//     for both, so one tile's softmax overlaps the other tile's MMAs;
+//   * head_dim 64 (attn_fwd_streams_kernel): four softmax warpgroups, each with 64 of the 128 keys of every key tile and sums and
+//     an O of its own, two per query tile, and two query tiles that run independently of each other;
+//   * S (fp32) and O (fp32, D columns) live in TMEM; P is written back over S as packed bf16 and consumed by the PV MMA
+//     straight from TMEM (A operand in TMEM), V is consumed from shared memory as an MN-major operand, so nothing is
+//     transposed and P never touches shared memory;
 //   * Q/K/V tiles arrive by per-CTA TMA (128-byte swizzle, no multicast) into two-stage K and V rings
 //     guarded by mbarriers; stages are released by tcgen05.commit;
 //   * the softmax works in the exp2 domain with scale*log2(e) folded into one FMA, and rescales O lazily:
@@ -23,8 +23,7 @@
 //     heads of one group are adjacent in launch order so they share K/V tiles in L2.
 //
 // Layout: bf16 token-major [B][H][S][D], D in {64,128}; LSE [B][Hq][Sq] fp32 (natural log).
-// TMEM map (512 columns): head_dim 128 S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D);
-// head_dim 64 S0 [0,128) P0 [128,192) S1 [192,320) P1 [320,384) O0 [384,448) O1 [448,512).
+// TMEM map (512 columns): head_dim 128 S0 [0,128) S1 [128,256) O0 [256,384) O1 [384,512); head_dim 64 four S of 64, then four O of 64.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_tile.cuh"
@@ -56,6 +55,7 @@ struct FwdParams {
     int causal;
     int window, global_tokens;   // sliding window and always-visible first keys (0, 0: plain causal)
     int n_qblk, tiles_per_cta;   // query blocks of that many 128-row tiles per (b, h)
+    int several_waves;           // more blocks than SMs
     float scale_log2; // scale * log2(e)
     // non-null: O and LSE leave as fp32 feature-major matrices (see MatrixOut)
     float *o_mat, *lse_mat;
@@ -64,8 +64,7 @@ struct FwdParams {
 
 // What one block of the grid computes.  A CTA computes its own block and then takes over blocks that have not started yet (as the
 // backward does): K, Q and the first S of one come in under the last softmax passes and the epilogue of the one before.
-// Cold: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108 us; B8 Hq12 S1024 D64 37.1 -> 35.3; B4 Hq32 Hkv8 S4096 D64 421 ->
-// 407.
+// Cold: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108 us.
 struct FwdWork {
     int bh, bh_kv, q0;         // q0: first of the one or two 128-row tiles
     int g_tiles, w_first;      // key tiles in ascending order: the g_tiles tiles holding global tokens, then from w_first up to the
@@ -107,12 +106,11 @@ struct FwdBarriers {
     // wait and one commit per key tile for the issuing warp instead of two each.  Barrier j & 1.
     uint64_t pair_full[2], pair_empty[2];
     uint64_t s_ready[2], p_ready[2];
-    uint64_t o_ready[2];     // head_dim 64: after every P V product; 128: after the tile's last one (s_ready covers the others)
+    uint64_t o_ready[2];     // after the tile's last P V product (s_ready covers the others)
     uint64_t p_half[2];      // the first 64 columns of P_t are written
     uint64_t final_bar;
     uint32_t tmem_base;
     uint32_t abort_flag;
-    uint64_t s_free[2];      // head_dim 64: the softmax warps have read S_j of tile t
 };
 
 // kMode: kPlain = causal / full attention of a whole sequence; kWindow adds the sliding window (separate so that the
@@ -120,7 +118,8 @@ struct FwdBarriers {
 enum FwdMode : int { kPlain = 0, kWindow = 1 };
 
 // kMat: O and LSE leave as fp32 feature-major matrices
-// kMany: CTAs take over blocks (FwdWork); without it each computes its own and the bookkeeping folds away
+// kMany: CTAs take over blocks (FwdWork); without it each computes its own and the bookkeeping folds away.  The plain kernel has no
+// such form: its softmax loop fills the registers, and with the bookkeeping it spills (B2 Hq28 Hkv4 S8192 737 -> 768 us).
 template <int D, int kMode, bool kMat, bool kMany>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -160,7 +159,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             mbar_init(&bars->pair_full[i], 1);
             mbar_init(&bars->pair_empty[i], 1);
             mbar_init(&bars->s_ready[i], 1);
-            if (D == 64) mbar_init(&bars->s_free[i], 128);
             mbar_init(&bars->p_ready[i], 128);
             mbar_init(&bars->p_half[i], 128);
             mbar_init(&bars->o_ready[i], 1);
@@ -178,19 +176,11 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
     wait_for_stream();      // nothing before this reads or writes global memory
-    // head_dim 64 (plain / window kernels) leaves room for P in columns of its own: S_t [192t, 192t+128), P_t the next 64,
-    // O_t [384+64t, +64).  The next S of a tile is then issued as soon as the softmax warps have READ the current one
-    // instead of behind the P V product that consumes P, which takes a tile's two products out of the chain between two of
-    // its softmax passes.  Otherwise (512 columns full at head_dim 128): S_t [128t, +128) with P written over it,
-    // O_t [256+128t, +128).
-    constexpr bool kOwnP = D == 64;
+    // P is written over S, so a tile's P V product and next S stay in the chain between two of its softmax passes; the first half of
+    // P V is issued as soon as the first 64 columns of P are written (-6 %).
     // (computed, not looked up: a two-element array indexed by the warp's tile would live in local memory)
-    auto tmem_S = [&](int t) { return tmem + (uint32_t)t * (kOwnP ? 192u : 128u); };
-    constexpr uint32_t kPOff = kOwnP ? 128u : 0u;   // P relative to the S of its tile
-    // head_dim 128 (plain / window): P is written over S, so a tile's P V product and next S stay in the chain between two of
-    // its softmax passes; there the first half of P V is issued as soon as the first 64 columns of P are written (-6 %)
-    constexpr bool kHalfP = !kOwnP;
-    auto tmem_O = [&](int t) { return tmem + (kOwnP ? 384u : 256u) + (uint32_t)t * (kOwnP ? 64u : 128u); };
+    auto tmem_S = [&](int t) { return tmem + (uint32_t)t * 128u; };
+    auto tmem_O = [&](int t) { return tmem + 256u + (uint32_t)t * 128u; };
 
     // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Counters of key
     // tiles run on over the blocks (all of them: c0; those of tile t: its steps), so stages and barrier phases continue where they
@@ -264,9 +254,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         setmaxnreg_dec<72>();
         // =========================== MMA issuer ===========================
         // All 32 lanes walk the loops (warp-uniform control flow keeps descriptors and addresses in uniform registers) and
-        // one elected lane issues each tcgen05 instruction: the warp shares its scheduler with two softmax warps and this
-        // form needs fewer of the issue slots it is given per MMA than a single-lane loop (-3.7 % at head_dim 64, where
-        // the issue order below makes this warp's pace count; no change at 128).
+        // one elected lane issues each tcgen05 instruction.
         {
             auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
                 return mbar_wait_prompt_warp(bar, parity, abort_flag, site);
@@ -287,18 +275,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     mma_ss_4<2, 2>(tmem_S(t), sdesc_advance(a, (uint32_t)(c * kChunkBytes)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_s, c > 0);
                 tc_commit_p(&bars->s_ready[t]);
             };
-            // With kHalfP, P V in two halves of the contraction: the first four k-steps need only the first 64 columns of P
-            // (p_half, which the caller has waited for), the rest the whole of it (p_ready) -- so half the product is issued
-            // while the softmax warps still compute the second half of their exponentials.  Otherwise the caller has waited
-            // for the whole of P.  Returns false when a wait gave up.
+            // P V in two halves of the contraction: the first four k-steps need only the first 64 columns of P (p_half, which the caller
+            // has waited for), the rest the whole of it (p_ready) -- so half the product is issued while the softmax warps still compute
+            // the second half of their exponentials.  Returns false when a wait gave up.
             auto issue_pv = [&](int t, int st, bool accumulate, uint32_t parity) {
                 const uint64_t b = st ? dv1 : dv0;
-                const uint32_t d = tmem_O(t), a = tmem_S(t) + kPOff;
+                const uint32_t d = tmem_O(t), a = tmem_S(t);
                 mma_ts_4<8, 128>(d, a, b, idesc_pv, accumulate);
-                if constexpr (kHalfP) {
-                    if (!wait(&bars->p_ready[t], parity, kSitePReady)) return false;
-                    tc_fence_after();
-                }
+                if (!wait(&bars->p_ready[t], parity, kSitePReady)) return false;
+                tc_fence_after();
                 mma_ts_4<8, 128>(d, a + 32u, sdesc_advance(b, 4 * 2048), idesc_pv, 1);
                 return true;
             };
@@ -311,73 +296,30 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             // (S of the last step of the block before has been read, and P over it consumed: this warp waited for p_ready and issued
             // the product; O is overwritten behind p_ready of the new block, which its warps give after their epilogue)
             issue_s(0, c0 & 1);          // (a block has rows in its first tile)
-            if constexpr (kOwnP) {
-                // With P in columns of its own the next S of a tile does not wait for the P V product that consumes P, and the two
-                // tiles are kept half a pass apart: S of tile 1 starts behind the first half of tile 0's first pass, and per key tile
-                // the order is S0_{j+1}, P1_{j-1} V, P0_j V, S1_{j+1}, which is the order in which their operands are ready then.
-                // One tile's loads, stores and hand-offs so fall into the other's exponentials.
-                const bool apart = n_max >= 4;   // short rows would pay more for the late start than they gain
-                if (!apart && n1 > 0) issue_s(1, c0 & 1);
-                if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
-                for (int j = 0; ok && j <= n_max; ++j) {
-                    const int c = c0 + j;
-                    if (j < n_max) {
-                        if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
-                    }
-                    const bool late = j == 0 && apart && n1 > 0;
-                    if (j + 1 < n0 || late) {
-                        if (!(ok = wait(&bars->s_free[0], (uint32_t)((s0 + j) & 1), kSiteIssue))) break;
-                        tc_fence_after();
-                        if (j + 1 < n0) issue_s(0, (c + 1) & 1);
-                        if (late) issue_s(1, c & 1);
-                    }
-                    if (j > 0 && j - 1 < n1) {
-                        if (!(ok = wait(&bars->p_ready[1], (uint32_t)((s1 + j - 1) & 1), kSitePReady))) break;
-                        tc_fence_after();
-                        issue_pv(1, (c - 1) & 1, j > 1, 0);
-                        tc_commit_p(&bars->o_ready[1]);
-                    }
-                    // pair c - 1; K_0 counts into the last pair of the block before, and this block's last into the next block's first
-                    if (j < n_max) tc_commit_p(&bars->pair_empty[(c - 1) & 1]);
-                    if (j < n0) {
-                        if (!(ok = wait(&bars->p_ready[0], (uint32_t)((s0 + j) & 1), kSitePReady))) break;
-                        tc_fence_after();
-                        issue_pv(0, c & 1, j > 0, 0);
-                        tc_commit_p(&bars->o_ready[0]);
-                    }
-                    if (j + 1 < n1) {
-                        if (!(ok = wait(&bars->s_free[1], (uint32_t)((s1 + j) & 1), kSiteIssue))) break;
-                        tc_fence_after();
-                        issue_s(1, (c + 1) & 1);
-                    }
-                    if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
-                }
-            } else {
-                // P is written over S: a tile's P V product, then its next S, as its P arrives
-                if (n1 > 0) issue_s(1, c0 & 1);
-                tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
-                if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
-                for (int j = 0; ok && j < n_max; ++j) {
-                    const int c = c0 + j;
-                    if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
+            // P is written over S: a tile's P V product, then its next S, as its P arrives
+            if (n1 > 0) issue_s(1, c0 & 1);
+            tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
+            if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
+            for (int j = 0; ok && j < n_max; ++j) {
+                const int c = c0 + j;
+                if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
 #pragma unroll
-                    for (int t = 0; t < 2; ++t) {
-                        const int n = t ? n1 : n0;
-                        const uint32_t parity = (uint32_t)(((t ? s1 : s0) + j) & 1);
-                        if (!ok || j >= n) continue;
-                        if (!(ok = wait(&bars->p_half[t], parity, kSitePReady))) continue;
-                        SNTL_TRACE_EV(tl8, 0, tn, 10 + t);
-                        tc_fence_after();
-                        if (!(ok = issue_pv(t, c & 1, j > 0, parity))) continue;
-                        SNTL_TRACE_EV(tl8, 0, tn, 20 + t);
-                        if (j + 1 < n) issue_s(t, (c + 1) & 1);
-                        else tc_commit_p(&bars->o_ready[t]);
-                        SNTL_TRACE_EV(tl8, 0, tn, 30 + t);
-                    }
-                    if (!ok) break;
-                    if (j + 1 < n_max) tc_commit_p(&bars->pair_empty[c & 1]);
-                    if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
+                for (int t = 0; t < 2; ++t) {
+                    const int n = t ? n1 : n0;
+                    const uint32_t parity = (uint32_t)(((t ? s1 : s0) + j) & 1);
+                    if (!ok || j >= n) continue;
+                    if (!(ok = wait(&bars->p_half[t], parity, kSitePReady))) continue;
+                    SNTL_TRACE_EV(tl8, 0, tn, 10 + t);
+                    tc_fence_after();
+                    if (!(ok = issue_pv(t, c & 1, j > 0, parity))) continue;
+                    SNTL_TRACE_EV(tl8, 0, tn, 20 + t);
+                    if (j + 1 < n) issue_s(t, (c + 1) & 1);
+                    else tc_commit_p(&bars->o_ready[t]);
+                    SNTL_TRACE_EV(tl8, 0, tn, 30 + t);
                 }
+                if (!ok) break;
+                if (j + 1 < n_max) tc_commit_p(&bars->pair_empty[c & 1]);
+                if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
             }
             if (!ok) break;
             c0 += n_max;
@@ -406,12 +348,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const int grow = q0 + t * kM + row;            // query row inside the (batch, head) slab
         auto key_tile = [&](int j) { return j < g_tiles ? j : w_first + (j - g_tiles); };
         float m_ref = -INFINITY, l = 0.0f;
-        // Barrier tests queue behind the exponentials in the same unit and take 200-400 cycles here; where a result is likely to be
-        // there already it is asked for ahead of its use, with other work in between.
-        bool s_seen = false;
         const int row_lo = q0 + t * kM + (warp & 3) * 32;      // first row of the warp
         for (int j = 0; j < n_mine; ++j, phase = kMany ? phase ^ 1u : (uint32_t)(j & 1)) {
-            if (!(ok = (s_seen || mbar_wait_prompt_warp(&bars->s_ready[t], phase, abort_flag, kSiteSReady)))) break;
+            if (!(ok = mbar_wait_prompt_warp(&bars->s_ready[t], phase, abort_flag, kSiteSReady))) break;
             SNTL_TRACE_EV(tw, 1 + t, tn, 1);
             tc_fence_after();
             uint32_t s[128];
@@ -429,7 +368,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             // than 2^8, which the lazy rule below leaves rare) is the first half done again.  The maximum and the decision were
             // a quarter of a tile's time in front of the exponentials.
             const int limit_lo = (p.causal ? min(p.Skv, row_lo + 1) : p.Skv) - key0, lo_hi = row_lo + 31 - p.window + 1 - key0;
-            const bool ahead = (kOwnP || kMode == kPlain) && j > 0 && limit_lo >= kN && !(kWin && lo_hi > 0 && glim < min(lo_hi, kN));   // (no row of the warp is cut)
+            const bool ahead = kMode == kPlain && j > 0 && limit_lo >= kN && !(kWin && lo_hi > 0 && glim < min(lo_hi, kN));   // (no row of the warp is cut)
             uint32_t pk[32];
             float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
             RowMax mx;
@@ -437,19 +376,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             float neg_m = shift();
             // whether some row of the warp has outgrown its reference (false when both are -inf: NaN compare)
             auto outgrown = [&](float m_new) { return j > 0 && __any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold); };
-            auto s_read = [&]() {       // nothing reads S_j any more: the next S of this tile may overwrite it
-                if constexpr (kOwnP) {
-                    tc_fence_before();
-                    mbar_arrive(&bars->s_free[t]);
-                }
-            };
-            bool o_seen = false;
-            auto o_done = [&]() {       // P_{j-1} has been consumed and O holds its product (head_dim 128: S_j was issued behind it)
-                if constexpr (kOwnP) {
-                    ok = o_seen || mbar_wait_prompt_warp(&bars->o_ready[t], phase ^ 1u, abort_flag, kSiteOReady);
-                    tc_fence_after();
-                }
-            };
             auto rescale = [&](float m_new) {
                 const bool need = (m_new - m_ref) > kRescaleThreshold;
                 const float factor = need ? ex2(m_ref - m_new) : 1.0f;
@@ -470,23 +396,16 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             if (ahead) {
                 exp_half<0, true>(s, p.scale_log2, neg_m, pk, sum, mx);
                 SNTL_TRACE_EV(tw, 1 + t, tn, 3);
-                if (kOwnP) o_seen = __all_sync(0xffffffffu, mbar_try_wait(&bars->o_ready[t], phase ^ 1u));
                 const float m_new = fmaxf(m_ref, mx.value() * p.scale_log2);
-                const bool again = outgrown(m_new);
-                if (!again) s_read();
-                o_done();
-                if (!ok) break;
-                if (again) {            // (S is read again: kept, it would take 64 registers more than there are)
+                if (outgrown(m_new)) {            // (S is read again: kept, it would take 64 registers more than there are)
                     rescale(m_new);
                     sum[0] = sum[1] = make_float2(0.0f, 0.0f);
 #pragma unroll
                     for (int c = 0; c < 2; ++c) tmem_ld32(tmem_S(t) + lane_off + (uint32_t)(c * 32), s + c * 32);
                     tmem_ld_wait();
-                    s_read();
                     exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
                 }
             } else {
-                s_read();
                 if (limit < kN) {
 #pragma unroll
                     for (int c = 0; c < kN; ++c)
@@ -498,24 +417,18 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                         if (c < lo && c >= glim) s[c] = 0xff800000u;
                 }
                 const float m_new = fmaxf(m_ref, row_max(s) * p.scale_log2);
-                const bool again = outgrown(m_new);
-                if (j > 0) o_done();
-                if (!ok) break;
                 if (j == 0) m_ref = m_new;
-                else if (again) rescale(m_new);
+                else if (outgrown(m_new)) rescale(m_new);
                 neg_m = shift();
                 SNTL_TRACE_EV(tw, 1 + t, tn, 4);
                 exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
             }
-            tmem_st32(tmem_S(t) + kPOff + lane_off, pk);
-            if (kHalfP) {   // the P V product may start on the first 64 keys while the rest is computed
-                tmem_st_wait();
-                tc_fence_before();
-                mbar_arrive(&bars->p_half[t]);
-            }
+            tmem_st32(tmem_S(t) + lane_off, pk);
+            tmem_st_wait();     // the P V product may start on the first 64 keys while the rest is computed
+            tc_fence_before();
+            mbar_arrive(&bars->p_half[t]);
             exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, mx);
-            if (kOwnP) s_seen = j + 1 < n_mine && __all_sync(0xffffffffu, mbar_try_wait(&bars->s_ready[t], phase ^ 1u));
-            tmem_st32(tmem_S(t) + kPOff + lane_off + 32u, pk);
+            tmem_st32(tmem_S(t) + lane_off + 32u, pk);
             l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             SNTL_TRACE_EV(tw, 1 + t, tn, 5);
             tmem_st_wait();
@@ -524,7 +437,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             SNTL_TRACE_EV(tw, 1 + t, tn, 6);
         }
         if (ok && n_mine > 0)
-            ok = mbar_wait_prompt_warp(&bars->o_ready[t], kOwnP ? phase ^ 1u : blocks & 1u, abort_flag, kSiteOReady);
+            ok = mbar_wait_prompt_warp(&bars->o_ready[t], blocks & 1u, abort_flag, kSiteOReady);
         if (ok && n_mine > 0) {
             ++blocks;
             tc_fence_after();
@@ -602,6 +515,387 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
 }
 
+// ---- head_dim 64 ----
+// Bound by the exponentials: 2048 cycles of the special-function unit for two tiles of 128 x 128, beside 1280 of products.  With two
+// softmax warps per scheduler, one per query tile, a step of two tiles took 3490 cycles: both warps wait for products, load, store
+// and hand over about as long as they compute.  Here four warps per scheduler work on four independent chains (S 64 columns and O 64
+// columns each fill the TMEM; 104 registers are enough for 64 columns), and a step takes 2500 to 2600.
+// The two query tiles of a CTA are halves that share nothing but the TMEM allocation and the queue of blocks: the end of a block
+// (about 5000 cycles from its last exponentials to the first of the next) then passes under the other half's steps, no tile waits for
+// the longer row of another, and blocks of one tile balance better.
+// us, before -> now: B4 Hq32 Hkv8 S4096 377 -> 351; B8 Hq12 S1024 31.0 -> 28.5; B2 Hq32 S1024 23.2 -> 19.4; B16 Hq8 S130 7.8 -> 7.5; a 300-key
+// window over B4 Hq12 S2048 35.6 -> 35.7; few long rows, B1 Hq4 S8192, 71.8 -> 71.6.  Also measured: both tiles
+// fed by one MMA warp, 351, 28.2 and 27.9; two softmax warpgroups with two S buffers of 64 columns each, 436, 32.0 and 25.2.
+constexpr int kHalf = 64;             // keys of a tile that one stream takes
+constexpr int kStreamThreads = 640;   // four softmax warpgroups, and one holding the MMA and the TMA warps
+
+// One half of a CTA: blocks of one query tile, two softmax warpgroups ("streams": stream b has keys [64 b, 64 b + 64) of every key
+// tile), an MMA warp and a TMA warp.
+struct StreamHalf {
+    uint4 response;                   // of the block scheduler
+    uint64_t response_full, work_full[2], work_empty[2];
+    struct alignas(16) { int n, q0, bh, unused, g_tiles, w_first; } work[2];    // blocks in turn (see FwdWork); n: key tiles, -1: no more blocks
+    uint64_t q_full, q_empty, k0_full, pair_full[2], pair_empty[2];    // as in FwdBarriers
+    uint64_t s_ready[2];              // S_j of the stream is there, and P_{j-1} V has been added to O
+    uint64_t o_ready[2];              // the last P V of a block has been.  (A phase of s_ready instead could be over before it is seen: the
+                                      // next block's first S does not wait for the softmax warps.)
+    uint64_t p_ready[2];
+    uint64_t final_bar;
+    float2 ml[2][kM];                 // reference maximum and sum of a row, for its other stream
+};
+struct StreamShared {
+    StreamHalf half[2];
+    uint32_t tmem_base;
+    uint32_t abort_flag;
+    uint32_t asking, none_left;       // a lock, and what it guards: no request may follow one that has failed
+};
+
+template <int kMode, bool kMat>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                        const __grid_constant__ CUtensorMap tmap_v, const FwdParams p)
+{
+    constexpr int D = 64, kTileBytes = 128 * D * 2;
+    constexpr uint32_t kHalfBytes = kHalf * 128;    // of a K or V tile
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* sOut = smem + 10 * kTileBytes;           // 2 KB per softmax warp
+    StreamShared* shared = (StreamShared*)(sOut + (kMat ? 0 : kOutBytes));
+    volatile uint32_t* abort_flag = &shared->abort_flag;
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp-uniform for the compiler)
+    constexpr bool kWin = kMode != kPlain;
+    const int inst = warp < 16 ? warp >> 3 : (warp >> 1) & 1;    // warps 0-7 and 8-15: softmax; 16, 18: MMA; 17, 19: TMA
+    StreamHalf* bars = &shared->half[inst];
+    uint8_t* sQ = smem + inst * 5 * kTileBytes;       // [kTileBytes]
+    uint8_t* sK = sQ + kTileBytes;                    // [2][kTileBytes]
+    uint8_t* sV = sK + 2 * kTileBytes;                // [2][kTileBytes]
+
+    // ---- setup ----
+    if (warp >= 16 && (warp & 1) && lane == 0) {
+        prefetch_tensormap(&tmap_q);
+        prefetch_tensormap(&tmap_k);
+        prefetch_tensormap(&tmap_v);
+        mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->q_empty, 1);
+        mbar_init(&bars->k0_full, 1);
+        mbar_init(&bars->response_full, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->work_full[i], 1);
+            mbar_init(&bars->work_empty[i], 9);    // the issuing warp and the softmax warps
+            mbar_init(&bars->pair_full[i], 1);
+            mbar_init(&bars->pair_empty[i], 1);
+            mbar_init(&bars->s_ready[i], 1);
+            mbar_init(&bars->o_ready[i], 1);
+            mbar_init(&bars->p_ready[i], 128);
+        }
+        mbar_init(&bars->final_bar, 1);
+        shared->abort_flag = shared->asking = shared->none_left = 0;
+        fence_mbar_init();
+    }
+    if (warp == 16) {
+        tmem_alloc(&shared->tmem_base, kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = shared->tmem_base;
+    wait_for_stream();      // nothing before this reads or writes global memory
+    auto tmem_S = [&](int b) { return tmem + (uint32_t)(inst * 2 * kHalf + b * kHalf); };
+    auto tmem_O = [&](int b) { return tmem + 256u + (uint32_t)(inst * 2 * D + b * D); };
+
+    // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Counters of key
+    // tiles run on over the blocks, so stages and barrier phases continue where they are.
+    int2 win = make_int2(0, 0);   // its g_tiles, w_first
+    // A warp's copy of block u (work: n, q0, bh); false when there is none.  Every access to shared memory waits some 250 cycles
+    // behind the other warps' exponentials, so there are few of them, and the softmax warps take the next block before their epilogue.
+    auto get = [&](int u, int4& work) {
+        if (!mbar_wait_prompt_warp(&bars->work_full[u & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext)) return false;
+        work = *reinterpret_cast<const int4*>(&bars->work[u & 1]);
+        if (kWin) win = *reinterpret_cast<const int2*>(&bars->work[u & 1].g_tiles);
+        work.x = warp_uniform(work.x);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->work_empty[u & 1]);
+        return work.x >= 0;
+    };
+
+    // 640 threads start with 96 registers each
+    if (warp >= 16 && (warp & 1)) {
+        setmaxnreg_dec<64>();
+        // =========================== TMA producer ===========================
+        if (lane == 0) {
+            // A block of the grid that has not started, or -1.  Both producers of the CTA ask, one at a time: none may ask once the
+            // answer was that there are no more.
+            uint32_t asked = 0;
+            auto ask = [&]() {
+                if (!p.several_waves) return -1;
+                uint32_t spins = 0;
+                while (atomicCAS(&shared->asking, 0u, 1u) != 0u) {
+                    __nanosleep(40);
+                    if (*abort_flag || ++spins > (1u << 24)) return -1;
+                }
+                int block = -1;
+                if (!*(volatile uint32_t*)&shared->none_left) {
+                    mbar_arrive_expect_tx(&bars->response_full, 16);
+                    clc_try_cancel(&bars->response, &bars->response_full);
+                    if (mbar_wait_prompt(&bars->response_full, asked++ & 1u, abort_flag, kSiteNext)) block = clc_first_block(&bars->response);
+                    fence_proxy_async_smem();
+                    if (block < 0) *(volatile uint32_t*)&shared->none_left = 1u;
+                }
+                __threadfence_block();
+                atomicExch(&shared->asking, 0u);
+                return block;
+            };
+            FwdWork w{};
+            int c0 = 0, block = inst == 0 ? (int)blockIdx.x : ask();
+            for (int u = 0;; ++u) {
+                w.n0 = -1;
+                if (block >= 0) w.decode<kWin>(p, block);
+                const int n = w.n0;
+                if (u >= 2 && !mbar_wait_prompt(&bars->work_empty[u & 1], (uint32_t)(((u >> 1) - 1) & 1), abort_flag, kSiteNext)) break;
+                bars->work[u & 1] = {n, w.q0, w.bh, 0, w.g_tiles, w.w_first};
+                mbar_arrive(&bars->work_full[u & 1]);
+                if (block < 0) break;
+                auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int j) {
+                    tma_load_3d(dst + ((c0 + j) & 1) * kTileBytes, map, bar, 0, w.key_tile(j) * kN, w.bh_kv);
+                };
+                // Q and K_0 once the last S product of the block before has run: Q is free then, and K_0's stage and barrier were free
+                // before (the barrier must not be armed again while the K_0 before is on its way or unseen: rows of a single
+                // key tile get here that early)
+                if (u > 0 && !mbar_wait_prompt(&bars->q_empty, (uint32_t)((u - 1) & 1), abort_flag, kSiteQEmpty)) break;
+                mbar_arrive_expect_tx(&bars->k0_full, (uint32_t)kTileBytes);
+                load(sK, &tmap_k, &bars->k0_full, 0);
+                mbar_arrive_expect_tx(&bars->q_full, (uint32_t)kTileBytes);
+                tma_load_3d(sQ, &tmap_q, &bars->q_full, 0, w.q0, w.bh);
+                bool ok = true;
+                for (int j = 0; j < n; ++j) {
+                    // (as in attn_fwd_tc_kernel)
+                    const int c = c0 + j;
+                    if (c >= 1 && !(ok = mbar_wait_prompt(&bars->pair_empty[c & 1], (uint32_t)((c >> 1) - (c & 1 ? 0 : 1)) & 1u, abort_flag, kSitePairEmpty))) break;
+                    const bool k_too = j + 1 < n;
+                    mbar_arrive_expect_tx(&bars->pair_full[c & 1], (uint32_t)(k_too ? 2 * kTileBytes : kTileBytes));
+                    if (k_too) load(sK, &tmap_k, &bars->pair_full[c & 1], j + 1);
+                    load(sV, &tmap_v, &bars->pair_full[c & 1], j);
+                }
+                if (!ok) break;
+                c0 += n;
+                // (about two steps before this block ends: in time, and not so early that blocks would go to this CTA although others
+                // are free sooner)
+                block = ask();
+            }
+        }
+    } else if (warp >= 16) {
+        setmaxnreg_dec<64>();
+        // =========================== MMA issuer ===========================
+        auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) { return mbar_wait_prompt_warp(bar, parity, abort_flag, site); };
+        constexpr uint32_t idesc_s = make_idesc(kM, kHalf, false, false);
+        constexpr uint32_t idesc_pv = make_idesc(kM, D, false, true);
+        const uint64_t dq = make_sdesc(smem_u32(sQ), 16, 1024), dk = make_sdesc(smem_u32(sK), 16, 1024), dv = make_sdesc(smem_u32(sV), 16384, 1024);
+        auto issue_s = [&](int b, int st) {
+            mma_ss_4<2, 2>(tmem_S(b), dq, sdesc_advance(dk, (uint32_t)(st * kTileBytes) + (uint32_t)b * kHalfBytes), idesc_s, 0);
+            tc_commit_p(&bars->s_ready[b]);
+        };
+        int c0 = 0;                        // key tiles of the blocks before
+        bool ok = true;
+        int4 work;
+        for (int u = 0; ok && get(u, work); ++u) {
+            const int n = work.x;
+            if (!(ok = wait(&bars->k0_full, (uint32_t)(u & 1), kSiteK0) && wait(&bars->q_full, (uint32_t)(u & 1), kSiteQ))) break;
+            tc_fence_after();
+            // (S of the block before has been read and P over it consumed: this warp waited for p_ready and issued the product; O is
+            // overwritten behind p_ready of the new block, which its warps give after their epilogue)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) issue_s(b, c0 & 1);
+            tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
+            if (n == 1) tc_commit_p(&bars->q_empty);
+            for (int j = 0; ok && j < n; ++j) {
+                const int c = c0 + j;
+                if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    if (!ok || !(ok = wait(&bars->p_ready[b], (uint32_t)(c & 1), kSitePReady))) continue;
+                    tc_fence_after();
+                    mma_ts_4<8, 128>(tmem_O(b), tmem_S(b), sdesc_advance(dv, (uint32_t)((c & 1) * kTileBytes) + (uint32_t)b * kHalfBytes), idesc_pv, j > 0);
+                    if (j + 1 < n) issue_s(b, (c + 1) & 1);
+                    else tc_commit_p(&bars->o_ready[b]);
+                }
+                if (!ok) break;
+                if (j + 1 < n) tc_commit_p(&bars->pair_empty[c & 1]);
+                if (j + 2 == n) tc_commit_p(&bars->q_empty);
+            }
+            c0 += n;
+        }
+        // every MMA issued above must have retired before shared memory / TMEM are given up
+        tc_commit_p(&bars->final_bar);
+        wait(&bars->final_bar, 0, kSiteFinal);
+    } else {
+        // =========================== softmax + epilogue warpgroups ===========================
+        setmaxnreg_inc<104>();
+        const int half = (warp >> 2) & 1;
+        const int row = (warp & 3) * 32 + lane;        // row inside the tile == TMEM lane
+        const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+        const uint32_t tmS = tmem_S(half) + lane_off, tmO = tmem_O(half) + lane_off;
+        bool ok = true;
+        uint32_t phase = 0, blocks = 0;                // of s_ready, of o_ready
+        int4 work;
+        bool more = get(0, work);
+        for (int u = 0; more; ++u) {
+            const int n_mine = work.x, q0 = work.y, bh = work.z;
+            const int g_tiles = kWin ? win.x : 0, w_first = kWin ? win.y : 0;
+            const int grow = q0 + row;                 // query row inside the (batch, head) slab
+            const int row_lo = q0 + (warp & 3) * 32;   // first row of the warp
+            float m_ref = -INFINITY, l = 0.0f;
+            for (int j = 0; j < n_mine; ++j) {
+                if (!(ok = mbar_wait_prompt_warp(&bars->s_ready[half], phase, abort_flag, kSiteSReady))) break;
+                phase ^= 1u;
+                tc_fence_after();
+                uint32_t s[kHalf];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) tmem_ld32(tmS + (uint32_t)(c * 32), s + c * 32);
+                tmem_ld_wait();
+                // number of visible keys of this row among these
+                const int key0 = (j < g_tiles ? j : w_first + (j - g_tiles)) * kN + half * kHalf;
+                const int limit_lo = (p.causal ? min(p.Skv, row_lo + 1) : p.Skv) - key0;
+                const int lo_hi = kWin ? row_lo + 31 - p.window + 1 - key0 : 0, glim = kWin ? p.global_tokens - key0 : 0;
+                const bool cut = limit_lo < kHalf || (kWin && lo_hi > 0 && glim < min(lo_hi, kHalf));   // (some row of the warp is)
+                uint32_t pk[32];
+                float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                auto shift = [&]() { return m_ref == -INFINITY ? 0.0f : -m_ref; };   // (no finite score so far: -inf + inf would be NaN)
+                // whether some row of the warp has outgrown its reference (false when both are -inf: NaN compare)
+                auto outgrown = [&](float m_new) { return __any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold); };
+                // Keys that the mask does not cut are exponentiated against the row's reference at once, with their maximum taken on the
+                // way (see attn_fwd_tc_kernel)
+                bool done = j > 0 && !cut;
+                if (done) {
+                    RowMax mx;
+                    exp_row<true>(s, p.scale_log2, shift(), pk, sum, mx);
+                    if (outgrown(fmaxf(m_ref, mx.value() * p.scale_log2))) {
+                        done = false;
+                        sum[0] = sum[1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) tmem_ld32(tmS + (uint32_t)(c * 32), s + c * 32);
+                        tmem_ld_wait();
+                    }
+                }
+                if (!done) {
+                    if (cut) {
+                        const int limit = (p.causal ? min(p.Skv, grow + 1) : p.Skv) - key0;
+#pragma unroll
+                        for (int c = 0; c < kHalf; ++c)
+                            if (c >= limit) s[c] = 0xff800000u;  // -inf
+                        const int lo = kWin ? grow - p.window + 1 - key0 : 0;
+                        if (kWin && lo > 0 && glim < min(lo, kHalf)) {      // keys below the window that are no global tokens
+#pragma unroll
+                            for (int c = 0; c < kHalf; ++c)
+                                if (c < lo && c >= glim) s[c] = 0xff800000u;
+                        }
+                    }
+                    const float m_new = fmaxf(m_ref, row_max(s) * p.scale_log2);
+                    if (j == 0) {
+                        m_ref = m_new;
+                    } else if (outgrown(m_new)) {
+                        // O and the sum of a row whose maximum has outgrown its reference (S_j was issued behind the product of P_{j-1})
+                        const bool need = (m_new - m_ref) > kRescaleThreshold;
+                        const float factor = need ? ex2(m_ref - m_new) : 1.0f;
+                        if (need) m_ref = m_new;
+                        l *= factor;
+#pragma unroll 1
+                        for (int c = 0; c < D / 8; ++c) {
+                            uint32_t o[8];
+                            tmem_ld8(tmO + (uint32_t)(c * 8), o);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+                            tmem_st8(tmO + (uint32_t)(c * 8), o);
+                        }
+                        tmem_st_wait();
+                    }
+                    RowMax unused;
+                    exp_row<false>(s, p.scale_log2, shift(), pk, sum, unused);
+                }
+                tmem_st32(tmS, pk);      // over S
+                l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(&bars->p_ready[half]);
+            }
+            if (!ok) break;
+            more = get(u + 1, work);
+            if (!(ok = mbar_wait_prompt_warp(&bars->o_ready[half], blocks, abort_flag, kSiteOReady))) break;
+            blocks ^= 1u;
+            // The two streams of a row are added here; each stores one half of the features.
+            bars->ml[half][row] = make_float2(m_ref, l);
+            tc_fence_before();
+            named_barrier_sync(1 + inst, 256);
+            tc_fence_after();
+            const float2 ml = bars->ml[half ^ 1][row];
+            uint32_t o[2][32];
+            tmem_ld32(tmO + (uint32_t)(half * 32), o[0]);
+            tmem_ld32(tmem_O(half ^ 1) + lane_off + (uint32_t)(half * 32), o[1]);
+            const float m = fmaxf(m_ref, ml.x);
+            float f0 = m_ref == -INFINITY ? 0.0f : ex2(m_ref - m), f1 = ml.x == -INFINITY ? 0.0f : ex2(ml.x - m);
+            // (the same order of the two in both, for the same bits)
+            const float total = half == 0 ? fmaf(l, f0, ml.y * f1) : fmaf(ml.y, f1, l * f0);
+            const float inv = total > 0.0f ? 1.0f / total : 0.0f;
+            f0 *= inv;
+            f1 *= inv;
+            tmem_ld_wait();
+            tc_fence_before();
+            named_barrier_sync(1 + inst, 256);      // the next block's first products may overwrite O
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[0][i] = __float_as_uint(fmaf(__uint_as_float(o[0][i]), f0, __uint_as_float(o[1][i]) * f1));
+            const bool store = grow < p.Sq;
+            if constexpr (kMat) {
+                // feature-major matrices: the 32 rows of a warp are 128 contiguous bytes of every feature's row
+                const int b = bh / p.Hq, h = bh - b * p.Hq;
+                float* dst = p.o_mat + (long long)(h * D + half * 32) * p.mat_stride + (long long)b * p.Sq + grow;
+                if (store) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) dst[i * p.mat_stride] = __uint_as_float(o[0][i]);
+                    if (half == 0)
+                        p.lse_mat[(long long)h * p.mat_stride + (long long)b * p.Sq + grow] = total > 0.0f ? (m + log2f(total)) * 0.6931471805599453f : -INFINITY;
+                }
+            } else {
+                // Through 2 KB of shared memory of the warp's own, so that a store instruction covers 64 bytes of each of eight rows; 16-byte
+                // units are XOR-swizzled by the row so that both sides spread over the banks.
+                uint8_t* stage = sOut + warp * 2048;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    uint4 v;
+                    v.x = pack_bf16(__uint_as_float(o[0][8 * i + 0]), __uint_as_float(o[0][8 * i + 1]));
+                    v.y = pack_bf16(__uint_as_float(o[0][8 * i + 2]), __uint_as_float(o[0][8 * i + 3]));
+                    v.z = pack_bf16(__uint_as_float(o[0][8 * i + 4]), __uint_as_float(o[0][8 * i + 5]));
+                    v.w = pack_bf16(__uint_as_float(o[0][8 * i + 6]), __uint_as_float(o[0][8 * i + 7]));
+                    *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = v;
+                }
+                __syncwarp();
+                __nv_bfloat16* dst = p.o + (size_t)bh * p.Sq * D;
+                const int sub = lane >> 2, unit = lane & 3, warp_row0 = grow - lane;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int r = i * 8 + sub;
+                    const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 64 + ((unit ^ ((r >> 1) & 3)) << 4));
+                    if (warp_row0 + r < p.Sq) *reinterpret_cast<uint4*>(dst + (size_t)(warp_row0 + r) * D + half * 32 + unit * 8) = v;
+                }
+                __syncwarp();
+                if (store && half == 0) p.lse[(size_t)bh * p.Sq + grow] = total > 0.0f ? (m + log2f(total)) * 0.6931471805599453f : -INFINITY;
+            }
+        }
+    }
+
+    // ---- teardown ----
+    if (*abort_flag) {
+        for (int i = 0; i < 64; ++i) __nanosleep(2000);      // (see attn_fwd_tc_kernel)
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 16) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kTmemCols);
+    }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -620,11 +914,10 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-// Two query tiles per CTA overlap one tile's softmax with the other's products; on a grid that leaves SMs idle or ends with one
-// long CTA, one tile per CTA finishes sooner: a step of one tile takes 0.7 (head_dim 64) or 0.83 (128) of a step of two.  The
-// estimate counts steps of two tiles: the longest CTA, or the SMs' average load and a short tail, with 1.3 steps per CTA of
-// set-up.  Cold, B1 Hq8 S2048: 33 -> 28 us at head_dim 128, 30 -> 21 at 64; B1 Hq4 S8192 D128 110 -> 92; equal at 128 CTAs of
-// 1024 rows, worse beyond (B8 Hq12 S1024 D64 37 -> 49).
+// head_dim 128.  Two query tiles per CTA overlap one tile's softmax with the other's products; on a grid that leaves SMs idle or ends
+// with one long CTA, one tile per CTA finishes sooner: a step of one tile takes 0.83 of a step of two.  The estimate counts steps of two
+// tiles: the longest CTA, or the SMs' average load and a short tail, with 1.3 steps per CTA of set-up.  Cold, B1 Hq8 S2048: 33 -> 28
+// us; B1 Hq4 S8192 110 -> 92.
 int fwd_tiles_per_cta(const AttnShape& s)
 {
     const int n = (s.Sq + kM - 1) / kM, n_keys = (s.Skv + kN - 1) / kN, heads = s.B * s.Hq, sms = sm_count();
@@ -637,15 +930,11 @@ int fwd_tiles_per_cta(const AttnShape& s)
         one += steps(i);
         if (i + 1 == n || (i & 1)) two += steps(i);
     }
-    const double cost = s.D == 64 ? 0.7 : 0.83, set_up = 1.3, longest = steps(n - 1);
+    const double cost = 0.83, set_up = 1.3, longest = steps(n - 1);
     const double t2 = std::max(longest + set_up, (two * heads + set_up * pairs) / sms + 0.1 * longest);
     const double t1 = std::max(cost * longest + set_up, (cost * one + set_up * n) * heads / sms + 0.1 * cost * longest);
     return t1 < 0.95 * t2 ? 1 : 2;
 }
-
-// Which kernels have a form that takes over blocks, for grids of more than one wave.  The plain one at head_dim 128 has not: its
-// softmax loop fills the registers, and with the bookkeeping it spills (B2 Hq28 Hkv4 S8192 737 -> 768 us).
-template <int D, int kMode> constexpr bool kTakesOver = D == 64 || kMode == kWindow;
 
 template <int D, int kMode, bool kMat>
 cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
@@ -664,21 +953,25 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     p.causal = s.causal;
     p.window = s.causal ? s.window : 0;
     p.global_tokens = s.global_tokens;
-    p.tiles_per_cta = fwd_tiles_per_cta(s);
+    p.tiles_per_cta = D == 64 ? 1 : fwd_tiles_per_cta(s);
     p.n_qblk = (s.Sq + p.tiles_per_cta * kM - 1) / (p.tiles_per_cta * kM);
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const long long ctas = (long long)p.n_qblk * s.B * s.Hq;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    const size_t smem = 6 * (size_t)(128 * D * 2) + (kMat ? 0 : kOutBytes) + sizeof(FwdBarriers) + 1024;
+    p.several_waves = ctas > sm_count();
+    const size_t smem = (D == 64 ? 10 : 6) * (size_t)(128 * D * 2) + (kMat ? 0 : kOutBytes) + (D == 64 ? sizeof(StreamShared) : sizeof(FwdBarriers)) + 1024;
     auto launch = [&](auto kernel, std::atomic<unsigned long long>& configured) {
         const cudaError_t err = ensure_dynamic_smem(kernel, smem, configured);
-        return err != cudaSuccess ? err : launch_kernel(kernel, (unsigned)ctas, kFwdThreads, smem, st, 1, tq, tk, tv, p);
+        return err != cudaSuccess ? err : launch_kernel(kernel, (unsigned)ctas, D == 64 ? kStreamThreads : kFwdThreads, smem, st, 1, tq, tk, tv, p);
     };
     static std::atomic<unsigned long long> configured_one{0}, configured_many{0};   // per instantiation, one bit per device
-    if constexpr (kTakesOver<D, kMode>) {
-        if (ctas > sm_count()) return launch(attn_fwd_tc_kernel<D, kMode, kMat, true>, configured_many);
+    if constexpr (D == 64) {
+        return launch(attn_fwd_streams_kernel<kMode, kMat>, configured_one);
+    } else {
+        if constexpr (kMode == kWindow)
+            if (p.several_waves) return launch(attn_fwd_tc_kernel<D, kMode, kMat, true>, configured_many);
+        return launch(attn_fwd_tc_kernel<D, kMode, kMat, false>, configured_one);
     }
-    return launch(attn_fwd_tc_kernel<D, kMode, kMat, false>, configured_one);
 }
 
 }  // namespace

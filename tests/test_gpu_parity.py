@@ -443,6 +443,37 @@ def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
         assert float((got.float() - want).norm() / want.norm()) <= tol
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,kw", [
+    (1, 1, 1, 1, 1, {}), (1, 2, 1, 64, 64, {}), (1, 2, 2, 65, 65, {}), (2, 3, 1, 128, 128, {}), (1, 2, 1, 129, 129, {}),   # edges of the key halves
+    (1, 2, 1, 200, 70, dict(causal=False)), (1, 2, 1, 70, 193, dict(causal=False)), (1, 1, 1, 130, 64, dict(causal=False)),
+    (5, 16, 4, 250, 250, {}),                                        # 160 blocks: a second half of a few CTAs has one
+    (9, 12, 12, 700, 700, {}),                                       # 648: every half takes over blocks
+    (6, 8, 2, 640, 640, dict(window=64)), (6, 8, 2, 650, 650, dict(window=65, global_tokens=3)), (4, 8, 8, 900, 900, dict(window=200, global_tokens=130)),
+])
+def test_head_dim_64_forward_streams(sb, B, Hq, Hkv, Sq, Sk, kw):
+    """The two streams of a row (64 keys of every key tile each) and the two halves of a CTA against fp64: rows whose first key tile
+    leaves one stream without a visible key, ragged ends in either half, blocks taken over; and large scores, for which the streams
+    rescale at different tiles."""
+    g = torch.Generator(device="cuda").manual_seed(Sq + B)
+    for std in (0.5, 6.0):
+        q, k, v = ((torch.randn(B, H, S, 64, generator=g, device="cuda") * x).to(torch.bfloat16) for H, S, x in ((Hq, Sq, std), (Hkv, Sk, std), (Hkv, Sk, 1.0)))
+        o, lse = sb.attention_forward(q, k, v, **kw)
+        assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+        kd, vd = (t.double().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+        s = q.double() @ kd.transpose(2, 3) * 64 ** -0.5
+        if kw.get("causal", True):
+            i, j = torch.arange(Sq, device="cuda")[:, None], torch.arange(Sk, device="cuda")[None, :]
+            seen = j <= i
+            if kw.get("window"):
+                seen &= (i - j < kw["window"]) | (j < kw.get("global_tokens", 0))
+            s = s.masked_fill(~seen, float("-inf"))
+        want = s.softmax(3) @ vd
+        assert float((lse.double() - s.logsumexp(3)).abs().max()) <= 2e-2
+        # P and O are rounded to bf16 once each, by 2^-8 of a weight and of a result at most
+        assert float((o.double() - want).norm() / want.norm()) <= BF16_REL
+        assert float((o.double() - want).abs().max()) <= 2.0 ** -7 * float(v.abs().max())
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,kw", [
     (40, 8, 8, 100, 100, 64, {}),                                 # 320 blocks of one step each
     (30, 6, 6, 129, 129, 128, {}),                                # one- and two-step blocks, the last with one query

@@ -6,7 +6,8 @@
 // asynchronous 16-byte copies, scores one key per thread, and accumulates P V with the lanes along the features while every
 // warp takes a quarter of the keys.  Partial (m, l, O) merge through distributed shared memory: one launch, no scratch.
 // 1 token x 777 keys x 12 heads, head_dim 64: 165 us with one warp per row, 11.7 us through the 16-row tiles of
-// attn_simt_fwd.cu (15 of 16 rows empty), 5 us here.
+// attn_simt_fwd.cu (15 of 16 rows empty), 5.1 us here (6.4 when the merge went through distributed shared memory once per peer and a
+// score was one chain of FMAs; 2000 keys x 4 sequences 11.9 -> 11.1, 100 keys 4.6 -> 4.0, 2 x 2048 keys of head_dim 128 14.1 -> 12.6).
 #include "attn_simt.cuh"
 
 #include <cooperative_groups.h>
@@ -19,6 +20,7 @@ namespace {
 
 constexpr int kChunk = kThreads;   // keys per pass: one per thread
 constexpr int kWarps = kThreads / 32;
+constexpr int kMaxSplit = 8;       // CTAs of a cluster
 
 template <int DP, int R> struct DecodeSmem {
     static constexpr int P = DP + 4;
@@ -90,18 +92,21 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
         for (int r = 0; r < R; ++r) sc[r] = 0.f;
         if ((int)threadIdx.x < n) {
             const float* kr = smem + L::k + threadIdx.x * L::P;
+            float part[R][4] = {};       // four chains of FMAs instead of one
 #pragma unroll 8
             for (int d = 0; d < DP; d += 4) {
                 const float4 x = *reinterpret_cast<const float4*>(kr + d);
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const float4 y = *reinterpret_cast<const float4*>(smem + L::q + r * DP + d);
-                    sc[r] = fmaf(x.x, y.x, sc[r]);
-                    sc[r] = fmaf(x.y, y.y, sc[r]);
-                    sc[r] = fmaf(x.z, y.z, sc[r]);
-                    sc[r] = fmaf(x.w, y.w, sc[r]);
+                    part[r][0] = fmaf(x.x, y.x, part[r][0]);
+                    part[r][1] = fmaf(x.y, y.y, part[r][1]);
+                    part[r][2] = fmaf(x.z, y.z, part[r][2]);
+                    part[r][3] = fmaf(x.w, y.w, part[r][3]);
                 }
             }
+#pragma unroll
+            for (int r = 0; r < R; ++r) sc[r] = (part[r][0] + part[r][1]) + (part[r][2] + part[r][3]);
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -143,7 +148,7 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
             for (int c = 0; c < kCols; ++c) acc[r][c] *= corr[r];
         }
         const int j_end = min(n, warp * 32 + 32);
-#pragma unroll 4
+#pragma unroll 8
         for (int j = warp * 32; j < j_end; ++j) {
             float v[kCols];
             load_vec<kCols>(v, smem + L::v + j * L::P + lane * kCols);
@@ -178,14 +183,27 @@ __global__ void __launch_bounds__(kThreads) simt_decode_kernel(const SimtArgs a,
     cluster.sync();
     for (int u = rank * kThreads + threadIdx.x; u < rows * DP; u += n_split * kThreads) {
         const int r = u / DP, d = u % DP;
+        // every peer's values are asked for before the first is used: one trip through distributed shared memory, not one per peer
+        float pm[kMaxSplit], pl[kMaxSplit], po[kMaxSplit];
+#pragma unroll
+        for (int p = 0; p < kMaxSplit; ++p)
+            if (p < n_split) {
+                const float* peer = cluster.map_shared_rank(smem, p);
+                pm[p] = peer[L::ml + r];
+                pl[p] = peer[L::ml + R + r];
+                po[p] = peer[L::out + u];
+            }
         float mx = -INFINITY, sum = 0.f, x = 0.f;
-        for (int p = 0; p < n_split; ++p) mx = fmaxf(mx, cluster.map_shared_rank(smem, p)[L::ml + r]);
-        for (int p = 0; p < n_split && mx > -INFINITY; ++p) {
-            const float* peer = cluster.map_shared_rank(smem, p);
-            const float w = expf(peer[L::ml + r] - mx);
-            sum = fmaf(w, peer[L::ml + R + r], sum);
-            x = fmaf(w, peer[L::out + u], x);
-        }
+#pragma unroll
+        for (int p = 0; p < kMaxSplit; ++p)
+            if (p < n_split) mx = fmaxf(mx, pm[p]);
+#pragma unroll
+        for (int p = 0; p < kMaxSplit; ++p)
+            if (p < n_split && mx > -INFINITY) {
+                const float w = expf(pm[p] - mx);
+                sum = fmaf(w, pl[p], sum);
+                x = fmaf(w, po[p], x);
+            }
         ((float*)a.o_out)[row_offset(r) + d] = sum > 0.f ? x / sum : 0.f;
         if (d == 0)
             a.lse_out[b * a.vlse.sb + (hk * group + r / s.Sq) * a.vlse.sh + (long long)(r % s.Sq) * a.vlse.ss] =
@@ -205,7 +223,7 @@ cudaError_t launch(const SimtArgs& a, cudaStream_t st)
     // split the keys while CTAs are fewer than about three per SM and a piece keeps at least half a pass of keys
     const long long slabs = (long long)a.s.B * a.s.Hkv;
     int split = 1;
-    while (split < 8 && slabs * split * 2 <= 3 * sm_count() && a.s.Skv >= split * kChunk) split *= 2;
+    while (split < kMaxSplit && slabs * split * 2 <= 3 * sm_count() && a.s.Skv >= split * kChunk) split *= 2;
     return launch_kernel(kernel, (unsigned)(slabs * split), kThreads, L::bytes, st, split, a, split);
 }
 

@@ -6,7 +6,7 @@
 // online softmax, O = P V, LSE = m + ln(l) -- re-designed for Blackwell:
 //
 //   * head_dim 128 (attn_fwd_tc_kernel): one CTA owns 256 (small grids: 128) consecutive query rows of one (batch, head) as two
-//     128-row tiles; each tile has its own softmax warpgroup (one thread per query row: tcgen05.ld's 32x32b shape hands thread i
+//     128-row tiles, whose key tiles are taken in halves of 64 keys; each tile has its own softmax warpgroup (one thread per query row: tcgen05.ld's 32x32b shape hands thread i
 //     row i, so the row max / row sum need no shuffles) while a single MMA-issuing warp (one elected lane) feeds the tensor core
 //     for both, so one tile's softmax overlaps the other tile's MMAs;
 //   * head_dim 64 (attn_fwd_streams_kernel): four softmax warpgroups, each with 64 of the 128 keys of every key tile and sums and
@@ -23,7 +23,8 @@
 //     heads of one group are adjacent in launch order so they share K/V tiles in L2.
 //
 // Layout: bf16 token-major [B][H][S][D], D in {64,128}; LSE [B][Hq][Sq] fp32 (natural log).
-// TMEM map (512 columns): head_dim 128 S0 [0,128) S1 [128,256) O0 [256,384) O1 [384,512); head_dim 64 four S of 64, then four O of 64.
+// TMEM map (512 columns): head_dim 128 two S of 64 columns for each tile, O0 [256,384) O1 [384,512); head_dim 64 four S of
+// 64, then four O of 64.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_tile.cuh"
@@ -39,6 +40,7 @@ namespace {
 
 constexpr int kM = 128;          // query rows per tile
 constexpr int kN = 128;          // keys per tile
+constexpr int kHalf = 64;        // keys of a tile per S product: one S buffer, or one stream
 constexpr int kFwdThreads = 384; // 2 softmax warpgroups + 1 warpgroup holding the MMA warp and the TMA warp
 constexpr uint32_t kTmemCols = 512;
 constexpr int kOutBytes = 8 * 4096;        // staging of O
@@ -64,7 +66,8 @@ struct FwdParams {
 
 // What one block of the grid computes.  A CTA computes its own block and then takes over blocks that have not started yet (as the
 // backward does): K, Q and the first S of one come in under the last softmax passes and the epilogue of the one before.
-// Cold: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108 us.
+// us: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108; B8 Hq28 Hkv4 S1024 D128 88.0 -> 71.9, B8 Hq16 S512 20.2 -> 18.3, B2 Hq16 Hkv4 S3000
+// 73.2 -> 69.6.
 struct FwdWork {
     int bh, bh_kv, q0;         // q0: first of the one or two 128-row tiles
     int g_tiles, w_first;      // key tiles in ascending order: the g_tiles tiles holding global tokens, then from w_first up to the
@@ -105,9 +108,10 @@ struct FwdBarriers {
     // Loads come in pairs {K_{j+1}, V_j} (K_0 alone first) and are released in the same pairs, {K_0} counting as pair -1: one
     // wait and one commit per key tile for the issuing warp instead of two each.  Barrier j & 1.
     uint64_t pair_full[2], pair_empty[2];
-    uint64_t s_ready[2], p_ready[2];
-    uint64_t o_ready[2];     // after the tile's last P V product (s_ready covers the others)
-    uint64_t p_half[2];      // the first 64 columns of P_t are written
+    // [tile][S buffer].  s_ready: S is there, and the product of the P that was in the buffer before has been added to O; buffer 0
+    // once more behind the last P that was in it.
+    uint64_t s_ready[2][2], p_ready[2][2];
+    uint64_t o_ready[2];     // the tile's last P V product has been added
     uint64_t final_bar;
     uint32_t tmem_base;
     uint32_t abort_flag;
@@ -118,8 +122,15 @@ struct FwdBarriers {
 enum FwdMode : int { kPlain = 0, kWindow = 1 };
 
 // kMat: O and LSE leave as fp32 feature-major matrices
-// kMany: CTAs take over blocks (FwdWork); without it each computes its own and the bookkeeping folds away.  The plain kernel has no
-// such form: its softmax loop fills the registers, and with the bookkeeping it spills (B2 Hq28 Hkv4 S8192 737 -> 768 us).
+// kMany: CTAs take over blocks (FwdWork); without it each computes its own and the bookkeeping folds away
+//
+// Bound by the chain of one tile between two of its softmax passes, beside 2048 cycles of exponentials and 2560 of products per step of two
+// tiles.  A key tile is taken as two halves of 64 keys, each with an S buffer of its own and its P written over it: while a
+// half is exponentiated, the other's P V and the S of the half after it run, which took the P V and S products (about 1150 cycles per
+// step) out of that chain.  S products of 64 keys are bound by their operands in shared memory (48 cycles per k-step instead of 32).
+// With 128 keys per S product, us, before -> now: B1 Hq4 S8192 88.0 -> 71.2 (one block per SM), B8 Hq16 S512 21.7 -> 20.2, B3 Hq16
+// Hkv4 S1237 28.7 -> 27.3, B8 Hq28 Hkv4 S1024 92.6 -> 88.0, B2 Hq28 Hkv4 S8192 within its spread (at the power limit: 1600 MHz).  64 columns
+// in registers instead of 128 also leave room for taking over blocks.
 template <int D, int kMode, bool kMat, bool kMany>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -158,9 +169,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             mbar_init(&bars->work_empty[i], 9);    // the issuing warp and the softmax warps
             mbar_init(&bars->pair_full[i], 1);
             mbar_init(&bars->pair_empty[i], 1);
-            mbar_init(&bars->s_ready[i], 1);
-            mbar_init(&bars->p_ready[i], 128);
-            mbar_init(&bars->p_half[i], 128);
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(&bars->s_ready[i][b], 1);
+                mbar_init(&bars->p_ready[i][b], 128);
+            }
             mbar_init(&bars->o_ready[i], 1);
         }
         mbar_init(&bars->final_bar, 1);
@@ -176,11 +188,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
     wait_for_stream();      // nothing before this reads or writes global memory
-    // P is written over S, so a tile's P V product and next S stay in the chain between two of its softmax passes; the first half of
-    // P V is issued as soon as the first 64 columns of P are written (-6 %).
     // (computed, not looked up: a two-element array indexed by the warp's tile would live in local memory)
-    auto tmem_S = [&](int t) { return tmem + (uint32_t)t * 128u; };
-    auto tmem_O = [&](int t) { return tmem + 256u + (uint32_t)t * 128u; };
+    auto tmem_S = [&](int t, int b) { return tmem + (uint32_t)(t * kN + b * kHalf); };
+    auto tmem_O = [&](int t) { return tmem + 256u + (uint32_t)(t * D); };
 
     // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Counters of key
     // tiles run on over the blocks (all of them: c0; those of tile t: its steps), so stages and barrier phases continue where they
@@ -197,9 +207,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
     // 384 threads start with 168 registers each; each role re-allocates inside its own branch
     if (warp >= 10) {
-        setmaxnreg_dec<72>();   // idle warps of the last warpgroup
+        setmaxnreg_dec<104>();   // idle warps of the last warpgroup
     } else if (warp == 9) {
-        setmaxnreg_dec<72>();
+        setmaxnreg_dec<104>();
         // =========================== TMA producer ===========================
         if (lane == 0) {
             int c0 = 0;
@@ -251,7 +261,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
         }
     } else if (warp == 8) {
-        setmaxnreg_dec<72>();
+        setmaxnreg_dec<104>();
         // =========================== MMA issuer ===========================
         // All 32 lanes walk the loops (warp-uniform control flow keeps descriptors and addresses in uniform registers) and
         // one elected lane issues each tcgen05 instruction.
@@ -262,69 +272,62 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             const bool tl8 = lane == 0;
             (void)tl8;
             SNTL_TRACE_DECL(tn);
-            constexpr uint32_t idesc_s = make_idesc(kM, kN, false, false);
+            constexpr uint32_t idesc_s = make_idesc(kM, kHalf, false, false);
             constexpr uint32_t idesc_pv = make_idesc(kM, D, false, true);
+            constexpr uint32_t kHalfBytes = kHalf * 128;    // of a K or V tile's 64-column chunk
             // one descriptor per tile, advanced per k-step by a 64-bit add
-            const uint64_t dq0 = make_sdesc(smem_u32(sQ), 16, 1024), dq1 = sdesc_advance(dq0, kTileBytes);
-            const uint64_t dk0 = make_sdesc(smem_u32(sK), 16, 1024), dk1 = sdesc_advance(dk0, kTileBytes);
-            const uint64_t dv0 = make_sdesc(smem_u32(sV), kChunkBytes, 1024), dv1 = sdesc_advance(dv0, kTileBytes);
-            auto issue_s = [&](int t, int st) {
-                const uint64_t a = t ? dq1 : dq0, b = st ? dk1 : dk0;
+            const uint64_t dq = make_sdesc(smem_u32(sQ), 16, 1024), dk = make_sdesc(smem_u32(sK), 16, 1024);
+            const uint64_t dv = make_sdesc(smem_u32(sV), kChunkBytes, 1024);
+            auto issue_s = [&](int t, int b, int st) {
+                const uint64_t q = sdesc_advance(dq, (uint32_t)(t * kTileBytes)), k = sdesc_advance(dk, (uint32_t)st * kTileBytes + (uint32_t)b * kHalfBytes);
 #pragma unroll
                 for (int c = 0; c < kChunks; ++c)
-                    mma_ss_4<2, 2>(tmem_S(t), sdesc_advance(a, (uint32_t)(c * kChunkBytes)), sdesc_advance(b, (uint32_t)(c * kChunkBytes)), idesc_s, c > 0);
-                tc_commit_p(&bars->s_ready[t]);
-            };
-            // P V in two halves of the contraction: the first four k-steps need only the first 64 columns of P (p_half, which the caller
-            // has waited for), the rest the whole of it (p_ready) -- so half the product is issued while the softmax warps still compute
-            // the second half of their exponentials.  Returns false when a wait gave up.
-            auto issue_pv = [&](int t, int st, bool accumulate, uint32_t parity) {
-                const uint64_t b = st ? dv1 : dv0;
-                const uint32_t d = tmem_O(t), a = tmem_S(t);
-                mma_ts_4<8, 128>(d, a, b, idesc_pv, accumulate);
-                if (!wait(&bars->p_ready[t], parity, kSitePReady)) return false;
-                tc_fence_after();
-                mma_ts_4<8, 128>(d, a + 32u, sdesc_advance(b, 4 * 2048), idesc_pv, 1);
-                return true;
+                    mma_ss_4<2, 2>(tmem_S(t, b), sdesc_advance(q, (uint32_t)(c * kChunkBytes)), sdesc_advance(k, (uint32_t)(c * kChunkBytes)), idesc_s, c > 0);
             };
             int c0 = 0, s0 = 0, s1 = 0;        // key tiles of the blocks before: all, those of tile 0, of tile 1
             bool ok = true, more = true;
             for (int u = 0; more; more = next(u++)) {
-            const int n0 = uniform(work(u).n0), n1 = uniform(work(u).n1), n_max = max(n0, n1);
-            if (!(ok = wait(&bars->k0_full, (uint32_t)(u & 1), kSiteK0) && wait(&bars->q_full, (uint32_t)(u & 1), kSiteQ))) break;
-            tc_fence_after();
-            // (S of the last step of the block before has been read, and P over it consumed: this warp waited for p_ready and issued
-            // the product; O is overwritten behind p_ready of the new block, which its warps give after their epilogue)
-            issue_s(0, c0 & 1);          // (a block has rows in its first tile)
-            // P is written over S: a tile's P V product, then its next S, as its P arrives
-            if (n1 > 0) issue_s(1, c0 & 1);
-            tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
-            if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
-            for (int j = 0; ok && j < n_max; ++j) {
-                const int c = c0 + j;
-                if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
+                const int n0 = uniform(work(u).n0), n1 = uniform(work(u).n1), n_max = max(n0, n1);
+                if (!(ok = wait(&bars->k0_full, (uint32_t)(u & 1), kSiteK0) && wait(&bars->q_full, (uint32_t)(u & 1), kSiteQ))) break;
+                tc_fence_after();
+                // (S of the last step of the block before has been read, and P over it consumed: this warp waited for p_ready and issued
+                // the product; O is overwritten behind p_ready of the new block, which its warps give after their epilogue)
 #pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const int n = t ? n1 : n0;
-                    const uint32_t parity = (uint32_t)(((t ? s1 : s0) + j) & 1);
-                    if (!ok || j >= n) continue;
-                    if (!(ok = wait(&bars->p_half[t], parity, kSitePReady))) continue;
-                    SNTL_TRACE_EV(tl8, 0, tn, 10 + t);
-                    tc_fence_after();
-                    if (!(ok = issue_pv(t, c & 1, j > 0, parity))) continue;
-                    SNTL_TRACE_EV(tl8, 0, tn, 20 + t);
-                    if (j + 1 < n) issue_s(t, (c + 1) & 1);
-                    else tc_commit_p(&bars->o_ready[t]);
-                    SNTL_TRACE_EV(tl8, 0, tn, 30 + t);
+                for (int b = 0; b < 2; ++b)
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+                        if (t == 0 || n1 > 0) {      // (a block has rows in its first tile)
+                            issue_s(t, b, c0 & 1);
+                            tc_commit_p(&bars->s_ready[t][b]);
+                        }
+                tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
+                if (kMany && n_max == 1) tc_commit_p(&bars->q_empty);
+                for (int j = 0; ok && j < n_max; ++j) {
+                    const int c = c0 + j;
+                    if (!(ok = wait(&bars->pair_full[c & 1], (uint32_t)((c >> 1) & 1), kSitePairFull))) break;
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            const int n = t ? n1 : n0;
+                            if (!ok || j >= n) continue;
+                            if (!(ok = wait(&bars->p_ready[t][b], (uint32_t)(((t ? s1 : s0) + j) & 1), kSitePReady))) continue;
+                            SNTL_TRACE_EV(tl8, 0, tn, 10 + 2 * b + t);
+                            tc_fence_after();
+                            mma_ts_4<8, 128>(tmem_O(t), tmem_S(t, b), sdesc_advance(dv, (uint32_t)(c & 1) * kTileBytes + (uint32_t)b * kHalfBytes), idesc_pv, j > 0 || b > 0);
+                            SNTL_TRACE_EV(tl8, 0, tn, 20 + 2 * b + t);
+                            if (j + 1 < n) issue_s(t, b, (c + 1) & 1);
+                            tc_commit_p(b == 1 && j + 1 == n ? &bars->o_ready[t] : &bars->s_ready[t][b]);
+                            SNTL_TRACE_EV(tl8, 0, tn, 30 + 2 * b + t);
+                        }
+                    if (!ok) break;
+                    if (j + 1 < n_max) tc_commit_p(&bars->pair_empty[c & 1]);
+                    if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
                 }
                 if (!ok) break;
-                if (j + 1 < n_max) tc_commit_p(&bars->pair_empty[c & 1]);
-                if (kMany && j + 2 == n_max) tc_commit_p(&bars->q_empty);
-            }
-            if (!ok) break;
-            c0 += n_max;
-            s0 += n0;
-            s1 += n1;
+                c0 += n_max;
+                s0 += n0;
+                s1 += n1;
             }
             // every MMA issued above must have retired before shared memory / TMEM are given up
             tc_commit_p(&bars->final_bar);
@@ -332,7 +335,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
     } else {
         // =========================== softmax + epilogue warpgroups ===========================
-        setmaxnreg_inc<216>();
+        setmaxnreg_inc<200>();
         const int t = warp >> 2;                       // tile 0 or 1
         const int row = (warp & 3) * 32 + lane;        // row inside the tile == TMEM lane
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
@@ -340,7 +343,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const bool tw = (warp & 3) == 0 && lane == 0;
         (void)tw;
         bool ok = true, more = true;
-        uint32_t phase = 0, blocks = 0;                // of this tile so far: parity of its key tiles, blocks with rows
+        uint32_t phase[2] = {0, 0}, blocks = 0;        // of the tile's s_ready barriers, blocks with rows
         for (int u = 0; ok && more; more = next(u++)) {
         const FwdWork& w = work(u);
         const int n_mine = uniform(t ? w.n1 : w.n0), q0 = uniform(w.q0);
@@ -348,40 +351,45 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const int grow = q0 + t * kM + row;            // query row inside the (batch, head) slab
         auto key_tile = [&](int j) { return j < g_tiles ? j : w_first + (j - g_tiles); };
         float m_ref = -INFINITY, l = 0.0f;
+        // Barrier tests queue behind the exponentials in the same unit and take 200-400 cycles here; where a result is likely to be
+        // there already it is asked for ahead of its use, with other work in between.
+        bool s_seen = false;
         const int row_lo = q0 + t * kM + (warp & 3) * 32;      // first row of the warp
-        for (int j = 0; j < n_mine; ++j, phase = kMany ? phase ^ 1u : (uint32_t)(j & 1)) {
-            if (!(ok = mbar_wait_prompt_warp(&bars->s_ready[t], phase, abort_flag, kSiteSReady))) break;
+        for (int h = 0; h < 2 * n_mine; ++h) {
+            const int b = h & 1;
+            const uint32_t tmS = tmem_S(t, b) + lane_off;
+            if (!(ok = s_seen || mbar_wait_prompt_warp(&bars->s_ready[t][b], b ? phase[1] : phase[0], abort_flag, kSiteSReady))) break;
             SNTL_TRACE_EV(tw, 1 + t, tn, 1);
             tc_fence_after();
-            uint32_t s[128];
+            uint32_t s[kHalf];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) tmem_ld32(tmem_S(t) + lane_off + (uint32_t)(c * 32), s + c * 32);
+            for (int c = 0; c < 2; ++c) tmem_ld32(tmS + (uint32_t)(c * 32), s + c * 32);
             tmem_ld_wait();
             SNTL_TRACE_EV(tw, 1 + t, tn, 2);
-            // number of visible keys of this row inside this tile
-            const int key0 = key_tile(j) * kN;
-            int limit = (p.causal ? min(p.Skv, grow + 1) : p.Skv) - key0;
-            const int lo = kWin ? grow - p.window + 1 - key0 : 0, glim = kWin ? p.global_tokens - key0 : 0;
-            const bool below = kWin && lo > 0 && glim < min(lo, kN);   // keys below the window that are no global tokens
-            // Once a row has a reference maximum, a tile that the mask does not cut is exponentiated against it at once, with the
-            // tile's own maximum taken on the way: only if some row of the warp then needs a rescale (its maximum grew by more
-            // than 2^8, which the lazy rule below leaves rare) is the first half done again.  The maximum and the decision were
-            // a quarter of a tile's time in front of the exponentials.
-            const int limit_lo = (p.causal ? min(p.Skv, row_lo + 1) : p.Skv) - key0, lo_hi = row_lo + 31 - p.window + 1 - key0;
-            const bool ahead = kMode == kPlain && j > 0 && limit_lo >= kN && !(kWin && lo_hi > 0 && glim < min(lo_hi, kN));   // (no row of the warp is cut)
+            // number of visible keys of this row among these
+            const int key0 = key_tile(h >> 1) * kN + b * kHalf;
+            const int limit = (p.causal ? min(p.Skv, grow + 1) : p.Skv) - key0;
+            // Once a row has a reference maximum, keys that the mask does not cut are exponentiated against it at once, with their
+            // own maximum taken on the way: only if some row of the warp then needs a rescale (its maximum grew by more than 2^8,
+            // which the lazy rule below leaves rare) is that done again.  The maximum and the decision were a quarter of a tile's time
+            // in front of the exponentials.  (Under a window many tiles are cut, and with both forms of the pass in use it is slower: a
+            // 512-key window over B2 Hq28 Hkv4 S2048 47.0 us, 44.4 without; 200 keys over B4 Hq16 S1024 27.5 and 26.1.)
+            const int limit_lo = (p.causal ? min(p.Skv, row_lo + 1) : p.Skv) - key0;
+            const int lo_hi = kWin ? row_lo + 31 - p.window + 1 - key0 : 0, glim = kWin ? p.global_tokens - key0 : 0;
+            const bool cut = limit_lo < kHalf || (kWin && lo_hi > 0 && glim < min(lo_hi, kHalf));   // (some row of the warp is)
             uint32_t pk[32];
             float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-            RowMax mx;
             auto shift = [&]() { return m_ref == -INFINITY ? 0.0f : -m_ref; };   // (no finite score so far: -inf + inf would be NaN)
-            float neg_m = shift();
-            // whether some row of the warp has outgrown its reference (false when both are -inf: NaN compare)
-            auto outgrown = [&](float m_new) { return j > 0 && __any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold); };
+            // O and the sum of a row whose maximum has outgrown its reference
             auto rescale = [&](float m_new) {
+                // the product of the P before has been added
+                if (!(ok = mbar_wait_prompt_warp(&bars->s_ready[t][b ^ 1], b ? phase[0] ^ 1u : phase[1], abort_flag, kSiteOReady))) return;
+                tc_fence_after();
                 const bool need = (m_new - m_ref) > kRescaleThreshold;
                 const float factor = need ? ex2(m_ref - m_new) : 1.0f;
                 if (need) m_ref = m_new;
                 l *= factor;
-#pragma unroll
+#pragma unroll 1
                 for (int c = 0; c < D / 32; ++c) {
                     uint32_t o[32];
                     tmem_ld32(tmem_O(t) + lane_off + (uint32_t)(c * 32), o);
@@ -391,55 +399,60 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     tmem_st32(tmem_O(t) + lane_off + (uint32_t)(c * 32), o);
                 }
                 tmem_st_wait();
-                neg_m = shift();
             };
-            if (ahead) {
-                exp_half<0, true>(s, p.scale_log2, neg_m, pk, sum, mx);
+            // whether some row of the warp has outgrown its reference (false when both are -inf: NaN compare)
+            auto outgrown = [&](float m_new) { return __any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold); };
+            bool plain = kMode == kPlain && h > 0 && !cut;
+            if (plain) {
+                RowMax mx;
+                exp_row<true>(s, p.scale_log2, shift(), pk, sum, mx);
                 SNTL_TRACE_EV(tw, 1 + t, tn, 3);
-                const float m_new = fmaxf(m_ref, mx.value() * p.scale_log2);
-                if (outgrown(m_new)) {            // (S is read again: kept, it would take 64 registers more than there are)
-                    rescale(m_new);
+                if (outgrown(fmaxf(m_ref, mx.value() * p.scale_log2))) {
+                    plain = false;
                     sum[0] = sum[1] = make_float2(0.0f, 0.0f);
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) tmem_ld32(tmem_S(t) + lane_off + (uint32_t)(c * 32), s + c * 32);
+                    for (int c = 0; c < 2; ++c) tmem_ld32(tmS + (uint32_t)(c * 32), s + c * 32);    // (kept, it would take 64 registers more)
                     tmem_ld_wait();
-                    exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
                 }
-            } else {
-                if (limit < kN) {
+            }
+            if (!plain) {
+                if (cut) {
+                    if (limit < kHalf) {
 #pragma unroll
-                    for (int c = 0; c < kN; ++c)
-                        if (c >= limit) s[c] = 0xff800000u;  // -inf
-                }
-                if (below) {
+                        for (int c = 0; c < kHalf; ++c)
+                            if (c >= limit) s[c] = 0xff800000u;  // -inf
+                    }
+                    const int lo = kWin ? grow - p.window + 1 - key0 : 0;
+                    if (kWin && lo > 0 && glim < min(lo, kHalf)) {      // keys below the window that are no global tokens
 #pragma unroll
-                    for (int c = 0; c < kN; ++c)
-                        if (c < lo && c >= glim) s[c] = 0xff800000u;
+                        for (int c = 0; c < kHalf; ++c)
+                            if (c < lo && c >= glim) s[c] = 0xff800000u;
+                    }
                 }
                 const float m_new = fmaxf(m_ref, row_max(s) * p.scale_log2);
-                if (j == 0) m_ref = m_new;
+                if (h == 0) m_ref = m_new;
                 else if (outgrown(m_new)) rescale(m_new);
-                neg_m = shift();
+                if (!ok) break;
                 SNTL_TRACE_EV(tw, 1 + t, tn, 4);
-                exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, mx);
+                RowMax unused;
+                exp_row<false>(s, p.scale_log2, shift(), pk, sum, unused);
             }
-            tmem_st32(tmem_S(t) + lane_off, pk);
-            tmem_st_wait();     // the P V product may start on the first 64 keys while the rest is computed
-            tc_fence_before();
-            mbar_arrive(&bars->p_half[t]);
-            exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, mx);
-            tmem_st32(tmem_S(t) + lane_off + 32u, pk);
+            if (b) phase[0] ^= 1u, phase[1] ^= 1u;
+            s_seen = h + 1 < 2 * n_mine && __all_sync(0xffffffffu, mbar_test(&bars->s_ready[t][b ^ 1], b ? phase[0] : phase[1]));
+            tmem_st32(tmS, pk);      // over S
             l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             SNTL_TRACE_EV(tw, 1 + t, tn, 5);
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(&bars->p_ready[t]);
+            mbar_arrive(&bars->p_ready[t][b]);
             SNTL_TRACE_EV(tw, 1 + t, tn, 6);
         }
-        if (ok && n_mine > 0)
-            ok = mbar_wait_prompt_warp(&bars->o_ready[t], blocks & 1u, abort_flag, kSiteOReady);
         if (ok && n_mine > 0) {
-            ++blocks;
+            ok = mbar_wait_prompt_warp(&bars->o_ready[t], blocks, abort_flag, kSiteOReady);
+            blocks ^= 1u;
+            phase[0] ^= 1u;
+        }
+        if (ok && n_mine > 0) {
             tc_fence_after();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             const bool store = grow < p.Sq;
@@ -526,7 +539,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 // us, before -> now: B4 Hq32 Hkv8 S4096 377 -> 351; B8 Hq12 S1024 31.0 -> 28.5; B2 Hq32 S1024 23.2 -> 19.4; B16 Hq8 S130 7.8 -> 7.5; a 300-key
 // window over B4 Hq12 S2048 35.6 -> 35.7; few long rows, B1 Hq4 S8192, 71.8 -> 71.6.  Also measured: both tiles
 // fed by one MMA warp, 351, 28.2 and 27.9; two softmax warpgroups with two S buffers of 64 columns each, 436, 32.0 and 25.2.
-constexpr int kHalf = 64;             // keys of a tile that one stream takes
 constexpr int kStreamThreads = 640;   // four softmax warpgroups, and one holding the MMA and the TMA warps
 
 // One half of a CTA: blocks of one query tile, two softmax warpgroups ("streams": stream b has keys [64 b, 64 b + 64) of every key
@@ -968,8 +980,7 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     if constexpr (D == 64) {
         return launch(attn_fwd_streams_kernel<kMode, kMat>, configured_one);
     } else {
-        if constexpr (kMode == kWindow)
-            if (p.several_waves) return launch(attn_fwd_tc_kernel<D, kMode, kMat, true>, configured_many);
+        if (p.several_waves) return launch(attn_fwd_tc_kernel<D, kMode, kMat, true>, configured_many);
         return launch(attn_fwd_tc_kernel<D, kMode, kMat, false>, configured_one);
     }
 }

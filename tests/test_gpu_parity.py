@@ -443,6 +443,7 @@ def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
         assert float((got.float() - want).norm() / want.norm()) <= tol
 
 
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,kw", [
     (1, 1, 1, 1, 1, {}), (1, 2, 1, 64, 64, {}), (1, 2, 2, 65, 65, {}), (2, 3, 1, 128, 128, {}), (1, 2, 1, 129, 129, {}),   # edges of the key halves
     (1, 2, 1, 200, 70, dict(causal=False)), (1, 2, 1, 70, 193, dict(causal=False)), (1, 1, 1, 130, 64, dict(causal=False)),
@@ -450,17 +451,17 @@ def test_backward_cut_pieces_vs_exact_kernels(sb, B, Hq, Hkv, S, D, kw):
     (9, 12, 12, 700, 700, {}),                                       # 648: every half takes over blocks
     (6, 8, 2, 640, 640, dict(window=64)), (6, 8, 2, 650, 650, dict(window=65, global_tokens=3)), (4, 8, 8, 900, 900, dict(window=200, global_tokens=130)),
 ])
-def test_head_dim_64_forward_streams(sb, B, Hq, Hkv, Sq, Sk, kw):
-    """The two streams of a row (64 keys of every key tile each) and the two halves of a CTA against fp64: rows whose first key tile
-    leaves one stream without a visible key, ragged ends in either half, blocks taken over; and large scores, for which the streams
-    rescale at different tiles."""
+def test_forward_key_halves(sb, B, Hq, Hkv, Sq, Sk, kw, D):
+    """Key tiles in halves of 64 keys, two streams of a row at head_dim 64 and one after the other at 128, against fp64: rows whose first
+    key tile leaves one half without a visible key, ragged ends in either half, blocks taken over by a CTA or by either half of one; and
+    large scores, for which rows rescale at every place."""
     g = torch.Generator(device="cuda").manual_seed(Sq + B)
     for std in (0.5, 6.0):
-        q, k, v = ((torch.randn(B, H, S, 64, generator=g, device="cuda") * x).to(torch.bfloat16) for H, S, x in ((Hq, Sq, std), (Hkv, Sk, std), (Hkv, Sk, 1.0)))
+        q, k, v = ((torch.randn(B, H, S, D, generator=g, device="cuda") * x).to(torch.bfloat16) for H, S, x in ((Hq, Sq, std), (Hkv, Sk, std), (Hkv, Sk, 1.0)))
         o, lse = sb.attention_forward(q, k, v, **kw)
         assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
         kd, vd = (t.double().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
-        s = q.double() @ kd.transpose(2, 3) * 64 ** -0.5
+        s = q.double() @ kd.transpose(2, 3) * D ** -0.5
         if kw.get("causal", True):
             i, j = torch.arange(Sq, device="cuda")[:, None], torch.arange(Sk, device="cuda")[None, :]
             seen = j <= i

@@ -179,7 +179,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             uint32_t lap = 0;                 // laps of the ring
             for (Walk<kMode> w(p); ok && w.next(); ++seg) {
                 const int slot = kMode == kPair ? 0 : seg & 1, use = kMode == kPair ? seg : seg >> 1;   // how often the slot was filled
-                if (use > 0 && !mbar_wait_prompt(&bars->q_empty[slot], (uint32_t)(use - 1) & 1u, abort_flag, kSiteQEmpty)) break;
+                if (use > 0 && !mbar_wait(&bars->q_empty[slot], (uint32_t)(use - 1) & 1u, abort_flag, kSiteQEmpty)) break;
                 const int blocks = kMode == kPair && w.both ? 2 : 1;
                 mbar_arrive_expect_tx(&bars->q_full[slot], (uint32_t)(blocks * L::kQBytes));
                 for (int i = 0; i < blocks; ++i)
@@ -187,11 +187,11 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                         tma_load_3d(sQ + (slot + i) * L::kQBytes + c * L::kQChunk, &tmap_q, &bars->q_full[slot], c * 64, w.row0 + i * kM, w.slab);
                 for (int j = 0; j < w.n; ++j) {
                     const int key0 = key_tile(w.tile + j) * kN;
-                    if (lap > 0 && !(ok = mbar_wait_prompt(&bars->k_empty[st], (lap - 1) & 1u, abort_flag, kSiteKEmpty))) break;
+                    if (lap > 0 && !(ok = mbar_wait(&bars->k_empty[st], (lap - 1) & 1u, abort_flag, kSiteKEmpty))) break;
                     mbar_arrive_expect_tx(&bars->k_full[st], (uint32_t)L::kTileBytes);
                     for (int c = 0; c < kChunks; ++c)
                         tma_load_3d(sK + st * L::kTileBytes + c * kChunkBytes, &tmap_k, &bars->k_full[st], c * 64, key0, w.slab);
-                    if (lap > 0 && !(ok = mbar_wait_prompt(&bars->v_empty[st], (lap - 1) & 1u, abort_flag, kSiteVEmpty))) break;
+                    if (lap > 0 && !(ok = mbar_wait(&bars->v_empty[st], (lap - 1) & 1u, abort_flag, kSiteVEmpty))) break;
                     mbar_arrive_expect_tx(&bars->v_full[st], (uint32_t)L::kTileBytes);
                     for (int c = 0; c < kChunks; ++c)
                         tma_load_3d(sV + st * L::kTileBytes + c * kChunkBytes, &tmap_v, &bars->v_full[st], c * 64, key0, w.slab);
@@ -210,7 +210,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const uint64_t dq0 = make_sdesc(smem_u32(sQ), 16, 1024), dk0 = make_sdesc(smem_u32(sK), 16, 1024);
             const uint64_t dv0 = make_sdesc(smem_u32(sV), kChunkBytes, 1024);
             auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t site) {
-                return mbar_wait_prompt_warp(bar, parity, abort_flag, site);
+                return mbar_wait_warp(bar, parity, abort_flag, site);
             };
             auto issue_s = [&](int t, int st, int slot) {
                 const uint64_t a = dq0 + (uint64_t)((slot * L::kQBytes - (kMode == kSmall ? (t + 1) * kSmallRows * 128 : 0)) >> 4);
@@ -335,7 +335,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                 int count = 0;
                 if (t == 1 && !w.both) continue;
                 for (int j = kMode == kPair || (n0 & 1) == t ? 0 : 1; j < w.n; j += kMode == kPair ? 1 : 2, ++count, ++mine) {
-                    if (!(ok = mbar_wait_prompt_warp(&bars->s_ready[t], mine & 1u, abort_flag, kSiteSReady))) break;
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_ready[t], mine & 1u, abort_flag, kSiteSReady)))) break;
                     tc_fence_after();
                     uint32_t s[128];
 #pragma unroll
@@ -361,7 +361,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     if (count == 0) {
                         m_ref = m_new;
                     } else if (__any_sync(0xffffffffu, need)) {
-                        if (!(ok = mbar_wait_prompt_warp(&bars->o_ready[t], (mine - 1u) & 1u, abort_flag, kSiteOReady))) break;
+                        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_ready[t], (mine - 1u) & 1u, abort_flag, kSiteOReady)))) break;
                         tc_fence_after();
                         const float factor = need ? ex2(m_ref - m_new) : 1.0f;
                         if (need) m_ref = m_new;
@@ -405,7 +405,7 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     if (live) p.lse_part[out_row] = -INFINITY;          // no tile: weighs nothing in the merge
                     continue;
                 }
-                if (!(ok = mbar_wait_prompt_warp(&bars->o_ready[t], (mine - 1u) & 1u, abort_flag, kSiteOReady))) break;
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_ready[t], (mine - 1u) & 1u, abort_flag, kSiteOReady)))) break;
                 tc_fence_after();
                 const float inv = l > 0.0f ? 1.0f / l : 0.0f;
 #pragma unroll

@@ -927,9 +927,10 @@ EncodeTiledFn encode_fn()
 }
 
 // head_dim 128.  Two query tiles per CTA overlap one tile's softmax with the other's products; on a grid that leaves SMs idle or ends
-// with one long CTA, one tile per CTA finishes sooner: a step of one tile takes 0.83 of a step of two.  The estimate counts steps of two
-// tiles: the longest CTA, or the SMs' average load and a short tail, with 1.3 steps per CTA of set-up.  Cold, B1 Hq8 S2048: 33 -> 28
-// us; B1 Hq4 S8192 110 -> 92.
+// with one long CTA, one tile per CTA finishes sooner: a step of one tile takes 0.62 to 0.7 of a step of two (2170 cycles of 3480).  The
+// estimate counts steps of two tiles: the longest CTA, or the SMs' average load and a short tail, with 1.3 steps per CTA of set-up.
+// us, with 0.83 (as measured before key tiles were taken in halves) -> 0.7: B2 Hq12 S1500 26.3 -> 24.2, B4 Hq8 S1000 19.1 -> 18.3, B1 Hq32 S1024 19.2 ->
+// 18.2, a 256-key window over B2 Hq16 S2048 25.6 -> 25.1; a dozen other grids within 1 %, and 0.62 as 0.7.
 int fwd_tiles_per_cta(const AttnShape& s)
 {
     const int n = (s.Sq + kM - 1) / kM, n_keys = (s.Skv + kN - 1) / kN, heads = s.B * s.Hq, sms = sm_count();
@@ -942,7 +943,7 @@ int fwd_tiles_per_cta(const AttnShape& s)
         one += steps(i);
         if (i + 1 == n || (i & 1)) two += steps(i);
     }
-    const double cost = 0.83, set_up = 1.3, longest = steps(n - 1);
+    const double cost = 0.7, set_up = 1.3, longest = steps(n - 1);
     const double t2 = std::max(longest + set_up, (two * heads + set_up * pairs) / sms + 0.1 * longest);
     const double t1 = std::max(cost * longest + set_up, (cost * one + set_up * n) * heads / sms + 0.1 * cost * longest);
     return t1 < 0.95 * t2 ? 1 : 2;

@@ -380,15 +380,14 @@ attn_cache_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                     const float neg_m = (m_ref == -INFINITY) ? 0.0f : -m_ref;
                     uint32_t pk[32];
                     float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-                    RowMax unused;
-                    exp_half<0, false>(s, p.scale_log2, neg_m, pk, sum, unused);
+                    exp_half<0>(s, p.scale_log2, neg_m, pk, sum);
                     tmem_st32(tmem_S(t) + lane_off, pk);
                     if (kMode == kPair) {
                         tmem_st_wait();
                         tc_fence_before();
                         mbar_arrive(&bars->p_half[t]);
                     }
-                    exp_half<1, false>(s, p.scale_log2, neg_m, pk, sum, unused);
+                    exp_half<1>(s, p.scale_log2, neg_m, pk, sum);
                     tmem_st32(tmem_S(t) + lane_off + 32u, pk);
                     l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
                     tmem_st_wait();

@@ -1,4 +1,4 @@
-// Pieces of the online softmax on one 128-column row of S per thread (forward and KV-cache kernels).
+// Pieces of the online softmax on one row of S per thread: 64 columns in the forward kernels, 128 in the KV-cache kernel.
 #pragma once
 
 #include "sm100_ptx.cuh"
@@ -34,26 +34,22 @@ template <int N> __device__ __forceinline__ float row_max(const uint32_t (&s)[N]
 }
 
 // Half a row: P = exp2(s * scale + shift) as packed bf16 in pk, and the sum of the fp32 values added to sum (two pairs of partial
-// sums).  kMax: the whole row's maximum is folded in on the way, in the issue slots that the special-function unit leaves free.
-template <int kHalf, bool kMax>
-__device__ __forceinline__ void exp_half(const uint32_t (&s)[128], float scale, float shift, uint32_t (&pk)[32], float2 (&sum)[2], RowMax& mx)
+// sums).
+template <int kHalf>
+__device__ __forceinline__ void exp_half(const uint32_t (&s)[128], float scale, float shift, uint32_t (&pk)[32], float2 (&sum)[2])
 {
     const float2 sc = make_float2(scale, scale), sh = make_float2(shift, shift);
-    if (kMax) mx.start(s);
 #pragma unroll
     for (int c = 0; c < 32; ++c) {
         const float2 x = ptx::ffma2(make_float2(__uint_as_float(s[kHalf * 64 + 2 * c]), __uint_as_float(s[kHalf * 64 + 2 * c + 1])), sc, sh);
         const float p0 = ptx::ex2(x.x), p1 = ptx::ex2(x.y);
-        if (kMax && c < 30) {
-            mx.step(s, 2 * c);
-            mx.step(s, 2 * c + 1);
-        }
         sum[c & 1] = ptx::fadd2(sum[c & 1], make_float2(p0, p1));
         pk[c] = ptx::pack_bf16(p0, p1);
     }
 }
 
-// The same for 64 columns.
+// The same for a row of 64 columns.  kMax: the row's maximum is taken on the way, in the issue slots that the special-function unit
+// leaves free.
 template <bool kMax>
 __device__ __forceinline__ void exp_row(const uint32_t (&s)[64], float scale, float shift, uint32_t (&pk)[32], float2 (&sum)[2], RowMax& mx)
 {

@@ -47,7 +47,7 @@ constexpr int kOutBytes = 8 * 4096;        // staging of O
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 enum WaitSite : uint32_t {
-    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue, kSiteQEmpty, kSiteNext
+    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue, kSiteQEmpty, kSiteNext, kSiteORead
 };
 
 struct FwdParams {
@@ -552,6 +552,7 @@ struct StreamHalf {
     uint64_t o_ready[2];              // the last P V of a block has been.  (A phase of s_ready instead could be over before it is seen: the
                                       // next block's first S does not wait for the softmax warps.)
     uint64_t p_ready[2];
+    uint64_t o_read;                  // every softmax warp has read O and ml of a block
     uint64_t final_bar;
     float2 ml[2][kM];                 // reference maximum and sum of a row, for its other stream
 };
@@ -601,6 +602,7 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             mbar_init(&bars->o_ready[i], 1);
             mbar_init(&bars->p_ready[i], 128);
         }
+        mbar_init(&bars->o_read, 8);
         mbar_init(&bars->final_bar, 1);
         shared->abort_flag = shared->asking = shared->none_left = 0;
         fence_mbar_init();
@@ -619,10 +621,13 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 
     // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Counters of key
     // tiles run on over the blocks, so stages and barrier phases continue where they are.
+    constexpr int kGaveUp = -2;
     int2 win = make_int2(0, 0);   // its g_tiles, w_first
-    // A warp's copy of block u (work: n, q0, bh); false when there is none.  Every access to shared memory waits some 250 cycles
-    // behind the other warps' exponentials, so there are few of them, and the softmax warps take the next block before their epilogue.
+    // A warp's copy of block u (work: n, q0, bh); false when there is none, or when the wait for it gave up (n = kGaveUp).  Every
+    // access to shared memory waits some 250 cycles behind the other warps' exponentials, so there are few of them, and the softmax
+    // warps take the next block before their epilogue.
     auto get = [&](int u, int4& work) {
+        work.x = kGaveUp;
         if (!mbar_wait_prompt_warp(&bars->work_full[u & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext)) return false;
         work = *reinterpret_cast<const int4*>(&bars->work[u & 1]);
         if (kWin) win = *reinterpret_cast<const int2*>(&bars->work[u & 1].g_tiles);
@@ -716,7 +721,7 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             if (!(ok = wait(&bars->k0_full, (uint32_t)(u & 1), kSiteK0) && wait(&bars->q_full, (uint32_t)(u & 1), kSiteQ))) break;
             tc_fence_after();
             // (S of the block before has been read and P over it consumed: this warp waited for p_ready and issued the product; O is
-            // overwritten behind p_ready of the new block, which its warps give after their epilogue)
+            // overwritten behind o_read)
 #pragma unroll
             for (int b = 0; b < 2; ++b) issue_s(b, c0 & 1);
             tc_commit_p(&bars->pair_empty[(c0 - 1) & 1]);        // K_0 and the last V of the block before
@@ -727,6 +732,7 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     if (!ok || !(ok = wait(&bars->p_ready[b], (uint32_t)(c & 1), kSitePReady))) continue;
+                    if (b == 0 && j == 0 && u > 0 && !(ok = wait(&bars->o_read, (uint32_t)((u - 1) & 1), kSiteORead))) continue;
                     tc_fence_after();
                     mma_ts_4<8, 128>(tmem_O(b), tmem_S(b), sdesc_advance(dv, (uint32_t)((c & 1) * kTileBytes) + (uint32_t)b * kHalfBytes), idesc_pv, j > 0);
                     if (j + 1 < n) issue_s(b, (c + 1) & 1);
@@ -749,9 +755,12 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t tmS = tmem_S(half) + lane_off, tmO = tmem_O(half) + lane_off;
         bool ok = true;
-        uint32_t phase = 0, blocks = 0;                // of s_ready, of o_ready
+        uint32_t phase = 0;                            // of s_ready
         int4 work;
         bool more = get(0, work);
+        // The eight warps of a half meet in a named barrier, which has no limit: here and at the end of each block.  A warp whose wait
+        // gave up goes there all the same and says so, and then all leave.
+        more = named_barrier_all(1 + inst, 256, work.x != kGaveUp) && more;
         for (int u = 0; more; ++u) {
             const int n_mine = work.x, q0 = work.y, bh = work.z;
             const int g_tiles = kWin ? win.x : 0, w_first = kWin ? win.y : 0;
@@ -832,14 +841,14 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 tc_fence_before();
                 mbar_arrive(&bars->p_ready[half]);
             }
-            if (!ok) break;
-            more = get(u + 1, work);
-            if (!(ok = mbar_wait_prompt_warp(&bars->o_ready[half], blocks, abort_flag, kSiteOReady))) break;
-            blocks ^= 1u;
+            if (!ok || (more = get(u + 1, work), work.x == kGaveUp) || !mbar_wait_prompt_warp(&bars->o_ready[half], (uint32_t)(u & 1), abort_flag, kSiteOReady)) {
+                named_barrier_all(1 + inst, 256, false);
+                break;
+            }
             // The two streams of a row are added here; each stores one half of the features.
             bars->ml[half][row] = make_float2(m_ref, l);
             tc_fence_before();
-            named_barrier_sync(1 + inst, 256);
+            if (!named_barrier_all(1 + inst, 256, true)) break;
             tc_fence_after();
             const float2 ml = bars->ml[half ^ 1][row];
             uint32_t o[2][32];
@@ -854,7 +863,8 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             f1 *= inv;
             tmem_ld_wait();
             tc_fence_before();
-            named_barrier_sync(1 + inst, 256);      // the next block's first products may overwrite O
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->o_read);      // (and ml: it is written behind products that wait for this)
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[0][i] = __float_as_uint(fmaf(__uint_as_float(o[0][i]), f0, __uint_as_float(o[1][i]) * f1));
             const bool store = grow < p.Sq;

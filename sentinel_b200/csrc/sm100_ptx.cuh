@@ -197,10 +197,25 @@ __device__ __forceinline__ int clc_first_block(const void* response)
 // the same value in all lanes, and known to be: what depends on it stays in uniform registers and branches
 __device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
-// barrier among a subset of the CTA's warps (id 1..15; `threads` a multiple of 32)
+// Barrier among a subset of the CTA's warps (id 1..15; `threads` a multiple of 32).  It has no limit of its own: between a wait that
+// may give up and a named barrier stands a named_barrier_all, at which the warps agree whether all of them go on.
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// the same, and whether `ok` holds in every thread
+__device__ __forceinline__ bool named_barrier_all(uint32_t id, uint32_t threads, bool ok)
+{
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "bar.red.and.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"(id), "r"(threads), "r"((uint32_t)ok)
+        : "memory");
+    return all != 0;
 }
 
 // per-warpgroup register re-allocation (all four warps of the warpgroup must execute it)

@@ -282,19 +282,25 @@ __device__ __forceinline__ uint64_t make_sdesc_plain(uint32_t smem_addr, uint32_
 // tile, kStageCols columns per piece.  Called by all 128 threads of the drain warpgroup (named barrier 1); `elected` is the
 // one thread that owns the bulk groups.  kStagingBytes of staging in all; `piece` counts pieces over the CTA's lifetime, so
 // that the rotation carries on from tile to tile (a buffer is rewritten only after the kStages - 1 groups issued since
-// its last use are all that may still be reading).
+// its last use are all that may still be reading).  A warp whose wait for the tile gave up takes part in the first barrier only,
+// with named_barrier_all(1, 128, false): then nothing is pushed and the result is false in all of them.
 template <int D, bool kDet, int kStageCols, int kStagingBytes>
-__device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile, uint8_t* sStage, int row, bool elected, uint32_t& piece)
+__device__ __forceinline__ bool push_dq_tile(const uint32_t (&r)[D], float* tile, uint8_t* sStage, int row, bool elected, uint32_t& piece)
 {
     constexpr int kStageBytes = kStageCols * kT * 4;
     constexpr int kStages = kStagingBytes / kStageBytes;
     static_assert(kStages >= 2 && kStages * kStageBytes == kStagingBytes, "staging must hold whole pieces");
+    auto stage_free = [&](int c) {
+        if (elected) bulk_wait_read<kStages - 1>();
+        if (c == 0) return named_barrier_all(1, 128, true);
+        named_barrier_sync(1, 128);
+        return true;
+    };
     if constexpr (!kDet) {
 #pragma unroll
         for (int c = 0; c < D / kStageCols; ++c) {
             uint8_t* stage = sStage + (piece++ % kStages) * kStageBytes;
-            if (elected) bulk_wait_read<kStages - 1>();
-            named_barrier_sync(1, 128);
+            if (!stage_free(c)) return false;
 #pragma unroll
             for (int v = 0; v < kStageCols / 4; ++v)
                 *reinterpret_cast<uint4*>(stage + ((size_t)v * kT + row) * 16) =
@@ -316,8 +322,7 @@ __device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile
 #pragma unroll
         for (int c = 0; c < D / kDetCols; ++c) {
             uint8_t* stage = sStage + (piece++ % kStages) * kStageBytes;
-            if (elected) bulk_wait_read<kStages - 1>();
-            named_barrier_sync(1, 128);
+            if (!stage_free(c)) return false;
 #pragma unroll
             for (int v = 0; v < kDetCols / 2; ++v) {
                 const long long a = __float2ll_rn(__uint_as_float(r[c * kDetCols + 2 * v]) * 4294967296.0f);
@@ -333,6 +338,7 @@ __device__ __forceinline__ void push_dq_tile(const uint32_t (&r)[D], float* tile
             }
         }
     }
+    return true;
 }
 
 // Epilogue of a compute warpgroup: its accumulator (dV for warpgroup 0, dK for warpgroup 1; `src` = TMEM address of this
@@ -575,12 +581,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
     // Every role walks the same blocks, which the producer decodes into shared memory: number u is work[u & 1].  Step counters run
     // on over the blocks (n0: steps before this block, blocks: how many before it had steps), so stages and barrier phases continue
-    // where they are.  next(u): done with block u; whether another follows.
-    auto next = [&](int u) {
+    // where they are.  next(u): done with block u; whether another follows (agree: whether the wait for it came through, for all warps that
+    // have to leave together).
+    auto next = [&](int u, auto agree) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->work_empty[u & 1]);
-        return mbar_wait_prompt_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext) && bars->work[(u + 1) & 1].n_iter >= 0;
+        return agree(mbar_wait_prompt_warp(&bars->work_full[(u + 1) & 1], (uint32_t)((u >> 1) & 1), abort_flag, kSiteNext)) && bars->work[(u + 1) & 1].n_iter >= 0;
     };
+    auto alone = [](bool came) { return came; };
 
     if (warp == 15) {
         setmaxnreg_dec<56>();
@@ -690,7 +698,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             int n0 = 0, blocks = 0;
             bool ok = true;
             bool more = true;
-            for (int u = 0; more; more = next(u++)) {
+            for (int u = 0; more; more = next(u++, alone)) {
                 const int end = n0 + bars->work[u & 1].n_iter;
                 if (end == n0) continue;
                 if (!(ok = wait(&bars->k_full, (uint32_t)(blocks & 1), kSiteKV))) break;
@@ -757,7 +765,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             int n0 = 0, blocks = 0;
             bool ok = true;
             bool more = true;
-            for (int u = 0; more; more = next(u++)) {
+            for (int u = 0; more; more = next(u++, alone)) {
                 const int end = n0 + bars->work[u & 1].n_iter;
                 if (end == n0) continue;
                 // dP^T of step n, into the columns that dQ of the step before has left
@@ -828,7 +836,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         uint32_t piece = 0;
         int n = 0;
         bool more = true;
-        for (int u = 0; ok && more; more = next(u++)) {
+        for (int u = 0; ok && more; ++u) {
         const BwdWork w = bars->work[u & 1];
         const int bh0 = w.slab * group;      // b * Hq + hk * group
         int g = w.g_first, tile_r = w.r_first;
@@ -839,7 +847,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             float* tile = p.dq_accum + ((size_t)bh * p.n_qt + qt) * (size_t)(kT * D) * (kDet ? 2 : 1);
             ok = mbar_wait_prompt_warp(&bars->dq_ready, (uint32_t)(n & 1), abort_flag, kSiteDQ);
             SNTL_TRACE_EV(tw, 3, tn, 1);
-            if (!ok) break;
+            if (!ok) {
+                named_barrier_all(1, 128, false);
+                break;
+            }
             tc_fence_after();
             // The whole dQ tile goes to registers first so that the TMEM columns are handed back to the MMA warp at
             // once; pushing 64 KB (D = 128) through the reduction path (~30 bytes/clock per SM) is the slow part and
@@ -856,9 +867,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             tc_fence_before();
             mbar_arrive(&bars->dq_drained);
             SNTL_TRACE_EV(tw, 3, tn, 2);
-            push_dq_tile<D, kDet, kStageCols, kStagingBytes>(r, tile, sStage, row, elected, piece);
+            ok = push_dq_tile<D, kDet, kStageCols, kStagingBytes>(r, tile, sStage, row, elected, piece);
             SNTL_TRACE_EV(tw, 3, tn, 3);
+            if (!ok) break;
         }
+        if (!ok) break;
+        more = next(u, [&](bool came) { return ok = named_barrier_all(1, 128, came); });      // (the four warps leave together)
         }
         if (elected) bulk_wait_all();   // the reductions read shared memory and must land before the CTA retires
     } else {
@@ -875,7 +889,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         bool ok = true;
         int n = 0, blocks = 0;
         bool more = true;
-        for (int u = 0; ok && more; more = next(u++)) {
+        for (int u = 0; ok && more; more = next(u++, alone)) {
         const BwdWork& w = bars->work[u & 1];
         const int qt_first = w.qt_first, per_head = w.per_head, n_iter = w.n_iter;
         const int kt = w.kt, k0 = kt * kT;

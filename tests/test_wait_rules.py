@@ -15,7 +15,7 @@ def roles(text):
     return re.split(r"\n    (?:if \(warp|\} else (?:if \(warp|\{))", text)
 
 
-@pytest.mark.parametrize("name", ["attn_fwd_sm100.cu"])
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith("_sm100.cu")))
 def test_warps_agree_after_bounded_waits_before_they_meet_in_a_named_barrier(name):
     """A named barrier has no limit.  If one warp's wait gives up and another's does not, and the second then stands in a barrier that
     counts the first, neither ever leaves.  So between a wait (or a call that waits) and a named barrier comes named_barrier_all, at
@@ -34,4 +34,4 @@ def test_warps_agree_after_bounded_waits_before_they_meet_in_a_named_barrier(nam
                 assert agreed, f"{name}: {token} behind a wait that may have given up in one warp alone"
             else:
                 agreed = False
-    assert met > 0
+    assert met > 0 or name not in ("attn_fwd_sm100.cu", "attn_bwd_sm100.cu")

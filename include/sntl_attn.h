@@ -288,9 +288,10 @@ int sntl_attn_poll_device_status_words(void* stream, uint32_t* forward_word, uin
  * cut short as well.  A caller therefore polls at the points where it synchronises anyway (end of a training step,
  * before reading results back) and discards the step on SNTL_ERR_DEVICE_TIMEOUT. */
 
-/* Self-test of that path, for test suites: launches one warp whose only wait can never complete, limited to
- * limit_us microseconds (1..100000).  The wait runs out, the kernel returns, and the next poll reports
- * SNTL_ERR_DEVICE_TIMEOUT with site code 0x7e in the top byte of the forward word.  Nothing hangs or faults.
+/* Self-test of that path, for test suites: launches four blocks, one for each form of wait that the kernels use, whose
+ * waits can never complete and are limited to limit_us microseconds (1..100000).  They run out, the kernel returns, and
+ * the next poll reports SNTL_ERR_DEVICE_TIMEOUT with site code 0x7e in the top byte of the forward word (0x7d: a form of
+ * wait did not do as it should, its number in the low bits).  Nothing hangs or faults.
  * Asynchronous on `stream`.  No counterpart in the reference. */
 int sntl_attn_selftest_wait_timeout(uint32_t limit_us, void* stream);
 

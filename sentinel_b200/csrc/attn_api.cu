@@ -588,7 +588,7 @@ int sntl_attn_selftest_wait_timeout(uint32_t limit_us, void* stream)
 {
     if (limit_us == 0 || limit_us > 100000u) return SNTL_ERR_BAD_ARGUMENT;   // 0.1 s at most: this is a test hook
     if (!device_ok()) return SNTL_ERR_NO_DEVICE;
-    return cuda_status(launch_wait_selftest((unsigned long long)limit_us * 1000ull, nullptr, (cudaStream_t)stream));
+    return cuda_status(launch_wait_selftest((unsigned long long)limit_us * 1000ull, (cudaStream_t)stream));
 }
 
 }  // extern "C"

@@ -1095,27 +1095,48 @@ extern "C" int sntl_debug_trace_fwd(unsigned long long* out, int n_words, int se
 }
 #endif
 
-// Self-test of the bounded wait: one warp waits on a barrier that by construction never receives its arrival, with a
-// limit of `limit_ns` instead of the kernels' one second.  The wait runs out, records kSiteSelfTest in the status word
-// exactly as a stuck production wait would, and the kernel returns normally (no trap, the context stays usable).
-constexpr uint32_t kSiteSelfTest = 0x7e;
-__global__ void wait_selftest_kernel(unsigned long long limit_ns, unsigned int* gave_up)
+// Self-test of the bounded waits, one form per block, on a barrier that by construction never receives its arrival and with a limit
+// of `limit_ns` instead of the kernels' one second: the wait of one thread (mbar_wait_for), its short form in one thread and in a
+// warp, and eight warps of which every other one gives up before they meet in a named barrier.  The waits run out, record
+// kSiteSelfTest in the status word as a stuck production wait records its own site, and the kernel returns normally (no trap, the
+// context stays usable).  A form that says that the phase completed, does not set the CTA's flag, gives up before half its limit without
+// being told to, or lets part of the warps go on records kSiteSelfTestFailed and its number instead.
+constexpr uint32_t kSiteSelfTest = 0x7e, kSiteSelfTestFailed = 0x7d;
+constexpr unsigned kSelfTestForms = 4;
+__global__ void __launch_bounds__(256) wait_selftest_kernel(unsigned long long limit_ns)
 {
-    __shared__ uint64_t bar;
+    __shared__ uint64_t never, done;
     __shared__ uint32_t abort_word;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned form = blockIdx.x;
     if (threadIdx.x == 0) {
-        ptx::mbar_init(&bar, 1);
+        ptx::mbar_init(&never, 1);
+        ptx::mbar_init(&done, 1);
         abort_word = 0;
         ptx::fence_mbar_init();
     }
     __syncthreads();
-    const bool done = ptx::mbar_wait_for(&bar, 0, &abort_word, kSiteSelfTest, limit_ns);
-    if (threadIdx.x == 0 && gave_up) *gave_up = done ? 0u : 1u;
+    if (threadIdx.x == 0) ptx::mbar_arrive(&done);
+    const unsigned long long t0 = ptx::global_timer_ns();
+    const bool told = t0 < *(volatile unsigned long long*)&ptx::g_abort_until_ns;      // (by a give-up before this launch)
+    bool fine = true;
+    if (form == 0 && threadIdx.x == 0) fine = !ptx::mbar_wait_for(&never, 0, &abort_word, kSiteSelfTest, limit_ns);
+    if (form == 1 && threadIdx.x == 0) fine = !ptx::mbar_wait_prompt(&never, 0, &abort_word, kSiteSelfTest, limit_ns);
+    if (form == 2 && warp == 0) fine = !ptx::mbar_wait_prompt_warp(&never, 0, &abort_word, kSiteSelfTest, limit_ns);
+    if (form == 3) {
+        const bool came = ptx::mbar_wait_prompt_warp(warp & 1 ? &done : &never, 0, &abort_word, kSiteSelfTest, limit_ns);
+        const bool some = ptx::named_barrier_all(1, 256, came), all = ptx::named_barrier_all(2, 256, true);     // (every warp meets in both)
+        fine = came == (bool)(warp & 1) && !some && all;
+    }
+    const bool early = !told && (ptx::global_timer_ns() - t0) * 2 < limit_ns;
+    __syncthreads();
+    if (lane == 0 && (!fine || (warp == 0 && (early || *(volatile uint32_t*)&abort_word != 1u))))
+        atomicExch(&ptx::g_device_status, (kSiteSelfTestFailed << 24) | form);
 }
 
-cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned int* gave_up, cudaStream_t st)
+cudaError_t launch_wait_selftest(unsigned long long limit_ns, cudaStream_t st)
 {
-    wait_selftest_kernel<<<1, 32, 0, st>>>(limit_ns, gave_up);
+    wait_selftest_kernel<<<kSelfTestForms, 256, 0, st>>>(limit_ns);
     count_launch();
     return cudaGetLastError();
 }

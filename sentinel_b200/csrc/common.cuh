@@ -238,7 +238,7 @@ cudaError_t merge_partials(int acc_dtype, int part_dtype, long long rows, int D,
 
 // A one-warp kernel whose only wait can never complete, limited to limit_ns (attn_fwd_sm100.cu): exercises the
 // give-up path of the bounded waits without hanging or faulting anything.  *gave_up (device memory, optional) <- 1.
-cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned int* gave_up, cudaStream_t st);
+cudaError_t launch_wait_selftest(unsigned long long limit_ns, cudaStream_t st);
 
 // Device status words written by bounded waits (one per tensor-core translation unit; the first reports the KV-cache kernel's and the fp32 forward's too, the second the
 // fp32 backward's).

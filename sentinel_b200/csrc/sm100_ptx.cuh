@@ -98,8 +98,9 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
 
 constexpr uint64_t kWaitLimitNs = 1000ull * 1000ull * 1000ull;  // 1 s
 
-// Bounded wait for the phase with the given parity.  `abort_flag` is a CTA-shared word any waiter sets when
-// it gives up; all later waits of the CTA then return false at once.  Returns true when the phase completed.
+// Bounded wait for the phase with the given parity.  `abort_flag` is a CTA-shared word any waiter sets when it gives up; later
+// waits of the CTA whose phase has not completed then return false soon (here at once; mbar_wait_prompt looks after 256 tries).
+// Returns true when the phase completed.
 __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t site,
                                               uint64_t limit_ns)
 {
@@ -375,34 +376,36 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 // barrier is looked at in the first tries, and little code (the wait is inlined at a dozen places of a loop that has to stay in the
 // instruction cache).  With these the forward of B8 Hq12 S1024 D64 takes 31.0 us instead of 34.0.  Kernels in which many warps wait for
 // long are better off with the waits above, whose tries are further apart (exact fp32, B8 H12 S512 D64: 218 us, 227 with these).
-__device__ __forceinline__ bool wait_gives_up(uint64_t& t0, volatile uint32_t* abort_flag, uint32_t site)
+__device__ __forceinline__ bool wait_gives_up(uint64_t& t0, volatile uint32_t* abort_flag, uint32_t site, uint64_t limit_ns)
 {
     if (*abort_flag) return true;
     const uint64_t now = global_timer_ns();
     if (t0 == 0) t0 = now;      // the wait's first look at the clock, 256 tries in
-    if (now >= *(volatile unsigned long long*)&g_abort_until_ns && now - t0 <= kWaitLimitNs) return false;
+    if (now >= *(volatile unsigned long long*)&g_abort_until_ns && now - t0 <= limit_ns) return false;
     atomicCAS(&g_device_status, 0u, (site << 24) | (blockIdx.x & 0xffffffu));
-    *(volatile unsigned long long*)&g_abort_until_ns = now + kWaitLimitNs;
+    *(volatile unsigned long long*)&g_abort_until_ns = now + limit_ns;
     *abort_flag = 1u;
     return true;
 }
-__device__ __forceinline__ bool mbar_wait_prompt(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t site)
+__device__ __forceinline__ bool mbar_wait_prompt(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t site,
+                                                 uint64_t limit_ns = kWaitLimitNs)
 {
     uint64_t t0 = 0;
 #pragma unroll 1
     for (uint32_t tries = 1;; ++tries) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((tries & 0xffu) == 0 && wait_gives_up(t0, abort_flag, site)) return false;
+        if ((tries & 0xffu) == 0 && wait_gives_up(t0, abort_flag, site, limit_ns)) return false;
     }
 }
 // for a fully active warp
-__device__ __forceinline__ bool mbar_wait_prompt_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t site)
+__device__ __forceinline__ bool mbar_wait_prompt_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t site,
+                                                      uint64_t limit_ns = kWaitLimitNs)
 {
     uint64_t t0 = 0;
 #pragma unroll 1
     for (uint32_t tries = 1;; ++tries) {
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-        if ((tries & 0xffu) == 0 && __any_sync(0xffffffffu, wait_gives_up(t0, abort_flag, site))) return false;
+        if ((tries & 0xffu) == 0 && __any_sync(0xffffffffu, wait_gives_up(t0, abort_flag, site, limit_ns))) return false;
     }
 }
 

@@ -119,6 +119,32 @@ def test_bounded_wait_runs_out_reports_and_leaves_the_context_usable(sb):
     assert lib.sntl_attn_selftest_wait_timeout(200000, stream) == _lib.ERR_BAD_ARGUMENT
 
 
+@pytest.mark.parametrize("limit_us", [1, 2000, 50000])
+def test_every_form_of_bounded_wait_runs_out(sb, limit_us):
+    """The wait of one thread, its short form in a thread and in a warp, and warps that meet in a named barrier after some of them have
+    given up: each returns false, sets the flag of its block and, when nothing else has given up, takes its limit, not the kernels' one
+    second (the self-test records site 0x7d instead of 0x7e if one does not).  The next call after it is clean."""
+    import ctypes as C
+    import time
+    from sentinel_b200 import _lib
+    lib = _lib.load()
+    assert sb.poll_device_status() == 0
+    time.sleep(0.12)                       # (past what an earlier self-test makes other waits give up early)
+    stream = torch.cuda.current_stream().cuda_stream
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    assert lib.sntl_attn_selftest_wait_timeout(limit_us, stream) == _lib.OK
+    torch.cuda.synchronize()
+    assert limit_us * 1e-6 <= time.perf_counter() - t0 < 0.5 + limit_us * 1e-6
+    fwd, bwd = C.c_uint32(0), C.c_uint32(0)
+    assert lib.sntl_attn_poll_device_status_words(stream, C.byref(fwd), C.byref(bwd)) == _lib.ERR_DEVICE_TIMEOUT
+    assert fwd.value >> 24 == 0x7e and fwd.value & 0xffffff < 4 and bwd.value == 0
+    time.sleep(0.12)
+    q = torch.randn(1, 2, 300, 64, device="cuda", dtype=torch.bfloat16)
+    o, _ = sb.attention_forward(q, q, q)
+    assert sb.poll_device_status() == 0 and bool(torch.isfinite(o).all())
+
+
 def test_deterministic_flag_makes_dq_bit_reproducible(sb):
     """SNTL_FLAG_DETERMINISTIC: dQ is summed in 64-bit fixed point, so it is bit-identical from run to run, between the
     one-stream and two-stream variants and through the chunked host-buffer pipeline -- and it meets the same oracle

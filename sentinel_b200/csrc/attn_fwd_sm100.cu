@@ -937,26 +937,37 @@ EncodeTiledFn encode_fn()
 }
 
 // head_dim 128.  Two query tiles per CTA overlap one tile's softmax with the other's products; on a grid that leaves SMs idle or ends
-// with one long CTA, one tile per CTA finishes sooner: a step of one tile takes 0.62 to 0.7 of a step of two (2170 cycles of 3480).  The
-// estimate counts steps of two tiles: the longest CTA, or the SMs' average load and a short tail, with 1.3 steps per CTA of set-up.
-// us, with 0.83 (as measured before key tiles were taken in halves) -> 0.7: B2 Hq12 S1500 26.3 -> 24.2, B4 Hq8 S1000 19.1 -> 18.3, B1 Hq32 S1024 19.2 ->
-// 18.2, a 256-key window over B2 Hq16 S2048 25.6 -> 25.1; a dozen other grids within 1 %, and 0.62 as 0.7.
+// with one long CTA, one tile per CTA finishes sooner.  The estimate counts steps of two tiles.  A step of one tile is 2/3 of one
+// (1.1 us of 1.65 over rows of 2 to 8 steps).  With at most one block per SM the longest decides.  With up to two, the lightest blocks
+// come second on the SMs that are free first (two sums bound that), and a second block costs 2.2 steps more than its own where a CTA has
+// one tile and 1.2 where it has two: its loads, its first products and the end of the block before pass with little else to do (192 blocks
+// of one tile and one or two steps 11.4 us, 148 or fewer of two steps 7.5).  With more, the SMs' average load and a tail.
+// Measured with either form on 200 grids (8 to 256 heads, 100 to 8192 queries, windows, no mask): the choice is the better one, or within
+// the 2 to 4 % by which two runs of such calls differ.  An estimate without the second block's cost took one tile for B4 Hq16 S333 (12.3 us, 9.5 with two) and B4 Hq12 S640
+// (15.2 and 13.0), and two for B6 Hq16 S333 (15.7 and 14.7).
 int fwd_tiles_per_cta(const AttnShape& s)
 {
     const int n = (s.Sq + kM - 1) / kM, n_keys = (s.Skv + kN - 1) / kN, heads = s.B * s.Hq, sms = sm_count();
-    const long long pairs = (long long)((n + 1) / 2) * heads;
-    if (pairs > 2 * sms) return 2;
+    if (n == 1) return 1;
+    if ((long long)((n + 1) / 2) * heads > 2 * sms) return 2;
     const int reach = s.causal && s.window > 0 ? (s.window + kN - 1) / kN + 1 + (s.global_tokens + kN - 1) / kN : n_keys;
-    auto steps = [&](int tile) { return std::min(s.causal ? tile + 1 : n_keys, reach); };
-    double two = 0.0, one = 0.0;
-    for (int i = 0; i < n; ++i) {
-        one += steps(i);
-        if (i + 1 == n || (i & 1)) two += steps(i);
-    }
-    const double cost = 0.7, set_up = 1.3, longest = steps(n - 1);
-    const double t2 = std::max(longest + set_up, (two * heads + set_up * pairs) / sms + 0.1 * longest);
-    const double t1 = std::max(cost * longest + set_up, (cost * one + set_up * n) * heads / sms + 0.1 * cost * longest);
-    return t1 < 0.95 * t2 ? 1 : 2;
+    auto time = [&](int tiles, double second) {
+        const int per_head = (n + tiles - 1) / tiles, blocks = per_head * heads;
+        // of the blocks of each head, in the order in which they start
+        auto cost = [&](int rank) {
+            const int first = (s.causal ? per_head - 1 - rank : rank) * tiles, last = std::min(n, first + tiles) - 1;
+            return std::min(s.causal ? last + 1 : n_keys, reach) * (last > first ? 1.0 : 2.0 / 3.0);
+        };
+        auto block = [&](int i) { return cost(i / heads); };
+        const double longest = std::max(cost(0), cost(std::min(1, per_head - 1)));     // (the first may be a lone tile)
+        if (blocks <= sms) return longest;
+        if (blocks <= 2 * sms)
+            return std::max(longest, std::max(block(sms - 1) + block(sms), block(2 * sms - blocks) + block(blocks - 1)) + second);
+        double sum = 0.0;
+        for (int i = 0; i < per_head; ++i) sum += cost(i);
+        return std::max(longest, (sum * heads + second * blocks) / sms - second + 0.2 * longest);
+    };
+    return time(1, 2.2) < 0.95 * time(2, 1.2) ? 1 : 2;
 }
 
 template <int D, int kMode, bool kMat>

@@ -802,9 +802,11 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 if (!done) {
                     if (cut) {
                         const int limit = (p.causal ? min(p.Skv, grow + 1) : p.Skv) - key0;
+                        if (limit < kHalf) {       // (under a window often only the other mask cuts)
 #pragma unroll
-                        for (int c = 0; c < kHalf; ++c)
-                            if (c >= limit) s[c] = 0xff800000u;  // -inf
+                            for (int c = 0; c < kHalf; ++c)
+                                if (c >= limit) s[c] = 0xff800000u;  // -inf
+                        }
                         const int lo = kWin ? grow - p.window + 1 - key0 : 0;
                         if (kWin && lo > 0 && glim < min(lo, kHalf)) {      // keys below the window that are no global tokens
 #pragma unroll

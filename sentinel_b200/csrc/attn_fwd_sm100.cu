@@ -57,7 +57,8 @@ struct FwdParams {
     int causal;
     int window, global_tokens;   // sliding window and always-visible first keys (0, 0: plain causal)
     int n_qblk, tiles_per_cta;   // query blocks of that many 128-row tiles per (b, h)
-    int several_waves;           // more blocks than SMs
+    int several_waves;           // CTAs ask for further blocks
+    int second_blocks;           // head_dim 64: blocks of the call where two per SM are enough and every half has its own, else 0
     float scale_log2; // scale * log2(e)
     // non-null: O and LSE leave as fp32 feature-major matrices (see MatrixOut)
     float *o_mat, *lse_mat;
@@ -584,7 +585,13 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     uint8_t* sK = sQ + kTileBytes;                    // [2][kTileBytes]
     uint8_t* sV = sK + 2 * kTileBytes;                // [2][kTileBytes]
 
+    // first block of this half, or -1: the second half either asks for one or has the light one that goes with the first half's heavy one
+    const int first = inst == 0 ? (int)blockIdx.x
+                      : p.second_blocks && 2 * (int)gridDim.x - 1 - (int)blockIdx.x < p.second_blocks ? 2 * (int)gridDim.x - 1 - (int)blockIdx.x
+                                                                                                      : -1;
+
     // ---- setup ----
+    FwdWork w{};        // (the producers')
     if (warp >= 16 && (warp & 1) && lane == 0) {
         prefetch_tensormap(&tmap_q);
         prefetch_tensormap(&tmap_k);
@@ -664,11 +671,10 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 atomicExch(&shared->asking, 0u);
                 return block;
             };
-            FwdWork w{};
-            int c0 = 0, block = inst == 0 ? (int)blockIdx.x : ask();
+            int c0 = 0, block = first >= 0 ? first : ask();
             for (int u = 0;; ++u) {
-                w.n0 = -1;
-                if (block >= 0) w.decode<kWin>(p, block);
+                if (block < 0) w.n0 = -1;
+                else w.decode<kWin>(p, block);
                 const int n = w.n0;
                 if (u >= 2 && !mbar_wait_prompt(&bars->work_empty[u & 1], (uint32_t)(((u >> 1) - 1) & 1), abort_flag, kSiteNext)) break;
                 bars->work[u & 1] = {n, w.q0, w.bh, 0, w.g_tiles, w.w_first};
@@ -994,11 +1000,16 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     p.scale_log2 = s.scale * 1.4426950408889634f;
     const long long ctas = (long long)p.n_qblk * s.B * s.Hq;
     if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    p.several_waves = ctas > sm_count();
+    // At head_dim 64 a CTA has two blocks at a time.  With up to two per SM, which half takes which is settled at the launch: asked for, a
+    // second block starts about 1 us later, beside whichever block is there, and a CTA that asks early may take one that an idle SM was
+    // about to start.  us: B1 Hq32 S1024 (256 blocks) 15.6 -> 13.4, B1 Hq16 S2048 24.5 -> 20.7, B4 Hq16 S333 (192) 9.3 -> 8.3.
+    const long long sms = sm_count();
+    p.several_waves = ctas > (D == 64 ? 2 * sms : sms);
+    p.second_blocks = D == 64 && ctas > sms && !p.several_waves ? (int)ctas : 0;
     const size_t smem = (D == 64 ? 10 : 6) * (size_t)(128 * D * 2) + (kMat ? 0 : kOutBytes) + (D == 64 ? sizeof(StreamShared) : sizeof(FwdBarriers)) + 1024;
     auto launch = [&](auto kernel, std::atomic<unsigned long long>& configured) {
         const cudaError_t err = ensure_dynamic_smem(kernel, smem, configured);
-        return err != cudaSuccess ? err : launch_kernel(kernel, (unsigned)ctas, D == 64 ? kStreamThreads : kFwdThreads, smem, st, 1, tq, tk, tv, p);
+        return err != cudaSuccess ? err : launch_kernel(kernel, (unsigned)(p.second_blocks ? sms : ctas), D == 64 ? kStreamThreads : kFwdThreads, smem, st, 1, tq, tk, tv, p);
     };
     static std::atomic<unsigned long long> configured_one{0}, configured_many{0};   // per instantiation, one bit per device
     if constexpr (D == 64) {

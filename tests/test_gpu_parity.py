@@ -475,6 +475,23 @@ def test_forward_key_halves(sb, B, Hq, Hkv, Sq, Sk, kw, D):
         assert float((o.double() - want).abs().max()) <= 2.0 ** -7 * float(v.abs().max())
 
 
+@pytest.mark.parametrize("S,kw", [(70, {}), (200, {}), (200, dict(causal=False)), (260, dict(window=64, global_tokens=5))])
+@pytest.mark.parametrize("per_sm,more", [(1, 0), (1, 1), (2, -1), (2, 0), (2, 1)])
+def test_forward_blocks_are_shared_out_at_one_and_two_per_sm(sb, per_sm, more, S, kw):
+    """head_dim 64: up to one block of 128 queries per SM, up to two (both halves of a CTA have theirs), and more (asked for).  Every row is
+    computed, once, with the same bits as in calls of few heads."""
+    tiles = -(-S // 128)
+    heads = per_sm * torch.cuda.get_device_properties(0).multi_processor_count // tiles + more
+    g = torch.Generator(device="cuda").manual_seed(S + heads)
+    q, k, v = (torch.randn(heads, 1, S, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(3))
+    o, lse = torch.full_like(q, float("nan")), torch.full((heads, 1, S), float("nan"), device="cuda")
+    sb.attention_forward(q, k, v, out=o, lse=lse, **kw)
+    assert sb.last_path() == "tcgen05" and sb.poll_device_status() == 0
+    for b in range(0, heads, 32):
+        want = sb.attention_forward(q[b:b + 32], k[b:b + 32], v[b:b + 32], **kw)
+        assert torch.equal(o[b:b + 32], want[0]) and torch.equal(lse[b:b + 32], want[1])
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk,D,kw", [
     (40, 8, 8, 100, 100, 64, {}),                                 # 320 blocks of one step each
     (30, 6, 6, 129, 129, 128, {}),                                # one- and two-step blocks, the last with one query

@@ -6,9 +6,9 @@
 // online softmax, O = P V, LSE = m + ln(l) -- re-designed for Blackwell:
 //
 //   * head_dim 128 (attn_fwd_tc_kernel): one CTA owns 256 (small grids: 128) consecutive query rows of one (batch, head) as two
-//     128-row tiles, whose key tiles are taken in halves of 64 keys; each tile has its own softmax warpgroup (one thread per query row: tcgen05.ld's 32x32b shape hands thread i
-//     row i, so the row max / row sum need no shuffles) while a single MMA-issuing warp (one elected lane) feeds the tensor core
-//     for both, so one tile's softmax overlaps the other tile's MMAs;
+//     128-row tiles, whose key tiles are taken in halves of 64 keys; each tile has its own softmax warpgroup (one thread per query
+//     row: tcgen05.ld's 32x32b shape hands thread i row i, so the row max / row sum need no shuffles) while a single MMA-issuing
+//     warp (one elected lane) feeds the tensor core for both, so one tile's softmax overlaps the other tile's MMAs;
 //   * head_dim 64 (attn_fwd_streams_kernel): four softmax warpgroups, each with 64 of the 128 keys of every key tile and sums and
 //     an O of its own, two per query tile, and two query tiles that run independently of each other;
 //   * S (fp32) and O (fp32, D columns) live in TMEM; P is written back over S as packed bf16 and consumed by the PV MMA
@@ -47,7 +47,7 @@ constexpr int kOutBytes = 8 * 4096;        // staging of O
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 enum WaitSite : uint32_t {
-    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteIssue, kSiteQEmpty, kSiteNext, kSiteORead
+    kSiteQ = 1, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteQEmpty = 10, kSiteNext
 };
 
 struct FwdParams {
@@ -67,8 +67,8 @@ struct FwdParams {
 
 // What one block of the grid computes.  A CTA computes its own block and then takes over blocks that have not started yet (as the
 // backward does): K, Q and the first S of one come in under the last softmax passes and the epilogue of the one before.
-// us: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108; B8 Hq28 Hkv4 S1024 D128 88.0 -> 71.9, B8 Hq16 S512 20.2 -> 18.3, B2 Hq16 Hkv4 S3000
-// 73.2 -> 69.6.
+// us: a 512-key window over B2 Hq28 Hkv4 S8192 D128 123 -> 108; B8 Hq28 Hkv4 S1024 D128 88.5 -> 72.0, B8 Hq16 S512 20.8 -> 18.9, B2 Hq16 Hkv4 S3000
+// 73.5 -> 69.9.  (A grid whose time is one long block's alone only pays for it: B1 Hq4 S8192 D128, 256 blocks of one tile, 71.5 -> 77.)
 struct FwdWork {
     int bh, bh_kv, q0;         // q0: first of the one or two 128-row tiles
     int g_tiles, w_first;      // key tiles in ascending order: the g_tiles tiles holding global tokens, then from w_first up to the
@@ -129,14 +129,19 @@ enum FwdMode : int { kPlain = 0, kWindow = 1 };
 // tiles.  A key tile is taken as two halves of 64 keys, each with an S buffer of its own and its P written over it: while a
 // half is exponentiated, the other's P V and the S of the half after it run, which took the P V and S products (about 1150 cycles per
 // step) out of that chain.  S products of 64 keys are bound by their operands in shared memory (48 cycles per k-step instead of 32).
-// With 128 keys per S product, us, before -> now: B1 Hq4 S8192 88.0 -> 71.2 (one block per SM), B8 Hq16 S512 21.7 -> 20.2, B3 Hq16
-// Hkv4 S1237 28.7 -> 27.3, B8 Hq28 Hkv4 S1024 92.6 -> 88.0, B2 Hq28 Hkv4 S8192 within its spread (at the power limit: 1600 MHz).  64 columns
-// in registers instead of 128 also leave room for taking over blocks.
-template <int D, int kMode, bool kMat, bool kMany>
+// With 128 keys per S product, us, before -> with halves, neither taking over blocks: B1 Hq4 S8192 88.0 -> 71.2 (256 blocks of one tile), B8
+// Hq16 S512 21.7 -> 20.2, B3 Hq16 Hkv4 S1237 28.7 -> 27.3, B8 Hq28 Hkv4 S1024 92.6 -> 88.0, B2 Hq28 Hkv4 S8192 within its spread (at the power
+// limit: 1600 MHz).  64 columns in registers instead of 128 also leave room for taking over blocks: the 168 registers that 384 threads
+// can have at compile time then spill 12 bytes (60 of loads, none of them without kMany and kWindow).
+// A row's reference maximum is that of 64 keys first and is renewed per 64 keys.  Taken from a whole first key tile, bits are those of
+// 128 keys per S product, and O of rows with scores of standard deviation 3 and more is 2 % nearer to its value; scores of 0.25 see no
+// difference, and the forward takes 3 to 10 % longer (B3 Hq16 Hkv4 S1237 26.1 -> 26.9, one tile 5.8 -> 6.2).
+template <int kMode, bool kMat, bool kMany>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const FwdParams p)
 {
+    constexpr int D = 128;
     constexpr int kTileBytes = 128 * D * 2;          // one 128-row tile of Q, K or V
     constexpr int kChunkBytes = 128 * 128;           // one 64-element-wide TMA box (128 rows x 128 B)
     constexpr int kChunks = D / 64;
@@ -533,13 +538,16 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 // Bound by the exponentials: 2048 cycles of the special-function unit for two tiles of 128 x 128, beside 1280 of products.  With two
 // softmax warps per scheduler, one per query tile, a step of two tiles took 3490 cycles: both warps wait for products, load, store
 // and hand over about as long as they compute.  Here four warps per scheduler work on four independent chains (S 64 columns and O 64
-// columns each fill the TMEM; 104 registers are enough for 64 columns), and a step takes 2500 to 2600.
+// columns each fill the TMEM; the 96 registers that 640 threads can have at compile time hold 64 columns, under a window with 16 bytes
+// spilled), and a step takes 2460 to 2520 cycles in long rows, 2700 to 2870 in rows of 16 key tiles.
 // The two query tiles of a CTA are halves that share nothing but the TMEM allocation and the queue of blocks: the end of a block
-// (about 5000 cycles from its last exponentials to the first of the next) then passes under the other half's steps, no tile waits for
+// (4700 to 5800 cycles from its last S to the first S of the next) then passes under the other half's steps, no tile waits for
 // the longer row of another, and blocks of one tile balance better.
-// us, before -> now: B4 Hq32 Hkv8 S4096 377 -> 351; B8 Hq12 S1024 31.0 -> 28.5; B2 Hq32 S1024 23.2 -> 19.4; B16 Hq8 S130 7.8 -> 7.5; a 300-key
-// window over B4 Hq12 S2048 35.6 -> 35.7; few long rows, B1 Hq4 S8192, 71.8 -> 71.6.  Also measured: both tiles
-// fed by one MMA warp, 351, 28.2 and 27.9; two softmax warpgroups with two S buffers of 64 columns each, 436, 32.0 and 25.2.
+// us, two warps per scheduler and the longer form of waits -> now: B4 Hq32 Hkv8 S4096 407 -> 343; B8 Hq12 S1024 34.6 -> 28.3; B2 Hq32 S1024 25.2 ->
+// 19.5; B16 Hq8 S130 8.3 -> 7.6; a 300-key window over B4 Hq12 S2048 39.2 -> 35.7; one block of one tile 5.3 -> 5.5 (its two streams meet once
+// more).  Of the first three 7 to 9 % are the waits' alone.  Also measured, when the streams took 351, 28.5 and 19.4: both tiles fed by one
+// MMA warp, 351, 28.2 and 27.9; two softmax warpgroups with two S buffers of 64 columns each, 436, 32.0 and 25.2.  The key loop is
+// sensitive to what the compiler does with code outside it: forms of the set-up that differ in nothing else came out up to 4 % apart.
 constexpr int kStreamThreads = 640;   // four softmax warpgroups, and one holding the MMA and the TMA warps
 
 // One half of a CTA: blocks of one query tile, two softmax warpgroups ("streams": stream b has keys [64 b, 64 b + 64) of every key
@@ -569,6 +577,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
 attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                         const __grid_constant__ CUtensorMap tmap_v, const FwdParams p)
 {
+    enum : uint32_t {       // (the status word tells the two kernels apart)
+        kSiteQ = 33, kSiteK0, kSitePairFull, kSitePairEmpty, kSiteSReady, kSitePReady, kSiteOReady, kSiteFinal, kSiteQEmpty, kSiteNext, kSiteORead
+    };
     constexpr int D = 64, kTileBytes = 128 * D * 2;
     constexpr uint32_t kHalfBytes = kHalf * 128;    // of a K or V tile
     extern __shared__ uint8_t smem_raw[];
@@ -760,6 +771,9 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         const int row = (warp & 3) * 32 + lane;        // row inside the tile == TMEM lane
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t tmS = tmem_S(half) + lane_off, tmO = tmem_O(half) + lane_off;
+        SNTL_TRACE_DECL(tn);
+        const bool tw = (warp & 3) == 0 && lane == 0;
+        (void)tw;
         bool ok = true;
         uint32_t phase = 0;                            // of s_ready
         int4 work;
@@ -775,12 +789,14 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             float m_ref = -INFINITY, l = 0.0f;
             for (int j = 0; j < n_mine; ++j) {
                 if (!(ok = mbar_wait_prompt_warp(&bars->s_ready[half], phase, abort_flag, kSiteSReady))) break;
+                SNTL_TRACE_EV(tw, warp >> 2, tn, 1);
                 phase ^= 1u;
                 tc_fence_after();
                 uint32_t s[kHalf];
 #pragma unroll
                 for (int c = 0; c < 2; ++c) tmem_ld32(tmS + (uint32_t)(c * 32), s + c * 32);
                 tmem_ld_wait();
+                SNTL_TRACE_EV(tw, warp >> 2, tn, 2);
                 // number of visible keys of this row among these
                 const int key0 = (j < g_tiles ? j : w_first + (j - g_tiles)) * kN + half * kHalf;
                 const int limit_lo = (p.causal ? min(p.Skv, row_lo + 1) : p.Skv) - key0;
@@ -843,17 +859,20 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                     RowMax unused;
                     exp_row<false>(s, p.scale_log2, shift(), pk, sum, unused);
                 }
+                SNTL_TRACE_EV(tw, warp >> 2, tn, 3);
                 tmem_st32(tmS, pk);      // over S
                 l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&bars->p_ready[half]);
+                SNTL_TRACE_EV(tw, warp >> 2, tn, 4);
             }
             if (!ok || (more = get(u + 1, work), work.x == kGaveUp) || !mbar_wait_prompt_warp(&bars->o_ready[half], (uint32_t)(u & 1), abort_flag, kSiteOReady)) {
                 named_barrier_all(1 + inst, 256, false);
                 break;
             }
             // The two streams of a row are added here; each stores one half of the features.
+            SNTL_TRACE_EV(tw, warp >> 2, tn, 5);
             bars->ml[half][row] = make_float2(m_ref, l);
             tc_fence_before();
             if (!named_barrier_all(1 + inst, 256, true)) break;
@@ -911,6 +930,7 @@ attn_fwd_streams_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 __syncwarp();
                 if (store && half == 0) p.lse[(size_t)bh * p.Sq + grow] = total > 0.0f ? (m + log2f(total)) * 0.6931471805599453f : -INFINITY;
             }
+            SNTL_TRACE_EV(tw, warp >> 2, tn, 6);
         }
     }
 
@@ -1015,8 +1035,8 @@ cudaError_t launch_fwd(const TcArgs& a, cudaStream_t st)
     if constexpr (D == 64) {
         return launch(attn_fwd_streams_kernel<kMode, kMat>, configured_one);
     } else {
-        if (p.several_waves) return launch(attn_fwd_tc_kernel<D, kMode, kMat, true>, configured_many);
-        return launch(attn_fwd_tc_kernel<D, kMode, kMat, false>, configured_one);
+        if (p.several_waves) return launch(attn_fwd_tc_kernel<kMode, kMat, true>, configured_many);
+        return launch(attn_fwd_tc_kernel<kMode, kMat, false>, configured_one);
     }
 }
 

@@ -372,10 +372,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site));
 }
 
-// The two waits in the form for loops whose pace depends on how soon a waiter goes on: warp-uniform control flow, nothing but the
-// barrier is looked at in the first tries, and little code (the wait is inlined at a dozen places of a loop that has to stay in the
-// instruction cache).  With these the forward of B8 Hq12 S1024 D64 takes 31.0 us instead of 34.0.  Kernels in which many warps wait for
-// long are better off with the waits above, whose tries are further apart (exact fp32, B8 H12 S512 D64: 218 us, 227 with these).
+// The two waits in a short form: warp-uniform control flow, nothing but the barrier is looked at in the first tries, and little code (the
+// wait is inlined at a dozen places of a loop that has to stay in the instruction cache).  A kernel has the form that measured better
+// in it.  The forward, whose pace is set by how soon a waiter goes on: 9.8 % slower with the waits above at head_dim 64 (B8 Hq12 S1024 28.3
+// -> 32.2 us, B4 Hq32 Hkv8 S4096 343 -> 372) and 7.4 % at 128 (mean of 25 shapes each).  The backward: no difference (0.1 % over 30 calls); it has
+// the short form.  The dQ kernel: none either (0.5 % over 16); it has the form above.  The KV-cache kernel: 1.5 to 2 % faster with the short
+// form on some shapes and 2 to 3 % slower on others; it has the form above.  Exact fp32, in which many warps wait for long: 218 us with the
+// form above, whose tries are further apart, 227 with the short one (B8 H12 S512 D64).
 __device__ __forceinline__ bool wait_gives_up(uint64_t& t0, volatile uint32_t* abort_flag, uint32_t site, uint64_t limit_ns)
 {
     if (*abort_flag) return true;

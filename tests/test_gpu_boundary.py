@@ -88,8 +88,8 @@ def test_calls_on_two_streams_keep_their_scratch_apart(sb):
 
 
 def test_bounded_wait_runs_out_reports_and_leaves_the_context_usable(sb):
-    """Failure detection without a fault: a one-warp kernel waits, with a 2 ms limit, on a barrier that by construction
-    never receives its arrival.  The wait runs out exactly as a stuck production wait would after its one second: the
+    """Failure detection without a fault: a small kernel waits, with a 2 ms limit, on barriers that by construction
+    never receive their arrival.  The waits run out as a stuck production wait would after its one second: the
     kernel returns normally, the poll reports SNTL_ERR_DEVICE_TIMEOUT with the self-test's site code, the report is
     cleared by that poll, and the next real call (made after the short give-up window has passed) is clean and exact."""
     import ctypes as C
